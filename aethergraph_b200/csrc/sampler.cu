@@ -58,9 +58,9 @@ namespace ag {
 namespace {
 
 constexpr int kTile = 512;      // threads per block of the assign kernel
-// Items per thread of the assign kernel.  The last stage holds no row bounds per item,
+// Most items per thread of the assign kernel.  The last stage holds no row bounds per item,
 // so it can afford twice as many table probes in flight per thread.
-template <bool HAS_NEXT> struct AssignShape { static constexpr int kIPT = HAS_NEXT ? 4 : 8; static constexpr int kTileItems = kTile * kIPT; };
+constexpr int kMaxIPT = 4, kMaxIPTLast = 8;
 constexpr int kPickThreads = 256;
 constexpr int kLargeK = 1024;   // largest fanout the k > 32 path keeps in shared memory
 
@@ -605,11 +605,11 @@ __device__ __forceinline__ void publish_counts(const SampleParams &p, BatchState
     bs->done_blocks = 0;
 }
 
-template <bool HAS_NEXT>
+template <bool HAS_NEXT, int IPT>
 __global__ void __launch_bounds__(kTile, 2)
 k_assign(const SampleParams *__restrict__ pa, uint32_t stage, uint32_t k) {
     constexpr bool has_next = HAS_NEXT;  // the last stage queues no frontier
-    constexpr int kIPT = AssignShape<HAS_NEXT>::kIPT, kTileItems = AssignShape<HAS_NEXT>::kTileItems;
+    constexpr int kIPT = IPT, kTileItems = kTile * IPT;
     chain_sync();
     __shared__ uint32_t s_tile;
     __shared__ ScanVal s_warp[kTile / 32];
@@ -642,9 +642,10 @@ k_assign(const SampleParams *__restrict__ pa, uint32_t stage, uint32_t k) {
     // The grid is sized for a typical batch, not for the worst case: a block
     // keeps drawing tile tickets until they run out.  Tickets are handed out in
     // order, so the tiles a look-back (or a pending vertex) waits for are always
-    // already running.  A thread owns kIPT (4, last stage 8) consecutive items of its tile,
-    // so that many table probes (and row-bound loads) are in flight per thread, and the
-    // barriers, the ticket and the look-back are paid once per kTile * kIPT items.
+    // already running.  A thread owns kIPT consecutive items of its tile (launch_assign
+    // picks kIPT), so that many table probes (and row-bound loads) are in flight per
+    // thread, and the barriers, the ticket and the look-back are paid once per
+    // kTile * kIPT items.
     for (;;) {
         if (threadIdx.x == 0) s_tile = atomicAdd(&bs->ticket, 1u);
         __syncthreads();
@@ -873,6 +874,31 @@ uint64_t next_pow2(uint64_t v) {
     uint64_t p = 1;
     while (p < v) p <<= 1;
     return p;
+}
+
+// Items per thread of an assign launch: the fewest with which the tiles of all batches
+// are resident at once (two blocks per SM).  A small stage is bound by the latency of its
+// dependent loads (slot, table entry, row bounds), so it wants its items on as many SMs
+// as there are; only a stage that fills the GPU gains from more items per thread.
+// (Always four, last stage eight: the last stage of 128 seeds with fanouts 15, 10 ran 22 us
+// on two blocks, now 13; a call of 1024 seeds with fanouts 25, 10 went from 167 to 140 us.)
+template <bool HAS_NEXT>
+void launch_assign(uint64_t items, uint32_t n_batches, cudaStream_t st, const SampleParams *pa, uint32_t stage, uint32_t k) {
+    const uint64_t resident = (uint64_t)kSMs * 2 * kTile;
+    const int most = HAS_NEXT ? kMaxIPT : kMaxIPTLast;
+    int ipt = 1;
+    while (ipt < most && items * n_batches > resident * ipt) ipt *= 2;
+    const uint64_t per = (uint64_t)kTile * ipt, blocks = (items + per - 1) / per;
+    // The grid covers the worst case only up to a few waves of resident blocks over the
+    // whole group; the kernel draws tile tickets beyond that, so a batch far below its
+    // bound does not pay for thousands of empty blocks.
+    const dim3 grid((uint32_t)std::max<uint64_t>(1, std::min<uint64_t>(blocks, std::max<uint64_t>(1, (uint64_t)kSMs * 8 / n_batches))), n_batches);
+    switch (ipt) {
+        case 1: launch_chained(k_assign<HAS_NEXT, 1>, grid, dim3(kTile), st, pa, stage, k); break;
+        case 2: launch_chained(k_assign<HAS_NEXT, 2>, grid, dim3(kTile), st, pa, stage, k); break;
+        case 4: launch_chained(k_assign<HAS_NEXT, 4>, grid, dim3(kTile), st, pa, stage, k); break;
+        default: launch_chained(k_assign<HAS_NEXT, HAS_NEXT ? kMaxIPT : kMaxIPTLast>, grid, dim3(kTile), st, pa, stage, k); break;
+    }
 }
 
 void launch_pick(int mode, uint32_t k, uint64_t frontier_est, uint32_t n_batches, cudaStream_t st,
@@ -1379,22 +1405,14 @@ int32_t launch_saved_impl(ag_sampler *s, bool relaunch) {
 
     const SampleParams *pa = s->params_dev;
     const uint32_t nmax = (uint32_t)max_n;
-    // Grids cover the worst case only up to about two waves of resident blocks
-    // over the whole group; the expand kernel draws tile tickets beyond that, so
-    // a batch far below its bound does not pay for thousands of empty blocks.
-    auto tiles_for = [&](uint64_t items, bool last) {
-        const uint64_t per = last ? AssignShape<false>::kTileItems : AssignShape<true>::kTileItems;
-        const uint64_t blocks = (items + per - 1) / per;
-        return (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>(blocks, std::max<uint64_t>(1, (uint64_t)kSMs * 8 / n_batches)));
-    };
     if (nmax) k_insert_seeds<<<dim3((nmax + 255) / 256, n_batches), 256, 0, st>>>(pa);
     uint64_t items = nmax;  // bound on the items of the stage being launched
     for (uint32_t stage = 0; stage <= H; ++stage) {
         const bool has_next = stage < H;
         const uint32_t k = has_next ? s->cfg.fanout[stage] : 0;
         const uint64_t expect = (stage && s->est_items[stage]) ? std::min(items, s->est_items[stage]) : items;
-        if (has_next) launch_chained(k_assign<true>, dim3(tiles_for(expect, false), n_batches), dim3(kTile), st, pa, stage, k);
-        else launch_chained(k_assign<false>, dim3(tiles_for(expect, true), n_batches), dim3(kTile), st, pa, stage, k);
+        if (has_next) launch_assign<true>(expect, n_batches, st, pa, stage, k);
+        else launch_assign<false>(expect, n_batches, st, pa, stage, k);
         if (has_next && k) {
             // the new vertices of this stage are at most its items
             launch_pick(s->mode, k, std::min<uint64_t>(expect, g->num_nodes), n_batches, st, pa, stage);
