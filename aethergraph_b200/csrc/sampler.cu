@@ -4,11 +4,12 @@
 // (crates/aethergraph-core/src/loader/sampler.rs:845-961 with the hop loop at
 // :754-842 and the per-node dispatch at :1178-1235), but as a short chain of
 // data-parallel kernels instead of one sequential loop.  A batch with H hops
-// is 2H + 2 launches:
+// is 2H + 1 launches (2H + 2 with more than kFusedSeeds seeds):
 //
 //   insert_seeds   every seed is inserted into a hash table keyed by vertex id
 //                  with atomicMin(position): the smallest position that names a
-//                  vertex is its first sighting.
+//                  vertex is its first sighting.  A batch of few seeds does this
+//                  at the head of assign(0).
 //   assign(s)      s = 0 .. H.  The items of stage s are the seeds (s = 0) or
 //                  the edges hop s - 1 emitted, in position order.  One
 //                  single-pass scan over them turns the first-sighting flags
@@ -138,18 +139,52 @@ __device__ __forceinline__ void chain_sync() {
     asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
-__global__ void k_insert_seeds(const SampleParams *__restrict__ pa) {
-    chain_sync();
-    const SampleParams &p = pa[blockIdx.y];
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= p.n_seeds) return;
-    const uint32_t id = p.seeds[i];
+// The parameter blocks, gather arguments and seeds of a chain are staged in pinned host
+// memory and the chain's first kernel reads them from there, leaving the device copies
+// the later kernels use.  A copy command each for the three costs more than the kernel
+// (measured on one batch of 128 seeds: 1.7 us each on the device with 3 - 4 us between
+// them, 3 - 5 us each on the launching thread); a read over PCIe is one round trip.
+// With the seed insertion at the head of stage 0 and the counts written straight to pinned
+// memory a call of 128 seeds went from 115 to 100 us, one of 1024 seeds from 140 to 123.
+struct StagedChain {
+    const SampleParams *params;  // pinned host, one per batch
+    const GatherArgs *gather;    // pinned host, one per batch; null: nothing to gather
+    SampleParams *params_dev;
+    GatherArgs *gather_dev;
+};
+static_assert(sizeof(SampleParams) % 8 == 0 && sizeof(GatherArgs) % 8 == 0, "staged blocks are copied as 8-byte words");
+
+// Loads batch blockIdx.y's parameters into shared memory (whole block); block 0 of the
+// batch leaves the device copies.
+__device__ __forceinline__ void load_staged(const StagedChain &c, SampleParams *s_params) {
+    constexpr uint32_t kWords = sizeof(SampleParams) / 8, kGatherWords = sizeof(GatherArgs) / 8;
+    const volatile uint64_t *src = (const volatile uint64_t *)(c.params + blockIdx.y);
+    const bool keep = blockIdx.x == 0;
+    for (uint32_t i = threadIdx.x; i < kWords + kGatherWords; i += blockDim.x) {
+        if (i < kWords) {
+            const uint64_t v = src[i];
+            ((uint64_t *)s_params)[i] = v;
+            if (keep) ((uint64_t *)(c.params_dev + blockIdx.y))[i] = v;
+        } else if (keep && c.gather) {
+            ((uint64_t *)(c.gather_dev + blockIdx.y))[i - kWords] = ((const volatile uint64_t *)(c.gather + blockIdx.y))[i - kWords];
+        }
+    }
+    __syncthreads();
+}
+
+__device__ __forceinline__ uint32_t insert_seed(const SampleParams &p, uint32_t i, uint32_t id) {
     if ((uint64_t)id >= p.num_nodes) {
         atomicOr(&p.state->error, kErrBadSeed);
-        p.slot_of_seed[i] = 0xFFFFFFFFu;
-        return;
+        return 0xFFFFFFFFu;
     }
-    p.slot_of_seed[i] = table_insert_min(p.table, id, enc_pending(p.table.gen, 0, i), &p.state->error);
+    return table_insert_min(p.table, id, enc_pending(p.table.gen, 0, i), &p.state->error);
+}
+
+__global__ void k_insert_seeds(StagedChain chain) {
+    __shared__ __align__(16) SampleParams p;
+    load_staged(chain, &p);
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < p.n_seeds) p.slot_of_seed[i] = insert_seed(p, i, p.seeds[i]);
 }
 
 // ----------------------------------------------------------------- expand --
@@ -605,17 +640,17 @@ __device__ __forceinline__ void publish_counts(const SampleParams &p, BatchState
     bs->done_blocks = 0;
 }
 
-template <bool HAS_NEXT, int IPT>
-__global__ void __launch_bounds__(kTile, 2)
-k_assign(const SampleParams *__restrict__ pa, uint32_t stage, uint32_t k) {
+// The body of an assign kernel.  FUSED: stage 0 of a batch whose seeds fit one tile; the
+// one block inserts the seeds itself and needs neither ticket nor look-back.
+template <bool HAS_NEXT, int IPT, bool FUSED>
+__device__ __forceinline__ void assign_stage(const SampleParams &p, uint32_t stage, uint32_t k) {
     constexpr bool has_next = HAS_NEXT;  // the last stage queues no frontier
     constexpr int kIPT = IPT, kTileItems = kTile * IPT;
-    chain_sync();
     __shared__ uint32_t s_tile;
     __shared__ ScanVal s_warp[kTile / 32];
     __shared__ ScanVal s_prefix;
+    __shared__ uint32_t s_seeds[FUSED ? kTileItems : 1];
 
-    const SampleParams &p = pa[blockIdx.y];
     BatchState *bs = p.state;
     StageInfo si = bs->stage[stage];
     if (stage == 0) {
@@ -631,14 +666,6 @@ k_assign(const SampleParams *__restrict__ pa, uint32_t stage, uint32_t k) {
     const uint32_t gen = p.table.gen;
     const uint32_t *slots_in = (stage == 0) ? p.slot_of_seed : p.slot_of_edge + si.n_edges;
 
-    if (!has_next && p.edge_index_local) {
-        // Last stage: every edge of the batch exists, so the row offset of the int64
-        // [2, E] local edge index is known.  Row 1 = the expanded vertex's local id.
-        const uint64_t total = min((uint64_t)edges_before_next, p.cap_edges);
-        for (uint64_t e = (uint64_t)blockIdx.x * kTile + threadIdx.x; e < total; e += (uint64_t)gridDim.x * kTile)
-            p.edge_index_local[total + e] = (int64_t)p.src_local[e];
-    }
-
     // The grid is sized for a typical batch, not for the worst case: a block
     // keeps drawing tile tickets until they run out.  Tickets are handed out in
     // order, so the tiles a look-back (or a pending vertex) waits for are always
@@ -647,9 +674,11 @@ k_assign(const SampleParams *__restrict__ pa, uint32_t stage, uint32_t k) {
     // thread, and the barriers, the ticket and the look-back are paid once per
     // kTile * kIPT items.
     for (;;) {
-        if (threadIdx.x == 0) s_tile = atomicAdd(&bs->ticket, 1u);
-        __syncthreads();
-        const uint32_t tile = s_tile;
+        if (!FUSED) {
+            if (threadIdx.x == 0) s_tile = atomicAdd(&bs->ticket, 1u);
+            __syncthreads();
+        }
+        const uint32_t tile = FUSED ? 0u : s_tile;
         if (tile >= n_tiles) {
             // n_tiles + gridDim.x tickets are drawn in all; the last one resets the counter.
             if (threadIdx.x == 0 && tile == n_tiles + gridDim.x - 1) bs->ticket = 0;
@@ -661,8 +690,22 @@ k_assign(const SampleParams *__restrict__ pa, uint32_t stage, uint32_t k) {
         // position that named the vertex.
         uint32_t slot[kIPT], id[kIPT], cur32[kIPT];
         bool first[kIPT];
+        if (FUSED) {
+            // the seeds may lie in host memory: read each sector of them once
 #pragma unroll
-        for (int j = 0; j < kIPT; ++j) slot[j] = (item0 + j < count) ? slots_in[item0 + j] : 0xFFFFFFFFu;
+            for (int j = 0; j < kIPT; ++j) {
+                const uint32_t i = threadIdx.x + j * kTile;
+                if (i < count) s_seeds[i] = p.seeds[i];
+            }
+            __syncthreads();
+#pragma unroll
+            for (int j = 0; j < kIPT; ++j) slot[j] = (item0 + j < count) ? insert_seed(p, item0 + j, s_seeds[item0 + j]) : 0xFFFFFFFFu;
+            __threadfence();  // every seed is in the table before any of them is looked at
+            __syncthreads();
+        } else {
+#pragma unroll
+            for (int j = 0; j < kIPT; ++j) slot[j] = (item0 + j < count) ? slots_in[item0 + j] : 0xFFFFFFFFu;
+        }
 #pragma unroll
         for (int j = 0; j < kIPT; ++j) {
             id[j] = 0; cur32[j] = 0; first[j] = false;
@@ -704,7 +747,8 @@ k_assign(const SampleParams *__restrict__ pa, uint32_t stage, uint32_t k) {
                                                 __shfl_sync(0xffffffffu, wi.take, 31),
                                                 __shfl_sync(0xffffffffu, wi.draws, 31)};
             if (lane < kTile / 32) s_warp[lane] = ScanVal{wi.flags - w.flags, wi.take - w.take, wi.draws - w.draws};
-            const ScanVal prefix = lookback_exclusive(p.tiles, tile, p.epoch_base + stage, block_total, lane, &bs->error);
+            const ScanVal prefix = FUSED ? ScanVal{0, 0, 0}
+                                         : lookback_exclusive(p.tiles, tile, p.epoch_base + stage, block_total, lane, &bs->error);
             if (lane == 0) {
                 s_prefix = prefix;
                 if (tile == n_tiles - 1) {
@@ -786,10 +830,18 @@ k_assign(const SampleParams *__restrict__ pa, uint32_t stage, uint32_t k) {
                 write_item_local(p, stage, si.n_edges, item0 + j, (v & kPendingBit) ? 0xFFFFFFFFu : (v & kPosMask));
             }
         }
+        if (FUSED) break;
     }
 
     if (has_next) return;
-    // Last stage: the block that finishes last publishes the batch's counts (every
+    if (p.edge_index_local) {
+        // Last stage: every edge of the batch exists, so the row offset of the int64
+        // [2, E] local edge index is known.  Row 1 = the expanded vertex's local id.
+        const uint64_t total = min((uint64_t)edges_before_next, p.cap_edges);
+        for (uint64_t e = (uint64_t)blockIdx.x * kTile + threadIdx.x; e < total; e += (uint64_t)gridDim.x * kTile)
+            p.edge_index_local[total + e] = (int64_t)p.src_local[e];
+    }
+    // The block that finishes last publishes the batch's counts (every
     // error bit any block raised is in by then) and leaves the state ready for the
     // handle's next batch.
     __shared__ bool s_last;
@@ -800,6 +852,24 @@ k_assign(const SampleParams *__restrict__ pa, uint32_t stage, uint32_t k) {
     __syncthreads();
     if (!s_last || threadIdx.x != 0) return;
     publish_counts(p, bs);
+}
+
+template <bool HAS_NEXT, int IPT>
+__global__ void __launch_bounds__(kTile, 2)
+k_assign(const SampleParams *__restrict__ pa, uint32_t stage, uint32_t k) {
+    chain_sync();
+    assign_stage<HAS_NEXT, IPT, false>(pa[blockIdx.y], stage, k);
+}
+
+// Seed insertion and stage 0 in one launch, a block per batch.
+constexpr uint32_t kFusedSeeds = kTile * kMaxIPT;
+
+template <int IPT>
+__global__ void __launch_bounds__(kTile, 2)
+k_assign_seeds(StagedChain chain, uint32_t k) {
+    __shared__ __align__(16) SampleParams p;
+    load_staged(chain, &p);
+    assign_stage<true, IPT, true>(p, 0, k);
 }
 
 // Hop `hop`: expand the frontier stage `hop` queued (stage[hop + 1] holds its
@@ -960,8 +1030,6 @@ struct ag_sampler {
     uint32_t *hub_list = nullptr;  // weighted only: per batch max_frontier queue slots + 1 counter word
     TileDesc *tiles = nullptr;
     BatchState *state = nullptr;
-    uint32_t *seeds_dev = nullptr;
-    ag_sample_counts *counts_dev = nullptr;
     SampleParams *params_dev = nullptr;
     GatherArgs *gather_dev = nullptr;
     // pinned host
@@ -1032,11 +1100,10 @@ void free_scratch(ag_sampler *s) {
     s->frontier = nullptr;
     cudaFree(s->slot_of_seed); cudaFree(s->slot_of_edge); cudaFree(s->tiles);
     cudaFree(s->hub_list); s->hub_list = nullptr;
-    cudaFree(s->seeds_dev);
     if (s->seeds_pinned) cudaFreeHost(s->seeds_pinned);
     s->table = nullptr;
     s->slot_of_seed = s->slot_of_edge = nullptr; s->tiles = nullptr;
-    s->seeds_dev = nullptr; s->seeds_pinned = nullptr;
+    s->seeds_pinned = nullptr;
 }
 
 // A finished continuing batch (no per-batch seed) moves the handle's stream on by
@@ -1072,7 +1139,6 @@ int32_t ensure_scratch(ag_sampler *s, uint64_t n_seeds) {
     s->n_tiles = std::max<uint64_t>(std::max(cap, s->max_hop_edges) / kTile + 2, 2);
     AG_CUDA(cudaMalloc(&s->tiles, G * s->n_tiles * sizeof(TileDesc)));
     AG_CUDA(cudaMemset(s->tiles, 0, G * s->n_tiles * sizeof(TileDesc)));
-    AG_CUDA(cudaMalloc(&s->seeds_dev, G * cap * 4));
     AG_CUDA(cudaHostAlloc(&s->seeds_pinned, G * cap * 4, cudaHostAllocDefault));
     s->cap_seeds = cap;
     s->epoch = 0;
@@ -1110,7 +1176,6 @@ extern "C" int32_t ag_sampler_create_group(const ag_graph *g, const ag_sampling_
     do {
         if (cudaMalloc(&s->state, group * sizeof(BatchState)) != cudaSuccess ||
             cudaMemset(s->state, 0, group * sizeof(BatchState)) != cudaSuccess ||
-            cudaMalloc(&s->counts_dev, group * sizeof(ag_sample_counts)) != cudaSuccess ||
             cudaMalloc(&s->params_dev, group * sizeof(SampleParams)) != cudaSuccess ||
             cudaMalloc(&s->gather_dev, group * sizeof(GatherArgs)) != cudaSuccess ||
             cudaHostAlloc(&s->counts_host, group * sizeof(ag_sample_counts), cudaHostAllocDefault) != cudaSuccess ||
@@ -1149,7 +1214,7 @@ extern "C" void ag_sampler_free(ag_sampler *s) {
     free_scratch(s);
     s->sort.release();
     for (void *p : s->owned) cudaFree(p);
-    cudaFree(s->state); cudaFree(s->counts_dev); cudaFree(s->params_dev); cudaFree(s->gather_dev);
+    cudaFree(s->state); cudaFree(s->params_dev); cudaFree(s->gather_dev);
     if (s->counts_host) cudaFreeHost(s->counts_host);
     if (s->params_host) cudaFreeHost(s->params_host);
     if (s->gather_host) cudaFreeHost(s->gather_host);
@@ -1274,7 +1339,7 @@ cudaEvent_t profile_origin(int device, cudaStream_t st) {
 int32_t launch_saved_impl(ag_sampler *s, bool relaunch);
 
 // Queues the chain described by s->last.  relaunch: the same chain once more with
-// full-size dedup tables (host seeds are already in the handle's device copy).
+// full-size dedup tables (host seeds are already in the handle's pinned copy).
 // A failure part way through leaves kernels of the chain queued: wait for them and
 // mark the handle's device state unknown, so that the next call clears it instead of
 // reusing staging buffers, table generation and batch state under running kernels.
@@ -1353,9 +1418,9 @@ int32_t launch_saved_impl(ag_sampler *s, bool relaunch) {
         p.tiles = s->tiles + (uint64_t)b * s->n_tiles;
         p.epoch_base = s->epoch + 1;
         p.n_seeds = n;
-        if (seeds_mem == AG_MEM_HOST) {
+        if (seeds_mem == AG_MEM_HOST) {  // read from the pinned copy by the chain's first kernel
             if (n && !relaunch) memcpy(s->seeds_pinned + (uint64_t)b * s->cap_seeds, seeds[b], (size_t)n * 4);
-            p.seeds = s->seeds_dev + (uint64_t)b * s->cap_seeds;
+            p.seeds = s->seeds_pinned + (uint64_t)b * s->cap_seeds;
         } else {
             p.seeds = seeds[b];
         }
@@ -1368,7 +1433,7 @@ int32_t launch_saved_impl(ag_sampler *s, bool relaunch) {
         p.edge_ids = s->cfg.track_edge_ids ? B.edge_ids : nullptr;
         p.cap_nodes = B.cap_nodes; p.cap_edges = B.cap_edges;
         p.n_id = B.n_id; p.edge_index_local = B.edge_index_local; p.e_id = B.e_id; p.seed_index = B.seed_index;
-        p.counts = s->counts_dev + b;
+        p.counts = s->counts_host + b;  // pinned: one posted write, visible once the chain's event is
         p.slot_of_seed = s->slot_of_seed + (uint64_t)b * s->cap_seeds;
         p.slot_of_edge = s->slot_of_edge + (uint64_t)b * ecap;
         p.frontier = s->frontier + (uint64_t)b * s->max_frontier;
@@ -1397,21 +1462,25 @@ int32_t launch_saved_impl(ag_sampler *s, bool relaunch) {
     s->pending_pos = (batch_seeds == nullptr);  // a continuing batch advances the handle's stream
     s->epoch += H + 2;
     s->gen += 1;
-    if (seeds_mem == AG_MEM_HOST && !relaunch)
-        AG_CUDA(cudaMemcpyAsync(s->seeds_dev, s->seeds_pinned, (uint64_t)n_batches * s->cap_seeds * 4, cudaMemcpyHostToDevice, st));
-    AG_CUDA(cudaMemcpyAsync(s->params_dev, s->params_host, n_batches * sizeof(SampleParams), cudaMemcpyHostToDevice, st));
-    if (want_x)
-        AG_CUDA(cudaMemcpyAsync(s->gather_dev, s->gather_host, n_batches * sizeof(GatherArgs), cudaMemcpyHostToDevice, st));
-
     const SampleParams *pa = s->params_dev;
     const uint32_t nmax = (uint32_t)max_n;
-    if (nmax) k_insert_seeds<<<dim3((nmax + 255) / 256, n_batches), 256, 0, st>>>(pa);
+    const StagedChain staged{s->params_host, want_x ? s->gather_host : nullptr, s->params_dev, s->gather_dev};
+    const bool fused = nmax <= kFusedSeeds;
+    if (!fused) {
+        k_insert_seeds<<<dim3((nmax + 255) / 256, n_batches), 256, 0, st>>>(staged);
+    } else {
+        const uint32_t k0 = s->cfg.fanout[0];
+        if (nmax <= kTile) k_assign_seeds<1><<<dim3(1, n_batches), kTile, 0, st>>>(staged, k0);
+        else if (nmax <= kTile * 2) k_assign_seeds<2><<<dim3(1, n_batches), kTile, 0, st>>>(staged, k0);
+        else k_assign_seeds<kMaxIPT><<<dim3(1, n_batches), kTile, 0, st>>>(staged, k0);
+    }
     uint64_t items = nmax;  // bound on the items of the stage being launched
     for (uint32_t stage = 0; stage <= H; ++stage) {
         const bool has_next = stage < H;
         const uint32_t k = has_next ? s->cfg.fanout[stage] : 0;
         const uint64_t expect = (stage && s->est_items[stage]) ? std::min(items, s->est_items[stage]) : items;
-        if (has_next) launch_assign<true>(expect, n_batches, st, pa, stage, k);
+        if (stage == 0 && fused) {}  // done above
+        else if (has_next) launch_assign<true>(expect, n_batches, st, pa, stage, k);
         else launch_assign<false>(expect, n_batches, st, pa, stage, k);
         if (has_next && k) {
             // the new vertices of this stage are at most its items
@@ -1421,7 +1490,6 @@ int32_t launch_saved_impl(ag_sampler *s, bool relaunch) {
     }
     AG_CUDA(cudaGetLastError());
     if (s->profile) AG_CUDA(cudaEventRecord(s->ev[1], st));
-    AG_CUDA(cudaMemcpyAsync(s->counts_host, s->counts_dev, n_batches * sizeof(ag_sample_counts), cudaMemcpyDeviceToHost, st));
     s->gathered = false;
     if (want_x) {
         bool aligned = ((uintptr_t)feats->payload % 16) == 0;
