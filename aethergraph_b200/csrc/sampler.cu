@@ -68,6 +68,12 @@ constexpr int kLargeK = 1024;   // largest fanout the k > 32 path keeps in share
 enum : int { kModeUniform = 0, kModeReplace = 1, kModeWeighted = 2, kModeWeightedReplace = 3 };
 enum : int { kPickSmall = 0, kPickLarge = 1, kPickWeighted = 2 };
 
+// A long row of a weighted hop, split into n_slices slices (0: it did not fit the queue).
+struct __align__(16) HubRow {
+    uint32_t batch, vertex;  // position in the batch's frontier
+    uint32_t slice_base, n_slices;
+};
+
 // Parameter block of one batch; a group's blocks sit in one device array that
 // the kernels index with blockIdx.y.
 struct SampleParams {
@@ -98,8 +104,13 @@ struct SampleParams {
     uint32_t *slot_of_edge;
     FrontierEntry *frontier;
     uint64_t frontier_cap;
-    uint32_t *hub_list;   // weighted only: frontier positions of the rows left to k_pick_hubs
-    uint32_t *hub_count;
+    // weighted only, shared by the batches of a chain: the rows left to k_pick_hub_slices
+    HubRow *hub_rows;                // [hub_cap]
+    unsigned long long *hub_count;   // rows queued << 32 | slices handed out
+    uint32_t *hub_thr, *hub_done;    // [hub_cap] per row: lowest k-th best key so far (float bits), slices finished
+    double *hub_key;                 // [hub_cap][k] the slices' best (key, position) pairs
+    uint32_t *hub_pos;
+    uint32_t hub_cap, hub_slice;     // slices the arrays hold, positions per slice
 };
 
 // Row bounds with the reference's guard (graph/csr.rs:318-335): an inverted
@@ -362,7 +373,6 @@ __device__ __forceinline__ void topk_insert_chunk(double key, uint32_t cpos, dou
     }
 }
 
-// Streams positions [begin, end) of the row of `fe` into the warp's sorted best k.
 // Exact key of position `pos` of the row (sampler.rs:1440-1452): u from the position's
 // own draw, key = -ln(u) / w, +inf for a weight that is not a positive finite number.
 __device__ __forceinline__ double weighted_key(const SampleParams &p, uint32_t hop, const FrontierEntry &fe, uint32_t pos) {
@@ -375,27 +385,51 @@ __device__ __forceinline__ double weighted_key(const SampleParams &p, uint32_t h
     return -log(u) / w;
 }
 
-// Streams positions [begin, end) of the row of `fe` into the warp's sorted best k.
+// Sorts the warp's 32 (key, position) pairs ascending across the lanes (bitonic).
+__device__ __forceinline__ void warp_sort_pairs(double &key, uint32_t &pos, int lane) {
+#pragma unroll
+    for (int size = 2; size <= 32; size <<= 1) {
+#pragma unroll
+        for (int stride = size >> 1; stride > 0; stride >>= 1) {
+            const double ok = __shfl_xor_sync(0xffffffffu, key, stride);
+            const uint32_t op = __shfl_xor_sync(0xffffffffu, pos, stride);
+            const bool want_small = ((lane & size) == 0) == ((lane & stride) == 0);
+            if (key_less(ok, op, key, pos) == want_small) { key = ok; pos = op; }
+        }
+    }
+}
+
+// Streams positions [begin, end) of the row of `fe` into the warp's sorted best k
+// (all sentinels on entry).
 //
 // Almost every position loses against the k-th best key, and the exact key costs an
 // f64 log and divide, so the stream works in two stages.  Stage 1, all lanes, single
-// precision: with uf >= u (u's top 24 bits, rounded up) -ln(uf) is a LOWER bound of
-// -ln(u); if even that bound, less the error of __logf (< 5e-7 absolute or relative),
-// exceeds thr * w (with slack for the f32 product), the exact key cannot be below the
-// threshold and the position is dropped.  Survivors are only queued (`buf`, 64 slots
-// of the warp's shared memory).  Stage 2, whenever 32 are queued: every lane evaluates
-// one queued position exactly and the winners are inserted.  The threshold is the k-th
-// best key at the last flush (and, when several warps stream slices of one row,
-// `shared_thr`, the lowest k-th best any of them holds; the bit pattern of a
-// non-negative float orders like the float).  It is always an upper bound of the
-// row's final k-th best key, so stage 1 only ever discards certain losers and the
+// precision, no log: with uf >= u (u's top 24 bits, rounded up),
+//     -ln(u) >= -ln(uf) >= 2 (1 - uf) / (1 + uf)
+// (the first term of the series of ln, all terms positive), tight where it matters: a
+// winner of a long row has u near 1.  If 2 (1 - uf) exceeds (1 + uf) * thr * w by more
+// than the rounding of the four f32 operations (< 4 * 2^-24 relative, 1e-5 is granted;
+// 1 - uf is exact, and at least 2^-24 unless it is 0 and nothing is dropped), the exact
+// key cannot be below the threshold and the position is dropped.  Survivors are only
+// queued (`buf`, 64 slots of the warp's shared memory).  Stage 2, whenever 32 are queued:
+// every lane evaluates one queued position exactly and the winners are inserted.  The
+// threshold is the k-th best key at the last flush (and, when several warps stream
+// slices of one row, `shared_thr`, the lowest k-th best any of them holds; the bit
+// pattern of a non-negative float orders like the float).  It is always an upper bound
+// of the row's final k-th best key, so stage 1 only ever discards certain losers and the
 // winners — and the output — are exactly those of evaluating every position.
+//
+// Bound: the 64 x 64 -> 128 bit multiply of the random stream and the weights' latency;
+// hence kChunks weight loads in flight per lane.
+constexpr uint32_t kChunks = 4;
+
 __device__ __forceinline__ void topk_stream(const SampleParams &p, uint32_t hop, const FrontierEntry &fe, uint32_t begin,
                                             uint32_t end, uint32_t k, int lane, double &best_key, uint32_t &best_pos,
                                             uint32_t *buf, uint32_t *shared_thr = nullptr) {
     const double inf = __longlong_as_double(0x7FF0000000000000ll);
     uint32_t queued = 0;  // warp-uniform
-    float thr = (float)__shfl_sync(0xffffffffu, best_key, k - 1);
+    bool fresh = true;    // nothing inserted yet
+    float thr = __uint_as_float(0x7F800000u);
     auto flush = [&](uint32_t count) {  // evaluate buf[0 .. count) exactly, one per lane, and insert the winners
         double key = inf;
         uint32_t cpos = 0xFFFFFFFFu;
@@ -403,7 +437,13 @@ __device__ __forceinline__ void topk_stream(const SampleParams &p, uint32_t hop,
             cpos = buf[lane];
             key = weighted_key(p, hop, fe, cpos);
         }
-        topk_insert_chunk(key, cpos, best_key, best_pos, k, lane);
+        if (fresh) {
+            warp_sort_pairs(key, cpos, lane);
+            best_key = key; best_pos = cpos;
+            fresh = false;
+        } else {
+            topk_insert_chunk(key, cpos, best_key, best_pos, k, lane);
+        }
         const double kth = __shfl_sync(0xffffffffu, best_key, k - 1);
         thr = (float)kth;
         if (shared_thr) {
@@ -411,42 +451,62 @@ __device__ __forceinline__ void topk_stream(const SampleParams &p, uint32_t hop,
             if (lane == 0 && up < 3.0e38f) atomicMin(shared_thr, __float_as_uint(up));
         }
     };
-    for (uint32_t c = begin; c < end; c += 32) {
-        const uint32_t pos = c + lane;
+    const float *w = p.weights + fe.off;
+    for (uint64_t c = begin; c < end; c += 32 * kChunks) {
         float t = thr;
-        if (shared_thr) t = fminf(t, __uint_as_float(*(volatile uint32_t *)shared_thr));
-        bool keep = pos < end;
-        if (keep && t >= 1.0e-30f) {  // a finite threshold in the normal range: no under- or overflow below
-            const uint64_t bits = (p.rng_mode == AG_RNG_PHILOX)
-                ? (((uint64_t)philox_u32(p.seed, hop, fe.id, 2 * pos) << 32) | philox_u32(p.seed, hop, fe.id, 2 * pos + 1))
-                : wyrand_at(p.seed, fe.dbase + pos);
-            const float wf = __ldg(p.weights + fe.off + pos);
-            if (wf > 0.0f && wf <= 3.0e38f) {
-                const float uf = (float)((uint32_t)(bits >> 40) + 1u) * 5.9604644775390625e-08f;  // 2^-24, exact
-                const float lower = -__logf(uf);
-                keep = !(lower * 0.999998f - 1.0e-6f > t * wf * 1.00001f + 1.0e-6f);
-            }
+        if (shared_thr) t = fminf(t, __uint_as_float(__ldcg(shared_thr)));
+        float wf[kChunks];
+#pragma unroll
+        for (uint32_t u = 0; u < kChunks; ++u) {
+            const uint64_t pos = c + u * 32 + lane;
+            wf[u] = pos < end ? __ldg(w + pos) : 0.0f;
         }
-        const uint32_t m = __ballot_sync(0xffffffffu, keep);
-        if (keep) buf[queued + __popc(m & ((1u << lane) - 1u))] = pos;
-        queued += __popc(m);
-        __syncwarp();
-        if (queued >= 32) {
-            flush(32);
+#pragma unroll
+        for (uint32_t u = 0; u < kChunks; ++u) {
+            const uint64_t pos64 = c + u * 32 + lane;
+            const uint32_t pos = (uint32_t)pos64;
+            bool keep = pos64 < end;
+            if (t >= 1.0e-30f) {  // in the normal range: no underflow below
+                if (wf[u] > 0.0f && isfinite(wf[u])) {  // thr * w may overflow: nothing is dropped
+                    const uint32_t n = 1u + ((p.rng_mode == AG_RNG_PHILOX) ? philox_u32(p.seed, hop, fe.id, 2 * pos) >> 8
+                                                                            : (uint32_t)(wyrand_at(p.seed, fe.dbase + pos) >> 40));
+                    const float twice_below = (float)(0x1000000u - n) * 1.1920928955078125e-07f;  // 2 (1 - uf), exact
+                    const float above = (float)(0x1000000u + n) * 5.9604644775390625e-08f;         // 1 + uf
+                    if (twice_below > above * (t * wf[u]) * 1.00001f) keep = false;
+                } else if (t <= 3.0e38f) {
+                    keep = false;  // key +inf against a finite k-th best
+                }
+            }
+            const uint32_t m = __ballot_sync(0xffffffffu, keep);
+            if (!m) continue;
+            if (keep) buf[queued + __popc(m & ((1u << lane) - 1u))] = pos;
+            queued += __popc(m);
             __syncwarp();
-            const uint32_t rest = queued - 32;  // < 32: move the tail to the front
-            const uint32_t moved = (uint32_t)lane < rest ? buf[32 + lane] : 0;
-            __syncwarp();
-            if ((uint32_t)lane < rest) buf[lane] = moved;
-            queued = rest;
-            __syncwarp();
+            if (queued >= 32) {
+                flush(32);
+                __syncwarp();
+                const uint32_t rest = queued - 32;  // < 32: move the tail to the front
+                const uint32_t moved = (uint32_t)lane < rest ? buf[32 + lane] : 0;
+                __syncwarp();
+                if ((uint32_t)lane < rest) buf[lane] = moved;
+                queued = rest;
+                __syncwarp();
+            }
         }
     }
     if (queued) { flush(queued); __syncwarp(); }
 }
 
-constexpr uint32_t kHubDegree = 4096;  // rows longer than this are left to k_pick_hubs (a whole block per row)
-constexpr int kHubThreads = 512;
+// Rows longer than kHubDegree are split into slices, a warp each, by k_pick_hub_slices;
+// a warp alone takes about 1 us per 1000 positions, so the rows left to one warp end
+// together with the rest of the hop.
+constexpr uint32_t kHubDegree = 2048;
+constexpr uint32_t kMaxHubSlices = 65536;   // slices a chain's queue holds; a row that does not fit stays with its warp
+constexpr uint32_t kMaxSlicesPerRow = 256;  // the merge of a row is one warp's work
+
+__device__ __forceinline__ uint32_t hub_slice_len(uint32_t deg, uint32_t slice) {
+    return max(slice, (deg / kMaxSlicesPerRow + 32u) & ~31u);
+}
 
 __device__ __forceinline__ void pick_weighted(const SampleParams &p, uint32_t hop, uint32_t k, uint32_t edges_before,
                                               const FrontierEntry *fes, uint32_t n, uint32_t *queue) {
@@ -461,9 +521,21 @@ __device__ __forceinline__ void pick_weighted(const SampleParams &p, uint32_t ho
             for (uint32_t t = lane; t < deg; t += 32) emit_edge(p, hop, edges_before, fe, t, fe.off + t);
             continue;
         }
-        if (deg > kHubDegree && p.hub_list) {  // queue the hub for the block-per-row kernel
-            if (lane == 0) p.hub_list[atomicAdd(p.hub_count, 1u)] = j;
-            continue;
+        if (deg > kHubDegree) {  // queue the row for the slice kernel
+            bool queued = false;
+            if (lane == 0) {
+                const uint32_t len = hub_slice_len(deg, p.hub_slice), slices = (deg - 1) / len + 1;
+                // one atomic for both counters: the rows' slice ranges ascend in queue order
+                const unsigned long long at = atomicAdd(p.hub_count, (1ull << 32) | slices);
+                const uint32_t h = (uint32_t)(at >> 32), base = (uint32_t)at;
+                queued = (uint64_t)base + slices <= p.hub_cap;
+                if (h < p.hub_cap) {
+                    p.hub_rows[h] = HubRow{blockIdx.y, j, base, queued ? slices : 0u};
+                    p.hub_thr[h] = 0x7F800000u;  // +inf
+                    p.hub_done[h] = 0;
+                }
+            }
+            if (__shfl_sync(0xffffffffu, queued, 0)) continue;
         }
         double best_key = inf;
         uint32_t best_pos = 0xFFFFFFFFu;  // sentinel: sorts after every real (key, position)
@@ -763,7 +835,7 @@ __device__ __forceinline__ void assign_stage(const SampleParams &p, uint32_t sta
                     nx.hop_draws = 0;
                     bs->stage[stage + 1] = nx;
                     bs->nodes_per_stage[stage] = tot.flags;
-                    if (p.hub_count) *p.hub_count = 0;  // the hop's hub queue starts empty
+                    if (p.hub_count) *p.hub_count = 0;  // the hop's hub queue starts empty (every batch says so)
                     if (stage == 0) bs->stage[0] = si;  // what the counts measure the draws against
                 }
             }
@@ -888,43 +960,64 @@ k_pick(const SampleParams *__restrict__ pa, uint32_t hop, uint32_t k) {
     else pick_small<G>(p, hop, k, nx.n_edges, p.frontier, nx.frontier_n);
 }
 
-// Hub rows of a weighted hop: one block per queued row.  Every warp streams an
-// equal slice of the row into its own best k, the slices' winners meet in shared
-// memory and warp 0 merges them; (key, position) is a total order, so the k
-// smallest — and their emission order — do not depend on how the row was split.
-__global__ void __launch_bounds__(kHubThreads)
-k_pick_hubs(const SampleParams *__restrict__ pa, uint32_t hop, uint32_t k) {
-    __shared__ double s_key[kHubThreads / 32][32];
-    __shared__ uint32_t s_pos[kHubThreads / 32][32];
-    __shared__ uint32_t s_thr;  // float bits: lowest k-th best key any warp holds for the current row
-    __shared__ uint32_t s_queue[(kHubThreads / 32) * 64];
+// The queued rows of a weighted hop, a warp per slice, whatever batch of the chain they
+// belong to.  Every slice leaves its best k; the warp that finishes a row's last slice
+// merges them and emits.  (key, position) is a total order, so the k smallest — and their
+// emission order — do not depend on how the row was split or which warp merges.
+//
+// A row of 500 K positions on one block of 512 threads took 450 us, as long for one batch
+// as for eight.  Twelve batches of 512 seeds, fanouts 15, 10, 5, on the 10 M vertex / 200 M
+// edge graph (28 M positions a batch): 5320 us with a block per row, 3600 us with slices.
+__global__ void __launch_bounds__(kPickThreads)
+k_pick_hub_slices(const SampleParams *__restrict__ pa, uint32_t hop, uint32_t k) {
+    __shared__ uint32_t s_queue[(kPickThreads / 32) * 64];
     chain_sync();
-    const SampleParams &p = pa[blockIdx.y];
-    const StageInfo nx = p.state->stage[hop + 1];
+    const SampleParams &q = pa[0];  // the queue is the same for every batch
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    constexpr int kWarps = kHubThreads / 32;
     const double inf = __longlong_as_double(0x7FF0000000000000ll);
-    const uint32_t hubs = min(*p.hub_count, nx.frontier_n);
-    for (uint32_t h = blockIdx.x; h < hubs; h += gridDim.x) {
-        const FrontierEntry fe = p.frontier[p.hub_list[h]];
-        const uint32_t deg = fe.deg;
-        const uint32_t per = ((deg + kWarps - 1) / kWarps + 31) & ~31u;  // slice per warp, whole chunks of 32
-        const uint32_t begin = min(deg, (uint32_t)warp * per), end = min(deg, begin + per);
+    const unsigned long long count = *q.hub_count;
+    const uint32_t rows = min((uint32_t)(count >> 32), q.hub_cap), slices = min((uint32_t)count, q.hub_cap);
+    for (uint32_t slice = blockIdx.x * (kPickThreads / 32) + warp; slice < slices; slice += gridDim.x * (kPickThreads / 32)) {
+        // the last row whose slices start at or before this one; 32 probes a step
+        uint32_t lo = 0, n = rows;
+        while (n > 1) {
+            const uint32_t step = (n + 31) / 32, at = lane * step;
+            const uint32_t m = __ballot_sync(0xffffffffu, at < n && q.hub_rows[lo + at].slice_base <= slice);
+            const uint32_t hit = 31 - __clz(m);  // lane 0 always holds
+            lo += hit * step;
+            n = min(step, n - hit * step);
+        }
+        const HubRow row = q.hub_rows[lo];
+        if (row.n_slices == 0) continue;  // did not fit: its own warp has done it
+        const SampleParams &p = pa[row.batch];
+        const FrontierEntry fe = p.frontier[row.vertex];
+        const uint32_t deg = fe.deg, len = hub_slice_len(deg, q.hub_slice);
+        const uint64_t first = (uint64_t)(slice - row.slice_base) * len;
+        const uint32_t begin = (uint32_t)min((uint64_t)deg, first), end = (uint32_t)min((uint64_t)deg, first + len);
         double best_key = inf;
         uint32_t best_pos = 0xFFFFFFFFu;
-        if (threadIdx.x == 0) s_thr = 0x7F800000u;  // +inf
-        __syncthreads();
-        topk_stream(p, hop, fe, begin, end, k, lane, best_key, best_pos, s_queue + warp * 64, &s_thr);
-        s_key[warp][lane] = best_key; s_pos[warp][lane] = best_pos;
-        __syncthreads();
-        if (warp == 0) {
-            for (int w = 1; w < kWarps; ++w) {
-                const bool have = (uint32_t)lane < k && s_pos[w][lane] != 0xFFFFFFFFu;
-                topk_insert_chunk(have ? s_key[w][lane] : inf, have ? s_pos[w][lane] : 0xFFFFFFFFu, best_key, best_pos, k, lane);
+        topk_stream(p, hop, fe, begin, end, k, lane, best_key, best_pos, s_queue + warp * 64, q.hub_thr + lo);
+        if (row.n_slices > 1) {
+            const uint64_t mine = (uint64_t)slice * k;
+            if ((uint32_t)lane < k) { q.hub_key[mine + lane] = best_key; q.hub_pos[mine + lane] = best_pos; }
+            __threadfence();
+            __syncwarp();
+            uint32_t before = 0;
+            if (lane == 0) before = atomicAdd(q.hub_done + lo, 1u);
+            if (__shfl_sync(0xffffffffu, before, 0) != row.n_slices - 1) continue;
+            __threadfence();
+            const uint64_t from = (uint64_t)row.slice_base * k;
+            const uint32_t cands = row.n_slices * k;
+            for (uint32_t c = 0; c < cands; c += 32) {
+                const uint32_t i = c + lane;
+                // this slice's own best are in the lanes already
+                const bool have = i < cands && i / k != slice - row.slice_base;
+                const double ck = have ? __ldcg(q.hub_key + from + i) : inf;
+                const uint32_t cp = have ? __ldcg(q.hub_pos + from + i) : 0xFFFFFFFFu;
+                topk_insert_chunk(ck, cp, best_key, best_pos, k, lane);
             }
-            if ((uint32_t)lane < k) emit_edge(p, hop, nx.n_edges, fe, lane, fe.off + best_pos);
         }
-        __syncthreads();
+        if ((uint32_t)lane < k) emit_edge(p, hop, p.state->stage[hop + 1].n_edges, fe, lane, fe.off + best_pos);
     }
 }
 
@@ -984,8 +1077,8 @@ void launch_pick(int mode, uint32_t k, uint64_t frontier_est, uint32_t n_batches
         launch_chained(k_pick_weighted_large, dim3(blocks_for(frontier_est, 1), n_batches), dim3(kWLThreads), st, pa, hop, k);
     } else if (mode == kModeWeighted) {
         launch_chained(k_pick<32, kPickWeighted>, dim3(blocks_for(frontier_est, kPickThreads / 32), n_batches), dim3(kPickThreads), st, pa, hop, k);
-        // rows longer than kHubDegree were only queued: one block per queued row
-        launch_chained(k_pick_hubs, dim3(std::max<uint32_t>(1, (uint32_t)(kSMs * 2 / n_batches)), n_batches), dim3(kHubThreads), st, pa, hop, k);
+        // rows longer than kHubDegree were only queued: a warp per slice of them
+        launch_chained(k_pick_hub_slices, dim3((uint32_t)kSMs * 4), dim3(kPickThreads), st, pa, hop, k);
     } else if (k > 32) {
         launch_chained(k_pick<32, kPickLarge>, dim3(blocks_for(frontier_est, 4), n_batches), dim3(128), st, pa, hop, k);
     } else {
@@ -1027,7 +1120,12 @@ struct ag_sampler {
     FrontierEntry *frontier = nullptr;
     uint64_t max_frontier = 0;
     uint32_t *slot_of_seed = nullptr, *slot_of_edge = nullptr;
-    uint32_t *hub_list = nullptr;  // weighted only: per batch max_frontier queue slots + 1 counter word
+    // weighted only: the queue of long rows, one for the chain (hub_rows is the allocation)
+    HubRow *hub_rows = nullptr;
+    unsigned long long *hub_count = nullptr;
+    uint32_t *hub_thr = nullptr, *hub_done = nullptr, *hub_pos = nullptr;
+    double *hub_key = nullptr;
+    uint32_t hub_cap = 0;
     TileDesc *tiles = nullptr;
     BatchState *state = nullptr;
     SampleParams *params_dev = nullptr;
@@ -1099,7 +1197,7 @@ void free_scratch(ag_sampler *s) {
     cudaFree(s->table); cudaFree(s->frontier);
     s->frontier = nullptr;
     cudaFree(s->slot_of_seed); cudaFree(s->slot_of_edge); cudaFree(s->tiles);
-    cudaFree(s->hub_list); s->hub_list = nullptr;
+    cudaFree(s->hub_rows); s->hub_rows = nullptr;
     if (s->seeds_pinned) cudaFreeHost(s->seeds_pinned);
     s->table = nullptr;
     s->slot_of_seed = s->slot_of_edge = nullptr; s->tiles = nullptr;
@@ -1133,8 +1231,21 @@ int32_t ensure_scratch(ag_sampler *s, uint64_t n_seeds) {
     AG_CUDA(cudaMalloc(&s->slot_of_seed, G * cap * 4));
     AG_CUDA(cudaMalloc(&s->slot_of_edge, G * std::max<uint64_t>(s->max_edges, 1) * 4));
     if (s->mode == kModeWeighted) {
-        AG_CUDA(cudaMalloc(&s->hub_list, G * (s->max_frontier + 1) * 4));
-        AG_CUDA(cudaMemset(s->hub_list, 0, G * (s->max_frontier + 1) * 4));
+        // A batch expands a vertex once, and a row of d > kHubDegree positions is at most
+        // 2 d / kHubDegree slices.
+        const uint64_t most = 2 * (s->g->num_edges / kHubDegree) * G;
+        uint64_t hop_k = 1;
+        for (uint32_t h = 0; h < s->cfg.num_hops; ++h) hop_k = std::max<uint64_t>(hop_k, std::min<uint32_t>(s->cfg.fanout[h], 32u));
+        s->hub_cap = (uint32_t)std::min<uint64_t>(std::max<uint64_t>(most, 1), kMaxHubSlices);
+        const uint64_t cap = s->hub_cap;
+        uint8_t *base = nullptr;
+        AG_CUDA(cudaMalloc(&base, cap * (sizeof(HubRow) + 8 * hop_k + 4 * hop_k + 8) + 8));
+        s->hub_rows = (HubRow *)base;
+        s->hub_key = (double *)(base + cap * sizeof(HubRow));
+        s->hub_count = (unsigned long long *)(s->hub_key + cap * hop_k);
+        s->hub_pos = (uint32_t *)(s->hub_count + 1);
+        s->hub_thr = s->hub_pos + cap * hop_k;
+        s->hub_done = s->hub_thr + cap;
     }
     s->n_tiles = std::max<uint64_t>(std::max(cap, s->max_hop_edges) / kTile + 2, 2);
     AG_CUDA(cudaMalloc(&s->tiles, G * s->n_tiles * sizeof(TileDesc)));
@@ -1438,9 +1549,11 @@ int32_t launch_saved_impl(ag_sampler *s, bool relaunch) {
         p.slot_of_edge = s->slot_of_edge + (uint64_t)b * ecap;
         p.frontier = s->frontier + (uint64_t)b * s->max_frontier;
         p.frontier_cap = s->max_frontier;
-        if (s->hub_list) {
-            p.hub_count = s->hub_list + (uint64_t)b * (s->max_frontier + 1);
-            p.hub_list = p.hub_count + 1;
+        if (s->hub_rows) {
+            p.hub_rows = s->hub_rows; p.hub_count = s->hub_count; p.hub_thr = s->hub_thr; p.hub_done = s->hub_done;
+            p.hub_key = s->hub_key; p.hub_pos = s->hub_pos; p.hub_cap = s->hub_cap;
+            // about as many slices whatever the chain's length: a slice of kHubDegree positions per batch
+            p.hub_slice = (uint32_t)std::min<uint64_t>(kHubDegree * next_pow2(n_batches), 16 * kHubDegree);
         }
         s->params_host[b] = p;
         uint64_t bn, be;

@@ -1,0 +1,68 @@
+"""Rows far longer than the rest of their hop, against the CPU oracle, at the edges of the
+slices they are split into."""
+import numpy as np
+import pytest
+
+from helpers import assert_same_subgraph, csr_from_edges
+
+pytestmark = pytest.mark.gpu
+
+
+def _hub_graph(degrees, n, seed, weights=None):
+    """Vertex i < len(degrees) has degrees[i] neighbours, every other vertex five of them hubs."""
+    rng = np.random.default_rng(seed)
+    src = [np.full(d, i) for i, d in enumerate(degrees)] + [np.repeat(np.arange(len(degrees), n), 5)]
+    src = np.concatenate(src).astype(np.uint32)
+    dst = rng.integers(0, n, len(src)).astype(np.uint32)
+    low = src >= len(degrees)
+    dst[low] = rng.integers(0, len(degrees), int(low.sum()))
+    w = None
+    if weights == "lognormal":
+        w = rng.lognormal(0.0, 1.0, len(src)).astype(np.float32)
+    elif weights == "equal":
+        w = np.ones(len(src), dtype=np.float32)
+    elif weights == "odd":  # zeros, negatives, infinities, NaN and subnormal weights never win before a real one
+        w = rng.lognormal(0.0, 1.0, len(src)).astype(np.float32)
+        w[rng.random(len(w)) < 0.9995] = 0.0
+        for value in (-1.0, np.inf, np.nan, 1e-42, 3.3e38, 1e-30):
+            w[rng.integers(0, len(w), 50)] = value
+    return csr_from_edges(n, src, dst, w)
+
+
+DEGREES = [2047, 2048, 2049, 4096, 4097, 31, 33, 70_000, 530_001, 9000, 0, 1, 16, 15]
+
+
+@pytest.mark.parametrize("weights", ["lognormal", "equal", "odd"])
+@pytest.mark.parametrize("fanout,rng_mode", [([15, 4], "wyrand_exact"), ([32], "wyrand_exact"), ([1, 1, 2], "wyrand_exact")])
+def test_weighted(weights, fanout, rng_mode):
+    import aethergraph_b200 as ag
+    from oracle import ago
+
+    n = 4000
+    off, dst, w = _hub_graph(DEGREES, n, 3, weights)
+    g = ag.Graph.from_csr(off, dst, w)
+    cfg = ag.SamplingConfig(num_neighbors=fanout, weighted=True, seed=11, rng_mode=rng_mode)
+    o = ago.Sampler(off, dst, fanout, weights=w, weighted=True, seed=11)
+    s = ag.NeighborSampler(g, cfg)
+    for count in (len(DEGREES), 1, 60):
+        seeds = np.arange(count, dtype=np.uint32)[::-1].copy()
+        assert_same_subgraph(s.sample(seeds).raw_u32(), o.sample(seeds))
+    batches = [np.arange(len(DEGREES) - i, dtype=np.uint32) for i in range(8)]
+    for i, sg in enumerate(ag.ParallelBatchSampler(g, cfg, group=8).sample_batches(batches)):
+        o.reseed(ago.batch_seed(11, i))
+        assert_same_subgraph(sg.raw_u32(), o.sample(batches[i]), ctx=f"batch {i}: ")
+
+
+def test_more_slices_than_the_queue_holds():
+    """64 batches that each expand 40 rows of 66 000 positions: 84 480 slices asked for."""
+    import aethergraph_b200 as ag
+    from oracle import ago
+
+    off, dst, w = _hub_graph([66_000] * 40, 2000, 5, "lognormal")
+    g = ag.Graph.from_csr(off, dst, w)
+    cfg = ag.SamplingConfig(num_neighbors=[10], weighted=True, seed=4)
+    o = ago.Sampler(off, dst, [10], weights=w, weighted=True, seed=4)
+    batches = [np.roll(np.arange(40, dtype=np.uint32), i) for i in range(64)]
+    for i, sg in enumerate(ag.ParallelBatchSampler(g, cfg, streams=1, group=64).sample_batches(batches)):
+        o.reseed(ago.batch_seed(4, i))
+        assert_same_subgraph(sg.raw_u32(), o.sample(batches[i]), ctx=f"batch {i}: ")
