@@ -173,89 +173,185 @@ extern "C" int32_t ag_subgraph_mirror(int32_t device, uint64_t n_edges, uint64_t
 // ------------------------------------------------------------------ induce --
 namespace {
 
-constexpr uint32_t kEmptyNode = 0xFFFFFFFFu;
+// The rows of the sampled nodes, one after the other in local order, form one list of
+// positions: the result is the hits of that list, in list order.  Every warp takes an
+// equal stretch of it, whatever rows it crosses, counts its hits (first walk) and, once
+// the counts are scanned, writes them behind the stretches before it (second walk).
+//
+// Rows differ by five orders of magnitude (a hub of an R-MAT graph of 64 M edges has
+// over 100 K neighbours, most vertices a few), so a warp per row left the two walks to
+// the warp with the longest one: 200 seeds, fanouts 10, 5 on that graph reach 3200 nodes
+// and 5.7 M positions, 2660 + 3080 us at 4 % of the warps busy.
+constexpr int kWalkThreads = 256;
+constexpr uint32_t kWalkWarpsPerSM = 32;
+constexpr uint32_t kWalkMin = 128;   // positions a warp takes at least
+constexpr uint32_t kWalkUnroll = 4;  // 32-position chunks in flight in a long row
 
 __device__ __forceinline__ uint32_t node_slot(uint32_t v, uint32_t mask) { return (uint32_t)(mix64(v) & mask); }
 
-// The sampled nodes are distinct: node -> local index.
-__global__ void k_induce_insert(const uint32_t *__restrict__ nodes, uint64_t n, uint32_t *keys, uint32_t *vals, uint32_t mask,
-                                uint32_t *err) {
+// The sampled nodes are distinct: table of node << 32 | local index, and every node's row.
+__global__ void k_induce_insert(const uint64_t *__restrict__ offsets, uint64_t num_graph_nodes, uint64_t num_edges,
+                                const uint32_t *__restrict__ nodes, uint64_t n, unsigned long long *table, uint32_t mask,
+                                uint64_t *row_off, uint64_t *row_len, uint32_t *err) {
     for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
         const uint32_t v = nodes[i];
+        uint64_t lo = 0, hi = 0;
+        if ((uint64_t)v < num_graph_nodes) { lo = offsets[v]; hi = offsets[(uint64_t)v + 1]; }
+        row_off[i] = lo;
+        row_len[i] = (hi > lo && hi <= num_edges) ? hi - lo : 0;
+        const unsigned long long entry = ((unsigned long long)v << 32) | (uint32_t)i;
         uint32_t slot = node_slot(v, mask);
         bool done = false;
         for (uint32_t probe = 0; probe <= mask && !done; ++probe) {
-            const uint32_t prev = atomicCAS(&keys[slot], kEmptyNode, v);
-            if (prev == kEmptyNode || prev == v) { vals[slot] = (uint32_t)i; done = true; }
-            else slot = (slot + 1) & mask;
+            done = atomicCAS(&table[slot], (unsigned long long)kEmptyKey, entry) == kEmptyKey;
+            slot = (slot + 1) & mask;
         }
         if (!done) atomicOr(err, 1u);
     }
 }
 
-__device__ __forceinline__ uint32_t node_lookup(const uint32_t *__restrict__ keys, const uint32_t *__restrict__ vals,
-                                                uint32_t mask, uint32_t v) {
+// Local index of node v, or 0xFFFFFFFF (never one: a plan holds fewer than 2^30 nodes).
+__device__ __forceinline__ uint32_t node_lookup(const unsigned long long *__restrict__ table, uint32_t mask, uint32_t v) {
     uint32_t slot = node_slot(v, mask);
     for (uint32_t probe = 0; probe <= mask; ++probe) {
-        const uint32_t k = keys[slot];
-        if (k == v) return vals[slot];
-        if (k == kEmptyNode) return kEmptyNode;
+        const unsigned long long e = __ldg(table + slot);
+        if (e == kEmptyKey) return 0xFFFFFFFFu;
+        if ((uint32_t)(e >> 32) == v) return (uint32_t)e;
         slot = (slot + 1) & mask;
     }
-    return kEmptyNode;
+    return 0xFFFFFFFFu;
 }
 
-// One warp per sampled node: walks the node's row 32 neighbours at a time.  With
-// FILL the hits are written in row order behind row_start[u_local]; without, they
-// are counted.
-template <bool FILL>
-__global__ void k_induce_rows(const uint64_t *__restrict__ offsets, const uint32_t *__restrict__ dst, uint64_t num_graph_nodes,
-                              const uint32_t *__restrict__ nodes, uint64_t n, const uint32_t *__restrict__ keys,
-                              const uint32_t *__restrict__ vals, uint32_t mask, uint64_t *row_count,
-                              const uint64_t *__restrict__ row_start, uint32_t *edge_src, uint32_t *edge_dst, uint32_t *sl,
-                              uint32_t *dl, uint64_t *edge_ids) {
-    const uint32_t lane = threadIdx.x & 31;
-    const uint64_t warps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
-    for (uint64_t u_local = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; u_local < n; u_local += warps) {
-        const uint32_t u = nodes[u_local];
-        uint64_t lo = 0, hi = 0;
-        if ((uint64_t)u < num_graph_nodes) { lo = offsets[u]; hi = offsets[(uint64_t)u + 1]; }
-        uint64_t out = FILL ? row_start[u_local] : 0, count = 0;
-        for (uint64_t base = lo; base < hi; base += 32) {
-            const uint64_t pos = base + lane;
-            uint32_t w = 0, w_local = kEmptyNode;
-            if (pos < hi) { w = dst[pos]; w_local = node_lookup(keys, vals, mask, w); }
-            const uint32_t hits = __ballot_sync(0xFFFFFFFFu, w_local != kEmptyNode);
-            if (FILL) {
-                if (w_local != kEmptyNode) {
-                    const uint64_t o = out + __popc(hits & ((1u << lane) - 1));
-                    edge_src[o] = u; edge_dst[o] = w; sl[o] = (uint32_t)u_local; dl[o] = w_local;
-                    if (edge_ids) edge_ids[o] = pos;
-                }
-                out += __popc(hits);
-            } else {
-                count += __popc(hits);
-            }
-        }
-        if (!FILL && lane == 0) row_count[u_local] = count;
+struct InduceWalk {
+    const uint32_t *dst, *nodes;
+    uint64_t n;
+    const uint64_t *row_off;    // [n] first CSR position of every node's row
+    const uint64_t *row_start;  // [n + 1] its first position in the list
+    const unsigned long long *table;
+    uint32_t mask, warps;
+    uint64_t *warp_start;       // [warps] hits, then (scanned) hits before the warp's stretch
+    uint64_t *total;            // [0] all hits, [1] blocks that have counted
+};
+
+struct InduceOut {
+    uint32_t *edge_src, *edge_dst, *sl, *dl;
+    uint64_t *edge_ids;
+    int64_t *edge_index_local;
+    uint64_t n_edges;
+};
+
+// Row that holds position g of the list, searched from row `lo` on.
+__device__ __forceinline__ uint64_t row_of(const uint64_t *__restrict__ row_start, uint64_t n, uint64_t lo, uint64_t g) {
+    uint64_t hi = n;  // row_start[lo] <= g < row_start[hi]
+    while (hi - lo > 1) {
+        const uint64_t mid = (lo + hi) >> 1;
+        if (__ldg(row_start + mid) <= g) lo = mid; else hi = mid;
     }
+    return lo;
+}
+
+template <bool FILL>
+__global__ void __launch_bounds__(kWalkThreads)
+k_induce_walk(InduceWalk a, InduceOut o) {
+    const uint32_t lane = threadIdx.x & 31, w = (blockIdx.x * kWalkThreads + threadIdx.x) >> 5;
+    const uint64_t all = a.row_start[a.n];
+    const uint64_t share = ((all + a.warps - 1) / a.warps + 31) & ~31ull;
+    const uint64_t per = share > kWalkMin ? share : kWalkMin;
+    uint64_t g = min(all, (uint64_t)w * per);
+    const uint64_t stop = min(all, g + per);
+    uint64_t out = FILL ? a.warp_start[w] : 0;
+    uint64_t count = 0;
+    // hits of 32 positions: lane's neighbour v at CSR position pos in the row of local index r
+    auto take = [&](uint32_t hit, uint32_t v, uint64_t pos, uint32_t r, uint32_t node) {
+        const uint32_t m = __ballot_sync(0xFFFFFFFFu, hit != 0xFFFFFFFFu);
+        if (FILL) {
+            if (hit != 0xFFFFFFFFu) {
+                const uint64_t at = out + __popc(m & ((1u << lane) - 1));
+                o.edge_src[at] = node; o.edge_dst[at] = v; o.sl[at] = r; o.dl[at] = hit;
+                if (o.edge_ids) o.edge_ids[at] = pos;
+                if (o.edge_index_local) { o.edge_index_local[at] = (int64_t)hit; o.edge_index_local[o.n_edges + at] = (int64_t)r; }
+            }
+            out += __popc(m);
+        } else {
+            count += __popc(m);
+        }
+    };
+    uint64_t row = 0;
+    while (g < stop) {
+        row = row_of(a.row_start, a.n, row, g);
+        const uint64_t begin = __ldg(a.row_start + row), end = min(stop, __ldg(a.row_start + row + 1));
+        if (end - g >= 32 * kWalkUnroll) {  // a long row: whole chunks of it
+            const uint64_t base = __ldg(a.row_off + row) - begin;  // list position -> CSR position
+            const uint32_t node = FILL ? __ldg(a.nodes + row) : 0;
+            for (; end - g >= 32 * kWalkUnroll; g += 32 * kWalkUnroll) {
+                uint32_t v[kWalkUnroll], hit[kWalkUnroll];
+#pragma unroll
+                for (uint32_t u = 0; u < kWalkUnroll; ++u) v[u] = ld_stream_u32(a.dst + base + g + u * 32 + lane);
+#pragma unroll
+                for (uint32_t u = 0; u < kWalkUnroll; ++u) hit[u] = node_lookup(a.table, a.mask, v[u]);
+#pragma unroll
+                for (uint32_t u = 0; u < kWalkUnroll; ++u) take(hit[u], v[u], base + g + u * 32 + lane, (uint32_t)row, node);
+            }
+        } else {  // 32 positions of whatever rows they lie in
+            const uint64_t mine = g + lane;
+            uint64_t r = row, pos = 0;
+            uint32_t v = 0, hit = 0xFFFFFFFFu;
+            if (mine < stop) {
+                r = row_of(a.row_start, a.n, row, mine);
+                pos = __ldg(a.row_off + r) + (mine - __ldg(a.row_start + r));
+                v = ld_stream_u32(a.dst + pos);
+                hit = node_lookup(a.table, a.mask, v);
+            }
+            const uint32_t node = (FILL && hit != 0xFFFFFFFFu) ? __ldg(a.nodes + r) : 0;
+            take(hit, v, pos, (uint32_t)r, node);
+            g += 32;
+        }
+    }
+    if (FILL) return;
+    if (lane == 0) a.warp_start[w] = count;
+    // The block that counts last scans the warps' counts.
+    __shared__ uint64_t s_sum[kWalkThreads];
+    __shared__ bool s_last;
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) s_last = atomicAdd((unsigned long long *)(a.total + 1), 1ull) == gridDim.x - 1;
+    __syncthreads();
+    if (!s_last) return;
+    __threadfence();
+    const uint32_t each = (a.warps + kWalkThreads - 1) / kWalkThreads;
+    const uint32_t from = min(a.warps, threadIdx.x * each), to = min(a.warps, from + each);
+    uint64_t sum = 0;
+    for (uint32_t i = from; i < to; ++i) sum += __ldcg(a.warp_start + i);
+    s_sum[threadIdx.x] = sum;
+    __syncthreads();
+    for (int d = 1; d < kWalkThreads; d <<= 1) {
+        const uint64_t add = (int)threadIdx.x >= d ? s_sum[threadIdx.x - d] : 0;
+        __syncthreads();
+        s_sum[threadIdx.x] += add;
+        __syncthreads();
+    }
+    uint64_t run = s_sum[threadIdx.x] - sum;
+    for (uint32_t i = from; i < to; ++i) {
+        const uint64_t c = __ldcg(a.warp_start + i);
+        a.warp_start[i] = run;
+        run += c;
+    }
+    if (threadIdx.x == kWalkThreads - 1) a.total[0] = run;
 }
 
 }  // namespace
 
 struct ag_induce_plan {
     int device = 0;
-    const ag_graph *g = nullptr;
-    const uint32_t *nodes = nullptr;
-    uint64_t n_nodes = 0, n_edges = 0;
-    uint32_t *keys = nullptr, *vals = nullptr, mask = 0;
-    uint64_t *row_count = nullptr, *row_start = nullptr;
+    uint64_t n_edges = 0;
+    void *scratch = nullptr;
+    InduceWalk walk{};
 };
 
 extern "C" void ag_subgraph_induce_free(ag_induce_plan *p) {
     if (!p) return;
     DeviceGuard guard(p->device);
-    cudaFree(p->keys); cudaFree(p->vals); cudaFree(p->row_count); cudaFree(p->row_start);
+    cudaFree(p->scratch);
     delete p;
 }
 
@@ -270,41 +366,39 @@ extern "C" int32_t ag_subgraph_induce_plan(const ag_graph *g, const uint32_t *no
     if (!guard.ok) return AG_ERR_CUDA;
     cudaStream_t st = (cudaStream_t)stream;
     ag_induce_plan *p = new ag_induce_plan();
-    p->device = g->device; p->g = g; p->nodes = nodes_dev; p->n_nodes = n_nodes;
+    p->device = g->device;
     *out = nullptr; *n_edges_out = 0;
     if (n_nodes == 0) { *out = p; return AG_OK; }
-    const uint64_t cap = pow2_at_least(2 * n_nodes);
-    p->mask = (uint32_t)(cap - 1);
-    void *temp = nullptr; uint32_t *err = nullptr;
-    auto bail = [&](int32_t rc) { cudaFree(temp); cudaFree(err); ag_subgraph_induce_free(p); return rc; };
+    auto bail = [&](int32_t rc) { ag_subgraph_induce_free(p); return rc; };
 #define AG_PLAN_CUDA(expr) do { const cudaError_t e_ = (expr); if (e_ != cudaSuccess) \
         return bail(fail(AG_ERR_CUDA, "%s failed: %s", #expr, cudaGetErrorString(e_))); } while (0)
-    AG_PLAN_CUDA(cudaMalloc(&p->keys, cap * 4));
-    AG_PLAN_CUDA(cudaMalloc(&p->vals, cap * 4));
-    AG_PLAN_CUDA(cudaMalloc(&p->row_count, (n_nodes + 1) * 8));
-    AG_PLAN_CUDA(cudaMalloc(&p->row_start, (n_nodes + 1) * 8));
-    AG_PLAN_CUDA(cudaMalloc(&err, 4));
-    AG_PLAN_CUDA(cudaMemsetAsync(p->keys, 0xFF, cap * 4, st));
-    AG_PLAN_CUDA(cudaMemsetAsync(err, 0, 4, st));
-    AG_PLAN_CUDA(cudaMemsetAsync(p->row_count + n_nodes, 0, 8, st));
-    k_induce_insert<<<grid_for(n_nodes), 256, 0, st>>>(nodes_dev, n_nodes, p->keys, p->vals, p->mask, err);
-    const uint32_t grid = grid_for(n_nodes * 32);
-    k_induce_rows<false><<<grid, 256, 0, st>>>(g->offsets, g->dst, g->num_nodes, nodes_dev, n_nodes, p->keys, p->vals, p->mask,
-                                               p->row_count, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr);
+    const uint64_t cap = pow2_at_least(2 * n_nodes);
+    const uint32_t warps = (uint32_t)kSMs * kWalkWarpsPerSM;
     size_t temp_bytes = 0;
-    AG_PLAN_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, temp_bytes, p->row_count, p->row_start, (int)(n_nodes + 1), st));
-    AG_PLAN_CUDA(cudaMalloc(&temp, std::max<size_t>(temp_bytes, 16)));
-    AG_PLAN_CUDA(cub::DeviceScan::ExclusiveSum(temp, temp_bytes, p->row_count, p->row_start, (int)(n_nodes + 1), st));
-    uint64_t total = 0; uint32_t herr = 0;
-    AG_PLAN_CUDA(cudaMemcpyAsync(&total, p->row_start + n_nodes, 8, cudaMemcpyDeviceToHost, st));
-    AG_PLAN_CUDA(cudaMemcpyAsync(&herr, err, 4, cudaMemcpyDeviceToHost, st));
-    AG_PLAN_CUDA(cudaStreamSynchronize(st));
+    AG_PLAN_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, temp_bytes, (uint64_t *)nullptr, (uint64_t *)nullptr, (int)(n_nodes + 1), st));
+    // one allocation: table, row offsets, row lengths and their scan, the warps' counts, totals, scan scratch
+    const uint64_t words = cap + n_nodes + 2 * (n_nodes + 1) + warps + 3;
+    const uint64_t temp_at = (words * 8 + 255) & ~255ull;
+    AG_PLAN_CUDA(cudaMalloc(&p->scratch, temp_at + temp_bytes));
+    unsigned long long *table = (unsigned long long *)p->scratch;
+    uint64_t *row_off = (uint64_t *)(table + cap), *row_len = row_off + n_nodes, *row_start = row_len + n_nodes + 1;
+    uint64_t *warp_start = row_start + n_nodes + 1, *total = warp_start + warps;  // total[2]: error bits
+    AG_PLAN_CUDA(cudaMemsetAsync(table, 0xFF, cap * 8, st));
+    AG_PLAN_CUDA(cudaMemsetAsync(total, 0, 24, st));
+    AG_PLAN_CUDA(cudaMemsetAsync(row_len + n_nodes, 0, 8, st));
+    k_induce_insert<<<grid_for(n_nodes), 256, 0, st>>>(g->offsets, g->num_nodes, g->num_edges, nodes_dev, n_nodes, table,
+                                                       (uint32_t)(cap - 1), row_off, row_len, (uint32_t *)(total + 2));
+    AG_PLAN_CUDA(cub::DeviceScan::ExclusiveSum((uint8_t *)p->scratch + temp_at, temp_bytes, row_len, row_start, (int)(n_nodes + 1), st));
+    p->walk = InduceWalk{g->dst, nodes_dev, n_nodes, row_off, row_start, table, (uint32_t)(cap - 1), warps, warp_start, total};
+    k_induce_walk<false><<<warps / (kWalkThreads / 32), kWalkThreads, 0, st>>>(p->walk, InduceOut{});
     AG_PLAN_CUDA(cudaGetLastError());
+    uint64_t got[3] = {0, 0, 0};
+    AG_PLAN_CUDA(cudaMemcpyAsync(got, total, 24, cudaMemcpyDeviceToHost, st));
+    AG_PLAN_CUDA(cudaStreamSynchronize(st));
 #undef AG_PLAN_CUDA
-    cudaFree(temp); cudaFree(err);
-    if (herr) { ag_subgraph_induce_free(p); return fail(AG_ERR_WORKER, "ag_subgraph_induce_plan: node table overflow"); }
-    p->n_edges = total;
-    *n_edges_out = total;
+    if ((uint32_t)got[2]) return bail(fail(AG_ERR_WORKER, "ag_subgraph_induce_plan: node table overflow"));
+    p->n_edges = got[0];
+    *n_edges_out = got[0];
     *out = p;
     return AG_OK;
 }
@@ -322,11 +416,8 @@ extern "C" int32_t ag_subgraph_induce_fill(ag_induce_plan *p, uint64_t cap_edges
     DeviceGuard guard(p->device);
     if (!guard.ok) return AG_ERR_CUDA;
     cudaStream_t st = (cudaStream_t)stream;
-    k_induce_rows<true><<<grid_for(p->n_nodes * 32), 256, 0, st>>>(p->g->offsets, p->g->dst, p->g->num_nodes, p->nodes, p->n_nodes,
-                                                                   p->keys, p->vals, p->mask, nullptr, p->row_start, edge_src,
-                                                                   edge_dst, src_local, dst_local, edge_ids);
-    if (edge_index_local)
-        k_edge_index_local<<<grid_for(p->n_edges), 256, 0, st>>>(src_local, dst_local, p->n_edges, edge_index_local);
+    const InduceOut o{edge_src, edge_dst, src_local, dst_local, edge_ids, edge_index_local, p->n_edges};
+    k_induce_walk<true><<<p->walk.warps / (kWalkThreads / 32), kWalkThreads, 0, st>>>(p->walk, o);
     AG_CUDA(cudaGetLastError());
     AG_CUDA(cudaStreamSynchronize(st));
     return AG_OK;

@@ -66,3 +66,22 @@ def test_more_slices_than_the_queue_holds():
     for i, sg in enumerate(ag.ParallelBatchSampler(g, cfg, streams=1, group=64).sample_batches(batches)):
         o.reseed(ago.batch_seed(4, i))
         assert_same_subgraph(sg.raw_u32(), o.sample(batches[i]), ctx=f"batch {i}: ")
+
+
+@pytest.mark.parametrize("track", [True, False])
+@pytest.mark.parametrize("degrees,seeds", [(DEGREES, 14), ([700_000], 1), ([0, 0, 0], 3), ([127, 128, 129, 160], 200), ([3] * 50, 0)])
+def test_induced(degrees, seeds, track):
+    import aethergraph_b200 as ag
+    from oracle import ago
+
+    n = 4000
+    off, dst, _ = _hub_graph(degrees, n, 7)
+    g = ag.Graph.from_csr(off, dst)
+    s = ag.NeighborSampler(g, ag.SamplingConfig(num_neighbors=[6, 4], subgraph_type="induced", seed=2, track_edge_ids=track))
+    o = ago.Sampler(off, dst, [6, 4], seed=2, track_edge_ids=track)
+    for ids in (np.arange(seeds), np.arange(seeds)[::-1] * 7 % n):
+        ids = ids.astype(np.uint32)
+        sg, want = s.sample(ids), ago.induce(off, dst, o.sample(ids))
+        assert_same_subgraph(sg.raw_u32(), want)
+        eil = sg.edge_index_local
+        assert np.array_equal(eil[0], want["dst_local"].astype(np.int64)) and np.array_equal(eil[1], want["src_local"].astype(np.int64))
