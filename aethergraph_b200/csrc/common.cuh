@@ -70,6 +70,18 @@ __device__ __forceinline__ uint64_t wyrand_at(uint64_t seed, uint64_t d) {
     return __umul64hi(st, b) ^ (st * b);
 }
 
+// Upper 32 bits of the draw with state `st` (that is, wyrand_at(seed, d) >> 32 for
+// st = seed + (d + 1) * C): four 32 x 32 -> 64 bit products instead of the seven of a high
+// and a low 64-bit product.
+__device__ __forceinline__ uint32_t wyrand_top32(uint64_t st) {
+    const uint64_t b = st ^ 0xe7037ed1a0b428dbull;
+    const uint32_t a0 = (uint32_t)st, a1 = (uint32_t)(st >> 32), b0 = (uint32_t)b, b1 = (uint32_t)(b >> 32);
+    const uint64_t m1 = (uint64_t)a0 * b1 + (((uint64_t)a0 * b0) >> 32);  // no sum here can overflow
+    const uint64_t m2 = (uint64_t)a1 * b0 + (uint32_t)m1;
+    const uint64_t hi = (uint64_t)a1 * b1 + (m1 >> 32) + (m2 >> 32);
+    return (uint32_t)(hi >> 32) ^ (uint32_t)m2;  // low half's upper word: m2 mod 2^32
+}
+
 // Philox4x32-10 (reference: internal/philox.rs:15-40): counter
 // (node_lo, node_hi, layer, draw_group), key (seed_lo, seed_hi).
 __device__ __forceinline__ uint4 philox4x32_10(uint64_t seed, uint32_t layer, uint64_t node,

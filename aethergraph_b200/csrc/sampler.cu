@@ -108,6 +108,7 @@ struct SampleParams {
     HubRow *hub_rows;                // [hub_cap]
     unsigned long long *hub_count;   // rows queued << 32 | slices handed out
     uint32_t *hub_thr, *hub_done;    // [hub_cap] per row: lowest k-th best key so far (float bits), slices finished
+    float *hub_guess;                // [hub_cap] the threshold the row started with
     double *hub_key;                 // [hub_cap][k] the slices' best (key, position) pairs
     uint32_t *hub_pos;
     uint32_t hub_cap, hub_slice;     // slices the arrays hold, positions per slice
@@ -350,15 +351,45 @@ __device__ __forceinline__ void pick_large(const SampleParams &p, uint32_t hop, 
 // emitted in ascending order.  A warp streams 32 positions at a time and keeps the
 // current best k sorted across its lanes.
 
+// Compare-exchange with the lane `stride` away; this lane keeps the smaller pair if `small`.
+__device__ __forceinline__ void warp_exchange(double &key, uint32_t &pos, int stride, bool small) {
+    const double ok = __shfl_xor_sync(0xffffffffu, key, stride);
+    const uint32_t op = __shfl_xor_sync(0xffffffffu, pos, stride);
+    if (key_less(ok, op, key, pos) == small) { key = ok; pos = op; }
+}
+
+// Sorts the warp's 32 (key, position) pairs ascending across the lanes (bitonic).
+__device__ __forceinline__ void warp_sort_pairs(double &key, uint32_t &pos, int lane) {
+#pragma unroll
+    for (int size = 2; size <= 32; size <<= 1) {
+#pragma unroll
+        for (int stride = size >> 1; stride > 0; stride >>= 1)
+            warp_exchange(key, pos, stride, ((lane & size) == 0) == ((lane & stride) == 0));
+    }
+}
+
+constexpr int kInsertFew = 6;  // winners inserted one by one (about 35 instructions each)
+
 // Inserts the chunk's candidates (one per lane, cpos == ~0 for none) that beat the
 // current k-th best into the sorted lanes.
 __device__ __forceinline__ void topk_insert_chunk(double key, uint32_t cpos, double &best_key, uint32_t &best_pos,
                                                   uint32_t k, int lane) {
-    for (;;) {
+    for (bool again = false;; again = true) {
         const double tk = __shfl_sync(0xffffffffu, best_key, k - 1);
         const uint32_t tp = __shfl_sync(0xffffffffu, best_pos, k - 1);
         const uint32_t m = __ballot_sync(0xffffffffu, cpos != 0xFFFFFFFFu && key_less(key, cpos, tk, tp));
         if (!m) break;
+        if (!again && __popc(m) > kInsertFew) {
+            // Many: sort them, keep the smaller of best[i] and candidate[31 - i] (the 32 smallest
+            // of the 64, a bitonic sequence) and sort that: 21 exchange steps.
+            warp_sort_pairs(key, cpos, lane);
+            const double rk = __shfl_sync(0xffffffffu, key, 31 - lane);
+            const uint32_t rp = __shfl_sync(0xffffffffu, cpos, 31 - lane);
+            if (key_less(rk, rp, best_key, best_pos)) { best_key = rk; best_pos = rp; }
+#pragma unroll
+            for (int stride = 16; stride > 0; stride >>= 1) warp_exchange(best_key, best_pos, stride, (lane & stride) == 0);
+            break;
+        }
         const int src = __ffs(m) - 1;
         const double ck = __shfl_sync(0xffffffffu, key, src);
         const uint32_t cp = __shfl_sync(0xffffffffu, cpos, src);
@@ -385,53 +416,47 @@ __device__ __forceinline__ double weighted_key(const SampleParams &p, uint32_t h
     return -log(u) / w;
 }
 
-// Sorts the warp's 32 (key, position) pairs ascending across the lanes (bitonic).
-__device__ __forceinline__ void warp_sort_pairs(double &key, uint32_t &pos, int lane) {
-#pragma unroll
-    for (int size = 2; size <= 32; size <<= 1) {
-#pragma unroll
-        for (int stride = size >> 1; stride > 0; stride >>= 1) {
-            const double ok = __shfl_xor_sync(0xffffffffu, key, stride);
-            const uint32_t op = __shfl_xor_sync(0xffffffffu, pos, stride);
-            const bool want_small = ((lane & size) == 0) == ((lane & stride) == 0);
-            if (key_less(ok, op, key, pos) == want_small) { key = ok; pos = op; }
-        }
-    }
-}
-
 // Streams positions [begin, end) of the row of `fe` into the warp's sorted best k
 // (all sentinels on entry).
 //
 // Almost every position loses against the k-th best key, and the exact key costs an
 // f64 log and divide, so the stream works in two stages.  Stage 1, all lanes, single
-// precision, no log: with uf >= u (u's top 24 bits, rounded up),
+// precision, no log: with uf >= u (u's top 23 bits, rounded up),
 //     -ln(u) >= -ln(uf) >= 2 (1 - uf) / (1 + uf)
 // (the first term of the series of ln, all terms positive), tight where it matters: a
 // winner of a long row has u near 1.  If 2 (1 - uf) exceeds (1 + uf) * thr * w by more
-// than the rounding of the four f32 operations (< 4 * 2^-24 relative, 1e-5 is granted;
-// 1 - uf is exact, and at least 2^-24 unless it is 0 and nothing is dropped), the exact
-// key cannot be below the threshold and the position is dropped.  Survivors are only
-// queued (`buf`, 64 slots of the warp's shared memory).  Stage 2, whenever 32 are queued:
-// every lane evaluates one queued position exactly and the winners are inserted.  The
-// threshold is the k-th best key at the last flush (and, when several warps stream
-// slices of one row, `shared_thr`, the lowest k-th best any of them holds; the bit
-// pattern of a non-negative float orders like the float).  It is always an upper bound
-// of the row's final k-th best key, so stage 1 only ever discards certain losers and the
-// winners — and the output — are exactly those of evaluating every position.
+// than the rounding of the three f32 products (3 * 2^-24 relative, 1e-5 is granted;
+// 1 + uf and 1 - uf are exact), the exact key cannot be below the threshold and the
+// position is dropped.  A weight that is not positive and finite has key +inf, which a
+// finite threshold beats: 0 and negative weights are dropped by the same comparison, NaN
+// and +inf (and a product that overflows) compare false and survive to stage 2.
+// Survivors are only queued (`buf`, 64 slots of the warp's shared memory).  Stage 2,
+// whenever 32 are queued: every lane evaluates one queued position exactly and the
+// winners are inserted.
 //
-// Bound: the 64 x 64 -> 128 bit multiply of the random stream and the weights' latency;
-// hence kChunks weight loads in flight per lane.
+// The threshold is the lowest of `guess`, the k-th best key at the last flush and, when
+// several warps stream slices of one row, `shared_thr`, the lowest k-th best any of them
+// holds (the bit pattern of a non-negative float orders like the float).  Without the
+// guess (+inf) it is always an upper bound of the row's final k-th best key, so stage 1
+// only ever discards certain losers and the output is exactly that of evaluating every
+// position.  With a guess the same holds if the k-th best found is at most the guess;
+// the caller checks that and streams again without one if not.
+//
+// Bound: instructions, about 30 for 32 positions in stage 1 and 500 for a flush, so what
+// counts is the multiply of the random stream (wyrand_top32) and the number of flushes
+// (guess_threshold).  kChunks * 32 positions are loaded and filtered together and only
+// then asked for survivors, with one vote.
 constexpr uint32_t kChunks = 4;
 
-__device__ __forceinline__ void topk_stream(const SampleParams &p, uint32_t hop, const FrontierEntry &fe, uint32_t begin,
-                                            uint32_t end, uint32_t k, int lane, double &best_key, uint32_t &best_pos,
-                                            uint32_t *buf, uint32_t *shared_thr = nullptr) {
-    const double inf = __longlong_as_double(0x7FF0000000000000ll);
+template <bool PHILOX>
+__device__ __forceinline__ void topk_stream_rng(const SampleParams &p, uint32_t hop, const FrontierEntry &fe, uint32_t begin,
+                                                uint32_t end, uint32_t k, int lane, double &best_key, uint32_t &best_pos,
+                                                uint32_t *buf, float guess, uint32_t *shared_thr) {
     uint32_t queued = 0;  // warp-uniform
     bool fresh = true;    // nothing inserted yet
-    float thr = __uint_as_float(0x7F800000u);
+    float thr = guess;
     auto flush = [&](uint32_t count) {  // evaluate buf[0 .. count) exactly, one per lane, and insert the winners
-        double key = inf;
+        double key = __longlong_as_double(0x7FF0000000000000ll);
         uint32_t cpos = 0xFFFFFFFFu;
         if ((uint32_t)lane < count) {
             cpos = buf[lane];
@@ -445,57 +470,102 @@ __device__ __forceinline__ void topk_stream(const SampleParams &p, uint32_t hop,
             topk_insert_chunk(key, cpos, best_key, best_pos, k, lane);
         }
         const double kth = __shfl_sync(0xffffffffu, best_key, k - 1);
-        thr = (float)kth;
+        thr = fminf(thr, (float)kth);
         if (shared_thr) {
             const float up = __double2float_ru(kth);  // rounded up: still an upper bound
             if (lane == 0 && up < 3.0e38f) atomicMin(shared_thr, __float_as_uint(up));
         }
     };
-    const float *w = p.weights + fe.off;
-    for (uint64_t c = begin; c < end; c += 32 * kChunks) {
+    const float *w = p.weights + fe.off + begin + lane;
+    constexpr uint64_t kStep = 0xa0761d6478bd642full;  // from one draw's state to the next (wyrand_at)
+    const uint64_t seed = p.seed;
+    uint32_t first = begin + lane;  // this lane's position in the next chunk
+    uint64_t state = seed + (fe.dbase + first + 1ull) * kStep;
+    for (uint32_t left = end - begin; left > 0;) {
         float t = thr;
         if (shared_thr) t = fminf(t, __uint_as_float(__ldcg(shared_thr)));
+        // NaN: nothing is dropped
+        const float ts = (t >= 1.0e-30f && t <= 3.0e38f) ? t * 1.00001f : __uint_as_float(0x7FC00000u);
         float wf[kChunks];
 #pragma unroll
-        for (uint32_t u = 0; u < kChunks; ++u) {
-            const uint64_t pos = c + u * 32 + lane;
-            wf[u] = pos < end ? __ldg(w + pos) : 0.0f;
-        }
+        for (uint32_t u = 0; u < kChunks; ++u) wf[u] = u * 32 + lane < left ? __ldg(w + u * 32) : 0.0f;
+        bool kept[kChunks], any = false;
 #pragma unroll
         for (uint32_t u = 0; u < kChunks; ++u) {
-            const uint64_t pos64 = c + u * 32 + lane;
-            const uint32_t pos = (uint32_t)pos64;
-            bool keep = pos64 < end;
-            if (t >= 1.0e-30f) {  // in the normal range: no underflow below
-                if (wf[u] > 0.0f && isfinite(wf[u])) {  // thr * w may overflow: nothing is dropped
-                    const uint32_t n = 1u + ((p.rng_mode == AG_RNG_PHILOX) ? philox_u32(p.seed, hop, fe.id, 2 * pos) >> 8
-                                                                            : (uint32_t)(wyrand_at(p.seed, fe.dbase + pos) >> 40));
-                    const float twice_below = (float)(0x1000000u - n) * 1.1920928955078125e-07f;  // 2 (1 - uf), exact
-                    const float above = (float)(0x1000000u + n) * 5.9604644775390625e-08f;         // 1 + uf
-                    if (twice_below > above * (t * wf[u]) * 1.00001f) keep = false;
-                } else if (t <= 3.0e38f) {
-                    keep = false;  // key +inf against a finite k-th best
+            const uint32_t top = PHILOX ? philox_u32(seed, hop, fe.id, 2 * (first + u * 32))
+                                        : wyrand_top32(state + u * 32 * kStep);
+            const float above = __uint_as_float(0x3F800000u | (top >> 9)) + 1.1920928955078125e-07f;  // 1 + uf
+            const float below = 2.0f - above;                                                           // 1 - uf
+            kept[u] = u * 32 + lane < left && !(2.0f * below > above * (ts * wf[u]));
+            any = any || kept[u];
+        }
+        if (__any_sync(0xffffffffu, any)) {
+#pragma unroll
+            for (uint32_t u = 0; u < kChunks; ++u) {
+                const uint32_t m = __ballot_sync(0xffffffffu, kept[u]);
+                if (!m) continue;
+                if (kept[u]) buf[queued + __popc(m & ((1u << lane) - 1u))] = first + u * 32;
+                queued += __popc(m);
+                __syncwarp();
+                if (queued >= 32) {
+                    flush(32);
+                    __syncwarp();
+                    const uint32_t rest = queued - 32;  // < 32: move the tail to the front
+                    const uint32_t moved = (uint32_t)lane < rest ? buf[32 + lane] : 0;
+                    __syncwarp();
+                    if ((uint32_t)lane < rest) buf[lane] = moved;
+                    queued = rest;
+                    __syncwarp();
                 }
             }
-            const uint32_t m = __ballot_sync(0xffffffffu, keep);
-            if (!m) continue;
-            if (keep) buf[queued + __popc(m & ((1u << lane) - 1u))] = pos;
-            queued += __popc(m);
-            __syncwarp();
-            if (queued >= 32) {
-                flush(32);
-                __syncwarp();
-                const uint32_t rest = queued - 32;  // < 32: move the tail to the front
-                const uint32_t moved = (uint32_t)lane < rest ? buf[32 + lane] : 0;
-                __syncwarp();
-                if ((uint32_t)lane < rest) buf[lane] = moved;
-                queued = rest;
-                __syncwarp();
-            }
         }
+        w += 32 * kChunks;
+        first += 32 * kChunks;
+        state += 32 * kChunks * kStep;
+        left -= min(left, 32 * kChunks);
     }
     if (queued) { flush(queued); __syncwarp(); }
 }
+
+__device__ __forceinline__ void topk_stream(const SampleParams &p, uint32_t hop, const FrontierEntry &fe, uint32_t begin,
+                                            uint32_t end, uint32_t k, int lane, double &best_key, uint32_t &best_pos,
+                                            uint32_t *buf, float guess, uint32_t *shared_thr = nullptr) {
+    best_key = __longlong_as_double(0x7FF0000000000000ll);
+    best_pos = 0xFFFFFFFFu;  // sentinel: sorts after every real (key, position)
+    if (p.rng_mode == AG_RNG_PHILOX) topk_stream_rng<true>(p, hop, fe, begin, end, k, lane, best_key, best_pos, buf, guess, shared_thr);
+    else topk_stream_rng<false>(p, hop, fe, begin, end, k, lane, best_key, best_pos, buf, guess, shared_thr);
+}
+
+// A threshold that about `want` of a row's `n` keys should fall below, given its positive
+// weights' mean: keys are exponential with rate w, so n (1 - exp(-t mean)) = want for equal
+// weights.  A hint only (see topk_stream): without one the threshold starts at +inf and
+// comes down flush by flush, four or five of them in a row of 500.
+__device__ __forceinline__ float guess_threshold(float mean, float n, float want) {
+    const float t = -__logf(1.0f - want / n) / mean;
+    return (want < 0.75f * n && t > 1.0e-30f && t < 3.0e38f) ? t : __uint_as_float(0x7F800000u);
+}
+
+// Sum of `count` weights of a row, `step` apart, that are positive and finite (warp-wide).
+__device__ __forceinline__ float weight_sum(const float *w, uint32_t count, uint64_t step, int lane) {
+    float sum = 0.0f;
+    for (uint32_t c = 0; c < count; c += 32 * kChunks) {
+        float v[kChunks];
+#pragma unroll
+        for (uint32_t u = 0; u < kChunks; ++u) {
+            const uint32_t i = c + u * 32 + lane;
+            v[u] = i < count ? __ldg(w + i * step) : 0.0f;
+        }
+#pragma unroll
+        for (uint32_t u = 0; u < kChunks; ++u) sum += (v[u] > 0.0f && v[u] < 3.0e38f) ? v[u] : 0.0f;
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+    return sum;
+}
+
+// Warps per block of the weighted picks: few, so that a block's slots are free again as
+// soon as its own rows are done (rows of a hop differ by a factor of 2000).
+constexpr int kWeightedThreads = 64;
 
 // Rows longer than kHubDegree are split into slices, a warp each, by k_pick_hub_slices;
 // a warp alone takes about 1 us per 1000 positions, so the rows left to one warp end
@@ -503,6 +573,8 @@ __device__ __forceinline__ void topk_stream(const SampleParams &p, uint32_t hop,
 constexpr uint32_t kHubDegree = 2048;
 constexpr uint32_t kMaxHubSlices = 65536;   // slices a chain's queue holds; a row that does not fit stays with its warp
 constexpr uint32_t kMaxSlicesPerRow = 256;  // the merge of a row is one warp's work
+constexpr uint32_t kGuessDegree = 128;      // rows from here on get a threshold to start with
+constexpr uint32_t kSampledWeights = 512;   // weights, evenly spaced, that a row's mean is taken from
 
 __device__ __forceinline__ uint32_t hub_slice_len(uint32_t deg, uint32_t slice) {
     return max(slice, (deg / kMaxSlicesPerRow + 32u) & ~31u);
@@ -512,8 +584,7 @@ __device__ __forceinline__ void pick_weighted(const SampleParams &p, uint32_t ho
                                               const FrontierEntry *fes, uint32_t n, uint32_t *queue) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (k == 0) return;
-    const double inf = __longlong_as_double(0x7FF0000000000000ll);
-    for (uint32_t j = blockIdx.x * (kPickThreads / 32) + warp; j < n; j += gridDim.x * (kPickThreads / 32)) {
+    for (uint32_t j = blockIdx.x * (kWeightedThreads / 32) + warp; j < n; j += gridDim.x * (kWeightedThreads / 32)) {
         const FrontierEntry fe = fes[j];
         const uint32_t deg = fe.deg;
         if (deg == 0) continue;
@@ -522,6 +593,9 @@ __device__ __forceinline__ void pick_weighted(const SampleParams &p, uint32_t ho
             continue;
         }
         if (deg > kHubDegree) {  // queue the row for the slice kernel
+            // Many more than k: one wrong guess costs the whole row again, by one warp.
+            const float guess = guess_threshold(weight_sum(p.weights + fe.off, kSampledWeights, deg / kSampledWeights, lane) / kSampledWeights,
+                                                (float)deg, 4.0f * (float)k + 64.0f);
             bool queued = false;
             if (lane == 0) {
                 const uint32_t len = hub_slice_len(deg, p.hub_slice), slices = (deg - 1) / len + 1;
@@ -531,15 +605,26 @@ __device__ __forceinline__ void pick_weighted(const SampleParams &p, uint32_t ho
                 queued = (uint64_t)base + slices <= p.hub_cap;
                 if (h < p.hub_cap) {
                     p.hub_rows[h] = HubRow{blockIdx.y, j, base, queued ? slices : 0u};
-                    p.hub_thr[h] = 0x7F800000u;  // +inf
+                    p.hub_guess[h] = guess;
+                    p.hub_thr[h] = __float_as_uint(guess);
                     p.hub_done[h] = 0;
                 }
             }
             if (__shfl_sync(0xffffffffu, queued, 0)) continue;
         }
-        double best_key = inf;
-        uint32_t best_pos = 0xFFFFFFFFu;  // sentinel: sorts after every real (key, position)
-        topk_stream(p, hop, fe, 0, deg, k, lane, best_key, best_pos, queue + warp * 64);
+        const float inff = __uint_as_float(0x7F800000u);
+        float guess = inff;
+        if (deg >= kGuessDegree) {
+            // enough to be right nineteen times in twenty or better, few enough for one flush
+            const float want = (float)k + 2.0f * sqrtf((float)k) + 2.0f;
+            guess = guess_threshold(weight_sum(p.weights + fe.off, min(deg, kSampledWeights), deg > kSampledWeights ? deg / kSampledWeights : 1, lane) /
+                                        (float)min(deg, kSampledWeights), (float)deg, want);
+        }
+        double best_key;
+        uint32_t best_pos;
+        topk_stream(p, hop, fe, 0, deg, k, lane, best_key, best_pos, queue + warp * 64, guess);
+        if (!(__shfl_sync(0xffffffffu, best_key, k - 1) <= (double)guess))
+            topk_stream(p, hop, fe, 0, deg, k, lane, best_key, best_pos, queue + warp * 64, inff);
         if ((uint32_t)lane < k) emit_edge(p, hop, edges_before, fe, lane, fe.off + best_pos);
     }
 }
@@ -948,10 +1033,10 @@ k_assign_seeds(StagedChain chain, uint32_t k) {
 // size and where the hop's edges start).  The lanes of the whole grid share the
 // frontier, so even a hop with few vertices spreads over the GPU.
 template <int G, int PICK>
-__global__ void __launch_bounds__(PICK == kPickLarge ? 128 : kPickThreads)
+__global__ void __launch_bounds__(PICK == kPickLarge ? 128 : PICK == kPickWeighted ? kWeightedThreads : kPickThreads)
 k_pick(const SampleParams *__restrict__ pa, uint32_t hop, uint32_t k) {
     __shared__ uint32_t s_picks[PICK == kPickLarge ? 4 : 1][PICK == kPickLarge ? kLargeK : 1];
-    __shared__ uint32_t s_queue[PICK == kPickWeighted ? (kPickThreads / 32) * 64 : 1];  // weighted: 64 queued positions per warp
+    __shared__ uint32_t s_queue[PICK == kPickWeighted ? (kWeightedThreads / 32) * 64 : 1];  // weighted: 64 queued positions per warp
     chain_sync();
     const SampleParams &p = pa[blockIdx.y];
     const StageInfo nx = p.state->stage[hop + 1];
@@ -967,17 +1052,18 @@ k_pick(const SampleParams *__restrict__ pa, uint32_t hop, uint32_t k) {
 //
 // A row of 500 K positions on one block of 512 threads took 450 us, as long for one batch
 // as for eight.  Twelve batches of 512 seeds, fanouts 15, 10, 5, on the 10 M vertex / 200 M
-// edge graph (28 M positions a batch): 5320 us with a block per row, 3600 us with slices.
-__global__ void __launch_bounds__(kPickThreads)
+// edge graph (28 M positions a batch): 5320 us with a block per row, 3600 us with slices,
+// 2730 us with the shorter filter and the first threshold guessed.
+__global__ void __launch_bounds__(kWeightedThreads)
 k_pick_hub_slices(const SampleParams *__restrict__ pa, uint32_t hop, uint32_t k) {
-    __shared__ uint32_t s_queue[(kPickThreads / 32) * 64];
+    __shared__ uint32_t s_queue[(kWeightedThreads / 32) * 64];
     chain_sync();
     const SampleParams &q = pa[0];  // the queue is the same for every batch
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const double inf = __longlong_as_double(0x7FF0000000000000ll);
     const unsigned long long count = *q.hub_count;
     const uint32_t rows = min((uint32_t)(count >> 32), q.hub_cap), slices = min((uint32_t)count, q.hub_cap);
-    for (uint32_t slice = blockIdx.x * (kPickThreads / 32) + warp; slice < slices; slice += gridDim.x * (kPickThreads / 32)) {
+    for (uint32_t slice = blockIdx.x * (kWeightedThreads / 32) + warp; slice < slices; slice += gridDim.x * (kWeightedThreads / 32)) {
         // the last row whose slices start at or before this one; 32 probes a step
         uint32_t lo = 0, n = rows;
         while (n > 1) {
@@ -994,9 +1080,10 @@ k_pick_hub_slices(const SampleParams *__restrict__ pa, uint32_t hop, uint32_t k)
         const uint32_t deg = fe.deg, len = hub_slice_len(deg, q.hub_slice);
         const uint64_t first = (uint64_t)(slice - row.slice_base) * len;
         const uint32_t begin = (uint32_t)min((uint64_t)deg, first), end = (uint32_t)min((uint64_t)deg, first + len);
-        double best_key = inf;
-        uint32_t best_pos = 0xFFFFFFFFu;
-        topk_stream(p, hop, fe, begin, end, k, lane, best_key, best_pos, s_queue + warp * 64, q.hub_thr + lo);
+        const float guess = q.hub_guess[lo];
+        double best_key;
+        uint32_t best_pos;
+        topk_stream(p, hop, fe, begin, end, k, lane, best_key, best_pos, s_queue + warp * 64, guess, q.hub_thr + lo);
         if (row.n_slices > 1) {
             const uint64_t mine = (uint64_t)slice * k;
             if ((uint32_t)lane < k) { q.hub_key[mine + lane] = best_key; q.hub_pos[mine + lane] = best_pos; }
@@ -1017,6 +1104,8 @@ k_pick_hub_slices(const SampleParams *__restrict__ pa, uint32_t hop, uint32_t k)
                 topk_insert_chunk(ck, cp, best_key, best_pos, k, lane);
             }
         }
+        if (!(__shfl_sync(0xffffffffu, best_key, k - 1) <= (double)guess))
+            topk_stream(p, hop, fe, 0, deg, k, lane, best_key, best_pos, s_queue + warp * 64, __uint_as_float(0x7F800000u));
         if ((uint32_t)lane < k) emit_edge(p, hop, p.state->stage[hop + 1].n_edges, fe, lane, fe.off + best_pos);
     }
 }
@@ -1076,9 +1165,11 @@ void launch_pick(int mode, uint32_t k, uint64_t frontier_est, uint32_t n_batches
     } else if (mode == kModeWeighted && k > 32) {
         launch_chained(k_pick_weighted_large, dim3(blocks_for(frontier_est, 1), n_batches), dim3(kWLThreads), st, pa, hop, k);
     } else if (mode == kModeWeighted) {
-        launch_chained(k_pick<32, kPickWeighted>, dim3(blocks_for(frontier_est, kPickThreads / 32), n_batches), dim3(kPickThreads), st, pa, hop, k);
+        const uint64_t blocks = std::min<uint64_t>((frontier_est + kWeightedThreads / 32 - 1) / (kWeightedThreads / 32),
+                                                   std::max<uint64_t>(1, (uint64_t)kSMs * 128 / n_batches));
+        launch_chained(k_pick<32, kPickWeighted>, dim3((uint32_t)std::max<uint64_t>(1, blocks), n_batches), dim3(kWeightedThreads), st, pa, hop, k);
         // rows longer than kHubDegree were only queued: a warp per slice of them
-        launch_chained(k_pick_hub_slices, dim3((uint32_t)kSMs * 4), dim3(kPickThreads), st, pa, hop, k);
+        launch_chained(k_pick_hub_slices, dim3((uint32_t)kSMs * 16), dim3(kWeightedThreads), st, pa, hop, k);
     } else if (k > 32) {
         launch_chained(k_pick<32, kPickLarge>, dim3(blocks_for(frontier_est, 4), n_batches), dim3(128), st, pa, hop, k);
     } else {
@@ -1124,6 +1215,7 @@ struct ag_sampler {
     HubRow *hub_rows = nullptr;
     unsigned long long *hub_count = nullptr;
     uint32_t *hub_thr = nullptr, *hub_done = nullptr, *hub_pos = nullptr;
+    float *hub_guess = nullptr;
     double *hub_key = nullptr;
     uint32_t hub_cap = 0;
     TileDesc *tiles = nullptr;
@@ -1239,13 +1331,14 @@ int32_t ensure_scratch(ag_sampler *s, uint64_t n_seeds) {
         s->hub_cap = (uint32_t)std::min<uint64_t>(std::max<uint64_t>(most, 1), kMaxHubSlices);
         const uint64_t cap = s->hub_cap;
         uint8_t *base = nullptr;
-        AG_CUDA(cudaMalloc(&base, cap * (sizeof(HubRow) + 8 * hop_k + 4 * hop_k + 8) + 8));
+        AG_CUDA(cudaMalloc(&base, cap * (sizeof(HubRow) + 8 * hop_k + 4 * hop_k + 12) + 8));
         s->hub_rows = (HubRow *)base;
         s->hub_key = (double *)(base + cap * sizeof(HubRow));
         s->hub_count = (unsigned long long *)(s->hub_key + cap * hop_k);
         s->hub_pos = (uint32_t *)(s->hub_count + 1);
         s->hub_thr = s->hub_pos + cap * hop_k;
         s->hub_done = s->hub_thr + cap;
+        s->hub_guess = (float *)(s->hub_done + cap);
     }
     s->n_tiles = std::max<uint64_t>(std::max(cap, s->max_hop_edges) / kTile + 2, 2);
     AG_CUDA(cudaMalloc(&s->tiles, G * s->n_tiles * sizeof(TileDesc)));
@@ -1550,7 +1643,7 @@ int32_t launch_saved_impl(ag_sampler *s, bool relaunch) {
         p.frontier = s->frontier + (uint64_t)b * s->max_frontier;
         p.frontier_cap = s->max_frontier;
         if (s->hub_rows) {
-            p.hub_rows = s->hub_rows; p.hub_count = s->hub_count; p.hub_thr = s->hub_thr; p.hub_done = s->hub_done;
+            p.hub_rows = s->hub_rows; p.hub_count = s->hub_count; p.hub_thr = s->hub_thr; p.hub_done = s->hub_done; p.hub_guess = s->hub_guess;
             p.hub_key = s->hub_key; p.hub_pos = s->hub_pos; p.hub_cap = s->hub_cap;
             // about as many slices whatever the chain's length: a slice of kHubDegree positions per batch
             p.hub_slice = (uint32_t)std::min<uint64_t>(kHubDegree * next_pow2(n_batches), 16 * kHubDegree);
