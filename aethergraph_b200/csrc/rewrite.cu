@@ -181,11 +181,19 @@ namespace {
 // Rows differ by five orders of magnitude (a hub of an R-MAT graph of 64 M edges has
 // over 100 K neighbours, most vertices a few), so a warp per row left the two walks to
 // the warp with the longest one: 200 seeds, fanouts 10, 5 on that graph reach 3200 nodes
-// and 5.7 M positions, 2660 + 3080 us at 4 % of the warps busy.
+// and 5.7 M positions, 2660 + 3080 us at 4 % of the warps busy.  Now 55 + 48 us (107 + 84
+// before the filter and the shuffled row search below), bound by warps in short rows.
 constexpr int kWalkThreads = 256;
 constexpr uint32_t kWalkWarpsPerSM = 32;
 constexpr uint32_t kWalkMin = 128;   // positions a warp takes at least
 constexpr uint32_t kWalkUnroll = 4;  // 32-position chunks in flight in a long row
+// Most neighbours are not in the sample, and a probe of the node table is 32 scattered
+// reads for a warp.  A bitmap of the nodes' hashes in shared memory answers for most of
+// them: kFilterMin - kFilterMax words a block, 16 bits or more per node where that fits
+// (up to 1 / 16 of the misses pass), built by every block from the node list; none above
+// kFilterNodes nodes, where it would be over a quarter full and slow to build.
+constexpr uint32_t kFilterMin = 1024, kFilterMax = 16384;
+constexpr uint64_t kFilterNodes = 1 << 17;
 
 __device__ __forceinline__ uint32_t node_slot(uint32_t v, uint32_t mask) { return (uint32_t)(mix64(v) & mask); }
 
@@ -229,6 +237,7 @@ struct InduceWalk {
     const uint64_t *row_start;  // [n + 1] its first position in the list
     const unsigned long long *table;
     uint32_t mask, warps;
+    uint32_t filter_words;      // a power of two, or 0: no filter
     uint64_t *warp_start;       // [warps] hits, then (scanned) hits before the warp's stretch
     uint64_t *total;            // [0] all hits, [1] blocks that have counted
 };
@@ -250,9 +259,26 @@ __device__ __forceinline__ uint64_t row_of(const uint64_t *__restrict__ row_star
     return lo;
 }
 
+// A node's bit in the filter: another hash than the table's.
+__device__ __forceinline__ uint32_t filter_bit(uint32_t v, uint32_t words) { return (v * 0x9E3779B1u) >> (32 - 5 - (31 - __clz(words))); }
+
+// Both walks.  In a long row the warp reads kWalkUnroll chunks of it at once.  Elsewhere the
+// 32 positions lie in several rows: the lanes hold the ends of the next 32 rows and every
+// lane finds its row among them by shuffles (a search through memory per lane took 4 us for
+// 32 positions); only a run of 32 empty rows falls back to the search.
 template <bool FILL>
 __global__ void __launch_bounds__(kWalkThreads)
 k_induce_walk(InduceWalk a, InduceOut o) {
+    extern __shared__ uint32_t s_filter[];
+    if (a.filter_words) {
+        for (uint32_t i = threadIdx.x; i < a.filter_words; i += kWalkThreads) s_filter[i] = 0;
+        __syncthreads();
+        for (uint64_t i = threadIdx.x; i < a.n; i += kWalkThreads) {
+            const uint32_t bit = filter_bit(__ldg(a.nodes + i), a.filter_words);
+            atomicOr(&s_filter[bit >> 5], 1u << (bit & 31));
+        }
+        __syncthreads();
+    }
     const uint32_t lane = threadIdx.x & 31, w = (blockIdx.x * kWalkThreads + threadIdx.x) >> 5;
     const uint64_t all = a.row_start[a.n];
     const uint64_t share = ((all + a.warps - 1) / a.warps + 31) & ~31ull;
@@ -276,36 +302,50 @@ k_induce_walk(InduceWalk a, InduceOut o) {
             count += __popc(m);
         }
     };
-    uint64_t row = 0;
+    auto find = [&](uint32_t v) {
+        if (!a.filter_words) return node_lookup(a.table, a.mask, v);
+        const uint32_t bit = filter_bit(v, a.filter_words);
+        return ((s_filter[bit >> 5] >> (bit & 31)) & 1u) ? node_lookup(a.table, a.mask, v) : 0xFFFFFFFFu;
+    };
+    uint64_t row = g < stop ? row_of(a.row_start, a.n, 0, g) : 0;  // row_start[row] <= g
     while (g < stop) {
-        row = row_of(a.row_start, a.n, row, g);
-        const uint64_t begin = __ldg(a.row_start + row), end = min(stop, __ldg(a.row_start + row + 1));
+        const uint64_t row_end = __ldg(a.row_start + min(row + 1 + lane, a.n));  // of row + lane
+        const uint32_t skip = __popc(__ballot_sync(0xFFFFFFFFu, row_end <= g));   // rows that end at or before g
+        if (skip == 32) { row = row_of(a.row_start, a.n, row, g); continue; }
+        const uint64_t end = min(stop, __shfl_sync(0xFFFFFFFFu, row_end, skip));
         if (end - g >= 32 * kWalkUnroll) {  // a long row: whole chunks of it
-            const uint64_t base = __ldg(a.row_off + row) - begin;  // list position -> CSR position
+            row += skip;
+            const uint64_t base = __ldg(a.row_off + row) - __ldg(a.row_start + row);  // list position -> CSR position
             const uint32_t node = FILL ? __ldg(a.nodes + row) : 0;
             for (; end - g >= 32 * kWalkUnroll; g += 32 * kWalkUnroll) {
                 uint32_t v[kWalkUnroll], hit[kWalkUnroll];
 #pragma unroll
                 for (uint32_t u = 0; u < kWalkUnroll; ++u) v[u] = ld_stream_u32(a.dst + base + g + u * 32 + lane);
 #pragma unroll
-                for (uint32_t u = 0; u < kWalkUnroll; ++u) hit[u] = node_lookup(a.table, a.mask, v[u]);
+                for (uint32_t u = 0; u < kWalkUnroll; ++u) hit[u] = find(v[u]);
 #pragma unroll
                 for (uint32_t u = 0; u < kWalkUnroll; ++u) take(hit[u], v[u], base + g + u * 32 + lane, (uint32_t)row, node);
             }
-        } else {  // 32 positions of whatever rows they lie in
-            const uint64_t mine = g + lane;
-            uint64_t r = row, pos = 0;
-            uint32_t v = 0, hit = 0xFFFFFFFFu;
-            if (mine < stop) {
-                r = row_of(a.row_start, a.n, row, mine);
-                pos = __ldg(a.row_off + r) + (mine - __ldg(a.row_start + r));
-                v = ld_stream_u32(a.dst + pos);
-                hit = node_lookup(a.table, a.mask, v);
-            }
-            const uint32_t node = (FILL && hit != 0xFFFFFFFFu) ? __ldg(a.nodes + r) : 0;
-            take(hit, v, pos, (uint32_t)r, node);
-            g += 32;
+            continue;
         }
+        const uint64_t mine = g + lane;
+        uint32_t r = 0;  // rows of the window that end at or before this lane's position
+#pragma unroll
+        for (uint32_t step = 16; step > 0; step >>= 1)
+            if (__shfl_sync(0xFFFFFFFFu, row_end, r + step - 1) <= mine) r += step;
+        const bool past = __shfl_sync(0xFFFFFFFFu, row_end, 31) <= mine;  // the window ends before it
+        uint64_t at = row + r, pos = 0;
+        uint32_t v = 0, hit = 0xFFFFFFFFu, node = 0;
+        if (mine < stop) {
+            if (past) at = row_of(a.row_start, a.n, row, mine);
+            pos = __ldg(a.row_off + at) + (mine - __ldg(a.row_start + at));
+            if (FILL) node = __ldg(a.nodes + at);
+            v = ld_stream_u32(a.dst + pos);
+            hit = find(v);
+        }
+        take(hit, v, pos, (uint32_t)at, node);
+        g += 32;
+        row = __shfl_sync(0xFFFFFFFFu, at, 31);  // at most the row of the next position
     }
     if (FILL) return;
     if (lane == 0) a.warp_start[w] = count;
@@ -389,8 +429,12 @@ extern "C" int32_t ag_subgraph_induce_plan(const ag_graph *g, const uint32_t *no
     k_induce_insert<<<grid_for(n_nodes), 256, 0, st>>>(g->offsets, g->num_nodes, g->num_edges, nodes_dev, n_nodes, table,
                                                        (uint32_t)(cap - 1), row_off, row_len, (uint32_t *)(total + 2));
     AG_PLAN_CUDA(cub::DeviceScan::ExclusiveSum((uint8_t *)p->scratch + temp_at, temp_bytes, row_len, row_start, (int)(n_nodes + 1), st));
-    p->walk = InduceWalk{g->dst, nodes_dev, n_nodes, row_off, row_start, table, (uint32_t)(cap - 1), warps, warp_start, total};
-    k_induce_walk<false><<<warps / (kWalkThreads / 32), kWalkThreads, 0, st>>>(p->walk, InduceOut{});
+    // cap >= 2 n: 16 bits or more per node
+    const uint32_t filter = n_nodes > kFilterNodes ? 0 : (uint32_t)std::min<uint64_t>(std::max<uint64_t>(cap / 4, kFilterMin), kFilterMax);
+    AG_PLAN_CUDA(cudaFuncSetAttribute(k_induce_walk<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kFilterMax * 4));
+    AG_PLAN_CUDA(cudaFuncSetAttribute(k_induce_walk<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kFilterMax * 4));
+    p->walk = InduceWalk{g->dst, nodes_dev, n_nodes, row_off, row_start, table, (uint32_t)(cap - 1), warps, filter, warp_start, total};
+    k_induce_walk<false><<<warps / (kWalkThreads / 32), kWalkThreads, filter * 4, st>>>(p->walk, InduceOut{});
     AG_PLAN_CUDA(cudaGetLastError());
     uint64_t got[3] = {0, 0, 0};
     AG_PLAN_CUDA(cudaMemcpyAsync(got, total, 24, cudaMemcpyDeviceToHost, st));
@@ -417,7 +461,7 @@ extern "C" int32_t ag_subgraph_induce_fill(ag_induce_plan *p, uint64_t cap_edges
     if (!guard.ok) return AG_ERR_CUDA;
     cudaStream_t st = (cudaStream_t)stream;
     const InduceOut o{edge_src, edge_dst, src_local, dst_local, edge_ids, edge_index_local, p->n_edges};
-    k_induce_walk<true><<<p->walk.warps / (kWalkThreads / 32), kWalkThreads, 0, st>>>(p->walk, o);
+    k_induce_walk<true><<<p->walk.warps / (kWalkThreads / 32), kWalkThreads, p->walk.filter_words * 4, st>>>(p->walk, o);
     AG_CUDA(cudaGetLastError());
     AG_CUDA(cudaStreamSynchronize(st));
     return AG_OK;
