@@ -20,6 +20,7 @@
 #include <mutex>
 
 #include <cub/device/device_radix_sort.cuh>
+#include <cuda_fp16.h>
 
 #include "common.cuh"
 #include "internal.h"
@@ -31,22 +32,12 @@ namespace {
 constexpr int kThreads = 256;
 constexpr int kInFlight = 4;
 
-__device__ __forceinline__ float bf16lo(uint32_t w) { return __uint_as_float(w << 16); }
-
 // IEEE binary16 -> binary32, exact; a NaN keeps its payload and comes out quiet
-// (what the reference's half / F16C converters produce).
+// (what the reference's half / F16C converters produce; the conversion instruction makes
+// every NaN the same one).
 __device__ __forceinline__ float f16_to_f32_bits(uint32_t h) {
-    const uint32_t sign = (h & 0x8000u) << 16;
-    const uint32_t exp = (h >> 10) & 0x1Fu;
-    uint32_t man = h & 0x3FFu;
-    if (exp == 0x1Fu) return __uint_as_float(man ? (sign | 0x7FC00000u | (man << 13)) : (sign | 0x7F800000u));
-    if (exp == 0) {
-        if (man == 0) return __uint_as_float(sign);
-        const int shift = __clz(man) - 21;  // bring the top set bit to bit 10
-        man = (man << shift) & 0x3FFu;
-        return __uint_as_float(sign | ((uint32_t)(113 - shift) << 23) | (man << 13));
-    }
-    return __uint_as_float(sign | ((exp + 112u) << 23) | (man << 13));
+    if ((h & 0x7FFFu) > 0x7C00u) return __uint_as_float(((h & 0x8000u) << 16) | 0x7FC00000u | ((h & 0x3FFu) << 13));
+    return __half2float(__ushort_as_half((unsigned short)h));
 }
 
 template <int DTYPE>
@@ -384,40 +375,164 @@ __global__ void k_encode_i8(const float *__restrict__ src, uint64_t rows, uint64
     }
 }
 
-// Element path for rows that are not a whole number of 16-byte vectors.
-template <int DTYPE>
+// Rows that are not a whole number of 16-byte vectors (or not 16-byte aligned): a row is
+// split into units of UNIT elements, the largest power of two up to four that divides the
+// row's length and that the bases' alignment allows, so that a unit is one aligned load of
+// UNIT * element bytes and one aligned store of UNIT floats.  A group of 2^lpr_log2 lanes
+// owns a row and walks its units; consecutive lanes touch consecutive bytes, and
+// kUnitRows x kUnitCols units are in flight per lane before any of them is stored.
+//
+// A thread per element (a 64-bit division, an id and a 2-byte load for every float) took
+// 127 us for 200 003 rows of 100 f16 (1.0 TB/s), bound by the instructions of the division
+// and of the decode; now 39 us.  100 M values: dim 301 bf16 625 -> 224 us, dim 50 f32 635 ->
+// 248 us, dim 33 int8 619 -> 275 us, dim 602 f16 643 -> 172 us; dim 1 f32 (20 M) 196 -> 141 us.
+constexpr int kUnitRows = 4, kUnitCols = 2;
+
+template <int BYTES> struct UnitWord;
+template <> struct UnitWord<1> { using T = uint8_t; };
+template <> struct UnitWord<2> { using T = uint16_t; };
+template <> struct UnitWord<4> { using T = uint32_t; };
+template <> struct UnitWord<8> { using T = uint2; };
+
+// STREAM: this GPU's own memory, read once; otherwise a plain load (peers' memory).
+template <int BYTES, bool STREAM>
+__device__ __forceinline__ typename UnitWord<BYTES>::T load_unit(const uint8_t *p) {
+    if constexpr (STREAM && BYTES == 8) return ld_stream_v2(p);
+    else if constexpr (STREAM && BYTES == 4) return ld_stream_u32(p);
+    else if constexpr (STREAM && BYTES == 2) return ld_stream_u16(p);
+    else if constexpr (STREAM) return __ldg(p);
+    else if constexpr (BYTES == 8) {
+        const unsigned long long v = *(const volatile unsigned long long *)p;
+        return make_uint2((uint32_t)v, (uint32_t)(v >> 32));
+    } else return *(const volatile typename UnitWord<BYTES>::T *)p;
+}
+
+__device__ __forceinline__ uint32_t unit_word(uint32_t w, int) { return w; }
+__device__ __forceinline__ uint32_t unit_word(uint2 w, int i) { return i ? w.y : w.x; }
+
+// Element e of a unit, as the bits of its f32 value.
+template <int DTYPE, typename W>
+__device__ __forceinline__ uint32_t unit_decode(W w, int e, float scale) {
+    if (DTYPE == AG_F32) return unit_word(w, e);
+    if (DTYPE == AG_I8) return __float_as_uint((float)(int)(signed char)(unit_word(w, 0) >> (8 * e)) * scale);
+    const uint32_t h = (unit_word(w, e >> 1) >> (16 * (e & 1))) & 0xFFFFu;
+    return DTYPE == AG_BF16 ? h << 16 : __float_as_uint(f16_to_f32_bits(h));
+}
+
+template <int DTYPE, int UNIT, bool SHARDED>
 __global__ void __launch_bounds__(kThreads)
-k_gather_elem(GatherArgs a, const GatherArgs *__restrict__ group) {
+k_gather_units(GatherArgs a, const GatherArgs *__restrict__ group, uint32_t lpr_log2) {
+    constexpr int kElem = DTYPE == AG_F32 ? 4 : DTYPE == AG_I8 ? 1 : 2, kBytes = kElem * UNIT;
+    using W = typename UnitWord<kBytes>::T;
     if (group) a = group[blockIdx.y];
     if (!a.payload) return;
     const uint64_t n = a.n_dev ? min((uint64_t)*a.n_dev, a.n) : a.n;
     if (a.ids_off) a.ids = (const uint32_t *)a.ids + *a.ids_off;
-    const uint64_t total = n * a.dim;
-    for (uint64_t g = (uint64_t)blockIdx.x * kThreads + threadIdx.x; g < total;
-         g += (uint64_t)gridDim.x * kThreads) {
-        const uint64_t r = g / a.dim;
-        const uint32_t j = (uint32_t)(g - r * a.dim);
-        const uint64_t id = load_id(a.ids, a.ids64, r);
-        const uint64_t local = id - a.row_begin;
-        float f = 0.f;
-        if (id >= a.row_begin && local < a.rows) {
-            if (a.shards) {  // sharded store: plain loads from the owner's memory
-                const uint8_t *row = shard_row(a.shards, id, a.row_bytes);
-                if (DTYPE == AG_F32) f = __uint_as_float(*(const volatile uint32_t *)(row + 4ull * j));
-                else if (DTYPE == AG_BF16) f = bf16lo(*(const volatile uint16_t *)(row + 2ull * j));
-                else f = f16_to_f32_bits(*(const volatile uint16_t *)(row + 2ull * j));
-            } else {
-                const uint8_t *row = a.payload + local * a.row_bytes;
-                if (DTYPE == AG_F32) f = __uint_as_float(ld_stream_u32(row + 4ull * j));
-                else if (DTYPE == AG_BF16) f = bf16lo(ld_stream_u16(row + 2ull * j));
-                else if (DTYPE == AG_I8) f = (float)(int)(signed char)row[j] *
-                                             a.scales[local * ((a.dim + kQuantBlock - 1) / kQuantBlock) + j / kQuantBlock];
-                else f = f16_to_f32_bits(ld_stream_u16(row + 2ull * j));
+    const uint32_t lpr = 1u << lpr_log2, lane = threadIdx.x & (lpr - 1), sub = threadIdx.x >> lpr_log2;
+    const uint32_t rows_per_wave = kThreads >> lpr_log2, units = a.dim / UNIT;
+    const uint32_t blocks_per_row = (a.dim + kQuantBlock - 1) / kQuantBlock;
+    const uint64_t chunk = (uint64_t)rows_per_wave * kUnitRows;
+    for (uint64_t base = blockIdx.x * chunk + sub; base < n; base += gridDim.x * chunk) {
+        const uint8_t *row[kUnitRows];
+        const float *scales[kUnitRows];
+#pragma unroll
+        for (int u = 0; u < kUnitRows; ++u) {
+            const uint64_t r = base + (uint64_t)u * rows_per_wave;
+            row[u] = nullptr; scales[u] = nullptr;
+            if (r < n) {
+                const uint64_t id = load_id(a.ids, a.ids64, r), local = id - a.row_begin;
+                if (id >= a.row_begin && local < a.rows) {
+                    row[u] = SHARDED ? shard_row(a.shards, id, a.row_bytes) : a.payload + local * a.row_bytes;
+                    if (DTYPE == AG_I8) scales[u] = a.scales + local * blocks_per_row;
+                } else if (lane == 0) {
+                    atomicOr(a.err, kErrBadId);
+                }
             }
-        } else if (j == 0) {
-            atomicOr(a.err, kErrBadId);
         }
-        a.out[g] = f;
+        for (uint32_t v0 = lane; v0 < units; v0 += lpr * kUnitCols) {
+            W val[kUnitRows][kUnitCols];
+            float scale[kUnitRows][kUnitCols];
+#pragma unroll
+            for (int u = 0; u < kUnitRows; ++u)
+#pragma unroll
+                for (int c = 0; c < kUnitCols; ++c) {
+                    const uint32_t v = v0 + c * lpr;
+                    val[u][c] = W{};  // a row outside the store decodes to zeros
+                    scale[u][c] = 0.f;
+                    if (row[u] && v < units) {
+                        val[u][c] = load_unit<kBytes, !SHARDED>(row[u] + (uint64_t)v * kBytes);
+                        if (DTYPE == AG_I8) scale[u][c] = __ldg(scales[u] + v * UNIT / kQuantBlock);
+                    }
+                }
+#pragma unroll
+            for (int u = 0; u < kUnitRows; ++u) {
+                const uint64_t r = base + (uint64_t)u * rows_per_wave;
+                if (r >= n) continue;
+#pragma unroll
+                for (int c = 0; c < kUnitCols; ++c) {
+                    const uint32_t v = v0 + c * lpr;
+                    if (v >= units) continue;
+                    float *dst = a.out + r * a.dim + (uint64_t)v * UNIT;
+                    uint32_t f[UNIT];
+#pragma unroll
+                    for (int e = 0; e < UNIT; ++e) f[e] = unit_decode<DTYPE>(val[u][c], e, scale[u][c]);
+                    if constexpr (UNIT == 4) st_stream_v4(dst, make_uint4(f[0], f[1], f[2], f[3]));
+                    else if constexpr (UNIT == 2) st_stream_v2(dst, make_uint2(f[0], f[1]));
+                    else st_stream_u32(dst, f[0]);
+                }
+            }
+        }
+    }
+}
+
+// Elements per unit: 4, 2 or 1 (f32: 2 or 1, four would be a vector row).  `payload` /
+// `out`: an OR of all base addresses concerned.
+uint32_t unit_elems(uint32_t dim, int dtype, uintptr_t payload, uintptr_t out) {
+    for (uint32_t u = dtype == AG_F32 ? 2 : 4; u > 1; u /= 2)
+        if (dim % u == 0 && payload % (u * elem_size(dtype)) == 0 && out % (u * 4) == 0) return u;
+    return 1;
+}
+
+// Lanes per row: the power of two that wastes the fewest lane slots on the row's last
+// units; of equal ones the largest.  At least eight lanes for a row that has the units,
+// so that a group's loads and stores fill whole sectors.
+uint32_t unit_lpr_log2(uint32_t units) {
+    uint32_t best = 0;
+    uint64_t best_slots = ~0ull;
+    for (uint32_t l = 0; l <= 5; ++l) {
+        if (l < 3 && units >= 8) continue;
+        const uint64_t lanes = 1ull << l, slots = (units + lanes - 1) / lanes * lanes;
+        if (slots <= best_slots) { best = l; best_slots = slots; }
+    }
+    return best;
+}
+
+// n: rows per batch the grid is sized for; max_blocks: over all batches.
+template <int DTYPE>
+cudaError_t launch_units(const GatherArgs &a, const GatherArgs *group, uint32_t n_batches, uint64_t n, uint32_t dim, uint32_t unit,
+                         bool sharded, cudaStream_t st) {
+    const uint32_t lg = unit_lpr_log2(dim / unit);
+    const uint64_t per = (uint64_t)(kThreads >> lg) * kUnitRows, need = (n + per - 1) / per;
+    const uint64_t cap = ((uint64_t)kSMs * 64 + n_batches - 1) / n_batches;
+    const dim3 grid((uint32_t)std::max<uint64_t>(1, std::min(need, cap)), n_batches);
+#define AG_LAUNCH_UNITS(U) do { if (sharded) k_gather_units<DTYPE, U, true><<<grid, kThreads, 0, st>>>(a, group, lg); \
+                                else k_gather_units<DTYPE, U, false><<<grid, kThreads, 0, st>>>(a, group, lg); } while (0)
+    if constexpr (DTYPE != AG_F32) {
+        if (unit == 4) { AG_LAUNCH_UNITS(4); return cudaGetLastError(); }
+    }
+    if (unit == 2) AG_LAUNCH_UNITS(2);
+    else AG_LAUNCH_UNITS(1);
+#undef AG_LAUNCH_UNITS
+    return cudaGetLastError();
+}
+
+cudaError_t launch_units(int dtype, const GatherArgs &a, const GatherArgs *group, uint32_t n_batches, uint64_t n, uint32_t dim,
+                         uint32_t unit, bool sharded, cudaStream_t st) {
+    switch (dtype) {
+        case AG_I8: return launch_units<AG_I8>(a, group, n_batches, n, dim, unit, sharded, st);
+        case AG_F32: return launch_units<AG_F32>(a, group, n_batches, n, dim, unit, sharded, st);
+        case AG_F16: return launch_units<AG_F16>(a, group, n_batches, n, dim, unit, sharded, st);
+        default: return launch_units<AG_BF16>(a, group, n_batches, n, dim, unit, sharded, st);
     }
 }
 
@@ -874,22 +989,15 @@ cudaError_t launch_gather(const GatherArgs &a, int dtype, cudaStream_t st) {
             default: return launch_vec<AG_BF16>(a, nullptr, a.row_bytes, grid, a.shards != nullptr, st);
         }
     }
-    const uint64_t total = a.n * a.dim;
-    uint64_t blocks = (total + kThreads - 1) / kThreads;
-    if (blocks > (uint64_t)kSMs * 8) blocks = (uint64_t)kSMs * 8;
-    switch (dtype) {
-        case AG_I8: k_gather_elem<AG_I8><<<(int)blocks, kThreads, 0, st>>>(a, nullptr); break;
-        case AG_F32: k_gather_elem<AG_F32><<<(int)blocks, kThreads, 0, st>>>(a, nullptr); break;
-        case AG_F16: k_gather_elem<AG_F16><<<(int)blocks, kThreads, 0, st>>>(a, nullptr); break;
-        default: k_gather_elem<AG_BF16><<<(int)blocks, kThreads, 0, st>>>(a, nullptr); break;
-    }
-    return cudaGetLastError();
+    return launch_units(dtype, a, nullptr, 1, a.n, a.dim, unit_elems(a.dim, dtype, (uintptr_t)a.payload, (uintptr_t)a.out),
+                        a.shards != nullptr, st);
 }
 
 // One launch for a group of batches: grid row b gathers the batch described by
 // group_dev[b].  The output buffers come from cudaMalloc / the torch allocator
 // (256- / 512-byte aligned) and the payload base is checked by the caller's
-// store, so only the row size decides between the vector and the element path.
+// store (`aligned`: all of them 16-byte aligned); rows of whole 16-byte vectors take the
+// vector path, others are walked in units.
 cudaError_t launch_gather_group(const GatherArgs *group_dev, uint32_t n_batches, uint32_t row_bytes,
                                 uint32_t dim, uint64_t n_bound, bool aligned, int dtype, bool sharded,
                                 cudaStream_t st) {
@@ -918,17 +1026,7 @@ cudaError_t launch_gather_group(const GatherArgs *group_dev, uint32_t n_batches,
             default: return launch_vec<AG_BF16>(none, group_dev, row_bytes, grid, sharded, st);
         }
     }
-    const uint64_t total = n_bound * dim;
-    uint64_t blocks = (total + kThreads - 1) / kThreads;
-    blocks = std::max<uint64_t>(1, std::min<uint64_t>(blocks, (uint64_t)kSMs * 8 / n_batches + 1));
-    const dim3 grid((uint32_t)blocks, n_batches);
-    switch (dtype) {
-        case AG_I8: k_gather_elem<AG_I8><<<grid, kThreads, 0, st>>>(none, group_dev); break;
-        case AG_F32: k_gather_elem<AG_F32><<<grid, kThreads, 0, st>>>(none, group_dev); break;
-        case AG_F16: k_gather_elem<AG_F16><<<grid, kThreads, 0, st>>>(none, group_dev); break;
-        default: k_gather_elem<AG_BF16><<<grid, kThreads, 0, st>>>(none, group_dev); break;
-    }
-    return cudaGetLastError();
+    return launch_units(dtype, none, group_dev, n_batches, n_bound, dim, unit_elems(dim, dtype, aligned ? 0 : 1, 0), sharded, st);
 }
 
 // ------------------------------------------------ sorted gather, host side --
