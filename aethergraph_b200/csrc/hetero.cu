@@ -686,8 +686,8 @@ void het_bounds(const ag_hetero_sampler *s, uint64_t n_seeds, uint64_t *nodes, u
 void het_free_scratch(ag_hetero_sampler *s) {
     void *ptrs[] = {s->table, s->slot_of_seed, s->slot_of_edge, s->node_key, s->node_rank, s->edge_exp, s->edge_rank,
                     s->class_tiles, s->seeds_dev, s->node_tag, s->edge_tag, s->frontier, s->tiles};
-    for (void *p : ptrs) cudaFree(p);
-    if (s->seeds_pinned) cudaFreeHost(s->seeds_pinned);
+    for (void *p : ptrs) workspace_free(p);
+    workspace_free(s->seeds_pinned);
     s->table = nullptr; s->slot_of_seed = s->slot_of_edge = s->node_key = s->node_rank = s->edge_exp = s->edge_rank = nullptr;
     s->class_tiles = s->seeds_dev = nullptr; s->node_tag = s->edge_tag = nullptr; s->frontier = nullptr; s->tiles = nullptr;
     s->seeds_pinned = nullptr;
@@ -713,24 +713,22 @@ int32_t het_ensure(ag_hetero_sampler *s, uint64_t n_seeds) {
                     (unsigned long long)s->max_hop_edges, (unsigned long long)kMaxPos - 1);
     const uint64_t cn = std::max<uint64_t>(s->max_nodes, 1), ce = std::max<uint64_t>(s->max_edges, 1);
     s->table_cap = std::max<uint64_t>(1024, next_pow2(2 * s->max_nodes));
-    AG_CUDA(cudaMalloc(&s->table, G * s->table_cap * 8));
-    AG_CUDA(cudaMalloc(&s->slot_of_seed, G * cap * 4));
-    AG_CUDA(cudaMalloc(&s->slot_of_edge, G * ce * 4));
-    AG_CUDA(cudaMalloc(&s->node_key, G * cn * 4));
-    AG_CUDA(cudaMalloc(&s->node_rank, G * cn * 4));
-    AG_CUDA(cudaMalloc(&s->node_tag, G * cn));
-    AG_CUDA(cudaMalloc(&s->edge_exp, G * ce * 4));
-    AG_CUDA(cudaMalloc(&s->edge_rank, G * ce * 4));
-    AG_CUDA(cudaMalloc(&s->edge_tag, G * ce));
-    AG_CUDA(cudaMalloc(&s->frontier, G * std::max<uint64_t>(s->max_frontier, 1) * sizeof(FrontierEntry)));
+    AG_CUDA(workspace_alloc(&s->table, G * s->table_cap * 8));
+    AG_CUDA(workspace_alloc(&s->slot_of_seed, G * cap * 4));
+    AG_CUDA(workspace_alloc(&s->slot_of_edge, G * ce * 4));
+    AG_CUDA(workspace_alloc(&s->node_key, G * cn * 4));
+    AG_CUDA(workspace_alloc(&s->node_rank, G * cn * 4));
+    AG_CUDA(workspace_alloc(&s->node_tag, G * cn));
+    AG_CUDA(workspace_alloc(&s->edge_exp, G * ce * 4));
+    AG_CUDA(workspace_alloc(&s->edge_rank, G * ce * 4));
+    AG_CUDA(workspace_alloc(&s->edge_tag, G * ce));
+    AG_CUDA(workspace_alloc(&s->frontier, G * std::max<uint64_t>(s->max_frontier, 1) * sizeof(FrontierEntry)));
     s->n_tiles = std::max<uint64_t>(std::max(cap, s->max_hop_edges) / kTile + 2, 2);
-    AG_CUDA(cudaMalloc(&s->tiles, G * s->n_tiles * sizeof(TileDesc)));
-    AG_CUDA(cudaMemset(s->tiles, 0, G * s->n_tiles * sizeof(TileDesc)));
+    AG_CUDA(workspace_alloc(&s->tiles, G * s->n_tiles * sizeof(TileDesc)));
     s->class_tiles_n = std::max(cn, ce) / kClassTile + 2;
-    AG_CUDA(cudaMalloc(&s->class_tiles, G * s->class_tiles_n * kDescWords * 4));
-    AG_CUDA(cudaMemset(s->class_tiles, 0, G * s->class_tiles_n * kDescWords * 4));
-    AG_CUDA(cudaMalloc(&s->seeds_dev, G * cap * 4));
-    AG_CUDA(cudaHostAlloc(&s->seeds_pinned, G * cap * 4, cudaHostAllocDefault));
+    AG_CUDA(workspace_alloc(&s->class_tiles, G * s->class_tiles_n * kDescWords * 4));
+    AG_CUDA(workspace_alloc(&s->seeds_dev, G * cap * 4));
+    AG_CUDA(workspace_alloc_host(&s->seeds_pinned, G * cap * 4));
     s->cap_seeds = cap; s->epoch = 0; s->class_epoch = 0; s->dirty = true;
     return AG_OK;
 }
@@ -742,11 +740,9 @@ extern "C" void ag_hetero_sampler_free(ag_hetero_sampler *s) {
     DeviceGuard guard(s->device);
     if (s->in_flight && s->done) cudaEventSynchronize(s->done);
     het_free_scratch(s);
-    cudaFree(s->meta_dev); cudaFree(s->state); cudaFree(s->counts_dev); cudaFree(s->class_misc);
-    cudaFree(s->params_dev); cudaFree(s->gather_dev);
-    if (s->params_host) cudaFreeHost(s->params_host);
-    if (s->gather_host) cudaFreeHost(s->gather_host);
-    if (s->counts_host) cudaFreeHost(s->counts_host);
+    void *ptrs[] = {s->meta_dev, s->state, s->counts_dev, s->class_misc, s->params_dev, s->gather_dev, s->params_host,
+                    s->gather_host, s->counts_host};
+    for (void *p : ptrs) workspace_free(p);
     if (s->done) cudaEventDestroy(s->done);
     delete s;
 }
@@ -785,18 +781,16 @@ extern "C" int32_t ag_hetero_sampler_create_group(const ag_hetero_graph *h, cons
     int32_t st = AG_OK;
     do {
         const size_t G = group;
-        if (cudaMalloc(&s->meta_dev, sizeof(HeteroMeta)) != cudaSuccess ||
+        if (workspace_alloc(&s->meta_dev, sizeof(HeteroMeta)) != cudaSuccess ||
             cudaMemcpy(s->meta_dev, &m, sizeof(HeteroMeta), cudaMemcpyHostToDevice) != cudaSuccess ||
-            cudaMalloc(&s->state, G * sizeof(BatchState)) != cudaSuccess ||
-            cudaMemset(s->state, 0, G * sizeof(BatchState)) != cudaSuccess ||
-            cudaMalloc(&s->counts_dev, G * sizeof(ag_hetero_counts)) != cudaSuccess ||
-            cudaMalloc(&s->class_misc, G * kMiscWords * 4) != cudaSuccess ||
-            cudaMemset(s->class_misc, 0, G * kMiscWords * 4) != cudaSuccess ||
-            cudaMalloc(&s->params_dev, G * sizeof(HParams)) != cudaSuccess ||
-            cudaMalloc(&s->gather_dev, G * kMaxNT * sizeof(GatherArgs)) != cudaSuccess ||
-            cudaHostAlloc(&s->params_host, G * sizeof(HParams), cudaHostAllocDefault) != cudaSuccess ||
-            cudaHostAlloc(&s->gather_host, G * kMaxNT * sizeof(GatherArgs), cudaHostAllocDefault) != cudaSuccess ||
-            cudaHostAlloc(&s->counts_host, G * sizeof(ag_hetero_counts), cudaHostAllocDefault) != cudaSuccess ||
+            workspace_alloc(&s->state, G * sizeof(BatchState)) != cudaSuccess ||
+            workspace_alloc(&s->counts_dev, G * sizeof(ag_hetero_counts)) != cudaSuccess ||
+            workspace_alloc(&s->class_misc, G * kMiscWords * 4) != cudaSuccess ||
+            workspace_alloc(&s->params_dev, G * sizeof(HParams)) != cudaSuccess ||
+            workspace_alloc(&s->gather_dev, G * kMaxNT * sizeof(GatherArgs)) != cudaSuccess ||
+            workspace_alloc_host(&s->params_host, G * sizeof(HParams)) != cudaSuccess ||
+            workspace_alloc_host(&s->gather_host, G * kMaxNT * sizeof(GatherArgs)) != cudaSuccess ||
+            workspace_alloc_host(&s->counts_host, G * sizeof(ag_hetero_counts)) != cudaSuccess ||
             cudaEventCreateWithFlags(&s->done, cudaEventDisableTiming) != cudaSuccess) {
             st = fail(AG_ERR_CUDA, "hetero sampler allocation failed: %s", cudaGetErrorString(cudaGetLastError()));
             break;
@@ -898,7 +892,14 @@ int32_t hetero_group_into(ag_hetero_sampler *s, uint32_t n_batches, uint32_t see
     AG_TRY(het_ensure(s, max_n));
     const uint64_t G = s->group;
     if (s->dirty || s->gen >= kGens) { AG_CUDA(cudaMemsetAsync(s->table, 0xFF, G * s->table_cap * 8, st)); s->gen = 0; }
-    if (s->dirty) { AG_CUDA(cudaMemsetAsync(s->state, 0, G * sizeof(BatchState), st)); s->dirty = false; }
+    if (s->dirty) {
+        AG_CUDA(cudaMemsetAsync(s->state, 0, G * sizeof(BatchState), st));
+        AG_CUDA(cudaMemsetAsync(s->class_misc, 0, G * kMiscWords * 4, st));
+        AG_CUDA(cudaMemsetAsync(s->tiles, 0, G * s->n_tiles * sizeof(TileDesc), st));
+        AG_CUDA(cudaMemsetAsync(s->class_tiles, 0, G * s->class_tiles_n * kDescWords * 4, st));
+        s->epoch = s->class_epoch = 0;
+        s->dirty = false;
+    }
     const uint32_t H = m.num_hops;
     if (s->epoch + (H + 2) > 0x3FFFFF00u) { AG_CUDA(cudaMemsetAsync(s->tiles, 0, G * s->n_tiles * sizeof(TileDesc), st)); s->epoch = 0; }
     if (s->class_epoch + 4 > 0x3FFFFF00u) {

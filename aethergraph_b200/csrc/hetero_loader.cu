@@ -98,8 +98,8 @@ uint64_t want_x_rows(const ag_hetero_loader *l, uint32_t t, uint64_t cn) {
 }
 
 void free_set(HPoolSet &p) {
-    if (p.last_use) cudaEventDestroy(p.last_use);
-    cudaFree(p.base);
+    if (p.last_use) { cudaEventSynchronize(p.last_use); cudaEventDestroy(p.last_use); }
+    workspace_free(p.base);
 }
 
 int32_t pool_take(ag_hetero_loader *l, uint64_t n_seeds, ag_hetero_buffers *out, cudaEvent_t *last_use) {
@@ -145,7 +145,7 @@ int32_t pool_take(ag_hetero_loader *l, uint64_t n_seeds, ag_hetero_buffers *out,
     for (uint32_t t = 0; t < l->nt; ++t)
         if (want[t]) o_x[t] = carve(want[t] * l->feats[t]->dim * 4);
     uint8_t *base = nullptr;
-    if (cudaMalloc(&base, std::max<uint64_t>(off, 256)) != cudaSuccess)
+    if (workspace_alloc(&base, std::max<uint64_t>(off, 256)) != cudaSuccess)
         return fail(AG_ERR_CUDA, "hetero loader: out of device memory for a %llu-byte batch buffer: %s",
                     (unsigned long long)off, cudaGetErrorString(cudaGetLastError()));
     HPoolSet s;
@@ -173,6 +173,8 @@ void pool_give(ag_hetero_loader *l, const ag_hetero_buffers &bufs, bool record, 
     if (record) {
         if (cudaEventCreateWithFlags(&s.last_use, cudaEventDisableTiming) != cudaSuccess ||
             cudaEventRecord(s.last_use, stream) != cudaSuccess) {
+            cudaDeviceSynchronize();
+            if (s.last_use) { cudaEventDestroy(s.last_use); s.last_use = nullptr; }
             free_set(s);  // cannot order the reuse: do not reuse
             return;
         }
@@ -359,14 +361,14 @@ extern "C" int32_t ag_hetero_loader_create(const ag_hetero_graph *g, uint32_t se
         if (st != AG_OK) break;
         l->samplers.push_back(s);
         cudaStream_t stream = nullptr;
-        if (cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking) != cudaSuccess)
+        if (workspace_stream(&stream, 0) != cudaSuccess)
             st = fail(AG_ERR_CUDA, "cudaStreamCreate failed: %s", cudaGetErrorString(cudaGetLastError()));
         else
             l->streams.push_back(stream);
     }
     if (st != AG_OK) {
         for (ag_hetero_sampler *s : l->samplers) ag_hetero_sampler_free(s);
-        for (cudaStream_t s : l->streams) cudaStreamDestroy(s);
+        for (cudaStream_t s : l->streams) workspace_stream_free(s, 0);
         delete l;
         return st;
     }
@@ -472,9 +474,9 @@ extern "C" void ag_hetero_loader_free(ag_hetero_loader *l) {
     for (HWork &w : l->queue) drop_work(l, w);
     for (auto &kv : l->ready) pool_give(l, kv.second.batch.bufs, false, nullptr);
     for (ag_hetero_sampler *s : l->samplers) ag_hetero_sampler_free(s);
-    for (cudaStream_t s : l->streams) cudaStreamDestroy(s);
+    for (cudaStream_t s : l->streams) workspace_stream_free(s, 0);
     // Batches still held by a consumer keep their memory valid until now.
     for (HPoolSet &p : l->pool_free) free_set(p);
-    for (auto &kv : l->pool_live) cudaFree(kv.second.base);
+    for (auto &kv : l->pool_live) workspace_free(kv.second.base);
     delete l;
 }

@@ -24,7 +24,28 @@ struct SortScratch {
 };
 }  // namespace ag
 
+namespace ag {
+// Memory and streams that outlive one handle (workspace.cu).  A block or stream is given
+// back only when all work on it has finished; contents of a new block are undefined.
+cudaError_t workspace_alloc(void **out, size_t bytes);       // current device
+cudaError_t workspace_alloc_host(void **out, size_t bytes);  // pinned
+void workspace_free(void *p);                                // either kind; null is ignored
+cudaError_t workspace_stream(cudaStream_t *out, int priority);  // non-blocking, current device
+void workspace_stream_free(cudaStream_t stream, int priority);
+template <typename T> cudaError_t workspace_alloc(T **out, size_t bytes) { return workspace_alloc((void **)out, bytes); }
+template <typename T> cudaError_t workspace_alloc_host(T **out, size_t bytes) { return workspace_alloc_host((void **)out, bytes); }
+// Held by every graph and feature store: kept blocks are freed when one is created and
+// when the last one goes.
+struct WorkspaceUser {
+    WorkspaceUser();
+    WorkspaceUser(const WorkspaceUser &);
+    WorkspaceUser &operator=(const WorkspaceUser &) = default;
+    ~WorkspaceUser();
+};
+}  // namespace ag
+
 struct ag_graph {
+    ag::WorkspaceUser workspace;
     int device = 0;
     uint64_t num_nodes = 0, num_edges = 0;
     uint64_t *offsets = nullptr;  // device, num_nodes + 1
@@ -47,6 +68,7 @@ void peer_handle_mark_legacy(void *handle);
 }  // namespace ag
 
 struct ag_features {
+    ag::WorkspaceUser workspace;
     int device = 0;
     uint64_t num_nodes = 0;   // rows of the whole store
     uint64_t row_begin = 0;   // first row held here (vertex-range shard)
@@ -88,6 +110,7 @@ struct ag_features {
 // Heterogeneous graph: per edge type only the transposed adjacency lives on the
 // device (for each destination, its sources ascending).
 struct ag_hetero_graph {
+    ag::WorkspaceUser workspace;
     int device = 0;
     uint32_t nt = 0, et = 0;
     uint64_t num_nodes[AG_MAX_NODE_TYPES] = {0};

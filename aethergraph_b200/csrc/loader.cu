@@ -40,7 +40,7 @@ bool yielding_waits() {
 namespace {
 
 struct PoolSet {
-    void *base = nullptr;              // one cudaMalloc: every array but x
+    void *base = nullptr;              // one allocation: every array but x
     void *x_base = nullptr;            // x on its own, so that a batch that outgrew it can get a larger one
     ag_subgraph_buffers bufs{};
     cudaEvent_t last_use = nullptr;    // consumer's last use of the memory, if any
@@ -92,6 +92,7 @@ struct ag_loader {
     std::vector<std::thread> workers;
     std::vector<ag_sampler *> samplers;
     std::vector<cudaStream_t> streams;
+    int priority = 0;                    // of `streams`
     ag_loader_stats stats{};
 
     // x of a pooled batch is reserved from the node counts batches really produce (the
@@ -140,9 +141,9 @@ int32_t pool_take(ag_loader *l, uint64_t n_seeds, ag_subgraph_buffers *out, cuda
                    o_nid = carve(cn * 8), o_eil = carve(ce * 16), o_sidx = carve(cs * 8);
     uint8_t *base = nullptr;
     float *xb = nullptr;
-    if (cudaMalloc(&base, std::max<uint64_t>(off, 256)) != cudaSuccess ||
-        (dim && cudaMalloc(&xb, std::max<uint64_t>(cx * dim * 4, 256)) != cudaSuccess)) {
-        cudaFree(base);
+    if (workspace_alloc(&base, std::max<uint64_t>(off, 256)) != cudaSuccess ||
+        (dim && workspace_alloc(&xb, std::max<uint64_t>(cx * dim * 4, 256)) != cudaSuccess)) {
+        workspace_free(base);
         return fail(AG_ERR_CUDA, "loader: out of device memory for a %llu-byte batch buffer: %s",
                     (unsigned long long)(off + cx * dim * 4), cudaGetErrorString(cudaGetLastError()));
     }
@@ -177,7 +178,8 @@ void pool_give(ag_loader *l, const ag_subgraph_buffers &bufs, bool record, cudaS
             cudaEventRecord(s.last_use, stream) != cudaSuccess) {
             // Cannot order the reuse: do not reuse.
             if (s.last_use) cudaEventDestroy(s.last_use);
-            cudaFree(s.base); cudaFree(s.x_base);
+            cudaDeviceSynchronize();
+            workspace_free(s.base); workspace_free(s.x_base);
             return;
         }
     }
@@ -282,18 +284,18 @@ void worker_main(ag_loader *l, uint32_t idx) {
                 float *bigger = nullptr;
                 const uint64_t rows = ((nn + nn / 4 + 4095) / 4096) * 4096;
                 int32_t g = AG_OK;
-                if (cudaMalloc(&bigger, rows * l->f->dim * 4) != cudaSuccess) g = fail(AG_ERR_CUDA, "loader: out of device memory for %llu feature rows", (unsigned long long)rows);
+                if (workspace_alloc(&bigger, rows * l->f->dim * 4) != cudaSuccess) g = fail(AG_ERR_CUDA, "loader: out of device memory for %llu feature rows", (unsigned long long)rows);
                 if (g == AG_OK) g = ag_gather(l->f, w.bufs.nodes, 0, nn, nullptr, bigger, st);
                 if (g == AG_OK && cudaStreamSynchronize(st) != cudaSuccess) g = fail(AG_ERR_CUDA, "loader: gathering an outgrown batch again failed");
-                if (g != AG_OK) { cudaFree(bigger); statuses[b] = g; err = ag_last_error(); if (rc == AG_OK) rc = g; continue; }
+                if (g != AG_OK) { cudaStreamSynchronize(st); workspace_free(bigger); statuses[b] = g; err = ag_last_error(); if (rc == AG_OK) rc = g; continue; }
                 std::lock_guard<std::mutex> pk(l->pool_m);
                 auto it = l->pool_live.find(w.bufs.nodes);
                 if (it != l->pool_live.end()) {
-                    cudaFree(it->second.x_base);
+                    workspace_free(it->second.x_base);
                     it->second.x_base = bigger; it->second.bufs.x = bigger; it->second.bufs.cap_x = rows;
                     w.bufs.x = bigger; w.bufs.cap_x = rows;
                 } else {
-                    cudaFree(bigger);
+                    workspace_free(bigger);
                 }
             }
         }
@@ -446,13 +448,14 @@ extern "C" int32_t ag_loader_create(const ag_graph *g, const ag_features *f, con
         // its own lowest-priority stream, so chains of other workers cut in.
         int lo = 0, hi = 0;
         cudaDeviceGetStreamPriorityRange(&lo, &hi);
-        if (st == AG_OK && cudaStreamCreateWithPriority(&stream, cudaStreamNonBlocking, hi) != cudaSuccess)
+        if (st == AG_OK && workspace_stream(&stream, hi) != cudaSuccess)
             st = fail(AG_ERR_CUDA, "cudaStreamCreate failed: %s", cudaGetErrorString(cudaGetLastError()));
+        l->priority = hi;
         if (st == AG_OK) l->streams.push_back(stream);
     }
     if (st != AG_OK) {
         for (ag_sampler *s : l->samplers) ag_sampler_free(s);
-        for (cudaStream_t s : l->streams) cudaStreamDestroy(s);
+        for (cudaStream_t s : l->streams) workspace_stream_free(s, l->priority);
         delete l;
         return st;
     }
@@ -613,9 +616,9 @@ extern "C" void ag_loader_free(ag_loader *l) {
     for (Work &w : l->queue) drop_work(l, w);
     for (auto &kv : l->ready) if (kv.second.batch.owned) pool_give(l, kv.second.batch.bufs, false, nullptr);
     for (ag_sampler *s : l->samplers) ag_sampler_free(s);
-    for (cudaStream_t s : l->streams) cudaStreamDestroy(s);
+    for (cudaStream_t s : l->streams) workspace_stream_free(s, l->priority);
     // Batches still held by a consumer keep their memory valid until now.
-    for (PoolSet &p : l->pool_free) { if (p.last_use) cudaEventDestroy(p.last_use); cudaFree(p.base); cudaFree(p.x_base); }
-    for (auto &kv : l->pool_live) { cudaFree(kv.second.base); cudaFree(kv.second.x_base); }
+    for (PoolSet &p : l->pool_free) { if (p.last_use) cudaEventDestroy(p.last_use); workspace_free(p.base); workspace_free(p.x_base); }
+    for (auto &kv : l->pool_live) { workspace_free(kv.second.base); workspace_free(kv.second.x_base); }
     delete l;
 }

@@ -111,8 +111,13 @@ uint64_t pow2_at_least(uint64_t v) {
 uint32_t grid_for(uint64_t n) { return (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>((n + 255) / 256, (uint64_t)kSMs * 8)); }
 
 struct Scratch {
+    cudaStream_t st;
     void *p[6] = {};
-    ~Scratch() { for (void *q : p) if (q) cudaFree(q); }
+    bool idle = false;  // nothing queued on `st` uses the blocks any more
+    ~Scratch() {
+        if (!idle) cudaStreamSynchronize(st);
+        for (void *q : p) workspace_free(q);
+    }
 };
 
 }  // namespace
@@ -135,13 +140,13 @@ extern "C" int32_t ag_subgraph_mirror(int32_t device, uint64_t n_edges, uint64_t
     if (!guard.ok) return AG_ERR_CUDA;
     cudaStream_t st = (cudaStream_t)stream;
     const uint64_t cap = pow2_at_least(4 * n_edges), mask = cap - 1;  // <= 2n keys: load <= 1/2
-    Scratch sc;
+    Scratch sc{st};
     unsigned long long *keys = nullptr; uint32_t *vals = nullptr, *flags = nullptr, *rank = nullptr, *err = nullptr;
-    AG_CUDA(cudaMalloc(&sc.p[0], cap * 8)); keys = (unsigned long long *)sc.p[0];
-    AG_CUDA(cudaMalloc(&sc.p[1], cap * 4)); vals = (uint32_t *)sc.p[1];
-    AG_CUDA(cudaMalloc(&sc.p[2], (n_edges + 1) * 4)); flags = (uint32_t *)sc.p[2];
-    AG_CUDA(cudaMalloc(&sc.p[3], (n_edges + 1) * 4)); rank = (uint32_t *)sc.p[3];
-    AG_CUDA(cudaMalloc(&sc.p[4], 4)); err = (uint32_t *)sc.p[4];
+    AG_CUDA(workspace_alloc(&sc.p[0], cap * 8)); keys = (unsigned long long *)sc.p[0];
+    AG_CUDA(workspace_alloc(&sc.p[1], cap * 4)); vals = (uint32_t *)sc.p[1];
+    AG_CUDA(workspace_alloc(&sc.p[2], (n_edges + 1) * 4)); flags = (uint32_t *)sc.p[2];
+    AG_CUDA(workspace_alloc(&sc.p[3], (n_edges + 1) * 4)); rank = (uint32_t *)sc.p[3];
+    AG_CUDA(workspace_alloc(&sc.p[4], 4)); err = (uint32_t *)sc.p[4];
     AG_CUDA(cudaMemsetAsync(keys, 0xFF, cap * 8, st));
     AG_CUDA(cudaMemsetAsync(vals, 0xFF, cap * 4, st));
     AG_CUDA(cudaMemsetAsync(err, 0, 4, st));
@@ -152,13 +157,14 @@ extern "C" int32_t ag_subgraph_mirror(int32_t device, uint64_t n_edges, uint64_t
     k_mirror_flags<<<grid, 256, 0, st>>>(src_local, dst_local, n_edges, keys, vals, mask, flags);
     size_t temp_bytes = 0;
     AG_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, temp_bytes, flags, rank, (int)(n_edges + 1), st));
-    AG_CUDA(cudaMalloc(&sc.p[5], std::max<size_t>(temp_bytes, 16)));
+    AG_CUDA(workspace_alloc(&sc.p[5], std::max<size_t>(temp_bytes, 16)));
     AG_CUDA(cub::DeviceScan::ExclusiveSum(sc.p[5], temp_bytes, flags, rank, (int)(n_edges + 1), st));
     k_mirror_append<<<grid, 256, 0, st>>>(edge_src, edge_dst, src_local, dst_local, edge_ids, n_edges, flags, rank);
     uint32_t added = 0, herr = 0;
     AG_CUDA(cudaMemcpyAsync(&added, rank + n_edges, 4, cudaMemcpyDeviceToHost, st));
     AG_CUDA(cudaMemcpyAsync(&herr, err, 4, cudaMemcpyDeviceToHost, st));
     AG_CUDA(cudaStreamSynchronize(st));
+    sc.idle = true;
     if (herr) return fail(AG_ERR_WORKER, "ag_subgraph_mirror: pair table overflow");
     const uint64_t total = n_edges + added;
     if (edge_index_local) {
@@ -384,6 +390,7 @@ k_induce_walk(InduceWalk a, InduceOut o) {
 struct ag_induce_plan {
     int device = 0;
     uint64_t n_edges = 0;
+    cudaStream_t stream = nullptr;  // the last call's
     void *scratch = nullptr;
     InduceWalk walk{};
 };
@@ -391,7 +398,8 @@ struct ag_induce_plan {
 extern "C" void ag_subgraph_induce_free(ag_induce_plan *p) {
     if (!p) return;
     DeviceGuard guard(p->device);
-    cudaFree(p->scratch);
+    if (p->scratch) cudaStreamSynchronize(p->stream);  // already idle unless a call failed
+    workspace_free(p->scratch);
     delete p;
 }
 
@@ -406,7 +414,7 @@ extern "C" int32_t ag_subgraph_induce_plan(const ag_graph *g, const uint32_t *no
     if (!guard.ok) return AG_ERR_CUDA;
     cudaStream_t st = (cudaStream_t)stream;
     ag_induce_plan *p = new ag_induce_plan();
-    p->device = g->device;
+    p->device = g->device; p->stream = st;
     *out = nullptr; *n_edges_out = 0;
     if (n_nodes == 0) { *out = p; return AG_OK; }
     auto bail = [&](int32_t rc) { ag_subgraph_induce_free(p); return rc; };
@@ -419,7 +427,7 @@ extern "C" int32_t ag_subgraph_induce_plan(const ag_graph *g, const uint32_t *no
     // one allocation: table, row offsets, row lengths and their scan, the warps' counts, totals, scan scratch
     const uint64_t words = cap + n_nodes + 2 * (n_nodes + 1) + warps + 3;
     const uint64_t temp_at = (words * 8 + 255) & ~255ull;
-    AG_PLAN_CUDA(cudaMalloc(&p->scratch, temp_at + temp_bytes));
+    AG_PLAN_CUDA(workspace_alloc(&p->scratch, temp_at + temp_bytes));
     unsigned long long *table = (unsigned long long *)p->scratch;
     uint64_t *row_off = (uint64_t *)(table + cap), *row_len = row_off + n_nodes, *row_start = row_len + n_nodes + 1;
     uint64_t *warp_start = row_start + n_nodes + 1, *total = warp_start + warps;  // total[2]: error bits
@@ -460,6 +468,7 @@ extern "C" int32_t ag_subgraph_induce_fill(ag_induce_plan *p, uint64_t cap_edges
     DeviceGuard guard(p->device);
     if (!guard.ok) return AG_ERR_CUDA;
     cudaStream_t st = (cudaStream_t)stream;
+    p->stream = st;
     const InduceOut o{edge_src, edge_dst, src_local, dst_local, edge_ids, edge_index_local, p->n_edges};
     k_induce_walk<true><<<p->walk.warps / (kWalkThreads / 32), kWalkThreads, p->walk.filter_words * 4, st>>>(p->walk, o);
     AG_CUDA(cudaGetLastError());

@@ -1237,8 +1237,10 @@ struct ag_sampler {
     cudaStream_t gstream = nullptr;
     cudaEvent_t sampled = nullptr;
     // Sharded stores: the remote part of a chain's rows is fetched by a launch of its own on
-    // this stream (between the two priorities), beside the local part on gstream.
+    // this stream (between the two priorities), beside the local part on gstream.  Made when
+    // the first such chain is launched.
     cudaStream_t rstream = nullptr;
+    int gpriority = 0, rpriority = 0;
     cudaEvent_t remote_done = nullptr;
     uint64_t est_rows_tight = 0;  // rows per batch the last chain produced, with little headroom (sort padding)
     SortScratch sort;  // sharded feature stores: the chain's row ids in address order (gather.cu)
@@ -1286,11 +1288,11 @@ void compute_bounds(const ag_sampler *s, uint64_t n_seeds, uint64_t *max_nodes, 
 }
 
 void free_scratch(ag_sampler *s) {
-    cudaFree(s->table); cudaFree(s->frontier);
+    workspace_free(s->table); workspace_free(s->frontier);
     s->frontier = nullptr;
-    cudaFree(s->slot_of_seed); cudaFree(s->slot_of_edge); cudaFree(s->tiles);
-    cudaFree(s->hub_rows); s->hub_rows = nullptr;
-    if (s->seeds_pinned) cudaFreeHost(s->seeds_pinned);
+    workspace_free(s->slot_of_seed); workspace_free(s->slot_of_edge); workspace_free(s->tiles);
+    workspace_free(s->hub_rows); s->hub_rows = nullptr;
+    workspace_free(s->seeds_pinned);
     s->table = nullptr;
     s->slot_of_seed = s->slot_of_edge = nullptr; s->tiles = nullptr;
     s->seeds_pinned = nullptr;
@@ -1316,12 +1318,12 @@ int32_t ensure_scratch(ag_sampler *s, uint64_t n_seeds) {
                     "in a hop (limit %llu each)", (unsigned long long)n_seeds, (unsigned long long)s->max_nodes,
                     (unsigned long long)s->max_hop_edges, (unsigned long long)kMaxPos - 1);
     s->table_cap = std::max<uint64_t>(1024, next_pow2(2 * s->max_nodes));
-    AG_CUDA(cudaMalloc(&s->table, G * s->table_cap * 8));
+    AG_CUDA(workspace_alloc(&s->table, G * s->table_cap * 8));
     // the frontier of a hop holds at most the vertices the previous stage found
     s->max_frontier = std::max<uint64_t>(std::min<uint64_t>(std::max(cap, s->max_hop_edges), s->g->num_nodes), 1);
-    AG_CUDA(cudaMalloc(&s->frontier, G * s->max_frontier * sizeof(FrontierEntry)));
-    AG_CUDA(cudaMalloc(&s->slot_of_seed, G * cap * 4));
-    AG_CUDA(cudaMalloc(&s->slot_of_edge, G * std::max<uint64_t>(s->max_edges, 1) * 4));
+    AG_CUDA(workspace_alloc(&s->frontier, G * s->max_frontier * sizeof(FrontierEntry)));
+    AG_CUDA(workspace_alloc(&s->slot_of_seed, G * cap * 4));
+    AG_CUDA(workspace_alloc(&s->slot_of_edge, G * std::max<uint64_t>(s->max_edges, 1) * 4));
     if (s->mode == kModeWeighted) {
         // A batch expands a vertex once, and a row of d > kHubDegree positions is at most
         // 2 d / kHubDegree slices.
@@ -1331,7 +1333,7 @@ int32_t ensure_scratch(ag_sampler *s, uint64_t n_seeds) {
         s->hub_cap = (uint32_t)std::min<uint64_t>(std::max<uint64_t>(most, 1), kMaxHubSlices);
         const uint64_t cap = s->hub_cap;
         uint8_t *base = nullptr;
-        AG_CUDA(cudaMalloc(&base, cap * (sizeof(HubRow) + 8 * hop_k + 4 * hop_k + 12) + 8));
+        AG_CUDA(workspace_alloc(&base, cap * (sizeof(HubRow) + 8 * hop_k + 4 * hop_k + 12) + 8));
         s->hub_rows = (HubRow *)base;
         s->hub_key = (double *)(base + cap * sizeof(HubRow));
         s->hub_count = (unsigned long long *)(s->hub_key + cap * hop_k);
@@ -1341,9 +1343,8 @@ int32_t ensure_scratch(ag_sampler *s, uint64_t n_seeds) {
         s->hub_guess = (float *)(s->hub_done + cap);
     }
     s->n_tiles = std::max<uint64_t>(std::max(cap, s->max_hop_edges) / kTile + 2, 2);
-    AG_CUDA(cudaMalloc(&s->tiles, G * s->n_tiles * sizeof(TileDesc)));
-    AG_CUDA(cudaMemset(s->tiles, 0, G * s->n_tiles * sizeof(TileDesc)));
-    AG_CUDA(cudaHostAlloc(&s->seeds_pinned, G * cap * 4, cudaHostAllocDefault));
+    AG_CUDA(workspace_alloc(&s->tiles, G * s->n_tiles * sizeof(TileDesc)));
+    AG_CUDA(workspace_alloc_host(&s->seeds_pinned, G * cap * 4));
     s->cap_seeds = cap;
     s->epoch = 0;
     s->dirty = true;
@@ -1378,13 +1379,12 @@ extern "C" int32_t ag_sampler_create_group(const ag_graph *g, const ag_sampling_
     s->seed = cfg->seed;
     int32_t st = AG_OK;
     do {
-        if (cudaMalloc(&s->state, group * sizeof(BatchState)) != cudaSuccess ||
-            cudaMemset(s->state, 0, group * sizeof(BatchState)) != cudaSuccess ||
-            cudaMalloc(&s->params_dev, group * sizeof(SampleParams)) != cudaSuccess ||
-            cudaMalloc(&s->gather_dev, group * sizeof(GatherArgs)) != cudaSuccess ||
-            cudaHostAlloc(&s->counts_host, group * sizeof(ag_sample_counts), cudaHostAllocDefault) != cudaSuccess ||
-            cudaHostAlloc(&s->params_host, group * sizeof(SampleParams), cudaHostAllocDefault) != cudaSuccess ||
-            cudaHostAlloc(&s->gather_host, group * sizeof(GatherArgs), cudaHostAllocDefault) != cudaSuccess ||
+        if (workspace_alloc(&s->state, group * sizeof(BatchState)) != cudaSuccess ||  // cleared by the first launch (`dirty`)
+            workspace_alloc(&s->params_dev, group * sizeof(SampleParams)) != cudaSuccess ||
+            workspace_alloc(&s->gather_dev, group * sizeof(GatherArgs)) != cudaSuccess ||
+            workspace_alloc_host(&s->counts_host, group * sizeof(ag_sample_counts)) != cudaSuccess ||
+            workspace_alloc_host(&s->params_host, group * sizeof(SampleParams)) != cudaSuccess ||
+            workspace_alloc_host(&s->gather_host, group * sizeof(GatherArgs)) != cudaSuccess ||
             cudaEventCreateWithFlags(&s->done, cudaEventDisableTiming) != cudaSuccess ||
             cudaEventCreateWithFlags(&s->sampled, cudaEventDisableTiming) != cudaSuccess) {
             st = fail(AG_ERR_CUDA, "sampler allocation failed: %s", cudaGetErrorString(cudaGetLastError()));
@@ -1394,9 +1394,9 @@ extern "C" int32_t ag_sampler_create_group(const ag_graph *g, const ag_sampling_
         cudaDeviceGetStreamPriorityRange(&lo, &hi);  // lo = least urgent
         // AG_GATHER_PRIORITY=high: the gather streams as urgent as the sampling streams (A/B measurements)
         static const bool gather_high = [] { const char *v = getenv("AG_GATHER_PRIORITY"); return v && v[0] == 'h'; }();
-        if (cudaStreamCreateWithPriority(&s->gstream, cudaStreamNonBlocking, gather_high ? hi : lo) != cudaSuccess ||
-            cudaStreamCreateWithPriority(&s->rstream, cudaStreamNonBlocking, (lo + hi) / 2) != cudaSuccess ||
-            cudaEventCreateWithFlags(&s->remote_done, cudaEventDisableTiming) != cudaSuccess) {
+        s->gpriority = gather_high ? hi : lo;
+        s->rpriority = (lo + hi) / 2;
+        if (workspace_stream(&s->gstream, s->gpriority) != cudaSuccess) {
             st = fail(AG_ERR_CUDA, "cudaStreamCreateWithPriority failed: %s", cudaGetErrorString(cudaGetLastError()));
             break;
         }
@@ -1418,14 +1418,12 @@ extern "C" void ag_sampler_free(ag_sampler *s) {
     free_scratch(s);
     s->sort.release();
     for (void *p : s->owned) cudaFree(p);
-    cudaFree(s->state); cudaFree(s->params_dev); cudaFree(s->gather_dev);
-    if (s->counts_host) cudaFreeHost(s->counts_host);
-    if (s->params_host) cudaFreeHost(s->params_host);
-    if (s->gather_host) cudaFreeHost(s->gather_host);
+    workspace_free(s->state); workspace_free(s->params_dev); workspace_free(s->gather_dev);
+    workspace_free(s->counts_host); workspace_free(s->params_host); workspace_free(s->gather_host);
     if (s->done) cudaEventDestroy(s->done);
     if (s->sampled) cudaEventDestroy(s->sampled);
-    if (s->gstream) cudaStreamDestroy(s->gstream);
-    if (s->rstream) cudaStreamDestroy(s->rstream);
+    workspace_stream_free(s->gstream, s->gpriority);
+    workspace_stream_free(s->rstream, s->rpriority);
     if (s->remote_done) cudaEventDestroy(s->remote_done);
     for (auto &e : s->ev) if (e) cudaEventDestroy(e);
     delete s;
@@ -1594,6 +1592,8 @@ int32_t launch_saved_impl(ag_sampler *s, bool relaunch) {
     }
     if (s->dirty) {
         AG_CUDA(cudaMemsetAsync(s->state, 0, s->group * sizeof(BatchState), st));
+        AG_CUDA(cudaMemsetAsync(s->tiles, 0, (uint64_t)s->group * s->n_tiles * sizeof(TileDesc), st));
+        s->epoch = 0;
         s->dirty = false;
     }
     const uint32_t H = s->cfg.num_hops;
@@ -1714,6 +1714,8 @@ int32_t launch_saved_impl(ag_sampler *s, bool relaunch) {
         AG_CUDA(cudaStreamWaitEvent(s->gstream, s->sampled, 0));
         if (s->profile) AG_CUDA(cudaEventRecord(s->ev[2], s->gstream));
         if (sorted) {
+            if (!s->rstream) AG_CUDA(workspace_stream(&s->rstream, s->rpriority));
+            if (!s->remote_done) AG_CUDA(cudaEventCreateWithFlags(&s->remote_done, cudaEventDisableTiming));
             AG_CUDA(cudaStreamWaitEvent(s->rstream, s->sampled, 0));
             AG_CUDA(launch_sorted_fetch(GatherArgs{}, s->gather_dev, n_batches, sort_rows, row_bytes, (uint32_t)feats->dim,
                                         feats->dtype, feats, s->sort, s->gstream, s->rstream));

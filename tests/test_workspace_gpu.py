@@ -1,0 +1,92 @@
+"""Scratch that short-lived handles share: batches out of reused blocks equal the oracle's,
+also from several threads, and the memory is bounded and given back."""
+import subprocess
+import sys
+import threading
+
+import numpy as np
+import pytest
+
+from helpers import assert_same_subgraph, rmat_csr
+
+pytestmark = pytest.mark.gpu
+
+
+def _run(ag, ago, g, off, dst, store, feats, fanout, size, seed, count):
+    import torch
+
+    rng = np.random.default_rng(seed)
+    n = len(off) - 1
+    batches = [rng.integers(0, n, size).astype(np.uint32) for _ in range(count)]
+    o = ago.Sampler(off, dst, fanout, seed=seed)
+    with ag.NeighborLoader(g, ag.SamplingConfig(num_neighbors=fanout, seed=seed), prefetch_depth=2, sampler_threads=2,
+                           features=store, group=2) as ld:
+        ld.submit_epoch(batches)
+        for i in range(count):
+            idx, sg, x = ld.next_batch()
+            o.reseed(ago.batch_seed(seed, i))
+            want = o.sample(batches[i])
+            assert_same_subgraph(sg.raw_u32(), want)
+            assert torch.equal(x.cpu(), torch.from_numpy(feats[want["nodes"].astype(np.int64)]))
+
+
+@pytest.mark.parametrize("threads", [1, 4])
+def test_loaders_one_after_the_other(threads):
+    import aethergraph_b200 as ag
+    from oracle import ago
+
+    n, off, dst, _ = rmat_csr(12, 12, seed=4)
+    feats = np.random.default_rng(0).standard_normal((n, 24)).astype(np.float32)
+    g, store = ag.Graph.from_csr(off, dst), ag.FeatureStore.from_array(feats)
+    errors = []
+
+    def work(t):
+        try:
+            for r in range(6):
+                fanout, size = [([5, 3], 64), ([4], 200), ([3, 3, 2], 30)][(r + t) % 3]
+                _run(ag, ago, g, off, dst, store, feats, fanout, size, 100 * t + r, 5)
+        except BaseException as e:  # handed to the test's own thread
+            errors.append(e)
+
+    ts = [threading.Thread(target=work, args=(t,)) for t in range(threads)]
+    for t in ts:
+        t.start()
+    for t in ts:
+        t.join()
+    if errors:
+        raise errors[0]
+
+
+_SCRIPT = """
+import gc, numpy as np, torch
+import aethergraph_b200 as ag
+def used():
+    gc.collect(); torch.cuda.synchronize(); torch.cuda.empty_cache()
+    free, total = torch.cuda.mem_get_info()
+    return (total - free) >> 20
+def make():
+    rng = np.random.default_rng(1)
+    off = np.arange(100_001, dtype=np.uint64) * 20
+    return ag.Graph.from_csr(off, rng.integers(0, 100_000, 2_000_000).astype(np.uint32))
+def loaders(g, sizes):
+    for size in sizes:
+        with ag.NeighborLoader(g, ag.SamplingConfig(num_neighbors=[10, 10], seed=1), sampler_threads=2) as ld:
+            ld.submit_epoch([np.arange(size, dtype=np.uint32)] * 4)
+            for _ in range(4): ld.next_batch()
+g = make(); loaders(g, [100]); del g
+before = used()          # kernels loaded, streams made
+g = make()
+alone = used()
+loaders(g, [100, 1000, 8000, 50, 20000, 700])
+kept = used() - alone
+assert kept <= 512 + 64, kept
+del g
+after = used()
+assert after <= before + 16, (before, after)
+print("ok", before, kept, after)
+"""
+
+
+def test_kept_memory_is_bounded_and_given_back():
+    r = subprocess.run([sys.executable, "-c", _SCRIPT], capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0 and "ok" in r.stdout, r.stdout + r.stderr
