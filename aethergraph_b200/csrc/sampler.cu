@@ -445,7 +445,7 @@ __device__ __forceinline__ double weighted_key(const SampleParams &p, uint32_t h
 // Bound: instructions, about 30 for 32 positions in stage 1 and 500 for a flush, so what
 // counts is the multiply of the random stream (wyrand_top32) and the number of flushes
 // (guess_threshold).  kChunks * 32 positions are loaded and filtered together and only
-// then asked for survivors, with one vote.
+// then asked for survivors, with one vote, while the next ones are loaded.
 constexpr uint32_t kChunks = 4;
 
 template <bool PHILOX>
@@ -481,14 +481,19 @@ __device__ __forceinline__ void topk_stream_rng(const SampleParams &p, uint32_t 
     const uint64_t seed = p.seed;
     uint32_t first = begin + lane;  // this lane's position in the next chunk
     uint64_t state = seed + (fe.dbase + first + 1ull) * kStep;
+    float wf[kChunks];  // the weights of the next kChunks * 32 positions
+#pragma unroll
+    for (uint32_t u = 0; u < kChunks; ++u) wf[u] = u * 32 + lane < end - begin ? __ldg(w + u * 32) : 0.0f;
     for (uint32_t left = end - begin; left > 0;) {
+        // those after them are on their way while these are filtered
+        float ahead[kChunks];
+#pragma unroll
+        for (uint32_t u = 0; u < kChunks; ++u)
+            ahead[u] = left > 32 * kChunks && u * 32 + lane < left - 32 * kChunks ? __ldg(w + 32 * kChunks + u * 32) : 0.0f;
         float t = thr;
         if (shared_thr) t = fminf(t, __uint_as_float(__ldcg(shared_thr)));
         // NaN: nothing is dropped
         const float ts = (t >= 1.0e-30f && t <= 3.0e38f) ? t * 1.00001f : __uint_as_float(0x7FC00000u);
-        float wf[kChunks];
-#pragma unroll
-        for (uint32_t u = 0; u < kChunks; ++u) wf[u] = u * 32 + lane < left ? __ldg(w + u * 32) : 0.0f;
         bool kept[kChunks], any = false;
 #pragma unroll
         for (uint32_t u = 0; u < kChunks; ++u) {
@@ -522,6 +527,8 @@ __device__ __forceinline__ void topk_stream_rng(const SampleParams &p, uint32_t 
         w += 32 * kChunks;
         first += 32 * kChunks;
         state += 32 * kChunks * kStep;
+#pragma unroll
+        for (uint32_t u = 0; u < kChunks; ++u) wf[u] = ahead[u];
         left -= min(left, 32 * kChunks);
     }
     if (queued) { flush(queued); __syncwarp(); }
@@ -622,9 +629,10 @@ __device__ __forceinline__ void pick_weighted(const SampleParams &p, uint32_t ho
         }
         double best_key;
         uint32_t best_pos;
-        topk_stream(p, hop, fe, 0, deg, k, lane, best_key, best_pos, queue + warp * 64, guess);
-        if (!(__shfl_sync(0xffffffffu, best_key, k - 1) <= (double)guess))
-            topk_stream(p, hop, fe, 0, deg, k, lane, best_key, best_pos, queue + warp * 64, inff);
+        for (;; guess = inff) {  // again without the guess if it was too low
+            topk_stream(p, hop, fe, 0, deg, k, lane, best_key, best_pos, queue + warp * 64, guess);
+            if (__shfl_sync(0xffffffffu, best_key, k - 1) <= (double)guess) break;
+        }
         if ((uint32_t)lane < k) emit_edge(p, hop, edges_before, fe, lane, fe.off + best_pos);
     }
 }
@@ -1033,7 +1041,7 @@ k_assign_seeds(StagedChain chain, uint32_t k) {
 // size and where the hop's edges start).  The lanes of the whole grid share the
 // frontier, so even a hop with few vertices spreads over the GPU.
 template <int G, int PICK>
-__global__ void __launch_bounds__(PICK == kPickLarge ? 128 : PICK == kPickWeighted ? kWeightedThreads : kPickThreads)
+__global__ void __launch_bounds__(PICK == kPickLarge ? 128 : PICK == kPickWeighted ? kWeightedThreads : kPickThreads, PICK == kPickWeighted ? 14 : 1)
 k_pick(const SampleParams *__restrict__ pa, uint32_t hop, uint32_t k) {
     __shared__ uint32_t s_picks[PICK == kPickLarge ? 4 : 1][PICK == kPickLarge ? kLargeK : 1];
     __shared__ uint32_t s_queue[PICK == kPickWeighted ? (kWeightedThreads / 32) * 64 : 1];  // weighted: 64 queued positions per warp
@@ -1053,8 +1061,9 @@ k_pick(const SampleParams *__restrict__ pa, uint32_t hop, uint32_t k) {
 // A row of 500 K positions on one block of 512 threads took 450 us, as long for one batch
 // as for eight.  Twelve batches of 512 seeds, fanouts 15, 10, 5, on the 10 M vertex / 200 M
 // edge graph (28 M positions a batch): 5320 us with a block per row, 3600 us with slices,
-// 2730 us with the shorter filter and the first threshold guessed.
-__global__ void __launch_bounds__(kWeightedThreads)
+// 2730 us with the shorter filter and the first threshold guessed, 2320 us with the next
+// weights loaded ahead and slices half as long.
+__global__ void __launch_bounds__(kWeightedThreads, 14)
 k_pick_hub_slices(const SampleParams *__restrict__ pa, uint32_t hop, uint32_t k) {
     __shared__ uint32_t s_queue[(kWeightedThreads / 32) * 64];
     chain_sync();
@@ -1079,33 +1088,40 @@ k_pick_hub_slices(const SampleParams *__restrict__ pa, uint32_t hop, uint32_t k)
         const FrontierEntry fe = p.frontier[row.vertex];
         const uint32_t deg = fe.deg, len = hub_slice_len(deg, q.hub_slice);
         const uint64_t first = (uint64_t)(slice - row.slice_base) * len;
-        const uint32_t begin = (uint32_t)min((uint64_t)deg, first), end = (uint32_t)min((uint64_t)deg, first + len);
-        const float guess = q.hub_guess[lo];
+        uint32_t begin = (uint32_t)min((uint64_t)deg, first), end = (uint32_t)min((uint64_t)deg, first + len);
+        float guess = q.hub_guess[lo];
+        uint32_t *shared_thr = q.hub_thr + lo;
         double best_key;
         uint32_t best_pos;
-        topk_stream(p, hop, fe, begin, end, k, lane, best_key, best_pos, s_queue + warp * 64, guess, q.hub_thr + lo);
-        if (row.n_slices > 1) {
-            const uint64_t mine = (uint64_t)slice * k;
-            if ((uint32_t)lane < k) { q.hub_key[mine + lane] = best_key; q.hub_pos[mine + lane] = best_pos; }
-            __threadfence();
-            __syncwarp();
-            uint32_t before = 0;
-            if (lane == 0) before = atomicAdd(q.hub_done + lo, 1u);
-            if (__shfl_sync(0xffffffffu, before, 0) != row.n_slices - 1) continue;
-            __threadfence();
-            const uint64_t from = (uint64_t)row.slice_base * k;
-            const uint32_t cands = row.n_slices * k;
-            for (uint32_t c = 0; c < cands; c += 32) {
-                const uint32_t i = c + lane;
-                // this slice's own best are in the lanes already
-                const bool have = i < cands && i / k != slice - row.slice_base;
-                const double ck = have ? __ldcg(q.hub_key + from + i) : inf;
-                const uint32_t cp = have ? __ldcg(q.hub_pos + from + i) : 0xFFFFFFFFu;
-                topk_insert_chunk(ck, cp, best_key, best_pos, k, lane);
+        bool mine = true;  // this warp finishes the row
+        for (bool whole = row.n_slices == 1;; whole = true) {
+            topk_stream(p, hop, fe, begin, end, k, lane, best_key, best_pos, s_queue + warp * 64, guess, shared_thr);
+            if (!whole) {
+                const uint64_t at = (uint64_t)slice * k;
+                if ((uint32_t)lane < k) { q.hub_key[at + lane] = best_key; q.hub_pos[at + lane] = best_pos; }
+                __threadfence();
+                __syncwarp();
+                uint32_t before = 0;
+                if (lane == 0) before = atomicAdd(q.hub_done + lo, 1u);
+                mine = __shfl_sync(0xffffffffu, before, 0) == row.n_slices - 1;
+                if (!mine) break;
+                __threadfence();
+                const uint64_t from = (uint64_t)row.slice_base * k;
+                const uint32_t cands = row.n_slices * k;
+                for (uint32_t c = 0; c < cands; c += 32) {
+                    const uint32_t i = c + lane;
+                    // this slice's own best are in the lanes already
+                    const bool have = i < cands && i / k != slice - row.slice_base;
+                    const double ck = have ? __ldcg(q.hub_key + from + i) : inf;
+                    const uint32_t cp = have ? __ldcg(q.hub_pos + from + i) : 0xFFFFFFFFu;
+                    topk_insert_chunk(ck, cp, best_key, best_pos, k, lane);
+                }
             }
+            if (__shfl_sync(0xffffffffu, best_key, k - 1) <= (double)guess) break;
+            // the guess was too low: the whole row once more without one
+            begin = 0; end = deg; guess = __uint_as_float(0x7F800000u); shared_thr = nullptr;
         }
-        if (!(__shfl_sync(0xffffffffu, best_key, k - 1) <= (double)guess))
-            topk_stream(p, hop, fe, 0, deg, k, lane, best_key, best_pos, s_queue + warp * 64, __uint_as_float(0x7F800000u));
+        if (!mine) continue;
         if ((uint32_t)lane < k) emit_edge(p, hop, p.state->stage[hop + 1].n_edges, fe, lane, fe.off + best_pos);
     }
 }
@@ -1645,8 +1661,8 @@ int32_t launch_saved_impl(ag_sampler *s, bool relaunch) {
         if (s->hub_rows) {
             p.hub_rows = s->hub_rows; p.hub_count = s->hub_count; p.hub_thr = s->hub_thr; p.hub_done = s->hub_done; p.hub_guess = s->hub_guess;
             p.hub_key = s->hub_key; p.hub_pos = s->hub_pos; p.hub_cap = s->hub_cap;
-            // about as many slices whatever the chain's length: a slice of kHubDegree positions per batch
-            p.hub_slice = (uint32_t)std::min<uint64_t>(kHubDegree * next_pow2(n_batches), 16 * kHubDegree);
+            // about as many slices whatever the chain's length, a few times what runs at once
+            p.hub_slice = (uint32_t)std::min<uint64_t>(kHubDegree * std::max<uint64_t>(next_pow2(n_batches) / 2, 1), 16 * kHubDegree);
         }
         s->params_host[b] = p;
         uint64_t bn, be;
