@@ -144,6 +144,31 @@ __device__ __forceinline__ void st_stream_u32(void *p, uint32_t v) {
     asm volatile("st.global.cs.u32 [%0], %1;" :: "l"(p), "r"(v) : "memory");
 }
 
+// ------------------------------------------------------- launch chains --
+// Programmatic dependent launch: the kernels of a chain are launched with
+// cudaLaunchAttributeProgrammaticStreamSerialization, so the next kernel's blocks
+// are scheduled as this one's blocks exit, without waiting for the grid's
+// completion to be reported first.  Every kernel starts by waiting for its
+// predecessor's results (griddepcontrol.wait; a no-op for a plain launch).  The
+// kernels do NOT release their successor early (no griddepcontrol.launch_dependents
+// before the work): measured, successor blocks parked in SM slots take those slots
+// from the gather of a neighbouring chain and the whole pipeline gets slower.
+__device__ __forceinline__ void chain_sync() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
+// Launches `kern` as a programmatic dependent of the previous kernel on the stream.
+template <typename... KArgs, typename... Args>
+void launch_chained(void (*kern)(KArgs...), dim3 grid, dim3 block, cudaStream_t st, Args... args) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = 0; cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr; cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, kern, KArgs(args)...);
+}
+
 // ------------------------------------------------------ release/acquire --
 __device__ __forceinline__ void st_release_u32(uint32_t *p, uint32_t v) {
     asm volatile("st.release.gpu.global.u32 [%0], %1;" :: "l"(p), "r"(v) : "memory");

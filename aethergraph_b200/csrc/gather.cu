@@ -113,11 +113,8 @@ __device__ __forceinline__ const uint8_t *shard_row(const ag_shard_table *t, uin
 // Vector path: row_bytes % 16 == 0 and the payload base is 16-byte aligned.
 // LPR lanes share a row; vecs = row_bytes / 16.
 template <int DTYPE, int LPR>
-__global__ void __launch_bounds__(kThreads)
-k_gather_vec(GatherArgs a, const GatherArgs *__restrict__ group, uint64_t first) {
+__device__ __forceinline__ void gather_vec_rows(GatherArgs &a, uint64_t first) {
     constexpr int kRowsPerBlock = kThreads / LPR;
-    if (group) a = group[blockIdx.y];  // one batch of a group per grid row
-    if (!a.payload) return;
     const uint64_t n = a.n_dev ? min((uint64_t)*a.n_dev, a.n) : a.n;
     if (a.ids_off) a.ids = (const uint32_t *)a.ids + *a.ids_off;  // a segment of a longer id array
     const int lane = threadIdx.x % LPR;
@@ -162,6 +159,29 @@ k_gather_vec(GatherArgs a, const GatherArgs *__restrict__ group, uint64_t first)
             }
         }
     }
+}
+
+template <int DTYPE, int LPR>
+__global__ void __launch_bounds__(kThreads)
+k_gather_vec(GatherArgs a, const GatherArgs *__restrict__ group, uint64_t first) {
+    if (group) a = group[blockIdx.y];  // one batch of a group per grid row
+    if (!a.payload) return;
+    gather_vec_rows<DTYPE, LPR>(a, first);
+}
+
+// The rows of several stores of one dtype (node types) in one launch: grid row y is the
+// batch, z the store, whose arguments are group[z * stride + y].
+template <int DTYPE>
+__global__ void __launch_bounds__(kThreads)
+k_gather_stores(const GatherArgs *__restrict__ group, uint32_t stride) {
+    chain_sync();
+    GatherArgs a = group[(uint64_t)blockIdx.z * stride + blockIdx.y];
+    if (!a.payload) return;
+    const uint32_t vecs = a.row_bytes >> 4;
+    if (vecs <= 4) gather_vec_rows<DTYPE, 4>(a, 0);
+    else if (vecs <= 8) gather_vec_rows<DTYPE, 8>(a, 0);
+    else if (vecs <= 16) gather_vec_rows<DTYPE, 16>(a, 0);
+    else gather_vec_rows<DTYPE, 32>(a, 0);
 }
 
 // Direct gather over a sharded store: every row is fetched straight from where it
@@ -1027,6 +1047,24 @@ cudaError_t launch_gather_group(const GatherArgs *group_dev, uint32_t n_batches,
         }
     }
     return launch_units(dtype, none, group_dev, n_batches, n_bound, dim, unit_elems(dim, dtype, aligned ? 0 : 1, 0), sharded, st);
+}
+
+// One launch for the stores of a heterogeneous chain; every store: the same 16- or 32-bit
+// dtype, whole 16-byte vectors, this GPU's memory.  rows[z] / row_bytes[z]: expected rows
+// per batch of store z and its row size; 0 rows: no such store.
+cudaError_t launch_gather_stores(const GatherArgs *group_dev, uint32_t stride, uint32_t n_stores, uint32_t n_batches,
+                                 const uint64_t *rows, const uint32_t *row_bytes, int dtype, cudaStream_t st) {
+    int per = 1;
+    for (uint32_t z = 0; z < n_stores; ++z)
+        if (rows[z]) per = std::max(per, gather_grid_blocks(rows[z], row_bytes[z]));
+    per = std::min(per, std::max(1, (kSMs * 64 + (int)n_batches - 1) / (int)n_batches));
+    const dim3 grid(per, n_batches, n_stores);
+    switch (dtype) {
+        case AG_F32: launch_chained(k_gather_stores<AG_F32>, grid, dim3(kThreads), st, group_dev, stride); break;
+        case AG_F16: launch_chained(k_gather_stores<AG_F16>, grid, dim3(kThreads), st, group_dev, stride); break;
+        default: launch_chained(k_gather_stores<AG_BF16>, grid, dim3(kThreads), st, group_dev, stride); break;
+    }
+    return cudaGetLastError();
 }
 
 // ------------------------------------------------ sorted gather, host side --

@@ -68,9 +68,10 @@ struct HParams {
     uint8_t *edge_tag;      // edge type
     uint32_t *edge_rank;    // rank within its edge type
     uint64_t cap_nodes, cap_edges;
-    uint32_t *class_tiles;  // descriptors of the class-rank scans
-    uint32_t class_epoch;   // the node scan runs under class_epoch, the edge scan under class_epoch + 1
-    uint32_t *class_ticket;
+    uint32_t *class_tiles;  // descriptors of the class-rank scans: class_tiles_n for the nodes, as many for the edges
+    uint64_t class_tiles_n;
+    uint32_t class_epoch;   // both scans run under it
+    uint32_t *class_ticket; // [0] nodes, [1] edges
     uint32_t *type_count, *et_count;  // totals per node type / edge type (device)
     uint32_t *type_start;   // first position of each node type's segment in `nodes`
     uint64_t start_draw;    // absolute index of the batch's first RNG draw (0 for a freshly seeded batch)
@@ -101,10 +102,37 @@ __device__ __forceinline__ void in_row(const HeteroMeta &m, uint32_t et, uint32_
     if (b > m.in_edges[et]) deg = 0;
 }
 
+// The chain's parameter blocks, gather arguments and seeds are staged in pinned host
+// memory; the first kernel reads them from there and leaves the device copies the later
+// kernels use (three copy commands fewer; see the homogeneous sampler).
+struct StagedHetero {
+    const HParams *params;     // pinned host, one per batch
+    const GatherArgs *gather;  // pinned host, [node type][group]; null: nothing to gather
+    HParams *params_dev;
+    GatherArgs *gather_dev;
+    uint32_t group, types;
+};
+static_assert(sizeof(HParams) % 8 == 0 && sizeof(GatherArgs) % 8 == 0, "staged blocks are copied as 8-byte words");
+
 // Every kernel's grid has the batch as blockIdx.y; the group's parameter blocks
 // sit in one device array.
-__global__ void k_het_insert_seeds(const HParams *__restrict__ pa) {
-    const HParams &p = pa[blockIdx.y];
+__global__ void k_het_insert_seeds(StagedHetero c) {
+    __shared__ __align__(16) HParams p;
+    constexpr uint32_t kWords = sizeof(HParams) / 8, kGatherWords = sizeof(GatherArgs) / 8;
+    const bool keep = blockIdx.x == 0;
+    const uint32_t words = kWords + ((keep && c.gather) ? c.types * kGatherWords : 0u);
+    for (uint32_t i = threadIdx.x; i < words; i += blockDim.x) {
+        if (i < kWords) {
+            const uint64_t v = ((const volatile uint64_t *)(c.params + blockIdx.y))[i];
+            ((uint64_t *)&p)[i] = v;
+            if (keep) ((uint64_t *)(c.params_dev + blockIdx.y))[i] = v;
+        } else {
+            const uint32_t t = (i - kWords) / kGatherWords, w = (i - kWords) % kGatherWords;
+            const uint64_t at = (uint64_t)t * c.group + blockIdx.y;
+            ((uint64_t *)(c.gather_dev + at))[w] = ((const volatile uint64_t *)(c.gather + at))[w];
+        }
+    }
+    __syncthreads();
     const HeteroMeta &m = *p.meta;
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= p.n_seeds) return;
@@ -125,6 +153,7 @@ k_het_assign(const HParams *__restrict__ pa, uint32_t stage, int has_next) {
     __shared__ uint32_t s_tile;
     __shared__ ScanVal s_warp[kTile / 32];
     __shared__ ScanVal s_prefix;
+    chain_sync();
     const HParams &p = pa[blockIdx.y];
     const HeteroMeta &m = *p.meta;
     BatchState *bs = p.state;
@@ -244,6 +273,7 @@ k_het_assign(const HParams *__restrict__ pa, uint32_t stage, int has_next) {
 // (hetero_sampler.rs:364-422) and emit the edges at consecutive slots.
 __global__ void __launch_bounds__(kPickThreads)
 k_het_pick(const HParams *__restrict__ pa, uint32_t hop) {
+    chain_sync();
     const HParams &p = pa[blockIdx.y];
     const HeteroMeta &m = *p.meta;
     const StageInfo nx = p.state->stage[hop + 1];
@@ -305,23 +335,31 @@ k_het_pick(const HParams *__restrict__ pa, uint32_t hop) {
 
 // Rank of every item among the items with the same tag, in item order, plus the
 // per-tag totals: a 16-channel single-pass scan (same look-back scheme, bounded
-// polls).  Descriptor layout per tile: status, agg[16], incl[16].
+// polls).  Descriptor layout per tile: status, agg[16], incl[16].  Grid z = 0 ranks the
+// nodes, z = 1 the edges, each with its own descriptors and ticket.
+//
+// The look-back reads 32 predecessors at a time: every lane polls one, then half a warp
+// adds up the channels of each.  One predecessor at a time, with the nodes and the edges
+// in launches of their own, the two took 18 us each on 30 K items.
 constexpr int kClassTile = 1024;
 constexpr int kClassThreads = 256;
 constexpr int kDescWords = 1 + 2 * kChan;
 
 __global__ void __launch_bounds__(kClassThreads)
-k_class_rank(const HParams *__restrict__ pa, int edges) {
+k_class_rank(const HParams *__restrict__ pa) {
     __shared__ uint32_t s_tile;
     __shared__ uint32_t s_cnt[kClassThreads / 32][kChan];   // per warp, per channel: count within the tile
     __shared__ uint32_t s_base[kChan];                      // exclusive prefix of the tile per channel
+    chain_sync();
     const HParams &p = pa[blockIdx.y];
+    const bool edges = blockIdx.z != 0;
     const StageInfo fin = p.state->stage[p.meta->num_hops + 1];
     const uint8_t *__restrict__ tags = edges ? p.edge_tag : p.node_tag;
     uint32_t *ranks = edges ? p.edge_rank : p.node_rank;
     uint32_t *totals = edges ? p.et_count : p.type_count;
-    uint32_t *tiles = p.class_tiles, *ticket = p.class_ticket, *err = &p.state->error;
-    const uint32_t epoch = p.class_epoch + (edges ? 1u : 0u);
+    uint32_t *tiles = p.class_tiles + (edges ? p.class_tiles_n * kDescWords : 0), *ticket = p.class_ticket + (edges ? 1 : 0);
+    uint32_t *err = &p.state->error;
+    const uint32_t epoch = p.class_epoch;
     const uint32_t n = edges ? (uint32_t)min((uint64_t)fin.n_edges, p.cap_edges) : (uint32_t)min((uint64_t)fin.n_nodes, p.cap_nodes);
     const uint32_t n_tiles = max(1u, (n + kClassTile - 1) / kClassTile);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -375,29 +413,32 @@ k_class_rank(const HParams *__restrict__ pa, int edges) {
                 if (lane < kChan) desc[1 + lane] = agg;
                 __syncwarp();
                 if (lane == 0) st_release_u32(&desc[0], (epoch << 2) | kTileAgg);
-                // lane c < 16 accumulates channel c while walking back one tile at a time
-                for (int look = (int)tile - 1; look >= 0; --look) {
-                    uint32_t *d = tiles + (uint64_t)look * kDescWords;
-                    uint32_t st = 0, spins = 0;
-                    if (lane == 0) {
+                for (int look = (int)tile - 1;; look -= 32) {
+                    const int t = look - lane;  // this lane polls tile t
+                    bool incl = true, lost = true;  // tiles before the first: an empty prefix
+                    if (t >= 0) {
+                        uint32_t st = 0, spins = 0;
                         for (;;) {
-                            st = ld_acquire_u32(&d[0]);
+                            st = ld_acquire_u32(tiles + (uint64_t)t * kDescWords);
                             if ((st >> 2) == epoch && (st & 3u) != 0) break;
                             if (++spins > kSpinLimit) { atomicOr(err, kErrSpinTimeout); st = (epoch << 2) | kTileIncl; break; }
                             __nanosleep(32);
                         }
+                        incl = (st & 3u) == kTileIncl;
+                        lost = spins > kSpinLimit;
                     }
-                    st = __shfl_sync(0xffffffffu, st, 0);
-                    spins = __shfl_sync(0xffffffffu, spins, 0);
-                    __syncwarp();
-                    const bool incl = (st & 3u) == kTileIncl;
-                    if (lane < kChan && spins <= kSpinLimit) {
-                        // the acquire above was done by lane 0; order this lane's reads behind it
-                        __threadfence();
-                        prefix += incl ? d[1 + kChan + lane] : d[1 + lane];
+                    const uint32_t incls = __ballot_sync(0xffffffffu, incl), losts = __ballot_sync(0xffffffffu, lost);
+                    __threadfence();  // the other lanes' acquires come before this lane's reads
+                    const int first = incls ? __ffs(incls) - 1 : 31;  // nearest inclusive prefix, or the whole window
+                    // lane = half * 16 + channel: tiles half, half + 2, ... of the window
+                    for (int i = lane >> 4; i <= first; i += 2) {
+                        if ((losts >> i) & 1u) continue;
+                        const uint32_t *d = tiles + (uint64_t)(look - i) * kDescWords + 1 + (((incls >> i) & 1u) ? kChan : 0);
+                        prefix += __ldcg(d + (lane & 15));
                     }
-                    if (incl) break;
+                    if (incls) break;
                 }
+                prefix += __shfl_xor_sync(0xffffffffu, prefix, 16);
                 if (lane < kChan) desc[1 + kChan + lane] = prefix + agg;
                 __syncwarp();
                 if (lane == 0) st_release_u32(&desc[0], (epoch << 2) | kTileIncl);
@@ -419,6 +460,7 @@ k_class_rank(const HParams *__restrict__ pa, int edges) {
 // Per-type arrays out of the global ones.  Segments: node type t starts at the
 // sum of the counts of the types before it; edge type likewise.
 __global__ void k_het_scatter(const HParams *__restrict__ pa) {
+    chain_sync();
     const HParams &p = pa[blockIdx.y];
     const HeteroMeta &m = *p.meta;
     BatchState *bs = p.state;
@@ -426,12 +468,18 @@ __global__ void k_het_scatter(const HParams *__restrict__ pa) {
     const uint32_t n_nodes = min((uint64_t)fin.n_nodes, p.cap_nodes);
     const uint32_t n_edges = min((uint64_t)fin.n_edges, p.cap_edges);
     __shared__ uint32_t s_toff[kChan + 1], s_eoff[kChan + 1];
-    if (threadIdx.x == 0) {
-        uint32_t a = 0, b = 0;
-        for (uint32_t t = 0; t < kChan; ++t) { s_toff[t] = a; a += (t < m.nt) ? p.type_count[t] : 0; }
-        for (uint32_t t = 0; t < kChan; ++t) { s_eoff[t] = b; b += (t < m.et) ? p.et_count[t] : 0; }
-        s_toff[kChan] = a; s_eoff[kChan] = b;
-        if (blockIdx.x == 0) for (uint32_t t = 0; t < kChan; ++t) p.type_start[t] = s_toff[t];  // for the gathers
+    if (threadIdx.x < 32) {  // lanes 0 - 15: node types, 16 - 31: edge types
+        const uint32_t t = threadIdx.x & 15, half = threadIdx.x >> 4;
+        const uint32_t c = half ? (t < m.et ? p.et_count[t] : 0) : (t < m.nt ? p.type_count[t] : 0);
+        uint32_t run = c;
+        for (int o = 1; o < kChan; o <<= 1) {
+            const uint32_t up = __shfl_up_sync(0xffffffffu, run, o, kChan);
+            if ((int)t >= o) run += up;
+        }
+        uint32_t *off = half ? s_eoff : s_toff;
+        off[t] = run - c;
+        if (t == kChan - 1) off[kChan] = run;
+        if (!half && blockIdx.x == 0) p.type_start[t] = run - c;  // for the gathers
     }
     __syncthreads();
     const uint64_t tid = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x, stride = (uint64_t)gridDim.x * blockDim.x;
@@ -535,19 +583,21 @@ struct ag_hetero_sampler {
     // scratch, each array x group
     uint64_t *table = nullptr;
     uint32_t *slot_of_seed = nullptr, *slot_of_edge = nullptr, *node_key = nullptr, *node_rank = nullptr,
-             *edge_exp = nullptr, *edge_rank = nullptr, *class_tiles = nullptr, *class_misc = nullptr, *seeds_dev = nullptr;
+             *edge_exp = nullptr, *edge_rank = nullptr, *class_tiles = nullptr, *class_misc = nullptr;
     uint8_t *node_tag = nullptr, *edge_tag = nullptr;
     FrontierEntry *frontier = nullptr;
     TileDesc *tiles = nullptr;
     BatchState *state = nullptr;
     HParams *params_dev = nullptr, *params_host = nullptr;
     GatherArgs *gather_dev = nullptr, *gather_host = nullptr;  // [node type][batch]
-    ag_hetero_counts *counts_dev = nullptr, *counts_host = nullptr;
+    ag_hetero_counts *counts_host = nullptr;
     uint32_t *seeds_pinned = nullptr;
     cudaEvent_t done = nullptr;
+    // what the last chain's largest batch produced, with headroom (0: nothing yet)
+    uint64_t est_nodes = 0, est_edges = 0, est_type[kMaxNT] = {0};
 };
 
-constexpr int kMiscWords = 3 * kChan + 2;  // type_count, et_count, type_start, ticket (per batch)
+constexpr int kMiscWords = 3 * kChan + 2;  // type_count, et_count, type_start, two tickets (per batch)
 
 extern "C" void ag_hetero_free(ag_hetero_graph *h) {
     if (!h) return;
@@ -685,11 +735,11 @@ void het_bounds(const ag_hetero_sampler *s, uint64_t n_seeds, uint64_t *nodes, u
 
 void het_free_scratch(ag_hetero_sampler *s) {
     void *ptrs[] = {s->table, s->slot_of_seed, s->slot_of_edge, s->node_key, s->node_rank, s->edge_exp, s->edge_rank,
-                    s->class_tiles, s->seeds_dev, s->node_tag, s->edge_tag, s->frontier, s->tiles};
+                    s->class_tiles, s->node_tag, s->edge_tag, s->frontier, s->tiles};
     for (void *p : ptrs) workspace_free(p);
     workspace_free(s->seeds_pinned);
     s->table = nullptr; s->slot_of_seed = s->slot_of_edge = s->node_key = s->node_rank = s->edge_exp = s->edge_rank = nullptr;
-    s->class_tiles = s->seeds_dev = nullptr; s->node_tag = s->edge_tag = nullptr; s->frontier = nullptr; s->tiles = nullptr;
+    s->class_tiles = nullptr; s->node_tag = s->edge_tag = nullptr; s->frontier = nullptr; s->tiles = nullptr;
     s->seeds_pinned = nullptr;
 }
 
@@ -726,8 +776,7 @@ int32_t het_ensure(ag_hetero_sampler *s, uint64_t n_seeds) {
     s->n_tiles = std::max<uint64_t>(std::max(cap, s->max_hop_edges) / kTile + 2, 2);
     AG_CUDA(workspace_alloc(&s->tiles, G * s->n_tiles * sizeof(TileDesc)));
     s->class_tiles_n = std::max(cn, ce) / kClassTile + 2;
-    AG_CUDA(workspace_alloc(&s->class_tiles, G * s->class_tiles_n * kDescWords * 4));
-    AG_CUDA(workspace_alloc(&s->seeds_dev, G * cap * 4));
+    AG_CUDA(workspace_alloc(&s->class_tiles, G * 2 * s->class_tiles_n * kDescWords * 4));
     AG_CUDA(workspace_alloc_host(&s->seeds_pinned, G * cap * 4));
     s->cap_seeds = cap; s->epoch = 0; s->class_epoch = 0; s->dirty = true;
     return AG_OK;
@@ -740,7 +789,7 @@ extern "C" void ag_hetero_sampler_free(ag_hetero_sampler *s) {
     DeviceGuard guard(s->device);
     if (s->in_flight && s->done) cudaEventSynchronize(s->done);
     het_free_scratch(s);
-    void *ptrs[] = {s->meta_dev, s->state, s->counts_dev, s->class_misc, s->params_dev, s->gather_dev, s->params_host,
+    void *ptrs[] = {s->meta_dev, s->state, s->class_misc, s->params_dev, s->gather_dev, s->params_host,
                     s->gather_host, s->counts_host};
     for (void *p : ptrs) workspace_free(p);
     if (s->done) cudaEventDestroy(s->done);
@@ -784,7 +833,6 @@ extern "C" int32_t ag_hetero_sampler_create_group(const ag_hetero_graph *h, cons
         if (workspace_alloc(&s->meta_dev, sizeof(HeteroMeta)) != cudaSuccess ||
             cudaMemcpy(s->meta_dev, &m, sizeof(HeteroMeta), cudaMemcpyHostToDevice) != cudaSuccess ||
             workspace_alloc(&s->state, G * sizeof(BatchState)) != cudaSuccess ||
-            workspace_alloc(&s->counts_dev, G * sizeof(ag_hetero_counts)) != cudaSuccess ||
             workspace_alloc(&s->class_misc, G * kMiscWords * 4) != cudaSuccess ||
             workspace_alloc(&s->params_dev, G * sizeof(HParams)) != cudaSuccess ||
             workspace_alloc(&s->gather_dev, G * kMaxNT * sizeof(GatherArgs)) != cudaSuccess ||
@@ -896,14 +944,14 @@ int32_t hetero_group_into(ag_hetero_sampler *s, uint32_t n_batches, uint32_t see
         AG_CUDA(cudaMemsetAsync(s->state, 0, G * sizeof(BatchState), st));
         AG_CUDA(cudaMemsetAsync(s->class_misc, 0, G * kMiscWords * 4, st));
         AG_CUDA(cudaMemsetAsync(s->tiles, 0, G * s->n_tiles * sizeof(TileDesc), st));
-        AG_CUDA(cudaMemsetAsync(s->class_tiles, 0, G * s->class_tiles_n * kDescWords * 4, st));
+        AG_CUDA(cudaMemsetAsync(s->class_tiles, 0, G * 2 * s->class_tiles_n * kDescWords * 4, st));
         s->epoch = s->class_epoch = 0;
         s->dirty = false;
     }
     const uint32_t H = m.num_hops;
     if (s->epoch + (H + 2) > 0x3FFFFF00u) { AG_CUDA(cudaMemsetAsync(s->tiles, 0, G * s->n_tiles * sizeof(TileDesc), st)); s->epoch = 0; }
     if (s->class_epoch + 4 > 0x3FFFFF00u) {
-        AG_CUDA(cudaMemsetAsync(s->class_tiles, 0, G * s->class_tiles_n * kDescWords * 4, st));
+        AG_CUDA(cudaMemsetAsync(s->class_tiles, 0, G * 2 * s->class_tiles_n * kDescWords * 4, st));
         s->class_epoch = 0;
     }
     uint32_t log2cap = 0;
@@ -920,7 +968,7 @@ int32_t hetero_group_into(ag_hetero_sampler *s, uint32_t n_batches, uint32_t see
         p.state = s->state + b; p.tiles = s->tiles + b * s->n_tiles; p.epoch_base = s->epoch + 1;
         p.n_seeds = n; p.seed_type = seed_type;
         if (n) memcpy(s->seeds_pinned + b * s->cap_seeds, seeds[b], (size_t)n * 4);
-        p.seeds = s->seeds_dev + b * s->cap_seeds;
+        p.seeds = s->seeds_pinned + b * s->cap_seeds;  // read by the chain's first kernel
         p.seed = batch_seeds ? batch_seeds[b] : s->seed;
         p.start_draw = batch_seeds ? 0ull : s->stream_pos;
         p.slot_of_seed = s->slot_of_seed + b * s->cap_seeds; p.slot_of_edge = s->slot_of_edge + b * ce;
@@ -929,13 +977,14 @@ int32_t hetero_group_into(ag_hetero_sampler *s, uint32_t n_batches, uint32_t see
         p.edge_exp = s->edge_exp + b * ce; p.edge_tag = s->edge_tag + b * ce; p.edge_rank = s->edge_rank + b * ce;
         p.cap_nodes = std::min<uint64_t>(B.cap_nodes, cn);
         p.cap_edges = std::min<uint64_t>(B.cap_edges, ce);
-        p.class_tiles = s->class_tiles + b * s->class_tiles_n * kDescWords;
+        p.class_tiles = s->class_tiles + b * 2 * s->class_tiles_n * kDescWords;
+        p.class_tiles_n = s->class_tiles_n;
         p.class_epoch = s->class_epoch + 1;
         uint32_t *misc = s->class_misc + b * kMiscWords;
         p.type_count = misc; p.et_count = misc + kChan; p.type_start = misc + 2 * kChan; p.class_ticket = misc + 3 * kChan;
         p.nodes = B.nodes; p.edge_src_local = B.edge_src_local; p.edge_dst_local = B.edge_dst_local;
         p.seed_indices = B.seed_indices; p.n_id = B.n_id; p.edge_index_local = B.edge_index_local;
-        p.seed_index = B.seed_index; p.counts = s->counts_dev + b;
+        p.seed_index = B.seed_index; p.counts = s->counts_host + b;  // pinned: a posted write
         s->params_host[b] = p;
         for (uint32_t t = 0; t < m.nt; ++t) {
             GatherArgs ga{};
@@ -953,24 +1002,25 @@ int32_t hetero_group_into(ag_hetero_sampler *s, uint32_t n_batches, uint32_t see
     }
     s->pending_pos = (batch_seeds == nullptr);
     s->epoch += H + 2; s->class_epoch += 2; s->gen += 1; s->last_batches = n_batches;
-    AG_CUDA(cudaMemcpyAsync(s->seeds_dev, s->seeds_pinned, (uint64_t)n_batches * s->cap_seeds * 4, cudaMemcpyHostToDevice, st));
-    AG_CUDA(cudaMemcpyAsync(s->params_dev, s->params_host, n_batches * sizeof(HParams), cudaMemcpyHostToDevice, st));
-    if (want_x) AG_CUDA(cudaMemcpyAsync(s->gather_dev, s->gather_host, G * kMaxNT * sizeof(GatherArgs), cudaMemcpyHostToDevice, st));
-
     const HParams *pa = s->params_dev;
     const uint32_t nmax = (uint32_t)max_n, nb = n_batches;
     auto tiles_for = [&](uint64_t items) {
         return (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>((items + kTile - 1) / kTile, std::max<uint64_t>(1, (uint64_t)kSMs * 8 / nb)));
     };
-    if (nmax) k_het_insert_seeds<<<dim3((nmax + 255) / 256, nb), 256, 0, st>>>(pa);
+    // Grids follow what the last chain produced (with headroom) where the bounds are far above it.
+    const uint64_t e_nodes = s->est_nodes ? std::min(s->max_nodes, s->est_nodes) : s->max_nodes;
+    const uint64_t e_edges = s->est_nodes ? std::min(s->max_edges, s->est_edges) : s->max_edges;
+    const StagedHetero staged{s->params_host, want_x ? s->gather_host : nullptr, s->params_dev, s->gather_dev, s->group, m.nt};
+    k_het_insert_seeds<<<dim3(std::max(1u, (nmax + 255) / 256), nb), 256, 0, st>>>(staged);
     uint64_t f_bound = nmax, items = nmax;
     for (uint32_t stage = 0; stage <= H; ++stage) {
         const bool has_next = stage < H;
-        k_het_assign<<<dim3(tiles_for(items), nb), kTile, 0, st>>>(pa, stage, has_next ? 1 : 0);
+        launch_chained(k_het_assign, dim3(tiles_for(stage ? std::min(items, e_edges) : items), nb), dim3(kTile), st, pa, stage, has_next ? 1 : 0);
         if (has_next) {
-            const uint32_t blocks = (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>((f_bound * 32 + kPickThreads - 1) / kPickThreads,
+            const uint64_t f = std::min(f_bound, std::max<uint64_t>(e_nodes, 1));
+            const uint32_t blocks = (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>((f * 32 + kPickThreads - 1) / kPickThreads,
                                                                                       std::max<uint64_t>(1, (uint64_t)kSMs * 16 / nb)));
-            k_het_pick<<<dim3(blocks, nb), kPickThreads, 0, st>>>(pa, stage);
+            launch_chained(k_het_pick, dim3(blocks, nb), dim3(kPickThreads), st, pa, stage);
             items = f_bound * het_per_node(m, stage);
             f_bound = std::min<uint64_t>(items, s->max_nodes);
         }
@@ -978,28 +1028,42 @@ int32_t hetero_group_into(ag_hetero_sampler *s, uint32_t n_batches, uint32_t see
     auto ctiles_for = [&](uint64_t n) {
         return (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>((n + kClassTile - 1) / kClassTile, std::max<uint64_t>(1, (uint64_t)kSMs * 4 / nb)));
     };
-    k_class_rank<<<dim3(ctiles_for(s->max_nodes), nb), kClassThreads, 0, st>>>(pa, 0);
-    k_class_rank<<<dim3(ctiles_for(s->max_edges), nb), kClassThreads, 0, st>>>(pa, 1);
+    launch_chained(k_class_rank, dim3(ctiles_for(std::max(e_nodes, e_edges)), nb, 2), dim3(kClassThreads), st, pa);
     {
-        const uint64_t work = std::max<uint64_t>(std::max(s->max_edges, s->max_nodes), std::max<uint64_t>(nmax, 1));
+        const uint64_t work = std::max<uint64_t>(std::max(e_edges, e_nodes), std::max<uint64_t>(nmax, 1));
         const uint32_t fx = (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>((work + 255) / 256, std::max<uint64_t>(1, (uint64_t)kSMs * 8 / nb)));
-        k_het_scatter<<<dim3(fx, nb), 256, 0, st>>>(pa);
+        launch_chained(k_het_scatter, dim3(fx, nb), dim3(256), st, pa);
     }
     AG_CUDA(cudaGetLastError());
     if (want_x) {
+        // One launch for all types where their stores are of one kind (latency: four launches
+        // of 5 - 9 us one after the other otherwise), else a launch per type.
+        bool any[kMaxNT] = {}, aligned[kMaxNT] = {}, together = true;
+        uint64_t rows[kMaxNT] = {};
+        uint32_t row_bytes[kMaxNT] = {};
+        int dtype = -1;
         for (uint32_t t = 0; t < m.nt; ++t) {
             if (!feats[t]) continue;
-            bool any = false, aligned = ((uintptr_t)feats[t]->payload % 16) == 0;
+            aligned[t] = ((uintptr_t)feats[t]->payload % 16) == 0;
             for (uint32_t b = 0; b < nb; ++b)
-                if (bufs[b].x[t]) { any = true; aligned = aligned && ((uintptr_t)bufs[b].x[t] % 16) == 0; }
-            if (!any) continue;
+                if (bufs[b].x[t]) { any[t] = true; aligned[t] = aligned[t] && ((uintptr_t)bufs[b].x[t] % 16) == 0; }
+            if (!any[t]) continue;
             const uint64_t bound = std::min<uint64_t>(s->max_nodes, m.type_nodes[t]);
-            AG_CUDA(launch_gather_group(s->gather_dev + (size_t)t * G, nb, (uint32_t)(feats[t]->dim * elem_size(feats[t]->dtype)),
-                                        (uint32_t)feats[t]->dim, std::max<uint64_t>(bound / 4, 1), aligned, feats[t]->dtype,
-                                        feats[t]->shards != nullptr, st));
+            rows[t] = std::max<uint64_t>(s->est_nodes ? std::min(bound, s->est_type[t]) : bound / 4, 1);
+            row_bytes[t] = (uint32_t)(feats[t]->dim * elem_size(feats[t]->dtype));
+            together = together && aligned[t] && row_bytes[t] % 16 == 0 && !feats[t]->shards && feats[t]->dtype != AG_I8 &&
+                       (dtype < 0 || dtype == feats[t]->dtype);
+            dtype = feats[t]->dtype;
+        }
+        if (together) {
+            AG_CUDA(launch_gather_stores(s->gather_dev, (uint32_t)G, m.nt, nb, rows, row_bytes, dtype, st));
+        } else {
+            for (uint32_t t = 0; t < m.nt; ++t)
+                if (any[t])
+                    AG_CUDA(launch_gather_group(s->gather_dev + (size_t)t * G, nb, row_bytes[t], (uint32_t)feats[t]->dim, rows[t],
+                                                aligned[t], feats[t]->dtype, feats[t]->shards != nullptr, st));
         }
     }
-    AG_CUDA(cudaMemcpyAsync(s->counts_host, s->counts_dev, nb * sizeof(ag_hetero_counts), cudaMemcpyDeviceToHost, st));
     AG_CUDA(cudaEventRecord(s->done, st));
     s->in_flight = true;
     return AG_OK;
@@ -1015,6 +1079,16 @@ extern "C" int32_t ag_hetero_sample_group_wait(ag_hetero_sampler *s, ag_hetero_c
     s->in_flight = false;
     if (e != cudaSuccess) { s->dirty = true; s->pending_pos = false; return fail(AG_ERR_CUDA, "hetero sampling kernels failed: %s", cudaGetErrorString(e)); }
     het_account(s);
+    uint64_t mx_nodes = 0, mx_edges = 0, mx_type[kMaxNT] = {0};
+    for (uint32_t b = 0; b < s->last_batches; ++b) {
+        const ag_hetero_counts &c = s->counts_host[b];
+        mx_nodes = std::max<uint64_t>(mx_nodes, c.total_nodes);
+        mx_edges = std::max<uint64_t>(mx_edges, c.total_edges);
+        for (uint32_t t = 0; t < s->meta.nt; ++t) mx_type[t] = std::max<uint64_t>(mx_type[t], c.nodes[t]);
+    }
+    s->est_nodes = mx_nodes + mx_nodes / 4 + 256;
+    s->est_edges = mx_edges + mx_edges / 4 + 512;
+    for (uint32_t t = 0; t < s->meta.nt; ++t) s->est_type[t] = mx_type[t] + mx_type[t] / 4 + 64;
     int32_t first = AG_OK;
     for (uint32_t b = 0; b < s->last_batches; ++b) {
         const ag_hetero_counts c = s->counts_host[b];

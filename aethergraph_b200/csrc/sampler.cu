@@ -139,18 +139,6 @@ __device__ __forceinline__ void row_demand(int mode, uint64_t deg, uint32_t k, u
 }
 
 // ------------------------------------------------------------ seed insert --
-// Programmatic dependent launch: the kernels of a chain are launched with
-// cudaLaunchAttributeProgrammaticStreamSerialization, so the next kernel's blocks
-// are scheduled as this one's blocks exit, without waiting for the grid's
-// completion to be reported first.  Every kernel starts by waiting for its
-// predecessor's results (griddepcontrol.wait; a no-op for a plain launch).  The
-// kernels do NOT release their successor early (no griddepcontrol.launch_dependents
-// before the work): measured, successor blocks parked in SM slots take those slots
-// from the gather of a neighbouring chain and the whole pipeline gets slower.
-__device__ __forceinline__ void chain_sync() {
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-}
-
 // The parameter blocks, gather arguments and seeds of a chain are staged in pinned host
 // memory and the chain's first kernel reads them from there, leaving the device copies
 // the later kernels use.  A copy command each for the three costs more than the kernel
@@ -1124,18 +1112,6 @@ k_pick_hub_slices(const SampleParams *__restrict__ pa, uint32_t hop, uint32_t k)
         if (!mine) continue;
         if ((uint32_t)lane < k) emit_edge(p, hop, p.state->stage[hop + 1].n_edges, fe, lane, fe.off + best_pos);
     }
-}
-
-// Launches `kern` as a programmatic dependent of the previous kernel on the stream.
-template <typename... KArgs, typename... Args>
-void launch_chained(void (*kern)(KArgs...), dim3 grid, dim3 block, cudaStream_t st, Args... args) {
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = 0; cfg.stream = st;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr; cfg.numAttrs = 1;
-    cudaLaunchKernelEx(&cfg, kern, KArgs(args)...);
 }
 
 uint64_t next_pow2(uint64_t v) {
