@@ -145,6 +145,15 @@ __device__ __forceinline__ void st_stream_u32(void *p, uint32_t v) {
 }
 
 // ------------------------------------------------------- launch chains --
+// What a chain's kernels need (parameter blocks, gather arguments, seeds) is staged as one
+// block of 8-byte words in pinned host memory.  A small block rides in the first kernel's own
+// parameters, and that kernel leaves the device copies the later ones use; a larger one is
+// copied first.  (Three copy commands: 1.7 us each on the device with 3 - 4 us between them.
+// The first kernel reading the pinned block itself: 9 us for 1 KB, 16 - 23 for 4 KB and
+// 24 - 38 for 16 KB on this host, page by page through the I/O address translation.)
+template <int BYTES> struct PackedWords { uint64_t w[BYTES / 8]; };
+constexpr int kPackedSmall = 4032, kPackedMedium = 8128, kPackedLarge = 16320;
+
 // Programmatic dependent launch: the kernels of a chain are launched with
 // cudaLaunchAttributeProgrammaticStreamSerialization, so the next kernel's blocks
 // are scheduled as this one's blocks exit, without waiting for the grid's

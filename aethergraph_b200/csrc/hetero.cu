@@ -19,6 +19,7 @@
 
 #include <algorithm>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "common.cuh"
@@ -102,41 +103,20 @@ __device__ __forceinline__ void in_row(const HeteroMeta &m, uint32_t et, uint32_
     if (b > m.in_edges[et]) deg = 0;
 }
 
-// The chain's parameter blocks, gather arguments and seeds are staged in pinned host
-// memory; the first kernel reads them from there and leaves the device copies the later
-// kernels use (three copy commands fewer; see the homogeneous sampler).
-struct StagedHetero {
-    const HParams *params;     // pinned host, one per batch
-    const GatherArgs *gather;  // pinned host, [node type][group]; null: nothing to gather
-    HParams *params_dev;
-    GatherArgs *gather_dev;
-    uint32_t group, types;
+// Where the parts of a chain's staged block are (see PackedWords): parameter blocks, gather
+// arguments [node type][batch] (if any), seeds.
+struct HStageLayout {
+    HParams *params_dev;      // the device copies
+    GatherArgs *gather_dev;   // null: nothing to gather
+    uint32_t types, seeds_at, seed_stride;
 };
-static_assert(sizeof(HParams) % 8 == 0 && sizeof(GatherArgs) % 8 == 0, "staged blocks are copied as 8-byte words");
+static_assert(sizeof(HParams) % 8 == 0 && sizeof(GatherArgs) % 8 == 0, "staged blocks are made of 8-byte words");
 
-// Every kernel's grid has the batch as blockIdx.y; the group's parameter blocks
-// sit in one device array.
-__global__ void k_het_insert_seeds(StagedHetero c) {
-    __shared__ __align__(16) HParams p;
-    constexpr uint32_t kWords = sizeof(HParams) / 8, kGatherWords = sizeof(GatherArgs) / 8;
-    const bool keep = blockIdx.x == 0;
-    const uint32_t words = kWords + ((keep && c.gather) ? c.types * kGatherWords : 0u);
-    for (uint32_t i = threadIdx.x; i < words; i += blockDim.x) {
-        if (i < kWords) {
-            const uint64_t v = ((const volatile uint64_t *)(c.params + blockIdx.y))[i];
-            ((uint64_t *)&p)[i] = v;
-            if (keep) ((uint64_t *)(c.params_dev + blockIdx.y))[i] = v;
-        } else {
-            const uint32_t t = (i - kWords) / kGatherWords, w = (i - kWords) % kGatherWords;
-            const uint64_t at = (uint64_t)t * c.group + blockIdx.y;
-            ((uint64_t *)(c.gather_dev + at))[w] = ((const volatile uint64_t *)(c.gather + at))[w];
-        }
-    }
-    __syncthreads();
+__device__ __forceinline__ void het_insert_seed(const HParams &p, const uint32_t *seeds) {
     const HeteroMeta &m = *p.meta;
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= p.n_seeds) return;
-    const uint32_t id = p.seeds[i];
+    const uint32_t id = seeds[i];
     if ((uint64_t)id >= m.type_nodes[p.seed_type]) {
         atomicOr(&p.state->error, kErrBadSeed);
         p.slot_of_seed[i] = 0xFFFFFFFFu;
@@ -144,6 +124,32 @@ __global__ void k_het_insert_seeds(StagedHetero c) {
     }
     p.slot_of_seed[i] = table_insert_min(p.table, m.type_base[p.seed_type] + id, enc_pending(p.table.gen, 0, i),
                                          &p.state->error);
+}
+
+// Every kernel's grid has the batch as blockIdx.y; the group's parameter blocks
+// sit in one device array.
+__global__ void k_het_insert_seeds(const HParams *__restrict__ pa) { het_insert_seed(pa[blockIdx.y], pa[blockIdx.y].seeds); }
+
+// The same with the staged block in the kernel's parameters; the batch's first block
+// leaves the device copies.
+template <int BYTES>
+__global__ void k_het_insert_seeds_packed(const __grid_constant__ PackedWords<BYTES> c, const HStageLayout at) {
+    __shared__ __align__(16) HParams p;
+    constexpr uint32_t kWords = sizeof(HParams) / 8, kGatherWords = sizeof(GatherArgs) / 8;
+    const bool keep = blockIdx.x == 0;
+    const uint32_t words = kWords + ((keep && at.gather_dev) ? at.types * kGatherWords : 0u);
+    for (uint32_t i = threadIdx.x; i < words; i += blockDim.x) {
+        if (i < kWords) {
+            const uint64_t v = c.w[blockIdx.y * kWords + i];
+            ((uint64_t *)&p)[i] = v;
+            if (keep) ((uint64_t *)(at.params_dev + blockIdx.y))[i] = v;
+        } else {
+            const uint32_t t = (i - kWords) / kGatherWords, w = (i - kWords) % kGatherWords, b = t * gridDim.y + blockIdx.y;
+            ((uint64_t *)(at.gather_dev + b))[w] = c.w[gridDim.y * kWords + b * kGatherWords + w];
+        }
+    }
+    __syncthreads();
+    het_insert_seed(p, (const uint32_t *)(c.w + at.seeds_at) + blockIdx.y * at.seed_stride);
 }
 
 // Same single-pass scan as the homogeneous assign; the demand of a new node is
@@ -588,10 +594,8 @@ struct ag_hetero_sampler {
     FrontierEntry *frontier = nullptr;
     TileDesc *tiles = nullptr;
     BatchState *state = nullptr;
-    HParams *params_dev = nullptr, *params_host = nullptr;
-    GatherArgs *gather_dev = nullptr, *gather_host = nullptr;  // [node type][batch]
+    uint8_t *stage_dev = nullptr, *stage_host = nullptr;  // see HStageLayout
     ag_hetero_counts *counts_host = nullptr;
-    uint32_t *seeds_pinned = nullptr;
     cudaEvent_t done = nullptr;
     // what the last chain's largest batch produced, with headroom (0: nothing yet)
     uint64_t est_nodes = 0, est_edges = 0, est_type[kMaxNT] = {0};
@@ -737,10 +741,10 @@ void het_free_scratch(ag_hetero_sampler *s) {
     void *ptrs[] = {s->table, s->slot_of_seed, s->slot_of_edge, s->node_key, s->node_rank, s->edge_exp, s->edge_rank,
                     s->class_tiles, s->node_tag, s->edge_tag, s->frontier, s->tiles};
     for (void *p : ptrs) workspace_free(p);
-    workspace_free(s->seeds_pinned);
+    workspace_free(s->stage_dev); workspace_free(s->stage_host);
     s->table = nullptr; s->slot_of_seed = s->slot_of_edge = s->node_key = s->node_rank = s->edge_exp = s->edge_rank = nullptr;
     s->class_tiles = nullptr; s->node_tag = s->edge_tag = nullptr; s->frontier = nullptr; s->tiles = nullptr;
-    s->seeds_pinned = nullptr;
+    s->stage_dev = s->stage_host = nullptr;
 }
 
 // A finished continuing batch moves the handle's stream on by the draws it consumed.
@@ -777,7 +781,9 @@ int32_t het_ensure(ag_hetero_sampler *s, uint64_t n_seeds) {
     AG_CUDA(workspace_alloc(&s->tiles, G * s->n_tiles * sizeof(TileDesc)));
     s->class_tiles_n = std::max(cn, ce) / kClassTile + 2;
     AG_CUDA(workspace_alloc(&s->class_tiles, G * 2 * s->class_tiles_n * kDescWords * 4));
-    AG_CUDA(workspace_alloc_host(&s->seeds_pinned, G * cap * 4));
+    const uint64_t stage = G * (sizeof(HParams) + kMaxNT * sizeof(GatherArgs) + (cap + 1) / 2 * 8);
+    AG_CUDA(workspace_alloc_host(&s->stage_host, stage));
+    AG_CUDA(workspace_alloc(&s->stage_dev, stage));
     s->cap_seeds = cap; s->epoch = 0; s->class_epoch = 0; s->dirty = true;
     return AG_OK;
 }
@@ -789,8 +795,7 @@ extern "C" void ag_hetero_sampler_free(ag_hetero_sampler *s) {
     DeviceGuard guard(s->device);
     if (s->in_flight && s->done) cudaEventSynchronize(s->done);
     het_free_scratch(s);
-    void *ptrs[] = {s->meta_dev, s->state, s->class_misc, s->params_dev, s->gather_dev, s->params_host,
-                    s->gather_host, s->counts_host};
+    void *ptrs[] = {s->meta_dev, s->state, s->class_misc, s->counts_host};
     for (void *p : ptrs) workspace_free(p);
     if (s->done) cudaEventDestroy(s->done);
     delete s;
@@ -834,10 +839,6 @@ extern "C" int32_t ag_hetero_sampler_create_group(const ag_hetero_graph *h, cons
             cudaMemcpy(s->meta_dev, &m, sizeof(HeteroMeta), cudaMemcpyHostToDevice) != cudaSuccess ||
             workspace_alloc(&s->state, G * sizeof(BatchState)) != cudaSuccess ||
             workspace_alloc(&s->class_misc, G * kMiscWords * 4) != cudaSuccess ||
-            workspace_alloc(&s->params_dev, G * sizeof(HParams)) != cudaSuccess ||
-            workspace_alloc(&s->gather_dev, G * kMaxNT * sizeof(GatherArgs)) != cudaSuccess ||
-            workspace_alloc_host(&s->params_host, G * sizeof(HParams)) != cudaSuccess ||
-            workspace_alloc_host(&s->gather_host, G * kMaxNT * sizeof(GatherArgs)) != cudaSuccess ||
             workspace_alloc_host(&s->counts_host, G * sizeof(ag_hetero_counts)) != cudaSuccess ||
             cudaEventCreateWithFlags(&s->done, cudaEventDisableTiming) != cudaSuccess) {
             st = fail(AG_ERR_CUDA, "hetero sampler allocation failed: %s", cudaGetErrorString(cudaGetLastError()));
@@ -959,6 +960,15 @@ int32_t hetero_group_into(ag_hetero_sampler *s, uint32_t n_batches, uint32_t see
     const uint64_t cn = std::max<uint64_t>(s->max_nodes, 1), ce = std::max<uint64_t>(s->max_edges, 1);
     const uint64_t fcap = std::max<uint64_t>(s->max_frontier, 1);
     bool want_x = false;
+    for (uint32_t b = 0; b < n_batches; ++b)
+        for (uint32_t t = 0; t < m.nt; ++t) want_x = want_x || (feats && feats[t] && bufs[b].x[t]);
+    const uint32_t nmax = (uint32_t)max_n, nb = n_batches, seed_stride = (nmax + 1) & ~1u;
+    const uint64_t gather_at = nb * sizeof(HParams), seeds_at = gather_at + (want_x ? (uint64_t)m.nt * nb * sizeof(GatherArgs) : 0);
+    const uint64_t stage_bytes = seeds_at + (uint64_t)nb * seed_stride * 4;
+    HParams *params_host = (HParams *)s->stage_host;
+    GatherArgs *gather_host = (GatherArgs *)(s->stage_host + gather_at), *gather_dev = (GatherArgs *)(s->stage_dev + gather_at);
+    uint32_t *seeds_host = (uint32_t *)(s->stage_host + seeds_at);
+    const uint32_t *seeds_dev = (const uint32_t *)(s->stage_dev + seeds_at);
     for (uint32_t b = 0; b < n_batches; ++b) {
         const ag_hetero_buffers &B = bufs[b];
         const uint32_t n = (uint32_t)n_seeds[b];
@@ -967,8 +977,8 @@ int32_t hetero_group_into(ag_hetero_sampler *s, uint32_t n_batches, uint32_t see
         p.table = DedupTable{s->table + b * s->table_cap, (uint32_t)(s->table_cap - 1), 32u - log2cap, s->gen};
         p.state = s->state + b; p.tiles = s->tiles + b * s->n_tiles; p.epoch_base = s->epoch + 1;
         p.n_seeds = n; p.seed_type = seed_type;
-        if (n) memcpy(s->seeds_pinned + b * s->cap_seeds, seeds[b], (size_t)n * 4);
-        p.seeds = s->seeds_pinned + b * s->cap_seeds;  // read by the chain's first kernel
+        if (n) memcpy(seeds_host + (uint64_t)b * seed_stride, seeds[b], (size_t)n * 4);
+        p.seeds = seeds_dev + (uint64_t)b * seed_stride;
         p.seed = batch_seeds ? batch_seeds[b] : s->seed;
         p.start_draw = batch_seeds ? 0ull : s->stream_pos;
         p.slot_of_seed = s->slot_of_seed + b * s->cap_seeds; p.slot_of_edge = s->slot_of_edge + b * ce;
@@ -985,7 +995,7 @@ int32_t hetero_group_into(ag_hetero_sampler *s, uint32_t n_batches, uint32_t see
         p.nodes = B.nodes; p.edge_src_local = B.edge_src_local; p.edge_dst_local = B.edge_dst_local;
         p.seed_indices = B.seed_indices; p.n_id = B.n_id; p.edge_index_local = B.edge_index_local;
         p.seed_index = B.seed_index; p.counts = s->counts_host + b;  // pinned: a posted write
-        s->params_host[b] = p;
+        params_host[b] = p;
         for (uint32_t t = 0; t < m.nt; ++t) {
             GatherArgs ga{};
             if (feats && feats[t] && B.x[t]) {
@@ -995,23 +1005,34 @@ int32_t hetero_group_into(ag_hetero_sampler *s, uint32_t n_batches, uint32_t see
                 if (B.cap_x[t]) ga.n = std::min<uint64_t>(ga.n, B.cap_x[t]);
                 ga.n_dev = p.type_count + t;
                 ga.out = B.x[t];
-                want_x = true;
             }
-            s->gather_host[(size_t)t * G + b] = ga;
+            if (want_x) gather_host[(size_t)t * nb + b] = ga;
         }
     }
     s->pending_pos = (batch_seeds == nullptr);
     s->epoch += H + 2; s->class_epoch += 2; s->gen += 1; s->last_batches = n_batches;
-    const HParams *pa = s->params_dev;
-    const uint32_t nmax = (uint32_t)max_n, nb = n_batches;
+    const HParams *pa = (const HParams *)s->stage_dev;
     auto tiles_for = [&](uint64_t items) {
         return (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>((items + kTile - 1) / kTile, std::max<uint64_t>(1, (uint64_t)kSMs * 8 / nb)));
     };
     // Grids follow what the last chain produced (with headroom) where the bounds are far above it.
     const uint64_t e_nodes = s->est_nodes ? std::min(s->max_nodes, s->est_nodes) : s->max_nodes;
     const uint64_t e_edges = s->est_nodes ? std::min(s->max_edges, s->est_edges) : s->max_edges;
-    const StagedHetero staged{s->params_host, want_x ? s->gather_host : nullptr, s->params_dev, s->gather_dev, s->group, m.nt};
-    k_het_insert_seeds<<<dim3(std::max(1u, (nmax + 255) / 256), nb), 256, 0, st>>>(staged);
+    const dim3 seed_grid(std::max(1u, (nmax + 255) / 256), nb);
+    const HStageLayout at{(HParams *)s->stage_dev, want_x ? gather_dev : nullptr, m.nt, (uint32_t)(seeds_at / 8), seed_stride};
+    auto launch_packed = [&](auto words) {
+        constexpr int kBytes = decltype(words)::value;
+        PackedWords<kBytes> c;
+        memcpy(&c, s->stage_host, stage_bytes);
+        k_het_insert_seeds_packed<kBytes><<<seed_grid, 256, 0, st>>>(c, at);
+    };
+    if (stage_bytes <= kPackedSmall) launch_packed(std::integral_constant<int, kPackedSmall>{});
+    else if (stage_bytes <= kPackedMedium) launch_packed(std::integral_constant<int, kPackedMedium>{});
+    else if (stage_bytes <= kPackedLarge) launch_packed(std::integral_constant<int, kPackedLarge>{});
+    else {
+        AG_CUDA(cudaMemcpyAsync(s->stage_dev, s->stage_host, stage_bytes, cudaMemcpyHostToDevice, st));
+        k_het_insert_seeds<<<seed_grid, 256, 0, st>>>(pa);
+    }
     uint64_t f_bound = nmax, items = nmax;
     for (uint32_t stage = 0; stage <= H; ++stage) {
         const bool has_next = stage < H;
@@ -1056,11 +1077,11 @@ int32_t hetero_group_into(ag_hetero_sampler *s, uint32_t n_batches, uint32_t see
             dtype = feats[t]->dtype;
         }
         if (together) {
-            AG_CUDA(launch_gather_stores(s->gather_dev, (uint32_t)G, m.nt, nb, rows, row_bytes, dtype, st));
+            AG_CUDA(launch_gather_stores(gather_dev, nb, m.nt, nb, rows, row_bytes, dtype, st));
         } else {
             for (uint32_t t = 0; t < m.nt; ++t)
                 if (any[t])
-                    AG_CUDA(launch_gather_group(s->gather_dev + (size_t)t * G, nb, row_bytes[t], (uint32_t)feats[t]->dim, rows[t],
+                    AG_CUDA(launch_gather_group(gather_dev + (size_t)t * nb, nb, row_bytes[t], (uint32_t)feats[t]->dim, rows[t],
                                                 aligned[t], feats[t]->dtype, feats[t]->shards != nullptr, st));
         }
     }

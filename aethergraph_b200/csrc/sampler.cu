@@ -46,6 +46,7 @@
 
 #include <algorithm>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include <sched.h>
@@ -139,38 +140,14 @@ __device__ __forceinline__ void row_demand(int mode, uint64_t deg, uint32_t k, u
 }
 
 // ------------------------------------------------------------ seed insert --
-// The parameter blocks, gather arguments and seeds of a chain are staged in pinned host
-// memory and the chain's first kernel reads them from there, leaving the device copies
-// the later kernels use.  A copy command each for the three costs more than the kernel
-// (measured on one batch of 128 seeds: 1.7 us each on the device with 3 - 4 us between
-// them, 3 - 5 us each on the launching thread); a read over PCIe is one round trip.
-// With the seed insertion at the head of stage 0 and the counts written straight to pinned
-// memory a call of 128 seeds went from 115 to 100 us, one of 1024 seeds from 140 to 123.
-struct StagedChain {
-    const SampleParams *params;  // pinned host, one per batch
-    const GatherArgs *gather;    // pinned host, one per batch; null: nothing to gather
-    SampleParams *params_dev;
-    GatherArgs *gather_dev;
+// Where the parts of a chain's staged block are.  Order: parameter blocks, gather
+// arguments (if any), seeds (if the caller's are in host memory).
+struct StageLayout {
+    SampleParams *params_dev;          // the device copies
+    GatherArgs *gather_dev;            // null: nothing to gather
+    uint32_t seeds_at, seed_stride;    // first word of the seeds (0: in device memory already), seeds reserved per batch
 };
-static_assert(sizeof(SampleParams) % 8 == 0 && sizeof(GatherArgs) % 8 == 0, "staged blocks are copied as 8-byte words");
-
-// Loads batch blockIdx.y's parameters into shared memory (whole block); block 0 of the
-// batch leaves the device copies.
-__device__ __forceinline__ void load_staged(const StagedChain &c, SampleParams *s_params) {
-    constexpr uint32_t kWords = sizeof(SampleParams) / 8, kGatherWords = sizeof(GatherArgs) / 8;
-    const volatile uint64_t *src = (const volatile uint64_t *)(c.params + blockIdx.y);
-    const bool keep = blockIdx.x == 0;
-    for (uint32_t i = threadIdx.x; i < kWords + kGatherWords; i += blockDim.x) {
-        if (i < kWords) {
-            const uint64_t v = src[i];
-            ((uint64_t *)s_params)[i] = v;
-            if (keep) ((uint64_t *)(c.params_dev + blockIdx.y))[i] = v;
-        } else if (keep && c.gather) {
-            ((uint64_t *)(c.gather_dev + blockIdx.y))[i - kWords] = ((const volatile uint64_t *)(c.gather + blockIdx.y))[i - kWords];
-        }
-    }
-    __syncthreads();
-}
+static_assert(sizeof(SampleParams) % 8 == 0 && sizeof(GatherArgs) % 8 == 0, "staged blocks are made of 8-byte words");
 
 __device__ __forceinline__ uint32_t insert_seed(const SampleParams &p, uint32_t i, uint32_t id) {
     if ((uint64_t)id >= p.num_nodes) {
@@ -180,9 +157,8 @@ __device__ __forceinline__ uint32_t insert_seed(const SampleParams &p, uint32_t 
     return table_insert_min(p.table, id, enc_pending(p.table.gen, 0, i), &p.state->error);
 }
 
-__global__ void k_insert_seeds(StagedChain chain) {
-    __shared__ __align__(16) SampleParams p;
-    load_staged(chain, &p);
+__global__ void k_insert_seeds(const SampleParams *__restrict__ pa) {
+    const SampleParams &p = pa[blockIdx.y];
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < p.n_seeds) p.slot_of_seed[i] = insert_seed(p, i, p.seeds[i]);
 }
@@ -844,7 +820,7 @@ __device__ __forceinline__ void assign_stage(const SampleParams &p, uint32_t sta
         uint32_t slot[kIPT], id[kIPT], cur32[kIPT];
         bool first[kIPT];
         if (FUSED) {
-            // the seeds may lie in host memory: read each sector of them once
+            // a coalesced read of the seeds, then each thread takes its own
 #pragma unroll
             for (int j = 0; j < kIPT; ++j) {
                 const uint32_t i = threadIdx.x + j * kTile;
@@ -1019,9 +995,29 @@ constexpr uint32_t kFusedSeeds = kTile * kMaxIPT;
 
 template <int IPT>
 __global__ void __launch_bounds__(kTile, 2)
-k_assign_seeds(StagedChain chain, uint32_t k) {
+k_assign_seeds(const SampleParams *__restrict__ pa, uint32_t k) {
+    assign_stage<true, IPT, true>(pa[blockIdx.y], 0, k);
+}
+
+// The same with the staged block in the kernel's parameters.
+template <int IPT, int BYTES>
+__global__ void __launch_bounds__(kTile, 2)
+k_assign_seeds_packed(const __grid_constant__ PackedWords<BYTES> c, const StageLayout at, uint32_t k) {
     __shared__ __align__(16) SampleParams p;
-    load_staged(chain, &p);
+    constexpr uint32_t kWords = sizeof(SampleParams) / 8, kGatherWords = sizeof(GatherArgs) / 8;
+    const uint32_t words = kWords + (at.gather_dev ? kGatherWords : 0u);
+    for (uint32_t i = threadIdx.x; i < words; i += kTile) {
+        if (i < kWords) {
+            const uint64_t v = c.w[blockIdx.y * kWords + i];
+            ((uint64_t *)&p)[i] = v;
+            ((uint64_t *)(at.params_dev + blockIdx.y))[i] = v;
+        } else {
+            ((uint64_t *)(at.gather_dev + blockIdx.y))[i - kWords] = c.w[gridDim.y * kWords + blockIdx.y * kGatherWords + i - kWords];
+        }
+    }
+    __syncthreads();
+    if (threadIdx.x == 0 && at.seeds_at) p.seeds = (const uint32_t *)(c.w + at.seeds_at) + blockIdx.y * at.seed_stride;
+    __syncthreads();
     assign_stage<true, IPT, true>(p, 0, k);
 }
 
@@ -1212,14 +1208,11 @@ struct ag_sampler {
     uint32_t hub_cap = 0;
     TileDesc *tiles = nullptr;
     BatchState *state = nullptr;
-    SampleParams *params_dev = nullptr;
-    GatherArgs *gather_dev = nullptr;
+    uint8_t *stage_dev = nullptr;   // parameter blocks, gather arguments and seeds of the chain (see StageLayout)
     // pinned host
-    uint32_t *seeds_pinned = nullptr;
     ag_sample_counts *counts_host = nullptr;
     bool yield_wait = false;  // ag_sample_group_wait polls and yields instead of spinning in the runtime
-    SampleParams *params_host = nullptr;
-    GatherArgs *gather_host = nullptr;
+    uint8_t *stage_host = nullptr;
     cudaEvent_t done = nullptr;
     bool in_flight = false, dirty = true;
     uint32_t in_flight_n = 0;
@@ -1284,10 +1277,10 @@ void free_scratch(ag_sampler *s) {
     s->frontier = nullptr;
     workspace_free(s->slot_of_seed); workspace_free(s->slot_of_edge); workspace_free(s->tiles);
     workspace_free(s->hub_rows); s->hub_rows = nullptr;
-    workspace_free(s->seeds_pinned);
+    workspace_free(s->stage_host); workspace_free(s->stage_dev);
     s->table = nullptr;
     s->slot_of_seed = s->slot_of_edge = nullptr; s->tiles = nullptr;
-    s->seeds_pinned = nullptr;
+    s->stage_host = s->stage_dev = nullptr;
 }
 
 // A finished continuing batch (no per-batch seed) moves the handle's stream on by
@@ -1336,7 +1329,9 @@ int32_t ensure_scratch(ag_sampler *s, uint64_t n_seeds) {
     }
     s->n_tiles = std::max<uint64_t>(std::max(cap, s->max_hop_edges) / kTile + 2, 2);
     AG_CUDA(workspace_alloc(&s->tiles, G * s->n_tiles * sizeof(TileDesc)));
-    AG_CUDA(workspace_alloc_host(&s->seeds_pinned, G * cap * 4));
+    const uint64_t stage = G * (sizeof(SampleParams) + sizeof(GatherArgs) + (cap + 1) / 2 * 8);
+    AG_CUDA(workspace_alloc_host(&s->stage_host, stage));
+    AG_CUDA(workspace_alloc(&s->stage_dev, stage));
     s->cap_seeds = cap;
     s->epoch = 0;
     s->dirty = true;
@@ -1372,11 +1367,7 @@ extern "C" int32_t ag_sampler_create_group(const ag_graph *g, const ag_sampling_
     int32_t st = AG_OK;
     do {
         if (workspace_alloc(&s->state, group * sizeof(BatchState)) != cudaSuccess ||  // cleared by the first launch (`dirty`)
-            workspace_alloc(&s->params_dev, group * sizeof(SampleParams)) != cudaSuccess ||
-            workspace_alloc(&s->gather_dev, group * sizeof(GatherArgs)) != cudaSuccess ||
             workspace_alloc_host(&s->counts_host, group * sizeof(ag_sample_counts)) != cudaSuccess ||
-            workspace_alloc_host(&s->params_host, group * sizeof(SampleParams)) != cudaSuccess ||
-            workspace_alloc_host(&s->gather_host, group * sizeof(GatherArgs)) != cudaSuccess ||
             cudaEventCreateWithFlags(&s->done, cudaEventDisableTiming) != cudaSuccess ||
             cudaEventCreateWithFlags(&s->sampled, cudaEventDisableTiming) != cudaSuccess) {
             st = fail(AG_ERR_CUDA, "sampler allocation failed: %s", cudaGetErrorString(cudaGetLastError()));
@@ -1410,8 +1401,7 @@ extern "C" void ag_sampler_free(ag_sampler *s) {
     free_scratch(s);
     s->sort.release();
     for (void *p : s->owned) cudaFree(p);
-    workspace_free(s->state); workspace_free(s->params_dev); workspace_free(s->gather_dev);
-    workspace_free(s->counts_host); workspace_free(s->params_host); workspace_free(s->gather_host);
+    workspace_free(s->state); workspace_free(s->counts_host);
     if (s->done) cudaEventDestroy(s->done);
     if (s->sampled) cudaEventDestroy(s->sampled);
     workspace_stream_free(s->gstream, s->gpriority);
@@ -1533,7 +1523,7 @@ cudaEvent_t profile_origin(int device, cudaStream_t st) {
 int32_t launch_saved_impl(ag_sampler *s, bool relaunch);
 
 // Queues the chain described by s->last.  relaunch: the same chain once more with
-// full-size dedup tables (host seeds are already in the handle's pinned copy).
+// full-size dedup tables (host seeds are already in the handle's staged block).
 // A failure part way through leaves kernels of the chain queued: wait for them and
 // mark the handle's device state unknown, so that the next call clears it instead of
 // reusing staging buffers, table generation and batch state under running kernels.
@@ -1602,6 +1592,19 @@ int32_t launch_saved_impl(ag_sampler *s, bool relaunch) {
     while ((1ull << log2cap) < used_cap) ++log2cap;
     const uint64_t ecap = std::max<uint64_t>(s->max_edges, 1);
 
+    // The staged block (see PackedWords): as kernel parameters where the seeds are inserted by
+    // stage 0 and the block is small, else copied to the device.
+    const bool host_seeds = seeds_mem == AG_MEM_HOST;
+    const uint32_t nmax = (uint32_t)max_n, seed_stride = (nmax + 1) & ~1u;
+    const uint64_t gather_at = n_batches * sizeof(SampleParams), seeds_at = gather_at + (want_x ? n_batches * sizeof(GatherArgs) : 0);
+    const uint64_t stage_bytes = seeds_at + (host_seeds ? (uint64_t)n_batches * seed_stride * 4 : 0);
+    const bool fused = nmax <= kFusedSeeds;
+    const uint64_t packed_most = nmax <= kTile ? kPackedSmall : nmax <= kTile * 2 ? kPackedMedium : kPackedLarge;
+    const bool packed = fused && stage_bytes <= packed_most;
+    SampleParams *params_host = (SampleParams *)s->stage_host;
+    GatherArgs *gather_host = (GatherArgs *)(s->stage_host + gather_at), *gather_dev = (GatherArgs *)(s->stage_dev + gather_at);
+    uint32_t *seeds_host = (uint32_t *)(s->stage_host + seeds_at);
+    const uint32_t *seeds_dev = (const uint32_t *)(s->stage_dev + seeds_at);
     uint64_t b_nodes = 0;
     for (uint32_t b = 0; b < n_batches; ++b) {
         const ag_subgraph_buffers &B = bufs[b];
@@ -1614,9 +1617,9 @@ int32_t launch_saved_impl(ag_sampler *s, bool relaunch) {
         p.tiles = s->tiles + (uint64_t)b * s->n_tiles;
         p.epoch_base = s->epoch + 1;
         p.n_seeds = n;
-        if (seeds_mem == AG_MEM_HOST) {  // read from the pinned copy by the chain's first kernel
-            if (n && !relaunch) memcpy(s->seeds_pinned + (uint64_t)b * s->cap_seeds, seeds[b], (size_t)n * 4);
-            p.seeds = s->seeds_pinned + (uint64_t)b * s->cap_seeds;
+        if (host_seeds) {  // (packed: the kernel fills in where they are)
+            if (n && !relaunch) memcpy(seeds_host + (uint64_t)b * seed_stride, seeds[b], (size_t)n * 4);
+            p.seeds = seeds_dev + (uint64_t)b * seed_stride;
         } else {
             p.seeds = seeds[b];
         }
@@ -1640,7 +1643,7 @@ int32_t launch_saved_impl(ag_sampler *s, bool relaunch) {
             // about as many slices whatever the chain's length, a few times what runs at once
             p.hub_slice = (uint32_t)std::min<uint64_t>(kHubDegree * std::max<uint64_t>(next_pow2(n_batches) / 2, 1), 16 * kHubDegree);
         }
-        s->params_host[b] = p;
+        params_host[b] = p;
         uint64_t bn, be;
         compute_bounds(s, n, &bn, &be, nullptr);
         b_nodes = std::max(b_nodes, bn);
@@ -1654,23 +1657,31 @@ int32_t launch_saved_impl(ag_sampler *s, bool relaunch) {
                 ga.n_dev = &s->state[b].stage[H + 1].n_nodes;
                 ga.out = B.x;
             }
-            s->gather_host[b] = ga;
+            gather_host[b] = ga;
         }
     }
     s->pending_pos = (batch_seeds == nullptr);  // a continuing batch advances the handle's stream
     s->epoch += H + 2;
     s->gen += 1;
-    const SampleParams *pa = s->params_dev;
-    const uint32_t nmax = (uint32_t)max_n;
-    const StagedChain staged{s->params_host, want_x ? s->gather_host : nullptr, s->params_dev, s->gather_dev};
-    const bool fused = nmax <= kFusedSeeds;
-    if (!fused) {
-        k_insert_seeds<<<dim3((nmax + 255) / 256, n_batches), 256, 0, st>>>(staged);
+    const SampleParams *pa = (const SampleParams *)s->stage_dev;
+    const uint32_t k0 = s->cfg.fanout[0];
+    if (packed) {
+        const StageLayout at{(SampleParams *)s->stage_dev, want_x ? gather_dev : nullptr, host_seeds ? (uint32_t)(seeds_at / 8) : 0u, seed_stride};
+        auto launch = [&](auto ipt, auto words) {
+            constexpr int kIPT = decltype(ipt)::value, kBytes = decltype(words)::value;
+            PackedWords<kBytes> c;
+            memcpy(&c, s->stage_host, stage_bytes);
+            k_assign_seeds_packed<kIPT, kBytes><<<dim3(1, n_batches), kTile, 0, st>>>(c, at, k0);
+        };
+        if (nmax <= kTile) launch(std::integral_constant<int, 1>{}, std::integral_constant<int, kPackedSmall>{});
+        else if (nmax <= kTile * 2) launch(std::integral_constant<int, 2>{}, std::integral_constant<int, kPackedMedium>{});
+        else launch(std::integral_constant<int, kMaxIPT>{}, std::integral_constant<int, kPackedLarge>{});
     } else {
-        const uint32_t k0 = s->cfg.fanout[0];
-        if (nmax <= kTile) k_assign_seeds<1><<<dim3(1, n_batches), kTile, 0, st>>>(staged, k0);
-        else if (nmax <= kTile * 2) k_assign_seeds<2><<<dim3(1, n_batches), kTile, 0, st>>>(staged, k0);
-        else k_assign_seeds<kMaxIPT><<<dim3(1, n_batches), kTile, 0, st>>>(staged, k0);
+        AG_CUDA(cudaMemcpyAsync(s->stage_dev, s->stage_host, stage_bytes, cudaMemcpyHostToDevice, st));
+        if (!fused) k_insert_seeds<<<dim3((nmax + 255) / 256, n_batches), 256, 0, st>>>(pa);
+        else if (nmax <= kTile) k_assign_seeds<1><<<dim3(1, n_batches), kTile, 0, st>>>(pa, k0);
+        else if (nmax <= kTile * 2) k_assign_seeds<2><<<dim3(1, n_batches), kTile, 0, st>>>(pa, k0);
+        else k_assign_seeds<kMaxIPT><<<dim3(1, n_batches), kTile, 0, st>>>(pa, k0);
     }
     uint64_t items = nmax;  // bound on the items of the stage being launched
     for (uint32_t stage = 0; stage <= H; ++stage) {
@@ -1700,7 +1711,7 @@ int32_t launch_saved_impl(ag_sampler *s, bool relaunch) {
         // kernels: it stays on the (high-priority) sampling stream.  (The handle's previous
         // chain has finished — its event was waited for — so the sort scratch is free.)
         const uint64_t sort_rows = s->est_rows_tight ? std::min(rows, s->est_rows_tight) : rows;  // less padding to sort
-        if (sorted) AG_CUDA(launch_sort_keys(GatherArgs{}, s->gather_dev, n_batches, sort_rows, feats, s->sort, st));
+        if (sorted) AG_CUDA(launch_sort_keys(GatherArgs{}, gather_dev, n_batches, sort_rows, feats, s->sort, st));
         // sampling chain -> event -> gather on the low-priority stream -> event -> caller's stream
         AG_CUDA(cudaEventRecord(s->sampled, st));
         AG_CUDA(cudaStreamWaitEvent(s->gstream, s->sampled, 0));
@@ -1709,12 +1720,12 @@ int32_t launch_saved_impl(ag_sampler *s, bool relaunch) {
             if (!s->rstream) AG_CUDA(workspace_stream(&s->rstream, s->rpriority));
             if (!s->remote_done) AG_CUDA(cudaEventCreateWithFlags(&s->remote_done, cudaEventDisableTiming));
             AG_CUDA(cudaStreamWaitEvent(s->rstream, s->sampled, 0));
-            AG_CUDA(launch_sorted_fetch(GatherArgs{}, s->gather_dev, n_batches, sort_rows, row_bytes, (uint32_t)feats->dim,
+            AG_CUDA(launch_sorted_fetch(GatherArgs{}, gather_dev, n_batches, sort_rows, row_bytes, (uint32_t)feats->dim,
                                         feats->dtype, feats, s->sort, s->gstream, s->rstream));
             AG_CUDA(cudaEventRecord(s->remote_done, s->rstream));
             AG_CUDA(cudaStreamWaitEvent(s->gstream, s->remote_done, 0));
         } else {
-            AG_CUDA(launch_gather_group(s->gather_dev, n_batches, row_bytes, (uint32_t)feats->dim, rows, aligned,
+            AG_CUDA(launch_gather_group(gather_dev, n_batches, row_bytes, (uint32_t)feats->dim, rows, aligned,
                                         feats->dtype, feats->shards != nullptr, s->gstream));
         }
         if (s->profile) AG_CUDA(cudaEventRecord(s->ev[3], s->gstream));
