@@ -441,6 +441,7 @@ extern "C" int32_t ag_loader_create(const ag_graph *g, const ag_features *f, con
         st = ag_sampler_create_group(g, &c, l->group, &s);
         if (st != AG_OK) break;
         l->samplers.push_back(s);
+        sampler_set_pipelined(s);
         if (profiling) st = ag_sampler_set_profiling(s, 1);
         if (st == AG_OK && yielding_waits()) st = sampler_set_yielding_wait(s, true);
         cudaStream_t stream = nullptr;

@@ -1216,10 +1216,14 @@ struct ag_sampler {
     cudaEvent_t done = nullptr;
     bool in_flight = false, dirty = true;
     uint32_t in_flight_n = 0;
-    // The gather runs on the handle's own low-priority stream, behind an event:
+    // A loader's handle gathers on its own low-priority stream, behind an event:
     // sampling kernels of other handles (latency-bound, few resources) then slip
     // in between the short-lived blocks of a running gather (bandwidth-bound).
+    // A handle that runs alone has no such neighbours and gathers on the caller's
+    // stream: the hop to another stream and back cost a call 5 us or so.  Made when
+    // the first such chain is launched.
     cudaStream_t gstream = nullptr;
+    bool pipelined = false;  // a loader's, or one of a group: sampler_set_pipelined
     cudaEvent_t sampled = nullptr;
     // Sharded stores: the remote part of a chain's rows is fetched by a launch of its own on
     // this stream (between the two priorities), beside the local part on gstream.  Made when
@@ -1362,6 +1366,7 @@ extern "C" int32_t ag_sampler_create_group(const ag_graph *g, const ag_sampling_
     s->cfg = *cfg;
     s->device = g->device;
     s->group = group;
+    s->pipelined = group > 1;
     s->mode = cfg->weighted ? (cfg->replace ? kModeWeightedReplace : kModeWeighted) : (cfg->replace ? kModeReplace : kModeUniform);
     s->seed = cfg->seed;
     int32_t st = AG_OK;
@@ -1379,10 +1384,6 @@ extern "C" int32_t ag_sampler_create_group(const ag_graph *g, const ag_sampling_
         static const bool gather_high = [] { const char *v = getenv("AG_GATHER_PRIORITY"); return v && v[0] == 'h'; }();
         s->gpriority = gather_high ? hi : lo;
         s->rpriority = (lo + hi) / 2;
-        if (workspace_stream(&s->gstream, s->gpriority) != cudaSuccess) {
-            st = fail(AG_ERR_CUDA, "cudaStreamCreateWithPriority failed: %s", cudaGetErrorString(cudaGetLastError()));
-            break;
-        }
         st = ensure_scratch(s, std::max<uint32_t>(cfg->max_seeds, 1));
     } while (0);
     if (st != AG_OK) { ag_sampler_free(s); return st; }
@@ -1429,6 +1430,8 @@ extern "C" int32_t ag_sampler_reseed(ag_sampler *s, uint64_t seed) {
 // host's cores, which the consumer's own thread needs; on an idle core a yield returns
 // at once, so nothing is lost when there are cores to spare.  (Sleeping on the event
 // — cudaEventBlockingSync — was measured too: -9 % on one GPU, the wake-up is too slow.)
+void ag::sampler_set_pipelined(ag_sampler *s) { s->pipelined = true; }
+
 int32_t ag::sampler_set_yielding_wait(ag_sampler *s, bool on) {
     s->yield_wait = on;
     return AG_OK;
@@ -1712,25 +1715,30 @@ int32_t launch_saved_impl(ag_sampler *s, bool relaunch) {
         // chain has finished — its event was waited for — so the sort scratch is free.)
         const uint64_t sort_rows = s->est_rows_tight ? std::min(rows, s->est_rows_tight) : rows;  // less padding to sort
         if (sorted) AG_CUDA(launch_sort_keys(GatherArgs{}, gather_dev, n_batches, sort_rows, feats, s->sort, st));
-        // sampling chain -> event -> gather on the low-priority stream -> event -> caller's stream
-        AG_CUDA(cudaEventRecord(s->sampled, st));
-        AG_CUDA(cudaStreamWaitEvent(s->gstream, s->sampled, 0));
-        if (s->profile) AG_CUDA(cudaEventRecord(s->ev[2], s->gstream));
+        cudaStream_t gs = st;
+        if (s->pipelined || sorted) {
+            // sampling chain -> event -> gather on the low-priority stream -> event -> caller's stream
+            if (!s->gstream) AG_CUDA(workspace_stream(&s->gstream, s->gpriority));
+            gs = s->gstream;
+            AG_CUDA(cudaEventRecord(s->sampled, st));
+            AG_CUDA(cudaStreamWaitEvent(gs, s->sampled, 0));
+        }
+        if (s->profile) AG_CUDA(cudaEventRecord(s->ev[2], gs));
         if (sorted) {
             if (!s->rstream) AG_CUDA(workspace_stream(&s->rstream, s->rpriority));
             if (!s->remote_done) AG_CUDA(cudaEventCreateWithFlags(&s->remote_done, cudaEventDisableTiming));
             AG_CUDA(cudaStreamWaitEvent(s->rstream, s->sampled, 0));
             AG_CUDA(launch_sorted_fetch(GatherArgs{}, gather_dev, n_batches, sort_rows, row_bytes, (uint32_t)feats->dim,
-                                        feats->dtype, feats, s->sort, s->gstream, s->rstream));
+                                        feats->dtype, feats, s->sort, gs, s->rstream));
             AG_CUDA(cudaEventRecord(s->remote_done, s->rstream));
-            AG_CUDA(cudaStreamWaitEvent(s->gstream, s->remote_done, 0));
+            AG_CUDA(cudaStreamWaitEvent(gs, s->remote_done, 0));
         } else {
             AG_CUDA(launch_gather_group(gather_dev, n_batches, row_bytes, (uint32_t)feats->dim, rows, aligned,
-                                        feats->dtype, feats->shards != nullptr, s->gstream));
+                                        feats->dtype, feats->shards != nullptr, gs));
         }
-        if (s->profile) AG_CUDA(cudaEventRecord(s->ev[3], s->gstream));
-        AG_CUDA(cudaEventRecord(s->done, s->gstream));
-        AG_CUDA(cudaStreamWaitEvent(st, s->done, 0));  // the caller's stream stays ordered behind the gather
+        if (s->profile) AG_CUDA(cudaEventRecord(s->ev[3], gs));
+        AG_CUDA(cudaEventRecord(s->done, gs));
+        if (gs != st) AG_CUDA(cudaStreamWaitEvent(st, s->done, 0));  // the caller's stream stays ordered behind the gather
         s->gathered = true;
     } else {
         AG_CUDA(cudaEventRecord(s->done, st));
