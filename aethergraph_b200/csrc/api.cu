@@ -1425,7 +1425,7 @@ extern "C" int32_t ag_features_get_batch(const ag_features *f, const int64_t *id
     float *out_dev = nullptr;
     int32_t st = AG_OK;
     do {
-        if (cudaMalloc(&ids_dev, n * 8) != cudaSuccess || cudaMalloc(&out_dev, n * f->dim * 4) != cudaSuccess) {
+        if (workspace_alloc(&ids_dev, n * 8) != cudaSuccess || workspace_alloc(&out_dev, n * f->dim * 4) != cudaSuccess) {
             st = fail(AG_ERR_CUDA, "out of device memory: %s", cudaGetErrorString(cudaGetLastError()));
             break;
         }
@@ -1437,6 +1437,7 @@ extern "C" int32_t ag_features_get_batch(const ag_features *f, const int64_t *id
         }
         if (e != cudaSuccess) st = fail(AG_ERR_CUDA, "get_batch failed: %s", cudaGetErrorString(e));
     } while (0);
-    cudaFree(ids_dev); cudaFree(out_dev);
+    if (st != AG_OK) cudaDeviceSynchronize();  // whatever was queued before the failure
+    workspace_free(ids_dev); workspace_free(out_dev);
     return st;
 }

@@ -1194,7 +1194,8 @@ struct ag_sampler {
     // sizing (per batch)
     uint64_t cap_seeds = 0, max_nodes = 0, max_edges = 0, max_hop_edges = 0;
     uint64_t table_cap = 0, n_tiles = 0;
-    // scratch (device), each `group` times the per-batch size
+    // scratch (device), each `group` times the per-batch size, carved out of one block
+    uint8_t *scratch = nullptr;
     uint64_t *table = nullptr;
     FrontierEntry *frontier = nullptr;
     uint64_t max_frontier = 0;
@@ -1277,14 +1278,10 @@ void compute_bounds(const ag_sampler *s, uint64_t n_seeds, uint64_t *max_nodes, 
 }
 
 void free_scratch(ag_sampler *s) {
-    workspace_free(s->table); workspace_free(s->frontier);
-    s->frontier = nullptr;
-    workspace_free(s->slot_of_seed); workspace_free(s->slot_of_edge); workspace_free(s->tiles);
-    workspace_free(s->hub_rows); s->hub_rows = nullptr;
-    workspace_free(s->stage_host); workspace_free(s->stage_dev);
-    s->table = nullptr;
-    s->slot_of_seed = s->slot_of_edge = nullptr; s->tiles = nullptr;
-    s->stage_host = s->stage_dev = nullptr;
+    workspace_free(s->scratch); workspace_free(s->stage_host);
+    s->scratch = nullptr; s->stage_host = s->stage_dev = nullptr;
+    s->table = nullptr; s->frontier = nullptr; s->tiles = nullptr; s->hub_rows = nullptr;
+    s->slot_of_seed = s->slot_of_edge = nullptr;
 }
 
 // A finished continuing batch (no per-batch seed) moves the handle's stream on by
@@ -1294,48 +1291,64 @@ void account_stream(ag_sampler *s) {
     s->pending_pos = false;
 }
 
-// Scratch for `group` batches of up to n_seeds seeds each.
+// Sizes of a batch of n_seeds seeds; refuses one past the per-batch limits.
+int32_t size_batch(ag_sampler *s, uint64_t n_seeds) {
+    const uint64_t cap = std::max<uint64_t>(n_seeds, 1);
+    compute_bounds(s, cap, &s->max_nodes, &s->max_edges, &s->max_hop_edges);
+    if (s->max_nodes >= kMaxPos || s->max_hop_edges >= kMaxPos || cap >= kMaxPos || s->max_edges >= 0xFFFFFFFFull)
+        return fail(AG_ERR_VALUE, "batch too large: %llu seeds with this fanout can reach %llu nodes and %llu edges "
+                    "in a hop (limit %llu each)", (unsigned long long)n_seeds, (unsigned long long)s->max_nodes,
+                    (unsigned long long)s->max_hop_edges, (unsigned long long)kMaxPos - 1);
+    return AG_OK;
+}
+
+// Scratch for `group` batches of up to n_seeds seeds each: one device block (an allocation
+// takes 0.1 to 1.5 ms when the driver has to map memory) and one pinned one.
 int32_t ensure_scratch(ag_sampler *s, uint64_t n_seeds) {
     if (n_seeds <= s->cap_seeds && s->table) return AG_OK;
     if (s->in_flight) { AG_CUDA(cudaEventSynchronize(s->done)); s->in_flight = false; account_stream(s); }
     free_scratch(s);
     s->cap_seeds = 0;
     const uint64_t cap = std::max<uint64_t>(n_seeds, 1), G = s->group;
-    compute_bounds(s, cap, &s->max_nodes, &s->max_edges, &s->max_hop_edges);
-    if (s->max_nodes >= kMaxPos || s->max_hop_edges >= kMaxPos || cap >= kMaxPos || s->max_edges >= 0xFFFFFFFFull)
-        return fail(AG_ERR_VALUE, "batch too large: %llu seeds with this fanout can reach %llu nodes and %llu edges "
-                    "in a hop (limit %llu each)", (unsigned long long)n_seeds, (unsigned long long)s->max_nodes,
-                    (unsigned long long)s->max_hop_edges, (unsigned long long)kMaxPos - 1);
+    AG_TRY(size_batch(s, n_seeds));
     s->table_cap = std::max<uint64_t>(1024, next_pow2(2 * s->max_nodes));
-    AG_CUDA(workspace_alloc(&s->table, G * s->table_cap * 8));
     // the frontier of a hop holds at most the vertices the previous stage found
     s->max_frontier = std::max<uint64_t>(std::min<uint64_t>(std::max(cap, s->max_hop_edges), s->g->num_nodes), 1);
-    AG_CUDA(workspace_alloc(&s->frontier, G * s->max_frontier * sizeof(FrontierEntry)));
-    AG_CUDA(workspace_alloc(&s->slot_of_seed, G * cap * 4));
-    AG_CUDA(workspace_alloc(&s->slot_of_edge, G * std::max<uint64_t>(s->max_edges, 1) * 4));
+    s->n_tiles = std::max<uint64_t>(std::max(cap, s->max_hop_edges) / kTile + 2, 2);
+    s->hub_cap = 0;
+    uint64_t hop_k = 1;
     if (s->mode == kModeWeighted) {
         // A batch expands a vertex once, and a row of d > kHubDegree positions is at most
         // 2 d / kHubDegree slices.
         const uint64_t most = 2 * (s->g->num_edges / kHubDegree) * G;
-        uint64_t hop_k = 1;
         for (uint32_t h = 0; h < s->cfg.num_hops; ++h) hop_k = std::max<uint64_t>(hop_k, std::min<uint32_t>(s->cfg.fanout[h], 32u));
         s->hub_cap = (uint32_t)std::min<uint64_t>(std::max<uint64_t>(most, 1), kMaxHubSlices);
-        const uint64_t cap = s->hub_cap;
-        uint8_t *base = nullptr;
-        AG_CUDA(workspace_alloc(&base, cap * (sizeof(HubRow) + 8 * hop_k + 4 * hop_k + 12) + 8));
-        s->hub_rows = (HubRow *)base;
-        s->hub_key = (double *)(base + cap * sizeof(HubRow));
-        s->hub_count = (unsigned long long *)(s->hub_key + cap * hop_k);
-        s->hub_pos = (uint32_t *)(s->hub_count + 1);
-        s->hub_thr = s->hub_pos + cap * hop_k;
-        s->hub_done = s->hub_thr + cap;
-        s->hub_guess = (float *)(s->hub_done + cap);
     }
-    s->n_tiles = std::max<uint64_t>(std::max(cap, s->max_hop_edges) / kTile + 2, 2);
-    AG_CUDA(workspace_alloc(&s->tiles, G * s->n_tiles * sizeof(TileDesc)));
-    const uint64_t stage = G * (sizeof(SampleParams) + sizeof(GatherArgs) + (cap + 1) / 2 * 8);
+    const uint64_t stage = G * (sizeof(SampleParams) + sizeof(GatherArgs) + (cap + 1) / 2 * 8), hubs = s->hub_cap;
     AG_CUDA(workspace_alloc_host(&s->stage_host, stage));
-    AG_CUDA(workspace_alloc(&s->stage_dev, stage));
+    uint8_t *base = nullptr;
+    for (int pass = 0; pass < 2; ++pass) {  // the sizes, then the places
+        uint64_t off = 0;
+        auto carve = [&](auto **p, uint64_t bytes) {
+            if (pass) *(uint8_t **)p = base + off;
+            off += (bytes + 255) & ~255ull;
+        };
+        carve(&s->table, G * s->table_cap * 8);
+        carve(&s->frontier, G * s->max_frontier * sizeof(FrontierEntry));
+        carve(&s->slot_of_seed, G * cap * 4);
+        carve(&s->slot_of_edge, G * std::max<uint64_t>(s->max_edges, 1) * 4);
+        carve(&s->tiles, G * s->n_tiles * sizeof(TileDesc));
+        carve(&s->stage_dev, stage);
+        if (hubs) {
+            carve(&s->hub_rows, hubs * sizeof(HubRow)); carve(&s->hub_count, 8);
+            carve(&s->hub_key, hubs * hop_k * 8); carve(&s->hub_pos, hubs * hop_k * 4);
+            carve(&s->hub_thr, hubs * 4); carve(&s->hub_done, hubs * 4); carve(&s->hub_guess, hubs * 4);
+        }
+        if (!pass) {
+            AG_CUDA(workspace_alloc(&base, off));
+            s->scratch = base;
+        }
+    }
     s->cap_seeds = cap;
     s->epoch = 0;
     s->dirty = true;
@@ -1384,7 +1397,8 @@ extern "C" int32_t ag_sampler_create_group(const ag_graph *g, const ag_sampling_
         static const bool gather_high = [] { const char *v = getenv("AG_GATHER_PRIORITY"); return v && v[0] == 'h'; }();
         s->gpriority = gather_high ? hi : lo;
         s->rpriority = (lo + hi) / 2;
-        st = ensure_scratch(s, std::max<uint32_t>(cfg->max_seeds, 1));
+        // Without a size to expect, the first batch brings it.
+        st = cfg->max_seeds ? ensure_scratch(s, cfg->max_seeds) : size_batch(s, 1);
     } while (0);
     if (st != AG_OK) { ag_sampler_free(s); return st; }
     *out = s;
