@@ -159,11 +159,16 @@ constexpr int kPackedSmall = 4032, kPackedMedium = 8128, kPackedLarge = 16320;
 // are scheduled as this one's blocks exit, without waiting for the grid's
 // completion to be reported first.  Every kernel starts by waiting for its
 // predecessor's results (griddepcontrol.wait; a no-op for a plain launch).  The
-// kernels do NOT release their successor early (no griddepcontrol.launch_dependents
-// before the work): measured, successor blocks parked in SM slots take those slots
-// from the gather of a neighbouring chain and the whole pipeline gets slower.
+// kernels of a loader's chain do NOT release their successor early: measured, successor
+// blocks parked in SM slots take those slots from the gather of a neighbouring chain and
+// the whole pipeline gets slower.  A chain that runs alone has no such neighbour, and
+// chain_release (after chain_sync, once all blocks have called it) lets the next kernel
+// be launched while this one works; it still waits for all of this one's results.
 __device__ __forceinline__ void chain_sync() {
     asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+__device__ __forceinline__ void chain_release(uint32_t alone) {
+    if (alone) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
 // Launches `kern` as a programmatic dependent of the previous kernel on the stream.

@@ -164,6 +164,7 @@ __device__ __forceinline__ void gather_vec_rows(GatherArgs &a, uint64_t first) {
 template <int DTYPE, int LPR>
 __global__ void __launch_bounds__(kThreads)
 k_gather_vec(GatherArgs a, const GatherArgs *__restrict__ group, uint64_t first) {
+    chain_sync();
     if (group) a = group[blockIdx.y];  // one batch of a group per grid row
     if (!a.payload) return;
     gather_vec_rows<DTYPE, LPR>(a, first);
@@ -574,6 +575,18 @@ cudaError_t launch_vec(const GatherArgs &a, const GatherArgs *group, uint32_t ro
     else if (vecs <= 8) k_gather_vec<DTYPE, 8><<<grid, kThreads, 0, st>>>(a, group, first);
     else if (vecs <= 16) k_gather_vec<DTYPE, 16><<<grid, kThreads, 0, st>>>(a, group, first);
     else k_gather_vec<DTYPE, 32><<<grid, kThreads, 0, st>>>(a, group, first);
+    return cudaGetLastError();
+}
+
+// The vector gather as a programmatic dependent of the chain's last kernel.
+template <int DTYPE>
+cudaError_t launch_vec_chained(const GatherArgs *group, uint32_t row_bytes, dim3 grid, cudaStream_t st) {
+    const uint32_t vecs = row_bytes >> 4;
+    const GatherArgs none{};
+    if (vecs <= 4) launch_chained(k_gather_vec<DTYPE, 4>, grid, dim3(kThreads), st, none, group, 0);
+    else if (vecs <= 8) launch_chained(k_gather_vec<DTYPE, 8>, grid, dim3(kThreads), st, none, group, 0);
+    else if (vecs <= 16) launch_chained(k_gather_vec<DTYPE, 16>, grid, dim3(kThreads), st, none, group, 0);
+    else launch_chained(k_gather_vec<DTYPE, 32>, grid, dim3(kThreads), st, none, group, 0);
     return cudaGetLastError();
 }
 
@@ -1020,7 +1033,7 @@ cudaError_t launch_gather(const GatherArgs &a, int dtype, cudaStream_t st) {
 // vector path, others are walked in units.
 cudaError_t launch_gather_group(const GatherArgs *group_dev, uint32_t n_batches, uint32_t row_bytes,
                                 uint32_t dim, uint64_t n_bound, bool aligned, int dtype, bool sharded,
-                                cudaStream_t st) {
+                                cudaStream_t st, bool chained) {
     if (n_batches == 0 || n_bound == 0) return cudaSuccess;
     GatherArgs none{};
     if (row_bytes % 16 == 0 && aligned) {
@@ -1037,6 +1050,13 @@ cudaError_t launch_gather_group(const GatherArgs *group_dev, uint32_t n_batches,
                 case AG_F32: return launch_bulk<AG_F32>(none, group_dev, row_bytes, n_bound, n_batches, st);
                 case AG_F16: return launch_bulk<AG_F16>(none, group_dev, row_bytes, n_bound, n_batches, st);
                 default: return launch_bulk<AG_BF16>(none, group_dev, row_bytes, n_bound, n_batches, st);
+            }
+        }
+        if (chained && !sharded && dtype != AG_I8) {
+            switch (dtype) {
+                case AG_F32: return launch_vec_chained<AG_F32>(group_dev, row_bytes, grid, st);
+                case AG_F16: return launch_vec_chained<AG_F16>(group_dev, row_bytes, grid, st);
+                default: return launch_vec_chained<AG_BF16>(group_dev, row_bytes, grid, st);
             }
         }
         switch (dtype) {

@@ -161,7 +161,7 @@ inline void set_gather_source(GatherArgs &a, const ag_features *f) {
 cudaError_t launch_gather(const GatherArgs &a, int dtype, cudaStream_t st);
 cudaError_t launch_gather_group(const GatherArgs *group_dev, uint32_t n_batches, uint32_t row_bytes,
                                 uint32_t dim, uint64_t n_bound, bool aligned, int dtype, bool sharded,
-                                cudaStream_t st);
+                                cudaStream_t st, bool chained = false);  // chained: behind a chain's kernels on the same stream
 cudaError_t launch_gather_stores(const GatherArgs *group_dev, uint32_t stride, uint32_t n_stores, uint32_t n_batches,
                                  const uint64_t *rows, const uint32_t *row_bytes, int dtype, cudaStream_t st);
 // Address-ordered gather over a sharded view (see gather.cu).

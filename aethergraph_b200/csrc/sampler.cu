@@ -113,6 +113,7 @@ struct SampleParams {
     double *hub_key;                 // [hub_cap][k] the slices' best (key, position) pairs
     uint32_t *hub_pos;
     uint32_t hub_cap, hub_slice;     // slices the arrays hold, positions per slice
+    uint32_t alone, pad;             // no other chain runs beside this one (chain_release)
 };
 
 // Row bounds with the reference's guard (graph/csr.rs:318-335): an inverted
@@ -643,6 +644,7 @@ __global__ void __launch_bounds__(kPickThreads)
 k_pick_weighted_replace(const SampleParams *__restrict__ pa, uint32_t hop, uint32_t k) {
     chain_sync();
     const SampleParams &p = pa[blockIdx.y];
+    chain_release(p.alone);
     const StageInfo nx = p.state->stage[hop + 1];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     for (uint32_t j = blockIdx.x * (kPickThreads / 32) + warp; j < nx.frontier_n; j += gridDim.x * (kPickThreads / 32)) {
@@ -708,6 +710,7 @@ k_pick_weighted_large(const SampleParams *__restrict__ pa, uint32_t hop, uint32_
     __shared__ uint32_t s_fill;
     chain_sync();
     const SampleParams &p = pa[blockIdx.y];
+    chain_release(p.alone);
     const StageInfo nx = p.state->stage[hop + 1];
     const double inf = __longlong_as_double(0x7FF0000000000000ll);
     for (uint32_t j = blockIdx.x; j < nx.frontier_n; j += gridDim.x) {
@@ -987,6 +990,7 @@ template <bool HAS_NEXT, int IPT>
 __global__ void __launch_bounds__(kTile, 2)
 k_assign(const SampleParams *__restrict__ pa, uint32_t stage, uint32_t k) {
     chain_sync();
+    chain_release(pa[blockIdx.y].alone);
     assign_stage<HAS_NEXT, IPT, false>(pa[blockIdx.y], stage, k);
 }
 
@@ -996,6 +1000,7 @@ constexpr uint32_t kFusedSeeds = kTile * kMaxIPT;
 template <int IPT>
 __global__ void __launch_bounds__(kTile, 2)
 k_assign_seeds(const SampleParams *__restrict__ pa, uint32_t k) {
+    chain_release(pa[blockIdx.y].alone);
     assign_stage<true, IPT, true>(pa[blockIdx.y], 0, k);
 }
 
@@ -1016,6 +1021,7 @@ k_assign_seeds_packed(const __grid_constant__ PackedWords<BYTES> c, const StageL
         }
     }
     __syncthreads();
+    chain_release(p.alone);
     if (threadIdx.x == 0 && at.seeds_at) p.seeds = (const uint32_t *)(c.w + at.seeds_at) + blockIdx.y * at.seed_stride;
     __syncthreads();
     assign_stage<true, IPT, true>(p, 0, k);
@@ -1031,6 +1037,7 @@ k_pick(const SampleParams *__restrict__ pa, uint32_t hop, uint32_t k) {
     __shared__ uint32_t s_queue[PICK == kPickWeighted ? (kWeightedThreads / 32) * 64 : 1];  // weighted: 64 queued positions per warp
     chain_sync();
     const SampleParams &p = pa[blockIdx.y];
+    chain_release(p.alone);
     const StageInfo nx = p.state->stage[hop + 1];
     if constexpr (PICK == kPickWeighted) pick_weighted(p, hop, k, nx.n_edges, p.frontier, nx.frontier_n, s_queue);
     else if constexpr (PICK == kPickLarge) pick_large(p, hop, k, nx.n_edges, p.frontier, nx.frontier_n, &s_picks[0][0]);
@@ -1052,6 +1059,7 @@ k_pick_hub_slices(const SampleParams *__restrict__ pa, uint32_t hop, uint32_t k)
     __shared__ uint32_t s_queue[(kWeightedThreads / 32) * 64];
     chain_sync();
     const SampleParams &q = pa[0];  // the queue is the same for every batch
+    chain_release(q.alone);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const double inf = __longlong_as_double(0x7FF0000000000000ll);
     const unsigned long long count = *q.hub_count;
@@ -1642,6 +1650,7 @@ int32_t launch_saved_impl(ag_sampler *s, bool relaunch) {
         }
         p.seed = batch_seeds ? batch_seeds[b] : s->seed;
         p.rng_mode = s->cfg.rng_mode; p.mode = s->mode;
+        p.alone = s->pipelined ? 0u : 1u;
         p.start_draw = batch_seeds ? 0ull : s->stream_pos;
         p.num_hops = H;
         p.nodes = B.nodes; p.edge_src = B.edge_src; p.edge_dst = B.edge_dst;
@@ -1748,7 +1757,7 @@ int32_t launch_saved_impl(ag_sampler *s, bool relaunch) {
             AG_CUDA(cudaStreamWaitEvent(gs, s->remote_done, 0));
         } else {
             AG_CUDA(launch_gather_group(gather_dev, n_batches, row_bytes, (uint32_t)feats->dim, rows, aligned,
-                                        feats->dtype, feats->shards != nullptr, gs));
+                                        feats->dtype, feats->shards != nullptr, gs, gs == st));
         }
         if (s->profile) AG_CUDA(cudaEventRecord(s->ev[3], gs));
         AG_CUDA(cudaEventRecord(s->done, gs));
