@@ -187,10 +187,13 @@ namespace {
 // Rows differ by five orders of magnitude (a hub of an R-MAT graph of 64 M edges has
 // over 100 K neighbours, most vertices a few), so a warp per row left the two walks to
 // the warp with the longest one: 200 seeds, fanouts 10, 5 on that graph reach 3200 nodes
-// and 5.7 M positions, 2660 + 3080 us at 4 % of the warps busy.  Now 55 + 48 us (107 + 84
-// before the filter and the shuffled row search below), bound by warps in short rows.
-constexpr int kWalkThreads = 256;
-constexpr uint32_t kWalkWarpsPerSM = 32;
+// and 5.7 M positions, 2660 + 3080 us at 4 % of the warps busy.  Now 39 + 44 us (107 + 84
+// before the filter and the shuffled row search below), bound by the probes of the node table.
+// One block per SM, so that the filter below is built once for 32 warps and the counts that
+// are scanned are one per block (256-thread blocks: 55 + 48 us, of it 25 us for the scan of
+// 4736 warp counts and up to 10 us for building the filter in waves of blocks).
+constexpr int kWalkThreads = 1024;
+constexpr uint32_t kWalkWarps = kWalkThreads / 32;
 constexpr uint32_t kWalkMin = 128;   // positions a warp takes at least
 constexpr uint32_t kWalkUnroll = 4;  // 32-position chunks in flight in a long row
 // Most neighbours are not in the sample, and a probe of the node table is 32 scattered
@@ -244,7 +247,8 @@ struct InduceWalk {
     const unsigned long long *table;
     uint32_t mask, warps;
     uint32_t filter_words;      // a power of two, or 0: no filter
-    uint64_t *warp_start;       // [warps] hits, then (scanned) hits before the warp's stretch
+    uint64_t *warp_start;       // [warps] hits of the block's earlier warps
+    uint64_t *block_start;      // [warps / kWalkWarps] hits of the block, then (scanned) of the blocks before it
     uint64_t *total;            // [0] all hits, [1] blocks that have counted
 };
 
@@ -269,9 +273,10 @@ __device__ __forceinline__ uint64_t row_of(const uint64_t *__restrict__ row_star
 __device__ __forceinline__ uint32_t filter_bit(uint32_t v, uint32_t words) { return (v * 0x9E3779B1u) >> (32 - 5 - (31 - __clz(words))); }
 
 // Both walks.  In a long row the warp reads kWalkUnroll chunks of it at once.  Elsewhere the
-// 32 positions lie in several rows: the lanes hold the ends of the next 32 rows and every
-// lane finds its row among them by shuffles (a search through memory per lane took 4 us for
-// 32 positions); only a run of 32 empty rows falls back to the search.
+// positions lie in several rows: the lanes hold the ends of the next 32 rows and every lane
+// finds its rows among them by shuffles (a search through memory per lane took 4 us for 32
+// positions), kWalkUnroll chunks at once (one at a time: 1 us each); only positions beyond
+// those 32 rows fall back to the search.
 template <bool FILL>
 __global__ void __launch_bounds__(kWalkThreads)
 k_induce_walk(InduceWalk a, InduceOut o) {
@@ -291,7 +296,7 @@ k_induce_walk(InduceWalk a, InduceOut o) {
     const uint64_t per = share > kWalkMin ? share : kWalkMin;
     uint64_t g = min(all, (uint64_t)w * per);
     const uint64_t stop = min(all, g + per);
-    uint64_t out = FILL ? a.warp_start[w] : 0;
+    uint64_t out = FILL ? a.block_start[blockIdx.x] + a.warp_start[w] : 0;
     uint64_t count = 0;
     // hits of 32 positions: lane's neighbour v at CSR position pos in the row of local index r
     auto take = [&](uint32_t hit, uint32_t v, uint64_t pos, uint32_t r, uint32_t node) {
@@ -334,55 +339,71 @@ k_induce_walk(InduceWalk a, InduceOut o) {
             }
             continue;
         }
-        const uint64_t mine = g + lane;
-        uint32_t r = 0;  // rows of the window that end at or before this lane's position
+        uint32_t at[kWalkUnroll], v[kWalkUnroll], hit[kWalkUnroll];
+        uint64_t pos[kWalkUnroll];
 #pragma unroll
-        for (uint32_t step = 16; step > 0; step >>= 1)
-            if (__shfl_sync(0xFFFFFFFFu, row_end, r + step - 1) <= mine) r += step;
-        const bool past = __shfl_sync(0xFFFFFFFFu, row_end, 31) <= mine;  // the window ends before it
-        uint64_t at = row + r, pos = 0;
-        uint32_t v = 0, hit = 0xFFFFFFFFu, node = 0;
-        if (mine < stop) {
-            if (past) at = row_of(a.row_start, a.n, row, mine);
-            pos = __ldg(a.row_off + at) + (mine - __ldg(a.row_start + at));
-            if (FILL) node = __ldg(a.nodes + at);
-            v = ld_stream_u32(a.dst + pos);
-            hit = find(v);
+        for (uint32_t u = 0; u < kWalkUnroll; ++u) {
+            const uint64_t mine = g + u * 32 + lane;
+            uint32_t r = 0;  // rows of the window that end at or before this lane's position
+#pragma unroll
+            for (uint32_t step = 16; step > 0; step >>= 1)
+                if (__shfl_sync(0xFFFFFFFFu, row_end, r + step - 1) <= mine) r += step;
+            const bool past = __shfl_sync(0xFFFFFFFFu, row_end, 31) <= mine;  // the window ends before it
+            at[u] = (uint32_t)row + r; pos[u] = 0; v[u] = 0;
+            if (mine < stop) {
+                if (past) at[u] = (uint32_t)row_of(a.row_start, a.n, row, mine);
+                pos[u] = __ldg(a.row_off + at[u]) + (mine - __ldg(a.row_start + at[u]));
+                v[u] = ld_stream_u32(a.dst + pos[u]);
+            }
         }
-        take(hit, v, pos, (uint32_t)at, node);
-        g += 32;
-        row = __shfl_sync(0xFFFFFFFFu, at, 31);  // at most the row of the next position
+#pragma unroll
+        for (uint32_t u = 0; u < kWalkUnroll; ++u) hit[u] = g + u * 32 + lane < stop ? find(v[u]) : 0xFFFFFFFFu;
+#pragma unroll
+        for (uint32_t u = 0; u < kWalkUnroll; ++u) {
+            const uint32_t node = (FILL && hit[u] != 0xFFFFFFFFu) ? __ldg(a.nodes + at[u]) : 0;
+            take(hit[u], v[u], pos[u], at[u], node);
+        }
+        g += 32 * kWalkUnroll;
+        row = __shfl_sync(0xFFFFFFFFu, at[kWalkUnroll - 1], 31);  // at most the row of the next position
     }
     if (FILL) return;
-    if (lane == 0) a.warp_start[w] = count;
-    // The block that counts last scans the warps' counts.
-    __shared__ uint64_t s_sum[kWalkThreads];
+    // Hits before every warp within its block; the block that counts last scans the blocks.
+    __shared__ uint64_t s_sum[kWalkWarps];
     __shared__ bool s_last;
+    auto scan_warp = [&](uint64_t v) {  // inclusive, over the lanes
+        for (int d = 1; d < 32; d <<= 1) {
+            const uint64_t up = __shfl_up_sync(0xFFFFFFFFu, v, d);
+            if ((int)lane >= d) v += up;
+        }
+        return v;
+    };
+    if (lane == 0) s_sum[threadIdx.x >> 5] = count;
+    __syncthreads();
+    if (threadIdx.x < 32) {
+        const uint64_t mine = s_sum[lane], upto = scan_warp(mine);
+        a.warp_start[blockIdx.x * kWalkWarps + lane] = upto - mine;
+        if (lane == 31) a.block_start[blockIdx.x] = upto;
+    }
     __threadfence();
     __syncthreads();
     if (threadIdx.x == 0) s_last = atomicAdd((unsigned long long *)(a.total + 1), 1ull) == gridDim.x - 1;
     __syncthreads();
     if (!s_last) return;
     __threadfence();
-    const uint32_t each = (a.warps + kWalkThreads - 1) / kWalkThreads;
-    const uint32_t from = min(a.warps, threadIdx.x * each), to = min(a.warps, from + each);
-    uint64_t sum = 0;
-    for (uint32_t i = from; i < to; ++i) sum += __ldcg(a.warp_start + i);
-    s_sum[threadIdx.x] = sum;
-    __syncthreads();
-    for (int d = 1; d < kWalkThreads; d <<= 1) {
-        const uint64_t add = (int)threadIdx.x >= d ? s_sum[threadIdx.x - d] : 0;
+    uint64_t before = 0;
+    for (uint32_t base = 0; base < gridDim.x; base += kWalkThreads) {
+        const uint32_t i = base + threadIdx.x;
+        const uint64_t mine = i < gridDim.x ? __ldcg(a.block_start + i) : 0, upto = scan_warp(mine);
         __syncthreads();
-        s_sum[threadIdx.x] += add;
+        if (lane == 31) s_sum[threadIdx.x >> 5] = upto;
         __syncthreads();
+        if (threadIdx.x < 32) s_sum[lane] = scan_warp(s_sum[lane]);
+        __syncthreads();
+        const uint64_t earlier = before + (threadIdx.x >= 32 ? s_sum[(threadIdx.x >> 5) - 1] : 0);
+        if (i < gridDim.x) a.block_start[i] = earlier + upto - mine;
+        before += s_sum[kWalkWarps - 1];
     }
-    uint64_t run = s_sum[threadIdx.x] - sum;
-    for (uint32_t i = from; i < to; ++i) {
-        const uint64_t c = __ldcg(a.warp_start + i);
-        a.warp_start[i] = run;
-        run += c;
-    }
-    if (threadIdx.x == kWalkThreads - 1) a.total[0] = run;
+    if (threadIdx.x == 0) a.total[0] = before;
 }
 
 }  // namespace
@@ -421,16 +442,16 @@ extern "C" int32_t ag_subgraph_induce_plan(const ag_graph *g, const uint32_t *no
 #define AG_PLAN_CUDA(expr) do { const cudaError_t e_ = (expr); if (e_ != cudaSuccess) \
         return bail(fail(AG_ERR_CUDA, "%s failed: %s", #expr, cudaGetErrorString(e_))); } while (0)
     const uint64_t cap = pow2_at_least(2 * n_nodes);
-    const uint32_t warps = (uint32_t)kSMs * kWalkWarpsPerSM;
+    const uint32_t blocks = (uint32_t)kSMs, warps = blocks * kWalkWarps;
     size_t temp_bytes = 0;
     AG_PLAN_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, temp_bytes, (uint64_t *)nullptr, (uint64_t *)nullptr, (int)(n_nodes + 1), st));
     // one allocation: table, row offsets, row lengths and their scan, the warps' counts, totals, scan scratch
-    const uint64_t words = cap + n_nodes + 2 * (n_nodes + 1) + warps + 3;
+    const uint64_t words = cap + n_nodes + 2 * (n_nodes + 1) + warps + blocks + 3;
     const uint64_t temp_at = (words * 8 + 255) & ~255ull;
     AG_PLAN_CUDA(workspace_alloc(&p->scratch, temp_at + temp_bytes));
     unsigned long long *table = (unsigned long long *)p->scratch;
     uint64_t *row_off = (uint64_t *)(table + cap), *row_len = row_off + n_nodes, *row_start = row_len + n_nodes + 1;
-    uint64_t *warp_start = row_start + n_nodes + 1, *total = warp_start + warps;  // total[2]: error bits
+    uint64_t *warp_start = row_start + n_nodes + 1, *block_start = warp_start + warps, *total = block_start + blocks;  // total[2]: error bits
     AG_PLAN_CUDA(cudaMemsetAsync(table, 0xFF, cap * 8, st));
     AG_PLAN_CUDA(cudaMemsetAsync(total, 0, 24, st));
     AG_PLAN_CUDA(cudaMemsetAsync(row_len + n_nodes, 0, 8, st));
@@ -441,8 +462,8 @@ extern "C" int32_t ag_subgraph_induce_plan(const ag_graph *g, const uint32_t *no
     const uint32_t filter = n_nodes > kFilterNodes ? 0 : (uint32_t)std::min<uint64_t>(std::max<uint64_t>(cap / 4, kFilterMin), kFilterMax);
     AG_PLAN_CUDA(cudaFuncSetAttribute(k_induce_walk<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kFilterMax * 4));
     AG_PLAN_CUDA(cudaFuncSetAttribute(k_induce_walk<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kFilterMax * 4));
-    p->walk = InduceWalk{g->dst, nodes_dev, n_nodes, row_off, row_start, table, (uint32_t)(cap - 1), warps, filter, warp_start, total};
-    k_induce_walk<false><<<warps / (kWalkThreads / 32), kWalkThreads, filter * 4, st>>>(p->walk, InduceOut{});
+    p->walk = InduceWalk{g->dst, nodes_dev, n_nodes, row_off, row_start, table, (uint32_t)(cap - 1), warps, filter, warp_start, block_start, total};
+    k_induce_walk<false><<<blocks, kWalkThreads, filter * 4, st>>>(p->walk, InduceOut{});
     AG_PLAN_CUDA(cudaGetLastError());
     uint64_t got[3] = {0, 0, 0};
     AG_PLAN_CUDA(cudaMemcpyAsync(got, total, 24, cudaMemcpyDeviceToHost, st));
@@ -470,7 +491,7 @@ extern "C" int32_t ag_subgraph_induce_fill(ag_induce_plan *p, uint64_t cap_edges
     cudaStream_t st = (cudaStream_t)stream;
     p->stream = st;
     const InduceOut o{edge_src, edge_dst, src_local, dst_local, edge_ids, edge_index_local, p->n_edges};
-    k_induce_walk<true><<<p->walk.warps / (kWalkThreads / 32), kWalkThreads, p->walk.filter_words * 4, st>>>(p->walk, o);
+    k_induce_walk<true><<<p->walk.warps / kWalkWarps, kWalkThreads, p->walk.filter_words * 4, st>>>(p->walk, o);
     AG_CUDA(cudaGetLastError());
     AG_CUDA(cudaStreamSynchronize(st));
     return AG_OK;
