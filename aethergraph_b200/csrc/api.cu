@@ -132,7 +132,7 @@ namespace {
 
 int32_t validate_on_device(const ag_graph *g, bool check_dst) {
     uint32_t *flag = nullptr;
-    AG_CUDA(cudaMalloc(&flag, 4));
+    AG_CUDA(device_malloc(&flag, 4));
     cudaMemset(flag, 0, 4);
     cudaError_t e = launch_validate_csr(g->offsets, check_dst ? g->dst : nullptr, g->num_nodes, g->num_edges,
                                         g->num_nodes, flag, 0);
@@ -148,7 +148,7 @@ int32_t validate_on_device(const ag_graph *g, bool check_dst) {
 }
 
 int32_t upload(void **dev, const void *src, uint64_t bytes, int mem_kind) {
-    AG_CUDA(cudaMalloc(dev, std::max<uint64_t>(bytes, 16)));
+    AG_CUDA(device_malloc(dev, std::max<uint64_t>(bytes, 16)));
     if (bytes)
         AG_CUDA(cudaMemcpy(*dev, src, bytes, mem_kind == AG_MEM_HOST ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToDevice));
     return AG_OK;
@@ -382,10 +382,10 @@ extern "C" int32_t ag_hetero_load(const char *path, int32_t device, ag_hetero_gr
         if (st != AG_OK) break;
         DeviceGuard guard(device);
         if (!guard.ok) { st = AG_ERR_CUDA; break; }
-        if (cudaMalloc(&flag, 4) != cudaSuccess) { st = fail(AG_ERR_CUDA, "out of device memory"); break; }
+        if (device_malloc(&flag, 4) != cudaSuccess) { st = fail(AG_ERR_CUDA, "out of device memory"); break; }
         for (uint32_t e = 0; e < num_et && st == AG_OK; ++e) {
             const uint64_t ns = num_nodes[src_type[e]], E = num_edges[e];
-            if (cudaMalloc(&off_dev[e], (ns + 1) * 8) != cudaSuccess || cudaMalloc(&dst_dev[e], std::max<uint64_t>(E, 1) * 4) != cudaSuccess) {
+            if (device_malloc(&off_dev[e], (ns + 1) * 8) != cudaSuccess || device_malloc(&dst_dev[e], std::max<uint64_t>(E, 1) * 4) != cudaSuccess) {
                 st = fail(AG_ERR_CUDA, "out of device memory for edge type '%s'", names->rel[e]);
                 break;
             }
@@ -452,7 +452,7 @@ extern "C" int32_t ag_hetero_save(const ag_hetero_graph *h, const ag_hetero_name
         const uint64_t E = h->num_edges[e], ns = h->num_nodes[h->src_type[e]], nd = h->num_nodes[h->dst_type[e]];
         uint64_t *keys = nullptr, *off = nullptr;
         uint32_t *dst = nullptr;
-        if (cudaMalloc(&keys, std::max<uint64_t>(E, 1) * 8) != cudaSuccess) { st = fail(AG_ERR_CUDA, "out of device memory"); break; }
+        if (device_malloc(&keys, std::max<uint64_t>(E, 1) * 8) != cudaSuccess) { st = fail(AG_ERR_CUDA, "out of device memory"); break; }
         if (E) k_in_adjacency_keys<<<grid_for(E), 256>>>(h->in_offsets[e], h->in_sources[e], nd, E, keys);
         st = keys_to_sorted_csr(keys, E, ns, &off, &dst);  // consumes keys
         auto dump = [&](const void *dev, uint64_t bytes) {
@@ -646,7 +646,7 @@ int32_t device_scan(T *d, uint64_t n, bool inclusive) {
     size_t temp_bytes = 0;
     cudaError_t e = inclusive ? cub::DeviceScan::InclusiveSum(nullptr, temp_bytes, d, d, (size_t)n)
                               : cub::DeviceScan::ExclusiveSum(nullptr, temp_bytes, d, d, (size_t)n);
-    if (e == cudaSuccess) e = cudaMalloc(&temp, std::max<size_t>(temp_bytes, 16));
+    if (e == cudaSuccess) e = device_malloc(&temp, std::max<size_t>(temp_bytes, 16));
     if (e == cudaSuccess)
         e = inclusive ? cub::DeviceScan::InclusiveSum(temp, temp_bytes, d, d, (size_t)n)
                       : cub::DeviceScan::ExclusiveSum(temp, temp_bytes, d, d, (size_t)n);
@@ -681,7 +681,7 @@ struct PayloadReader {
 struct DevBuf {  // frees what a failed load leaves behind
     void *p = nullptr;
     ~DevBuf() { cudaFree(p); }
-    cudaError_t alloc(uint64_t bytes) { return cudaMalloc(&p, std::max<uint64_t>(bytes, 16)); }
+    cudaError_t alloc(uint64_t bytes) { return device_malloc(&p, std::max<uint64_t>(bytes, 16)); }
     template <typename T> T *as() { return (T *)p; }
     void *release() { void *q = p; p = nullptr; return q; }
 };
@@ -905,9 +905,9 @@ extern "C" int32_t ag_graph_load(const char *path, int32_t validation, int32_t d
     uint32_t crc = 0;
     const bool want_crc = validation == AG_VALIDATE_FULL && checksum != 0;
     do {
-        if (cudaMalloc(&g->offsets, std::max<uint64_t>(off_bytes, 16)) != cudaSuccess ||
-            cudaMalloc(&g->dst, std::max<uint64_t>(edge_bytes, 16)) != cudaSuccess ||
-            (has_w && cudaMalloc(&g->weights, std::max<uint64_t>(w_bytes, 16)) != cudaSuccess)) {
+        if (device_malloc(&g->offsets, std::max<uint64_t>(off_bytes, 16)) != cudaSuccess ||
+            device_malloc(&g->dst, std::max<uint64_t>(edge_bytes, 16)) != cudaSuccess ||
+            (has_w && device_malloc(&g->weights, std::max<uint64_t>(w_bytes, 16)) != cudaSuccess)) {
             st = fail(AG_ERR_CUDA, "out of device memory loading %s: %s", path, cudaGetErrorString(cudaGetLastError()));
             break;
         }
@@ -1005,7 +1005,7 @@ extern "C" int32_t ag_graph_degrees(const ag_graph *g, const uint32_t *ids, uint
     int32_t st = AG_OK;
     do {
         if (ids && (st = upload((void **)&ids_dev, ids, n * 4, AG_MEM_HOST)) != AG_OK) break;
-        if (cudaMalloc(&out_dev, n * 4) != cudaSuccess) { st = fail(AG_ERR_CUDA, "out of device memory"); break; }
+        if (device_malloc(&out_dev, n * 4) != cudaSuccess) { st = fail(AG_ERR_CUDA, "out of device memory"); break; }
         cudaError_t e = launch_degrees(g->offsets, g->num_nodes, ids_dev, n, out_dev, 0);
         if (e == cudaSuccess) e = cudaMemcpy(out, out_dev, n * 4, cudaMemcpyDeviceToHost);
         if (e != cudaSuccess) st = fail(AG_ERR_CUDA, "degrees failed: %s", cudaGetErrorString(e));
@@ -1080,8 +1080,8 @@ int32_t alloc_features(ag_features *f, bool alloc_payload) {
                                      &f->block));
     }
     if (alloc_payload && f->dtype == AG_I8)
-        AG_CUDA(cudaMalloc(&f->scales, std::max<uint64_t>(f->rows * ((f->dim + kQuantBlock - 1) / kQuantBlock) * 4, 16)));
-    AG_CUDA(cudaMalloc(&f->err, 32));  // error bits, then the gather counters (internal.h)
+        AG_CUDA(device_malloc(&f->scales, std::max<uint64_t>(f->rows * ((f->dim + kQuantBlock - 1) / kQuantBlock) * 4, 16)));
+    AG_CUDA(device_malloc(&f->err, 32));  // error bits, then the gather counters (internal.h)
     AG_CUDA(cudaMemset(f->err, 0, 32));
     return AG_OK;
 }
@@ -1276,7 +1276,7 @@ extern "C" int32_t ag_features_from_f32(const float *features, uint64_t num_node
         if (st != AG_OK || count == 0) break;
         const float *src = features;
         if (mem_kind == AG_MEM_HOST) {
-            if (cudaMalloc(&staged, count * 4) != cudaSuccess ||
+            if (device_malloc(&staged, count * 4) != cudaSuccess ||
                 cudaMemcpy(staged, features, count * 4, cudaMemcpyHostToDevice) != cudaSuccess) {
                 st = fail(AG_ERR_CUDA, "feature upload failed: %s", cudaGetErrorString(cudaGetLastError()));
                 break;
@@ -1286,7 +1286,7 @@ extern "C" int32_t ag_features_from_f32(const float *features, uint64_t num_node
         cudaError_t e;
         if (dtype == AG_I8) {
             uint32_t hbad = 0;
-            e = cudaMalloc(&bad, 4);
+            e = device_malloc(&bad, 4);
             if (e == cudaSuccess) e = cudaMemset(bad, 0, 4);
             if (e == cudaSuccess) e = launch_encode_i8(src, num_nodes, dim, (int8_t *)f->payload, f->scales, bad, 0);
             if (e == cudaSuccess) e = cudaMemcpy(&hbad, bad, 4, cudaMemcpyDeviceToHost);

@@ -1103,11 +1103,11 @@ cudaError_t SortScratch::ensure(uint64_t items) {
                                                     (const uint32_t *)nullptr, (uint32_t *)nullptr, want, 0, 32, (cudaStream_t)0);
     if (e != cudaSuccess) return e;
     for (int i = 0; i < 2 && e == cudaSuccess; ++i) {
-        e = cudaMalloc(&keys[i], want * 4);
-        if (e == cudaSuccess) e = cudaMalloc(&vals[i], want * 4);
+        e = device_malloc(&keys[i], want * 4);
+        if (e == cudaSuccess) e = device_malloc(&vals[i], want * 4);
     }
-    if (e == cudaSuccess) e = cudaMalloc(&temp, std::max<size_t>(tb, 16));
-    if (e == cudaSuccess) e = cudaMalloc(&counts, 16);
+    if (e == cudaSuccess) e = device_malloc(&temp, std::max<size_t>(tb, 16));
+    if (e == cudaSuccess) e = device_malloc(&counts, 16);
     if (e != cudaSuccess) { release(); return e; }
     cap = want; temp_bytes = tb;
     return cudaSuccess;

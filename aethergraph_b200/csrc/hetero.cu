@@ -638,7 +638,7 @@ extern "C" int32_t ag_hetero_create(uint32_t num_node_types, const uint64_t *num
     for (uint32_t t = 0; t < num_node_types; ++t) h->num_nodes[t] = num_nodes[t];
     int32_t st = AG_OK;
     uint32_t *bad = nullptr;
-    if (cudaMalloc(&bad, 4) != cudaSuccess) { delete h; return fail(AG_ERR_CUDA, "out of device memory"); }
+    if (device_malloc(&bad, 4) != cudaSuccess) { delete h; return fail(AG_ERR_CUDA, "out of device memory"); }
     for (uint32_t e = 0; e < num_edge_types && st == AG_OK; ++e) {
         if (src_type[e] >= num_node_types || dst_type[e] >= num_node_types) { st = fail(AG_ERR_VALUE, "edge type %u names an unknown node type", e); break; }
         h->src_type[e] = src_type[e]; h->dst_type[e] = dst_type[e]; h->num_edges[e] = num_edges[e];
@@ -648,16 +648,16 @@ extern "C" int32_t ag_hetero_create(uint32_t num_node_types, const uint64_t *num
         uint32_t *a_dev = nullptr, *b_dev = nullptr;
         bool own = false;
         do {
-            if (cudaMalloc(&keys, std::max<uint64_t>(E, 1) * 8) != cudaSuccess) { st = fail(AG_ERR_CUDA, "out of device memory"); break; }
+            if (device_malloc(&keys, std::max<uint64_t>(E, 1) * 8) != cudaSuccess) { st = fail(AG_ERR_CUDA, "out of device memory"); break; }
             cudaMemset(bad, 0, 4);
             if (mem_kind == AG_MEM_HOST) {
                 own = true;
                 if (csr) {
-                    if (cudaMalloc(&off_dev, (ns + 1) * 8) != cudaSuccess || cudaMemcpy(off_dev, rel_offsets[e], (ns + 1) * 8, cudaMemcpyHostToDevice) != cudaSuccess) { st = fail(AG_ERR_CUDA, "upload failed"); break; }
+                    if (device_malloc(&off_dev, (ns + 1) * 8) != cudaSuccess || cudaMemcpy(off_dev, rel_offsets[e], (ns + 1) * 8, cudaMemcpyHostToDevice) != cudaSuccess) { st = fail(AG_ERR_CUDA, "upload failed"); break; }
                 } else if (E) {
-                    if (cudaMalloc(&a_dev, E * 4) != cudaSuccess || cudaMemcpy(a_dev, rel_a[e], E * 4, cudaMemcpyHostToDevice) != cudaSuccess) { st = fail(AG_ERR_CUDA, "upload failed"); break; }
+                    if (device_malloc(&a_dev, E * 4) != cudaSuccess || cudaMemcpy(a_dev, rel_a[e], E * 4, cudaMemcpyHostToDevice) != cudaSuccess) { st = fail(AG_ERR_CUDA, "upload failed"); break; }
                 }
-                if (E && (cudaMalloc(&b_dev, E * 4) != cudaSuccess || cudaMemcpy(b_dev, rel_b[e], E * 4, cudaMemcpyHostToDevice) != cudaSuccess)) { st = fail(AG_ERR_CUDA, "upload failed"); break; }
+                if (E && (device_malloc(&b_dev, E * 4) != cudaSuccess || cudaMemcpy(b_dev, rel_b[e], E * 4, cudaMemcpyHostToDevice) != cudaSuccess)) { st = fail(AG_ERR_CUDA, "upload failed"); break; }
             } else {
                 off_dev = csr ? (uint64_t *)rel_offsets[e] : nullptr;
                 a_dev = csr ? nullptr : (uint32_t *)rel_a[e];

@@ -69,15 +69,15 @@ extern "C" int32_t ag_graph_hot_vertices(const ag_graph *g, uint64_t max_rows, u
         return e == cudaSuccess;
     };
     do {
-        if (!ok(cudaMalloc(&cnt, n * 4), "cudaMalloc(in-degrees)") || !ok(cudaMemset(cnt, 0, n * 4), "cudaMemset")) break;
+        if (!ok(device_malloc(&cnt, n * 4), "device_malloc(in-degrees)") || !ok(cudaMemset(cnt, 0, n * 4), "cudaMemset")) break;
         k_in_degree<<<grid_of(g->num_edges), 256>>>(g->dst, g->num_edges, n, cnt);
         for (int i = 0; i < 2; ++i)
-            if (!ok(cudaMalloc(&keys[i], n * 4), "cudaMalloc(sort keys)") || !ok(cudaMalloc(&vals[i], n * 4), "cudaMalloc(sort values)")) break;
+            if (!ok(device_malloc(&keys[i], n * 4), "device_malloc(sort keys)") || !ok(device_malloc(&vals[i], n * 4), "device_malloc(sort values)")) break;
         if (st != AG_OK) break;
         k_degree_keys<<<grid_of(n), 256>>>(cnt, n, keys[0], vals[0]);
         size_t tb = 0;
         if (!ok(cub::DeviceRadixSort::SortPairs(nullptr, tb, (const uint32_t *)keys[0], keys[1], (const uint32_t *)vals[0], vals[1], n), "sort sizing")) break;
-        if (!ok(cudaMalloc(&temp, std::max<size_t>(tb, 16)), "cudaMalloc(sort temp)")) break;
+        if (!ok(device_malloc(&temp, std::max<size_t>(tb, 16)), "device_malloc(sort temp)")) break;
         if (!ok(cub::DeviceRadixSort::SortPairs(temp, tb, (const uint32_t *)keys[0], keys[1], (const uint32_t *)vals[0], vals[1], n), "radix sort")) break;
         // drop the tail of vertices with in-degree 0 (key 0xFFFFFFFF): find how many of the first max_rows have one
         uint64_t take = std::min<uint64_t>(max_rows, n);
@@ -96,7 +96,7 @@ extern "C" int32_t ag_graph_hot_vertices(const ag_graph *g, uint64_t max_rows, u
             take = lo;
         }
         if (take == 0) break;
-        if (!ok(cudaMalloc(&out, take * 4), "cudaMalloc(hot ids)")) break;
+        if (!ok(device_malloc(&out, take * 4), "device_malloc(hot ids)")) break;
         if (!ok(cudaMemcpy(out, vals[1], take * 4, cudaMemcpyDeviceToDevice), "copy")) break;
         *ids_dev = out; *n_out = take;
         out = nullptr;
@@ -130,7 +130,7 @@ extern "C" int32_t ag_features_cache_rows(ag_features *view, const uint32_t *ids
     uint32_t *slot = nullptr;
     int32_t st = AG_OK;
     do {
-        if (cudaMalloc(&rows, n * row_bytes) != cudaSuccess || cudaMalloc(&slot, view->num_nodes * 4) != cudaSuccess ||
+        if (device_malloc(&rows, n * row_bytes) != cudaSuccess || device_malloc(&slot, view->num_nodes * 4) != cudaSuccess ||
             cudaMemset(slot, 0xFF, view->num_nodes * 4) != cudaSuccess) {
             st = fail(AG_ERR_CUDA, "ag_features_cache_rows: out of device memory for %llu rows: %s", (unsigned long long)n,
                       cudaGetErrorString(cudaGetLastError()));

@@ -34,8 +34,11 @@ cudaError_t workspace_stream(cudaStream_t *out, int priority);  // non-blocking,
 void workspace_stream_free(cudaStream_t stream, int priority);
 template <typename T> cudaError_t workspace_alloc(T **out, size_t bytes) { return workspace_alloc((void **)out, bytes); }
 template <typename T> cudaError_t workspace_alloc_host(T **out, size_t bytes) { return workspace_alloc_host((void **)out, bytes); }
-// Held by every graph and feature store: kept blocks are freed when one is created and
-// when the last one goes.
+// cudaMalloc; when memory is short, once more after the kept blocks are freed.
+cudaError_t device_malloc(void **out, size_t bytes);
+template <typename T> cudaError_t device_malloc(T **out, size_t bytes) { return device_malloc((void **)out, bytes); }
+void workspace_drop();  // frees every kept block and stream
+// Held by every graph and feature store: kept blocks are freed when the last one goes.
 struct WorkspaceUser {
     WorkspaceUser();
     WorkspaceUser(const WorkspaceUser &);

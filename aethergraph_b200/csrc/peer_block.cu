@@ -179,7 +179,7 @@ int32_t alloc_feature_payload(int device, size_t bytes, uint8_t **ptr, PeerBlock
     }();
     *block = nullptr;
     if (plain) {
-        AG_CUDA(cudaMalloc(ptr, bytes));
+        AG_CUDA(device_malloc(ptr, bytes));
         return AG_OK;
     }
     if (peer_block_alloc(device, bytes, block) == AG_OK) {
@@ -195,7 +195,7 @@ int32_t alloc_feature_payload(int device, size_t bytes, uint8_t **ptr, PeerBlock
                         "cudaMalloc, and shards mapped by other processes to legacy CUDA IPC handles\n", ag_last_error());
     });
     *block = nullptr;
-    AG_CUDA(cudaMalloc(ptr, bytes));
+    AG_CUDA(device_malloc(ptr, bytes));
     return AG_OK;
 }
 
@@ -210,6 +210,10 @@ int32_t peer_block_alloc(int device, size_t bytes, PeerBlock **out) {
     PeerBlock *b = new PeerBlock();
     b->device = device; b->size = size;
     CUresult r = d.Create(&b->handle, size, &prop, 0);
+    if (r == CUDA_ERROR_OUT_OF_MEMORY) {
+        workspace_drop();
+        r = d.Create(&b->handle, size, &prop, 0);
+    }
     if (r != CUDA_SUCCESS) {
         delete b;
         return fail(AG_ERR_CUDA, "cuMemCreate of %zu bytes on GPU %d failed: %s", size, device, cu_str(r));

@@ -80,7 +80,7 @@ __global__ void k_fill_permuted(const uint64_t *__restrict__ old_offsets, const 
 struct Dev {
     void *p = nullptr;
     ~Dev() { cudaFree(p); }
-    cudaError_t alloc(uint64_t bytes) { return cudaMalloc(&p, std::max<uint64_t>(bytes, 16)); }
+    cudaError_t alloc(uint64_t bytes) { return device_malloc(&p, std::max<uint64_t>(bytes, 16)); }
     template <typename T> T *as() { return (T *)p; }
     void *release() { void *q = p; p = nullptr; return q; }
 };

@@ -1869,7 +1869,7 @@ extern "C" int32_t ag_sample(ag_sampler *s, const uint32_t *seeds, uint64_t n_se
     b.cap_seeds = std::max<uint64_t>(n_seeds, 1);
     std::vector<void *> mine;
     auto alloc = [&](void **ptr, uint64_t bytes) -> bool {
-        if (cudaMalloc(ptr, bytes) != cudaSuccess) return false;
+        if (device_malloc(ptr, bytes) != cudaSuccess) return false;
         mine.push_back(*ptr);
         return true;
     };

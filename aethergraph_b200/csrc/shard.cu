@@ -56,8 +56,8 @@ int32_t make_view(const ag_features *local, uint32_t world, uint32_t rank, bool 
     t.self = rank;
     t.hot_slot = nullptr;
     t.cyclic = cyclic ? 1u : 0u;
-    if (cudaMalloc(&v->err, 32) != cudaSuccess || cudaMemset(v->err, 0, 32) != cudaSuccess ||
-        cudaMalloc(&v->shards, sizeof(ag_shard_table)) != cudaSuccess ||
+    if (device_malloc(&v->err, 32) != cudaSuccess || cudaMemset(v->err, 0, 32) != cudaSuccess ||
+        device_malloc(&v->shards, sizeof(ag_shard_table)) != cudaSuccess ||
         cudaMemcpy(v->shards, &t, sizeof(t), cudaMemcpyHostToDevice) != cudaSuccess) {
         const int32_t st = fail(AG_ERR_CUDA, "sharded view allocation failed: %s", cudaGetErrorString(cudaGetLastError()));
         ag_features_free(v);

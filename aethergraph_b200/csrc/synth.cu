@@ -247,27 +247,27 @@ int32_t build_relation(uint64_t num_src, uint64_t num_dst, uint64_t num_edges, c
     };
     do {
         const uint64_t kb = std::max<uint64_t>(num_edges, 1) * 8;
-        if (!cuda_ok(cudaMalloc(&keys_a, kb), "cudaMalloc(keys)")) break;
-        if (!cuda_ok(cudaMalloc(&keys_b, kb), "cudaMalloc(keys)")) break;
+        if (!cuda_ok(device_malloc(&keys_a, kb), "device_malloc(keys)")) break;
+        if (!cuda_ok(device_malloc(&keys_b, kb), "device_malloc(keys)")) break;
         k_rmat_keys<<<grid_for(num_edges), 256>>>(p, keys_a);
         if (!cuda_ok(cudaGetLastError(), "k_rmat_keys")) break;
         cub::DoubleBuffer<uint64_t> buf(keys_a, keys_b);
         size_t temp_bytes = 0;
         const int end_bit = 32 + (int)p.bits_src;
         if (!cuda_ok(cub::DeviceRadixSort::SortKeys(nullptr, temp_bytes, buf, (uint64_t)num_edges, 0, end_bit), "sort sizing")) break;
-        if (!cuda_ok(cudaMalloc(&temp, std::max<size_t>(temp_bytes, 16)), "cudaMalloc(sort temp)")) break;
+        if (!cuda_ok(device_malloc(&temp, std::max<size_t>(temp_bytes, 16)), "device_malloc(sort temp)")) break;
         if (!cuda_ok(cub::DeviceRadixSort::SortKeys(temp, temp_bytes, buf, (uint64_t)num_edges, 0, end_bit), "radix sort")) break;
         if (!cuda_ok(cudaDeviceSynchronize(), "radix sort")) break;
         cudaFree(temp); temp = nullptr;
         // keep only the sorted buffer
         uint64_t *sorted = buf.Current();
         if (sorted == keys_a) { cudaFree(keys_b); keys_b = nullptr; } else { cudaFree(keys_a); keys_a = nullptr; }
-        if (!cuda_ok(cudaMalloc(&offsets, (num_src + 1) * 8), "cudaMalloc(offsets)")) break;
-        if (!cuda_ok(cudaMalloc(&dst, std::max<uint64_t>(num_edges, 1) * 4), "cudaMalloc(dst)")) break;
+        if (!cuda_ok(device_malloc(&offsets, (num_src + 1) * 8), "device_malloc(offsets)")) break;
+        if (!cuda_ok(device_malloc(&dst, std::max<uint64_t>(num_edges, 1) * 4), "device_malloc(dst)")) break;
         k_keys_to_csr<<<grid_for(std::max<uint64_t>(num_edges, num_src + 1)), 256>>>(sorted, num_edges, num_src, offsets, dst);
         if (!cuda_ok(cudaGetLastError(), "k_keys_to_csr")) break;
         if (weight_sigma > 0.f) {
-            if (!cuda_ok(cudaMalloc(&w, std::max<uint64_t>(num_edges, 1) * 4), "cudaMalloc(weights)")) break;
+            if (!cuda_ok(device_malloc(&w, std::max<uint64_t>(num_edges, 1) * 4), "device_malloc(weights)")) break;
             k_weights<<<grid_for(num_edges), 256>>>(w, num_edges, mix(seed ^ 0x77656967687473ull), weight_sigma);
             if (!cuda_ok(cudaGetLastError(), "k_weights")) break;
         }
@@ -296,9 +296,9 @@ int32_t build_relation_partitioned(const RmatParams &p, float weight_sigma, uint
         return e == cudaSuccess;
     };
     do {
-        if (!cuda_ok(cudaMalloc(&offsets, (num_src + 1) * 8), "cudaMalloc(offsets)")) break;
-        if (!cuda_ok(cudaMalloc(&dst, std::max<uint64_t>(num_edges, 1) * 4), "cudaMalloc(dst)")) break;
-        if (!cuda_ok(cudaMalloc(&hist_dev, (bins + 1) * 8), "cudaMalloc(histogram)")) break;
+        if (!cuda_ok(device_malloc(&offsets, (num_src + 1) * 8), "device_malloc(offsets)")) break;
+        if (!cuda_ok(device_malloc(&dst, std::max<uint64_t>(num_edges, 1) * 4), "device_malloc(dst)")) break;
+        if (!cuda_ok(device_malloc(&hist_dev, (bins + 1) * 8), "device_malloc(histogram)")) break;
         if (!cuda_ok(cudaMemset(hist_dev, 0, (bins + 1) * 8), "cudaMemset")) break;
         count_dev = hist_dev + bins;
         k_rmat_hist<<<grid_for(num_edges), 256>>>(p, shift, hist_dev);
@@ -316,15 +316,15 @@ int32_t build_relation_partitioned(const RmatParams &p, float weight_sigma, uint
             b = q.hi;
         }
         const uint64_t kb = std::max<uint64_t>(biggest, 1) * 8;
-        if (!cuda_ok(cudaMalloc(&keys_a, kb), "cudaMalloc(keys)")) break;
-        if (!cuda_ok(cudaMalloc(&keys_b, kb), "cudaMalloc(keys)")) break;
+        if (!cuda_ok(device_malloc(&keys_a, kb), "device_malloc(keys)")) break;
+        if (!cuda_ok(device_malloc(&keys_b, kb), "device_malloc(keys)")) break;
         size_t temp_bytes = 0;
         const int end_bit = 32 + (int)p.bits_src;
         {
             cub::DoubleBuffer<uint64_t> probe(keys_a, keys_b);
             if (!cuda_ok(cub::DeviceRadixSort::SortKeys(nullptr, temp_bytes, probe, biggest, 0, end_bit), "sort sizing")) break;
         }
-        if (!cuda_ok(cudaMalloc(&temp, std::max<size_t>(temp_bytes, 16)), "cudaMalloc(sort temp)")) break;
+        if (!cuda_ok(device_malloc(&temp, std::max<size_t>(temp_bytes, 16)), "device_malloc(sort temp)")) break;
         uint64_t base = 0;
         for (const Part &q : parts) {
             const uint64_t row_lo = std::min<uint64_t>((uint64_t)q.lo << shift, num_src);
@@ -347,7 +347,7 @@ int32_t build_relation_partitioned(const RmatParams &p, float weight_sigma, uint
         cudaFree(keys_a); cudaFree(keys_b); cudaFree(temp);
         keys_a = keys_b = nullptr; temp = nullptr;
         if (weight_sigma > 0.f) {
-            if (!cuda_ok(cudaMalloc(&w, std::max<uint64_t>(num_edges, 1) * 4), "cudaMalloc(weights)")) break;
+            if (!cuda_ok(device_malloc(&w, std::max<uint64_t>(num_edges, 1) * 4), "device_malloc(weights)")) break;
             k_weights<<<grid_for(num_edges), 256>>>(w, num_edges, mix(p.seed ^ 0x77656967687473ull), weight_sigma);
             if (!cuda_ok(cudaGetLastError(), "k_weights")) break;
         }
@@ -376,20 +376,20 @@ int32_t keys_to_sorted_csr(uint64_t *keys, uint64_t n, uint64_t num_rows, uint64
     uint64_t *sorted = keys;
     do {
         if (n) {
-            if (!ok(cudaMalloc(&alt, n * 8), "cudaMalloc(sort buffer)")) break;
+            if (!ok(device_malloc(&alt, n * 8), "device_malloc(sort buffer)")) break;
             cub::DoubleBuffer<uint64_t> buf(keys, alt);
             size_t temp_bytes = 0;
             const int end_bit = 32 + (int)bits_for(std::max<uint64_t>(num_rows, 2));
             if (!ok(cub::DeviceRadixSort::SortKeys(nullptr, temp_bytes, buf, n, 0, end_bit), "sort sizing")) break;
-            if (!ok(cudaMalloc(&temp, std::max<size_t>(temp_bytes, 16)), "cudaMalloc(sort temp)")) break;
+            if (!ok(device_malloc(&temp, std::max<size_t>(temp_bytes, 16)), "device_malloc(sort temp)")) break;
             if (!ok(cub::DeviceRadixSort::SortKeys(temp, temp_bytes, buf, n, 0, end_bit), "radix sort")) break;
             if (!ok(cudaDeviceSynchronize(), "radix sort")) break;
             sorted = buf.Current();
             cudaFree(temp); temp = nullptr;
             if (sorted == keys) { cudaFree(alt); alt = nullptr; } else { cudaFree(keys); keys = nullptr; }
         }
-        if (!ok(cudaMalloc(&offsets, (num_rows + 1) * 8), "cudaMalloc(offsets)")) break;
-        if (!ok(cudaMalloc(&vals, std::max<uint64_t>(n, 1) * 4), "cudaMalloc(values)")) break;
+        if (!ok(device_malloc(&offsets, (num_rows + 1) * 8), "device_malloc(offsets)")) break;
+        if (!ok(device_malloc(&vals, std::max<uint64_t>(n, 1) * 4), "device_malloc(values)")) break;
         k_keys_to_csr<<<grid_for(std::max<uint64_t>(n, num_rows + 1)), 256>>>(sorted, n, num_rows, offsets, vals);
         if (!ok(cudaGetLastError(), "k_keys_to_csr")) break;
         ok(cudaDeviceSynchronize(), "k_keys_to_csr");
@@ -434,8 +434,8 @@ extern "C" int32_t ag_synth_fixed_degree_csr(uint64_t num_src, uint64_t num_dst,
     if (!guard.ok) return AG_ERR_CUDA;
     uint64_t *off = nullptr;
     uint32_t *dst = nullptr;
-    AG_CUDA(cudaMalloc(&off, (num_src + 1) * 8));
-    if (cudaMalloc(&dst, std::max<uint64_t>(num_src * degree, 1) * 4) != cudaSuccess) {
+    AG_CUDA(device_malloc(&off, (num_src + 1) * 8));
+    if (device_malloc(&dst, std::max<uint64_t>(num_src * degree, 1) * 4) != cudaSuccess) {
         cudaFree(off);
         return fail(AG_ERR_CUDA, "out of device memory");
     }
@@ -468,10 +468,10 @@ int32_t synth_feature_rows(uint64_t num_nodes, uint64_t dim, int32_t dtype, uint
         float *scales = nullptr, *slab = nullptr;
         uint32_t *bad = nullptr;
         const uint64_t slab_rows = std::max<uint64_t>(1, std::min<uint64_t>(rows, (256ull << 20) / (dim * 4)));
-        cudaError_t e = cudaMalloc(&codes, std::max<uint64_t>(rows * dim, 16));
-        if (e == cudaSuccess) e = cudaMalloc(&scales, std::max<uint64_t>(rows * bpr * 4, 16));
-        if (e == cudaSuccess) e = cudaMalloc(&slab, slab_rows * dim * 4);
-        if (e == cudaSuccess) e = cudaMalloc(&bad, 4);
+        cudaError_t e = device_malloc(&codes, std::max<uint64_t>(rows * dim, 16));
+        if (e == cudaSuccess) e = device_malloc(&scales, std::max<uint64_t>(rows * bpr * 4, 16));
+        if (e == cudaSuccess) e = device_malloc(&slab, slab_rows * dim * 4);
+        if (e == cudaSuccess) e = device_malloc(&bad, 4);
         if (e == cudaSuccess) e = cudaMemset(bad, 0, 4);
         for (uint64_t r0 = 0; r0 < rows && e == cudaSuccess; r0 += slab_rows) {
             const uint64_t m = std::min(slab_rows, rows - r0);

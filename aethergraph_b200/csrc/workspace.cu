@@ -7,8 +7,8 @@
 // Blocks that a handle gives back are kept for the next handle that asks for the size.
 //
 //   * Bounded: kMaxHeld bytes per device and kMaxHeldHost pinned; the blocks kept longest go first.
-//   * Given back: when the last graph and feature store are freed, whenever a new one is
-//     created (those are the large allocations), and when an allocation here fails.
+//   * Given back: when the last graph and feature store are freed, and whenever a device
+//     allocation of the library fails, which is then tried again (device_malloc).
 //   * Ordered: a block is given back only once all work on it has finished, so the next
 //     owner needs no event; contents are whatever they were.
 //   * One lock, held for list operations only; any thread may take and give.
@@ -110,13 +110,17 @@ cudaError_t take(int device, void **out, size_t bytes) {
             return cudaSuccess;
         }
     }
-    auto get = [&](void **p) { return device == kHost ? cudaHostAlloc(p, want, cudaHostAllocDefault) : cudaMalloc(p, want); };
     void *p = nullptr;
-    cudaError_t e = get(&p);
-    if (e == cudaErrorMemoryAllocation) {
-        cudaGetLastError();
-        drop_all();
-        e = get(&p);
+    cudaError_t e;
+    if (device == kHost) {
+        e = cudaHostAlloc(&p, want, cudaHostAllocDefault);
+        if (e == cudaErrorMemoryAllocation) {
+            cudaGetLastError();
+            drop_all();
+            e = cudaHostAlloc(&p, want, cudaHostAllocDefault);
+        }
+    } else {
+        e = device_malloc(&p, want);
     }
     if (e != cudaSuccess) return e;
     std::lock_guard<std::mutex> lk(c.m);
@@ -148,6 +152,16 @@ void give(void *p) {
 }
 
 }  // namespace
+
+cudaError_t device_malloc(void **out, size_t bytes) {
+    const cudaError_t e = cudaMalloc(out, bytes);
+    if (e != cudaErrorMemoryAllocation) return e;
+    cudaGetLastError();
+    drop_all();
+    return cudaMalloc(out, bytes);
+}
+
+void workspace_drop() { drop_all(); }
 
 cudaError_t workspace_alloc(void **out, size_t bytes) {
     int device = 0;
@@ -193,7 +207,6 @@ void workspace_stream_free(cudaStream_t stream, int priority) {
 }
 
 WorkspaceUser::WorkspaceUser() {
-    drop_all();  // a graph or feature table is about to be allocated
     Cache &c = cache();
     std::lock_guard<std::mutex> lk(c.m);
     ++c.users;
