@@ -839,9 +839,10 @@ def run_device(args, w):
                                  "note": "same calls, every batch (int64 ids, local edge index, f32 feature rows) "
                                          "also copied to pinned host memory: PCIe-bound"}},
             "sharded": sharded, "int8_payload": int8_leg, "secondary": secondary,
-            # one launch chain per group of batches (the batch is blockIdx.y): seed insert,
-            # hops + 1 assign, hops pick, gather (sharded: + key, sorted gather, overflow)
-            "gpu_launches": world * chains * (2 * hops + 3 + (3 if sharded_main else 0)),
+            # one launch chain per group of batches (the batch is blockIdx.y): hops + 1 assign (the
+            # first inserts the seeds, up to 2048 a batch; more: a launch of its own), hops pick,
+            # gather (sharded: + key, sorted gather, overflow)
+            "gpu_launches": world * chains * (2 * hops + (2 if bs <= 2048 else 3) + (3 if sharded_main else 0)),
         }
         print(json.dumps(line), flush=True)
     if world > 1:
