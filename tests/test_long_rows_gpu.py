@@ -85,3 +85,16 @@ def test_induced(degrees, seeds, track):
         assert_same_subgraph(sg.raw_u32(), want)
         eil = sg.edge_index_local
         assert np.array_equal(eil[0], want["dst_local"].astype(np.int64)) and np.array_equal(eil[1], want["src_local"].astype(np.int64))
+
+
+def test_induced_without_the_node_filter():
+    """More sampled nodes than the walk keeps a filter for."""
+    import aethergraph_b200 as ag
+    from oracle import ago
+
+    rng = np.random.default_rng(9)
+    n = 200_000
+    off, dst, _ = csr_from_edges(n, rng.integers(0, n, 3 * n).astype(np.uint32), rng.integers(0, n, 3 * n).astype(np.uint32))
+    seeds = rng.permutation(n)[:140_000].astype(np.uint32)
+    s = ag.NeighborSampler(ag.Graph.from_csr(off, dst), ag.SamplingConfig(num_neighbors=[1], subgraph_type="induced", seed=2))
+    assert_same_subgraph(s.sample(seeds).raw_u32(), ago.induce(off, dst, ago.Sampler(off, dst, [1], seed=2).sample(seeds)))
