@@ -164,8 +164,24 @@ constexpr int kPackedSmall = 4032, kPackedMedium = 8128, kPackedLarge = 16320;
 // the whole pipeline gets slower.  A chain that runs alone has no such neighbour, and
 // chain_release (after chain_sync, once all blocks have called it) lets the next kernel
 // be launched while this one works; it still waits for all of this one's results.
+//
+// A dependent kernel can be resident before its predecessor has written what it reads, and a
+// read-only load promises data that does not change while the kernel is resident: neither the
+// compiler nor the cache behind it has to order it behind chain_sync.  So what an earlier
+// kernel of the chain writes (parameter blocks, gather arguments, stage records, tags, ids) is
+// read by ordinary loads after chain_sync, never through a __restrict__ parameter, __ldg or
+// ld.global.nc.  Graph arrays, weights and feature rows are older than the chain.
 __device__ __forceinline__ void chain_sync() {
     asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+// The batch's parameter block in shared memory (behind ordinary stores the compiler would load
+// every field from global memory again).  The whole block calls it, after chain_sync.
+template <typename T>
+__device__ __forceinline__ const T &chain_block(const T *from, T &shared) {
+    static_assert(sizeof(T) % 8 == 0, "copied as 8-byte words");
+    for (uint32_t i = threadIdx.x; i < sizeof(T) / 8; i += blockDim.x) ((uint64_t *)&shared)[i] = ((const uint64_t *)from)[i];
+    __syncthreads();
+    return shared;
 }
 __device__ __forceinline__ void chain_release(uint32_t alone) {
     if (alone) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");

@@ -163,7 +163,7 @@ __device__ __forceinline__ void gather_vec_rows(GatherArgs &a, uint64_t first) {
 
 template <int DTYPE, int LPR>
 __global__ void __launch_bounds__(kThreads)
-k_gather_vec(GatherArgs a, const GatherArgs *__restrict__ group, uint64_t first) {
+k_gather_vec(GatherArgs a, const GatherArgs *group, uint64_t first) {
     chain_sync();
     if (group) a = group[blockIdx.y];  // one batch of a group per grid row
     if (!a.payload) return;
@@ -174,7 +174,7 @@ k_gather_vec(GatherArgs a, const GatherArgs *__restrict__ group, uint64_t first)
 // batch, z the store, whose arguments are group[z * stride + y].
 template <int DTYPE>
 __global__ void __launch_bounds__(kThreads)
-k_gather_stores(const GatherArgs *__restrict__ group, uint32_t stride) {
+k_gather_stores(const GatherArgs *group, uint32_t stride) {
     chain_sync();
     GatherArgs a = group[(uint64_t)blockIdx.z * stride + blockIdx.y];
     if (!a.payload) return;

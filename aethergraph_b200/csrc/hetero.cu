@@ -155,12 +155,13 @@ __global__ void k_het_insert_seeds_packed(const __grid_constant__ PackedWords<BY
 // Same single-pass scan as the homogeneous assign; the demand of a new node is
 // the sum over the edge types into its type.
 __global__ void __launch_bounds__(kTile)
-k_het_assign(const HParams *__restrict__ pa, uint32_t stage, int has_next) {
+k_het_assign(const HParams *pa, uint32_t stage, int has_next) {
     __shared__ uint32_t s_tile;
     __shared__ ScanVal s_warp[kTile / 32];
     __shared__ ScanVal s_prefix;
+    __shared__ __align__(16) HParams s_params;
     chain_sync();
-    const HParams &p = pa[blockIdx.y];
+    const HParams &p = chain_block(pa + blockIdx.y, s_params);
     const HeteroMeta &m = *p.meta;
     BatchState *bs = p.state;
     StageInfo si = bs->stage[stage];
@@ -278,9 +279,10 @@ k_het_assign(const HParams *__restrict__ pa, uint32_t stage, int has_next) {
 // edge type id, the lanes reproduce take-all / Floyd / replace
 // (hetero_sampler.rs:364-422) and emit the edges at consecutive slots.
 __global__ void __launch_bounds__(kPickThreads)
-k_het_pick(const HParams *__restrict__ pa, uint32_t hop) {
+k_het_pick(const HParams *pa, uint32_t hop) {
+    __shared__ __align__(16) HParams s_params;
     chain_sync();
-    const HParams &p = pa[blockIdx.y];
+    const HParams &p = chain_block(pa + blockIdx.y, s_params);
     const HeteroMeta &m = *p.meta;
     const StageInfo nx = p.state->stage[hop + 1];
     const int lane = threadIdx.x & 31;
@@ -352,15 +354,16 @@ constexpr int kClassThreads = 256;
 constexpr int kDescWords = 1 + 2 * kChan;
 
 __global__ void __launch_bounds__(kClassThreads)
-k_class_rank(const HParams *__restrict__ pa) {
+k_class_rank(const HParams *pa) {
     __shared__ uint32_t s_tile;
     __shared__ uint32_t s_cnt[kClassThreads / 32][kChan];   // per warp, per channel: count within the tile
     __shared__ uint32_t s_base[kChan];                      // exclusive prefix of the tile per channel
+    __shared__ __align__(16) HParams s_params;
     chain_sync();
-    const HParams &p = pa[blockIdx.y];
+    const HParams &p = chain_block(pa + blockIdx.y, s_params);
     const bool edges = blockIdx.z != 0;
     const StageInfo fin = p.state->stage[p.meta->num_hops + 1];
-    const uint8_t *__restrict__ tags = edges ? p.edge_tag : p.node_tag;
+    const uint8_t *tags = edges ? p.edge_tag : p.node_tag;
     uint32_t *ranks = edges ? p.edge_rank : p.node_rank;
     uint32_t *totals = edges ? p.et_count : p.type_count;
     uint32_t *tiles = p.class_tiles + (edges ? p.class_tiles_n * kDescWords : 0), *ticket = p.class_ticket + (edges ? 1 : 0);
@@ -465,9 +468,10 @@ k_class_rank(const HParams *__restrict__ pa) {
 
 // Per-type arrays out of the global ones.  Segments: node type t starts at the
 // sum of the counts of the types before it; edge type likewise.
-__global__ void k_het_scatter(const HParams *__restrict__ pa) {
+__global__ void k_het_scatter(const HParams *pa) {
+    __shared__ __align__(16) HParams s_params;
     chain_sync();
-    const HParams &p = pa[blockIdx.y];
+    const HParams &p = chain_block(pa + blockIdx.y, s_params);
     const HeteroMeta &m = *p.meta;
     BatchState *bs = p.state;
     const StageInfo fin = bs->stage[m.num_hops + 1];

@@ -641,9 +641,10 @@ __device__ __forceinline__ void write_item_local(const SampleParams &p, uint32_t
 // broadcasts) — once for the total, once more to place its own draw.  Lane t owns draw t
 // of the current round of 32.
 __global__ void __launch_bounds__(kPickThreads)
-k_pick_weighted_replace(const SampleParams *__restrict__ pa, uint32_t hop, uint32_t k) {
+k_pick_weighted_replace(const SampleParams *pa, uint32_t hop, uint32_t k) {
+    __shared__ __align__(16) SampleParams s_params;
     chain_sync();
-    const SampleParams &p = pa[blockIdx.y];
+    const SampleParams &p = chain_block(pa + blockIdx.y, s_params);
     chain_release(p.alone);
     const StageInfo nx = p.state->stage[hop + 1];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -704,12 +705,13 @@ __device__ __forceinline__ void wl_sort(double *key, uint32_t *pos) {  // whole 
 }
 
 __global__ void __launch_bounds__(kWLThreads)
-k_pick_weighted_large(const SampleParams *__restrict__ pa, uint32_t hop, uint32_t k) {
+k_pick_weighted_large(const SampleParams *pa, uint32_t hop, uint32_t k) {
     __shared__ double s_key[kWLBuf];
     __shared__ uint32_t s_pos[kWLBuf];
     __shared__ uint32_t s_fill;
+    __shared__ __align__(16) SampleParams s_params;
     chain_sync();
-    const SampleParams &p = pa[blockIdx.y];
+    const SampleParams &p = chain_block(pa + blockIdx.y, s_params);
     chain_release(p.alone);
     const StageInfo nx = p.state->stage[hop + 1];
     const double inf = __longlong_as_double(0x7FF0000000000000ll);
@@ -988,10 +990,12 @@ __device__ __forceinline__ void assign_stage(const SampleParams &p, uint32_t sta
 
 template <bool HAS_NEXT, int IPT>
 __global__ void __launch_bounds__(kTile, 2)
-k_assign(const SampleParams *__restrict__ pa, uint32_t stage, uint32_t k) {
+k_assign(const SampleParams *pa, uint32_t stage, uint32_t k) {
+    __shared__ __align__(16) SampleParams s_params;
     chain_sync();
-    chain_release(pa[blockIdx.y].alone);
-    assign_stage<HAS_NEXT, IPT, false>(pa[blockIdx.y], stage, k);
+    const SampleParams &p = chain_block(pa + blockIdx.y, s_params);
+    chain_release(p.alone);
+    assign_stage<HAS_NEXT, IPT, false>(p, stage, k);
 }
 
 // Seed insertion and stage 0 in one launch, a block per batch.
@@ -1032,11 +1036,12 @@ k_assign_seeds_packed(const __grid_constant__ PackedWords<BYTES> c, const StageL
 // frontier, so even a hop with few vertices spreads over the GPU.
 template <int G, int PICK>
 __global__ void __launch_bounds__(PICK == kPickLarge ? 128 : PICK == kPickWeighted ? kWeightedThreads : kPickThreads, PICK == kPickWeighted ? 14 : 1)
-k_pick(const SampleParams *__restrict__ pa, uint32_t hop, uint32_t k) {
+k_pick(const SampleParams *pa, uint32_t hop, uint32_t k) {
     __shared__ uint32_t s_picks[PICK == kPickLarge ? 4 : 1][PICK == kPickLarge ? kLargeK : 1];
     __shared__ uint32_t s_queue[PICK == kPickWeighted ? (kWeightedThreads / 32) * 64 : 1];  // weighted: 64 queued positions per warp
+    __shared__ __align__(16) SampleParams s_params;
     chain_sync();
-    const SampleParams &p = pa[blockIdx.y];
+    const SampleParams &p = chain_block(pa + blockIdx.y, s_params);
     chain_release(p.alone);
     const StageInfo nx = p.state->stage[hop + 1];
     if constexpr (PICK == kPickWeighted) pick_weighted(p, hop, k, nx.n_edges, p.frontier, nx.frontier_n, s_queue);
@@ -1055,34 +1060,43 @@ k_pick(const SampleParams *__restrict__ pa, uint32_t hop, uint32_t k) {
 // 2730 us with the shorter filter and the first threshold guessed, 2320 us with the next
 // weights loaded ahead and slices half as long.
 __global__ void __launch_bounds__(kWeightedThreads, 14)
-k_pick_hub_slices(const SampleParams *__restrict__ pa, uint32_t hop, uint32_t k) {
+k_pick_hub_slices(const SampleParams *pa, uint32_t hop, uint32_t k) {
     __shared__ uint32_t s_queue[(kWeightedThreads / 32) * 64];
+    __shared__ __align__(16) SampleParams s_params[kWeightedThreads / 32];
     chain_sync();
-    const SampleParams &q = pa[0];  // the queue is the same for every batch
-    chain_release(q.alone);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    // the parameter block of the batch this warp is at; what concerns the queue is in every one
+    const SampleParams &p = s_params[warp];
+    uint32_t batch = 0;
+    auto load_params = [&] {
+        __syncwarp();
+        for (uint32_t i = lane; i < sizeof(SampleParams) / 8; i += 32) ((uint64_t *)&s_params[warp])[i] = ((const uint64_t *)(pa + batch))[i];
+        __syncwarp();
+    };
+    load_params();
+    chain_release(p.alone);
     const double inf = __longlong_as_double(0x7FF0000000000000ll);
-    const unsigned long long count = *q.hub_count;
-    const uint32_t rows = min((uint32_t)(count >> 32), q.hub_cap), slices = min((uint32_t)count, q.hub_cap);
+    const unsigned long long count = *p.hub_count;
+    const uint32_t rows = min((uint32_t)(count >> 32), p.hub_cap), slices = min((uint32_t)count, p.hub_cap);
     for (uint32_t slice = blockIdx.x * (kWeightedThreads / 32) + warp; slice < slices; slice += gridDim.x * (kWeightedThreads / 32)) {
         // the last row whose slices start at or before this one; 32 probes a step
         uint32_t lo = 0, n = rows;
         while (n > 1) {
             const uint32_t step = (n + 31) / 32, at = lane * step;
-            const uint32_t m = __ballot_sync(0xffffffffu, at < n && q.hub_rows[lo + at].slice_base <= slice);
+            const uint32_t m = __ballot_sync(0xffffffffu, at < n && p.hub_rows[lo + at].slice_base <= slice);
             const uint32_t hit = 31 - __clz(m);  // lane 0 always holds
             lo += hit * step;
             n = min(step, n - hit * step);
         }
-        const HubRow row = q.hub_rows[lo];
+        const HubRow row = p.hub_rows[lo];
         if (row.n_slices == 0) continue;  // did not fit: its own warp has done it
-        const SampleParams &p = pa[row.batch];
+        if (row.batch != batch) { batch = row.batch; load_params(); }
         const FrontierEntry fe = p.frontier[row.vertex];
-        const uint32_t deg = fe.deg, len = hub_slice_len(deg, q.hub_slice);
+        const uint32_t deg = fe.deg, len = hub_slice_len(deg, p.hub_slice);
         const uint64_t first = (uint64_t)(slice - row.slice_base) * len;
         uint32_t begin = (uint32_t)min((uint64_t)deg, first), end = (uint32_t)min((uint64_t)deg, first + len);
-        float guess = q.hub_guess[lo];
-        uint32_t *shared_thr = q.hub_thr + lo;
+        float guess = p.hub_guess[lo];
+        uint32_t *shared_thr = p.hub_thr + lo;
         double best_key;
         uint32_t best_pos;
         bool mine = true;  // this warp finishes the row
@@ -1090,11 +1104,11 @@ k_pick_hub_slices(const SampleParams *__restrict__ pa, uint32_t hop, uint32_t k)
             topk_stream(p, hop, fe, begin, end, k, lane, best_key, best_pos, s_queue + warp * 64, guess, shared_thr);
             if (!whole) {
                 const uint64_t at = (uint64_t)slice * k;
-                if ((uint32_t)lane < k) { q.hub_key[at + lane] = best_key; q.hub_pos[at + lane] = best_pos; }
+                if ((uint32_t)lane < k) { p.hub_key[at + lane] = best_key; p.hub_pos[at + lane] = best_pos; }
                 __threadfence();
                 __syncwarp();
                 uint32_t before = 0;
-                if (lane == 0) before = atomicAdd(q.hub_done + lo, 1u);
+                if (lane == 0) before = atomicAdd(p.hub_done + lo, 1u);
                 mine = __shfl_sync(0xffffffffu, before, 0) == row.n_slices - 1;
                 if (!mine) break;
                 __threadfence();
@@ -1104,8 +1118,8 @@ k_pick_hub_slices(const SampleParams *__restrict__ pa, uint32_t hop, uint32_t k)
                     const uint32_t i = c + lane;
                     // this slice's own best are in the lanes already
                     const bool have = i < cands && i / k != slice - row.slice_base;
-                    const double ck = have ? __ldcg(q.hub_key + from + i) : inf;
-                    const uint32_t cp = have ? __ldcg(q.hub_pos + from + i) : 0xFFFFFFFFu;
+                    const double ck = have ? __ldcg(p.hub_key + from + i) : inf;
+                    const uint32_t cp = have ? __ldcg(p.hub_pos + from + i) : 0xFFFFFFFFu;
                     topk_insert_chunk(ck, cp, best_key, best_pos, k, lane);
                 }
             }
