@@ -437,7 +437,7 @@ k_class_rank(const HParams *pa) {
                         lost = spins > kSpinLimit;
                     }
                     const uint32_t incls = __ballot_sync(0xffffffffu, incl), losts = __ballot_sync(0xffffffffu, lost);
-                    __threadfence();  // the other lanes' acquires come before this lane's reads
+                    __syncwarp();  // the other lanes' acquires come before this lane's reads
                     const int first = incls ? __ffs(incls) - 1 : 31;  // nearest inclusive prefix, or the whole window
                     // lane = half * 16 + channel: tiles half, half + 2, ... of the window
                     for (int i = lane >> 4; i <= first; i += 2) {

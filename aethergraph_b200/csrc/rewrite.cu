@@ -386,10 +386,12 @@ k_induce_walk(InduceWalk a, InduceOut o) {
     }
     __threadfence();
     __syncthreads();
-    if (threadIdx.x == 0) s_last = atomicAdd((unsigned long long *)(a.total + 1), 1ull) == gridDim.x - 1;
+    if (threadIdx.x == 0) {
+        s_last = atomicAdd((unsigned long long *)(a.total + 1), 1ull) == gridDim.x - 1;
+        __threadfence();  // before the other threads' reads, by the barrier
+    }
     __syncthreads();
     if (!s_last) return;
-    __threadfence();
     uint64_t before = 0;
     for (uint32_t base = 0; base < gridDim.x; base += kWalkThreads) {
         const uint32_t i = base + threadIdx.x;

@@ -1108,10 +1108,10 @@ k_pick_hub_slices(const SampleParams *pa, uint32_t hop, uint32_t k) {
                 __threadfence();
                 __syncwarp();
                 uint32_t before = 0;
-                if (lane == 0) before = atomicAdd(p.hub_done + lo, 1u);
+                if (lane == 0) { before = atomicAdd(p.hub_done + lo, 1u); __threadfence(); }
                 mine = __shfl_sync(0xffffffffu, before, 0) == row.n_slices - 1;
                 if (!mine) break;
-                __threadfence();
+                __syncwarp();  // lane 0's fence comes before the other lanes' reads
                 const uint64_t from = (uint64_t)row.slice_base * k;
                 const uint32_t cands = row.n_slices * k;
                 for (uint32_t c = 0; c < cands; c += 32) {

@@ -50,3 +50,17 @@ def test_no_read_only_view_of_chain_data(params, body):
 
 def test_the_chains_kernels_are_found():
     assert len(list(_chained())) >= 10
+
+
+@pytest.mark.parametrize("file,kernel,observed,read,order", [
+    ("hetero.cu", "k_class_rank", "ld_acquire_u32(tiles", "__ldcg(d", r"__syncwarp\(\)"),
+    ("sampler.cu", "k_pick_hub_slices", "atomicAdd(p.hub_done", "__ldcg(p.hub_key", r"__threadfence\(\).*__syncwarp\(\)"),
+    ("rewrite.cu", "k_induce_walk", "atomicAdd((unsigned long long *)(a.total", "__ldcg(a.block_start", r"__threadfence\(\).*?__syncthreads\(\)"),
+])
+def test_what_one_thread_observes_is_passed_on_by_a_barrier(file, kernel, observed, read, order):
+    """One thread sees that data is complete, others read it: its acquire (or fence) has to come
+    before their reads through a barrier; a vote or a shuffle orders no memory."""
+    body = next(b for n, _, b in _kernels(os.path.join(CSRC, file)) if n == kernel)
+    at = body.index(observed)
+    between = body[at:body.index(read, at)]
+    assert re.search(order, between, re.S), between
