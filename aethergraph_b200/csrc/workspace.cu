@@ -4,7 +4,7 @@
 // worker, two arrays per batch in flight, streams and staging buffers.  cudaMalloc and
 // cudaFree of megabytes take 0.3 - 1.7 ms each while kernels run (cudaFree waits for the
 // whole device), so ten batches of 128 seeds spent 12 - 24 ms on 0.3 ms of kernels.
-// Blocks that a handle gives back are kept for the next handle that asks for the size.
+// Blocks that a handle gives back are kept for the next handle that asks for about the size.
 //
 //   * Bounded: kMaxHeld bytes per device and kMaxHeldHost pinned; the blocks kept longest go first.
 //   * Given back: when the last graph and feature store are freed, and whenever a device
@@ -52,8 +52,12 @@ Cache &cache() {  // never destroyed: handles may be freed during process exit
     return *c;
 }
 
-// Eight sizes per power of two: at most an eighth is rounded up.
-size_t size_class(size_t bytes) {
+// What is asked of the driver for a block.  Large blocks: whole 2 MiB pages, which the driver
+// maps in any case, so that a loader of several GB holds no more than it asked for.  Below that
+// eight sizes per power of two, so that requests which differ from call to call meet again.
+constexpr size_t kPage = 2ull << 20;
+size_t block_size(size_t bytes) {
+    if (bytes >= kPage) return (bytes + kPage - 1) / kPage * kPage;
     size_t step = 512;
     while (step * 16 <= bytes) step *= 2;
     return (std::max<size_t>(bytes, 1) + step - 1) / step * step;
@@ -95,16 +99,20 @@ void drop_all() {
 
 cudaError_t take(int device, void **out, size_t bytes) {
     Cache &c = cache();
-    const size_t want = size_class(bytes);
+    const size_t want = block_size(bytes);
     *out = nullptr;
     {
+        // the smallest kept block that holds the request and is at most an eighth larger
         std::lock_guard<std::mutex> lk(c.m);
-        for (auto it = c.idle.end(); it != c.idle.begin();) {  // newest first
-            --it;
-            if (it->device != device || it->bytes != want) continue;
-            const Block b = *it;
-            c.idle.erase(it);
-            c.held[device] -= want;
+        auto best = c.idle.end();
+        for (auto it = c.idle.begin(); it != c.idle.end(); ++it) {
+            if (it->device != device || it->bytes < want || it->bytes > want + want / 8) continue;
+            if (best == c.idle.end() || it->bytes <= best->bytes) best = it;  // of equal ones the newest
+        }
+        if (best != c.idle.end()) {
+            const Block b = *best;
+            c.idle.erase(best);
+            c.held[device] -= b.bytes;
             c.live.emplace(b.ptr, b);
             *out = b.ptr;
             return cudaSuccess;
