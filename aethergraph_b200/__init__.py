@@ -5,7 +5,7 @@ local edge index, and the feature-row gather with fused f16/bf16 -> f32 upcast,
 as hand-written CUDA kernels (sm_100a) behind a C ABI (include/aethergpu.h) and
 the reference's Python sampler / feature-store / loader surface.
 """
-from ._lib import GraphLoadError, SamplingError
+from ._lib import GraphLoadError, SamplingError, release_kept_memory
 from .features import FeatureStore, save_features
 from .graph import CsrGraph, Graph, partition_aligned_batches
 from .loader import NeighborLoader, PrefetchStats
@@ -20,5 +20,5 @@ __all__ = [
     "HeteroNeighborSampler", "HeteroSampledSubgraph", "HeteroSamplingConfig", "NeighborLoader", "NeighborSampler",
     "ParallelBatchSampler", "PrefetchStats",
     "SampledSubgraph", "Sampler", "SamplingConfig", "SamplingError", "__version__", "partition_aligned_batches",
-    "save_features",
+    "release_kept_memory", "save_features",
 ]

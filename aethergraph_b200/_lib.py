@@ -108,6 +108,7 @@ _I32P = C.POINTER(C.c_int32)
 SIGNATURES = {
     "ag_last_error": (C.c_char_p, []),
     "ag_abi_version": (C.c_int32, []),
+    "ag_release_kept_memory": (None, []),
     "ag_batch_seed": (C.c_uint64, [C.c_uint64, C.c_uint64]),
     "ag_graph_load": (C.c_int32, [C.c_char_p, C.c_int32, C.c_int32, _PP]),
     "ag_graph_from_csr": (C.c_int32, [C.c_uint64, C.c_uint64, _P, _P, _P, C.c_int32, C.c_int32, _PP]),
@@ -232,6 +233,13 @@ def lib():
             fn.argtypes = args
         _lib = L
     return _lib
+
+
+def release_kept_memory() -> None:
+    """Give the GPU back what freed samplers and loaders have left for the next ones (at most
+    512 MiB a device): torch's allocator does not know of it and cannot ask for it when it
+    runs out.  Safe at any time; the next sampler or loader allocates anew."""
+    lib().ag_release_kept_memory()
 
 
 def last_error() -> str:

@@ -8,7 +8,8 @@
 //
 //   * Bounded: kMaxHeld bytes per device and kMaxHeldHost pinned; the blocks kept longest go first.
 //   * Given back: when the last graph and feature store are freed, and whenever a device
-//     allocation of the library fails, which is then tried again (device_malloc).
+//     allocation of the library fails, which is then tried again (device_malloc).  Another
+//     allocator of the process asks for it with ag_release_kept_memory.
 //   * Ordered: a block is given back only once all work on it has finished, so the next
 //     owner needs no event; contents are whatever they were.
 //   * One lock, held for list operations only; any thread may take and give.
@@ -231,3 +232,5 @@ WorkspaceUser::~WorkspaceUser() {
 }
 
 }  // namespace ag
+
+extern "C" void ag_release_kept_memory(void) { ag::workspace_drop(); }

@@ -58,6 +58,11 @@ typedef struct ag_loader ag_loader;
 const char *ag_last_error(void);
 /* ABI version of this header; bumped on any incompatible change. */
 int32_t ag_abi_version(void);
+/* Handles that were freed leave device blocks (at most 512 MiB a device), pinned
+ * blocks (64 MiB) and idle streams for the next handle, until the last graph and
+ * feature store are freed or an allocation of this library fails.  This gives them
+ * back now, for a caller whose own allocator has run out; any thread, any time. */
+void ag_release_kept_memory(void);
 
 /* ------------------------------------------------------------------ RNG --
  * crates/aethergraph-core/src/loader/sampler.rs:69-75 (batch_seed). */

@@ -121,6 +121,15 @@ def test_a_failed_request_is_tried_again_without_the_kept_blocks(ws):
     assert ws.t_alloc(500 * MiB)
 
 
+def test_kept_memory_can_be_asked_back(ws):
+    held = ws.t_alloc(10 * MiB)
+    ws.t_free(ws.t_alloc(100 * MiB))
+    ws.ag_release_kept_memory()
+    assert ws.t_used() == 10 * MiB
+    ws.t_free(held)
+    assert ws.t_alloc(10 * MiB) == held
+
+
 def test_the_last_user_gives_everything_back(ws):
     second = ws.t_user()
     ws.t_free(ws.t_alloc(100 * MiB))

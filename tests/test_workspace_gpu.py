@@ -80,6 +80,10 @@ alone = used()
 loaders(g, [100, 1000, 8000, 50, 20000, 700])
 kept = used() - alone
 assert kept <= 512 + 64, kept
+ag.release_kept_memory()
+released = used() - alone
+assert kept > 64 and released <= 16, (kept, released)
+loaders(g, [100, 20000])  # and work goes on
 del g
 after = used()
 assert after <= before + 16, (before, after)
