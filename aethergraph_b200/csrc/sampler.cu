@@ -1034,8 +1034,13 @@ k_assign_seeds_packed(const __grid_constant__ PackedWords<BYTES> c, const StageL
 // Hop `hop`: expand the frontier stage `hop` queued (stage[hop + 1] holds its
 // size and where the hop's edges start).  The lanes of the whole grid share the
 // frontier, so even a hop with few vertices spreads over the GPU.
+//
+// Latency-bound, so resident warps count: six blocks of 256 threads per SM, which leaves 40
+// registers a thread.  Asked for one block the compiler takes 48 to 53, and the long chains of
+// two workers lose 1.3 % (64 batches of 1024 seeds, fanouts 25, 10, on 100 M vertices / 2 B
+// edges: 6.54 ms for 512 batches against 6.45).
 template <int G, int PICK>
-__global__ void __launch_bounds__(PICK == kPickLarge ? 128 : PICK == kPickWeighted ? kWeightedThreads : kPickThreads, PICK == kPickWeighted ? 14 : 1)
+__global__ void __launch_bounds__(PICK == kPickLarge ? 128 : PICK == kPickWeighted ? kWeightedThreads : kPickThreads, PICK == kPickWeighted ? 14 : PICK == kPickLarge ? 12 : 6)
 k_pick(const SampleParams *pa, uint32_t hop, uint32_t k) {
     __shared__ uint32_t s_picks[PICK == kPickLarge ? 4 : 1][PICK == kPickLarge ? kLargeK : 1];
     __shared__ uint32_t s_queue[PICK == kPickWeighted ? (kWeightedThreads / 32) * 64 : 1];  // weighted: 64 queued positions per warp
