@@ -106,9 +106,10 @@ struct SampleParams {
     FrontierEntry *frontier;
     uint64_t frontier_cap;
     // weighted only, shared by the batches of a chain: the rows left to k_pick_hub_slices
-    HubRow *hub_rows;                // [hub_cap]
-    unsigned long long *hub_count;   // rows queued << 32 | slices handed out
-    uint32_t *hub_thr, *hub_done;    // [hub_cap] per row: lowest k-th best key so far (float bits), slices finished
+    // rows, thresholds and done counts twice: [0] the hop's rows, [1] those whose guess was too low
+    HubRow *hub_rows;                // [2][hub_cap]
+    unsigned long long *hub_count;   // [2] rows queued << 32 | slices handed out
+    uint32_t *hub_thr, *hub_done;    // [2][hub_cap] per row: lowest k-th best key so far (float bits), slices finished
     float *hub_guess;                // [hub_cap] the threshold the row started with
     double *hub_key;                 // [hub_cap][k] the slices' best (key, position) pairs
     uint32_t *hub_pos;
@@ -393,11 +394,15 @@ __device__ __forceinline__ double weighted_key(const SampleParams &p, uint32_t h
 // than the rounding of the three f32 products (3 * 2^-24 relative, 1e-5 is granted;
 // 1 + uf and 1 - uf are exact), the exact key cannot be below the threshold and the
 // position is dropped.  A weight that is not positive and finite has key +inf, which a
-// finite threshold beats: 0 and negative weights are dropped by the same comparison, NaN
-// and +inf (and a product that overflows) compare false and survive to stage 2.
-// Survivors are only queued (`buf`, 64 slots of the warp's shared memory).  Stage 2,
-// whenever 32 are queued: every lane evaluates one queued position exactly and the
-// winners are inserted.
+// finite threshold beats: 0, negative weights and NaN are dropped by the same comparison,
+// +inf (and a product that overflows) survives to stage 2.  Survivors are only queued
+// (`buf`, kQueue slots of the warp's shared memory).  Stage 2, whenever 32 are queued: every
+// lane evaluates one queued position exactly and the winners are inserted.
+//
+// Without a threshold the first 32 positions are evaluated at once, which holds k of them.
+// If the k-th best key is still +inf then, a later position whose key is +inf as well comes
+// after the k held (equal keys go by position), so weights that are not positive can be
+// dropped from there on: the factor +inf keeps exactly the positive ones.
 //
 // The threshold is the lowest of `guess`, the k-th best key at the last flush and, when
 // several warps stream slices of one row, `shared_thr`, the lowest k-th best any of them
@@ -409,9 +414,11 @@ __device__ __forceinline__ double weighted_key(const SampleParams &p, uint32_t h
 //
 // Bound: instructions, about 30 for 32 positions in stage 1 and 500 for a flush, so what
 // counts is the multiply of the random stream (wyrand_top32) and the number of flushes
-// (guess_threshold).  kChunks * 32 positions are loaded and filtered together and only
+// (guess_threshold, and the first chunk on its own where there is no threshold).  One place
+// in the code flushes: with three inlined copies the kernels spill.  kChunks * 32 positions are loaded and filtered together and only
 // then asked for survivors, with one vote, while the next ones are loaded.
 constexpr uint32_t kChunks = 4;
+constexpr uint32_t kQueue = 32 + 32 * kChunks;  // what a flush leaves (fewer than 32) and one round's survivors
 
 template <bool PHILOX>
 __device__ __forceinline__ void topk_stream_rng(const SampleParams &p, uint32_t hop, const FrontierEntry &fe, uint32_t begin,
@@ -420,45 +427,56 @@ __device__ __forceinline__ void topk_stream_rng(const SampleParams &p, uint32_t 
     uint32_t queued = 0;  // warp-uniform
     bool fresh = true;    // nothing inserted yet
     float thr = guess;
-    auto flush = [&](uint32_t count) {  // evaluate buf[0 .. count) exactly, one per lane, and insert the winners
-        double key = __longlong_as_double(0x7FF0000000000000ll);
-        uint32_t cpos = 0xFFFFFFFFu;
-        if ((uint32_t)lane < count) {
-            cpos = buf[lane];
-            key = weighted_key(p, hop, fe, cpos);
-        }
-        if (fresh) {
-            warp_sort_pairs(key, cpos, lane);
-            best_key = key; best_pos = cpos;
-            fresh = false;
-        } else {
-            topk_insert_chunk(key, cpos, best_key, best_pos, k, lane);
-        }
-        const double kth = __shfl_sync(0xffffffffu, best_key, k - 1);
-        thr = fminf(thr, (float)kth);
-        if (shared_thr) {
-            const float up = __double2float_ru(kth);  // rounded up: still an upper bound
-            if (lane == 0 && up < 3.0e38f) atomicMin(shared_thr, __float_as_uint(up));
-        }
-    };
+    auto threshold = [&] { return shared_thr ? fminf(thr, __uint_as_float(__ldcg(shared_thr))) : thr; };
     const float *w = p.weights + fe.off + begin + lane;
     constexpr uint64_t kStep = 0xa0761d6478bd642full;  // from one draw's state to the next (wyrand_at)
     const uint64_t seed = p.seed;
     uint32_t first = begin + lane;  // this lane's position in the next chunk
     uint64_t state = seed + (fe.dbase + first + 1ull) * kStep;
-    float wf[kChunks];  // the weights of the next kChunks * 32 positions
+    float wf[kChunks];  // the weights of the next kChunks * 32 positions; past the end: negative, dropped
 #pragma unroll
-    for (uint32_t u = 0; u < kChunks; ++u) wf[u] = u * 32 + lane < end - begin ? __ldg(w + u * 32) : 0.0f;
-    for (uint32_t left = end - begin; left > 0;) {
+    for (uint32_t u = 0; u < kChunks; ++u) wf[u] = u * 32 + lane < end - begin ? __ldg(w + u * 32) : -1.0f;
+    uint32_t left = end - begin;
+    __syncwarp();  // the queue may have been another stream's
+    if (!(__shfl_sync(0xffffffffu, threshold(), 0) <= 3.0e38f)) {  // no threshold: the first chunk as it is
+        buf[lane] = first;
+        queued = min(32u, left);
+        wf[0] = -1.0f;
+    }
+    for (bool drain = queued > 0;;) {
+        // evaluate 32 queued positions exactly, one per lane, and insert the winners
+        while (queued >= 32 || (drain && queued > 0)) {
+            const uint32_t count = min(queued, 32u);
+            queued -= count;
+            __syncwarp();
+            double key = __longlong_as_double(0x7FF0000000000000ll);
+            uint32_t cpos = 0xFFFFFFFFu;
+            if ((uint32_t)lane < count) {
+                cpos = buf[queued + lane];
+                key = weighted_key(p, hop, fe, cpos);
+            }
+            if (fresh) {
+                warp_sort_pairs(key, cpos, lane);
+                best_key = key; best_pos = cpos;
+                fresh = false;
+            } else {
+                topk_insert_chunk(key, cpos, best_key, best_pos, k, lane);
+            }
+            const double kth = __shfl_sync(0xffffffffu, best_key, k - 1);
+            thr = fminf(thr, (float)kth);
+            if (shared_thr) {
+                const float up = __double2float_ru(kth);  // rounded up: still an upper bound
+                if (lane == 0 && up < 3.0e38f) atomicMin(shared_thr, __float_as_uint(up));
+            }
+        }
+        if (left == 0) break;
         // those after them are on their way while these are filtered
         float ahead[kChunks];
 #pragma unroll
         for (uint32_t u = 0; u < kChunks; ++u)
-            ahead[u] = left > 32 * kChunks && u * 32 + lane < left - 32 * kChunks ? __ldg(w + 32 * kChunks + u * 32) : 0.0f;
-        float t = thr;
-        if (shared_thr) t = fminf(t, __uint_as_float(__ldcg(shared_thr)));
-        // NaN: nothing is dropped
-        const float ts = (t >= 1.0e-30f && t <= 3.0e38f) ? t * 1.00001f : __uint_as_float(0x7FC00000u);
+            ahead[u] = left > 32 * kChunks && u * 32 + lane < left - 32 * kChunks ? __ldg(w + 32 * kChunks + u * 32) : -1.0f;
+        const float t = threshold();
+        const float ts = (t >= 1.0e-30f && t <= 3.0e38f) ? t * 1.00001f : __uint_as_float(0x7F800000u);
         bool kept[kChunks], any = false;
 #pragma unroll
         for (uint32_t u = 0; u < kChunks; ++u) {
@@ -466,27 +484,16 @@ __device__ __forceinline__ void topk_stream_rng(const SampleParams &p, uint32_t 
                                         : wyrand_top32(state + u * 32 * kStep);
             const float above = __uint_as_float(0x3F800000u | (top >> 9)) + 1.1920928955078125e-07f;  // 1 + uf
             const float below = 2.0f - above;                                                           // 1 - uf
-            kept[u] = u * 32 + lane < left && !(2.0f * below > above * (ts * wf[u]));
+            kept[u] = 2.0f * below <= above * (ts * wf[u]);
             any = any || kept[u];
         }
         if (__any_sync(0xffffffffu, any)) {
+            __syncwarp();  // the queue's last reads are done
 #pragma unroll
             for (uint32_t u = 0; u < kChunks; ++u) {
                 const uint32_t m = __ballot_sync(0xffffffffu, kept[u]);
-                if (!m) continue;
                 if (kept[u]) buf[queued + __popc(m & ((1u << lane) - 1u))] = first + u * 32;
                 queued += __popc(m);
-                __syncwarp();
-                if (queued >= 32) {
-                    flush(32);
-                    __syncwarp();
-                    const uint32_t rest = queued - 32;  // < 32: move the tail to the front
-                    const uint32_t moved = (uint32_t)lane < rest ? buf[32 + lane] : 0;
-                    __syncwarp();
-                    if ((uint32_t)lane < rest) buf[lane] = moved;
-                    queued = rest;
-                    __syncwarp();
-                }
             }
         }
         w += 32 * kChunks;
@@ -495,8 +502,8 @@ __device__ __forceinline__ void topk_stream_rng(const SampleParams &p, uint32_t 
 #pragma unroll
         for (uint32_t u = 0; u < kChunks; ++u) wf[u] = ahead[u];
         left -= min(left, 32 * kChunks);
+        drain = left == 0;
     }
-    if (queued) { flush(queued); __syncwarp(); }
 }
 
 __device__ __forceinline__ void topk_stream(const SampleParams &p, uint32_t hop, const FrontierEntry &fe, uint32_t begin,
@@ -517,8 +524,15 @@ __device__ __forceinline__ float guess_threshold(float mean, float n, float want
     return (want < 0.75f * n && t > 1.0e-30f && t < 3.0e38f) ? t : __uint_as_float(0x7F800000u);
 }
 
+// A lane's share of a row's weight above which the row counts as skewed, in means.  Weights of
+// one size stay below, log-normal ones of sigma 1 nearly always.  Eight batches of 1024 seeds,
+// fanouts 15, 10, rows of 128 to 2048 positions: Pareto weights (exponent 1/2) 765 us, 1810
+// from the mean alone (most rows streamed twice); log-normal 655.
+constexpr float kSkew = 6.0f;
+
 // Sum of `count` weights of a row, `step` apart, that are positive and finite (warp-wide).
-__device__ __forceinline__ float weight_sum(const float *w, uint32_t count, uint64_t step, int lane) {
+// *skewed: a lane's share is far from the others', so the mean says little about the keys.
+__device__ __forceinline__ float weight_sum(const float *w, uint32_t count, uint64_t step, int lane, bool *skewed) {
     float sum = 0.0f;
     for (uint32_t c = 0; c < count; c += 32 * kChunks) {
         float v[kChunks];
@@ -530,9 +544,41 @@ __device__ __forceinline__ float weight_sum(const float *w, uint32_t count, uint
 #pragma unroll
         for (uint32_t u = 0; u < kChunks; ++u) sum += (v[u] > 0.0f && v[u] < 3.0e38f) ? v[u] : 0.0f;
     }
+    const float share = sum;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+    *skewed = __any_sync(0xffffffffu, !(share > 0.0f && share * 32.0f < sum * kSkew));
     return sum;
+}
+
+// The threshold for a skewed row: of the sampled weights about `target` keys should fall below
+// t.  A key does with probability 1 - exp(-t w), bounded by min(t w, 1); the sum of the bounds
+// is concave in t and linear between the places where a weight reaches 1, so from the left
+// Newton's steps approach the place where it is `target`, and a third more makes up for the
+// bound.  +inf if fewer weights than that are positive.
+__device__ __forceinline__ float skewed_threshold(const float *w, uint32_t count, uint64_t step, float t, float target, int lane) {
+    const float inff = __uint_as_float(0x7F800000u);
+    if (!(t < 3.0e38f)) return inff;
+    for (int round = 0; round < 12; ++round) {
+        float rest = 0.0f, full = 0.0f;  // weights with t w < 1, number of the others
+        for (uint32_t i = lane; i < count; i += 32) {
+            const float v = __ldg(w + i * step);
+            if (!(v > 0.0f && v < 3.0e38f)) continue;
+            if (t * v < 1.0f) rest += v; else full += 1.0f;
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            rest += __shfl_xor_sync(0xffffffffu, rest, o);
+            full += __shfl_xor_sync(0xffffffffu, full, o);
+        }
+        if (full >= target) break;
+        if (!(rest > 0.0f)) return inff;
+        const float next = (target - full) / rest;
+        if (!(next > 1.05f * t)) break;
+        t = next;
+    }
+    t *= 1.33f;
+    return t > 1.0e-30f && t < 3.0e38f ? t : inff;
 }
 
 // Warps per block of the weighted picks: few, so that a block's slots are free again as
@@ -552,6 +598,28 @@ __device__ __forceinline__ uint32_t hub_slice_len(uint32_t deg, uint32_t slice) 
     return max(slice, (deg / kMaxSlicesPerRow + 32u) & ~31u);
 }
 
+// Queues a long row for k_pick_hub_slices<again> with a threshold to start from; false if its
+// slices do not fit the queue.  Warp-wide.
+__device__ __forceinline__ bool queue_long_row(const SampleParams &p, uint32_t again, uint32_t batch, uint32_t vertex, uint32_t deg,
+                                               float thr, int lane) {
+    bool queued = false;
+    if (lane == 0) {
+        const uint32_t len = hub_slice_len(deg, again ? kHubDegree : p.hub_slice), slices = (deg - 1) / len + 1;
+        // one atomic for both counters: the rows' slice ranges ascend in queue order
+        const unsigned long long at = atomicAdd(p.hub_count + again, (1ull << 32) | slices);
+        const uint32_t h = (uint32_t)(at >> 32), base = (uint32_t)at;
+        queued = (uint64_t)base + slices <= p.hub_cap;
+        if (h < p.hub_cap) {
+            const uint32_t to = again * p.hub_cap + h;
+            p.hub_rows[to] = HubRow{batch, vertex, base, queued ? slices : 0u};
+            p.hub_thr[to] = __float_as_uint(thr);
+            p.hub_done[to] = 0;
+            if (!again) p.hub_guess[h] = thr;
+        }
+    }
+    return __shfl_sync(0xffffffffu, queued, 0);
+}
+
 __device__ __forceinline__ void pick_weighted(const SampleParams &p, uint32_t hop, uint32_t k, uint32_t edges_before,
                                               const FrontierEntry *fes, uint32_t n, uint32_t *queue) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -565,37 +633,27 @@ __device__ __forceinline__ void pick_weighted(const SampleParams &p, uint32_t ho
             continue;
         }
         if (deg > kHubDegree) {  // queue the row for the slice kernel
-            // Many more than k: one wrong guess costs the whole row again, by one warp.
-            const float guess = guess_threshold(weight_sum(p.weights + fe.off, kSampledWeights, deg / kSampledWeights, lane) / kSampledWeights,
+            // Many more than k: a wrong guess costs the whole row again.
+            bool skewed;
+            const float guess = guess_threshold(weight_sum(p.weights + fe.off, kSampledWeights, deg / kSampledWeights, lane, &skewed) / kSampledWeights,
                                                 (float)deg, 4.0f * (float)k + 64.0f);
-            bool queued = false;
-            if (lane == 0) {
-                const uint32_t len = hub_slice_len(deg, p.hub_slice), slices = (deg - 1) / len + 1;
-                // one atomic for both counters: the rows' slice ranges ascend in queue order
-                const unsigned long long at = atomicAdd(p.hub_count, (1ull << 32) | slices);
-                const uint32_t h = (uint32_t)(at >> 32), base = (uint32_t)at;
-                queued = (uint64_t)base + slices <= p.hub_cap;
-                if (h < p.hub_cap) {
-                    p.hub_rows[h] = HubRow{blockIdx.y, j, base, queued ? slices : 0u};
-                    p.hub_guess[h] = guess;
-                    p.hub_thr[h] = __float_as_uint(guess);
-                    p.hub_done[h] = 0;
-                }
-            }
-            if (__shfl_sync(0xffffffffu, queued, 0)) continue;
+            if (queue_long_row(p, 0, blockIdx.y, j, deg, guess, lane)) continue;
         }
         const float inff = __uint_as_float(0x7F800000u);
         float guess = inff;
         if (deg >= kGuessDegree) {
             // enough to be right nineteen times in twenty or better, few enough for one flush
             const float want = (float)k + 2.0f * sqrtf((float)k) + 2.0f;
-            guess = guess_threshold(weight_sum(p.weights + fe.off, min(deg, kSampledWeights), deg > kSampledWeights ? deg / kSampledWeights : 1, lane) /
-                                        (float)min(deg, kSampledWeights), (float)deg, want);
+            const uint32_t count = min(deg, kSampledWeights), step = deg > kSampledWeights ? deg / kSampledWeights : 1;
+            const float *w = p.weights + fe.off;
+            bool skewed;
+            guess = guess_threshold(weight_sum(w, count, step, lane, &skewed) / (float)count, (float)deg, want);
+            if (skewed) guess = skewed_threshold(w, count, step, guess, want * ((float)count / (float)deg), lane);
         }
         double best_key;
         uint32_t best_pos;
         for (;; guess = inff) {  // again without the guess if it was too low
-            topk_stream(p, hop, fe, 0, deg, k, lane, best_key, best_pos, queue + warp * 64, guess);
+            topk_stream(p, hop, fe, 0, deg, k, lane, best_key, best_pos, queue + warp * kQueue, guess);
             if (__shfl_sync(0xffffffffu, best_key, k - 1) <= (double)guess) break;
         }
         if ((uint32_t)lane < k) emit_edge(p, hop, edges_before, fe, lane, fe.off + best_pos);
@@ -897,7 +955,7 @@ __device__ __forceinline__ void assign_stage(const SampleParams &p, uint32_t sta
                     nx.hop_draws = 0;
                     bs->stage[stage + 1] = nx;
                     bs->nodes_per_stage[stage] = tot.flags;
-                    if (p.hub_count) *p.hub_count = 0;  // the hop's hub queue starts empty (every batch says so)
+                    if (p.hub_count) p.hub_count[0] = p.hub_count[1] = 0;  // the hop's queues start empty (every batch says so)
                     if (stage == 0) bs->stage[0] = si;  // what the counts measure the draws against
                 }
             }
@@ -1043,7 +1101,7 @@ template <int G, int PICK>
 __global__ void __launch_bounds__(PICK == kPickLarge ? 128 : PICK == kPickWeighted ? kWeightedThreads : kPickThreads, PICK == kPickWeighted ? 14 : PICK == kPickLarge ? 12 : 6)
 k_pick(const SampleParams *pa, uint32_t hop, uint32_t k) {
     __shared__ uint32_t s_picks[PICK == kPickLarge ? 4 : 1][PICK == kPickLarge ? kLargeK : 1];
-    __shared__ uint32_t s_queue[PICK == kPickWeighted ? (kWeightedThreads / 32) * 64 : 1];  // weighted: 64 queued positions per warp
+    __shared__ uint32_t s_queue[PICK == kPickWeighted ? (kWeightedThreads / 32) * kQueue : 1];  // weighted: queued positions per warp
     __shared__ __align__(16) SampleParams s_params;
     chain_sync();
     const SampleParams &p = chain_block(pa + blockIdx.y, s_params);
@@ -1059,14 +1117,19 @@ k_pick(const SampleParams *pa, uint32_t hop, uint32_t k) {
 // merges them and emits.  (key, position) is a total order, so the k smallest — and their
 // emission order — do not depend on how the row was split or which warp merges.
 //
-// A row of 500 K positions on one block of 512 threads took 450 us, as long for one batch
-// as for eight.  Twelve batches of 512 seeds, fanouts 15, 10, 5, on the 10 M vertex / 200 M
-// edge graph (28 M positions a batch): 5320 us with a block per row, 3600 us with slices,
-// 2730 us with the shorter filter and the first threshold guessed, 2320 us with the next
-// weights loaded ahead and slices half as long.
+// Why slices: a row of 500 K positions takes one block of 512 threads 450 us, whatever the rest
+// of the chain does.  Twelve batches of 512 seeds, fanouts 15, 10, 5, on a graph of 10 M vertices
+// and 200 M edges (28 M positions a batch): 5330 us with a block per row, 2070 us in slices.
+//
+// A guessed threshold below the row's k-th best key shows at the merge.  The row is then queued
+// once more and a second launch (AGAIN) streams it in slices without a guess.  512 seeds,
+// fanouts 15, 10, rows of up to 220 K positions: log-normal weights 175 us; one weight of a
+// row 1e6 times the others 240 (870 if the merging warp streams the row alone); eight positive
+// weights a row, the rest zero, 210 (3870 alone).
+template <bool AGAIN>
 __global__ void __launch_bounds__(kWeightedThreads, 14)
 k_pick_hub_slices(const SampleParams *pa, uint32_t hop, uint32_t k) {
-    __shared__ uint32_t s_queue[(kWeightedThreads / 32) * 64];
+    __shared__ uint32_t s_queue[(kWeightedThreads / 32) * kQueue];
     __shared__ __align__(16) SampleParams s_params[kWeightedThreads / 32];
     chain_sync();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -1081,39 +1144,40 @@ k_pick_hub_slices(const SampleParams *pa, uint32_t hop, uint32_t k) {
     load_params();
     chain_release(p.alone);
     const double inf = __longlong_as_double(0x7FF0000000000000ll);
-    const unsigned long long count = *p.hub_count;
+    const unsigned long long count = p.hub_count[AGAIN];
     const uint32_t rows = min((uint32_t)(count >> 32), p.hub_cap), slices = min((uint32_t)count, p.hub_cap);
+    const uint32_t half = AGAIN ? p.hub_cap : 0u;
     for (uint32_t slice = blockIdx.x * (kWeightedThreads / 32) + warp; slice < slices; slice += gridDim.x * (kWeightedThreads / 32)) {
         // the last row whose slices start at or before this one; 32 probes a step
         uint32_t lo = 0, n = rows;
         while (n > 1) {
             const uint32_t step = (n + 31) / 32, at = lane * step;
-            const uint32_t m = __ballot_sync(0xffffffffu, at < n && p.hub_rows[lo + at].slice_base <= slice);
+            const uint32_t m = __ballot_sync(0xffffffffu, at < n && p.hub_rows[half + lo + at].slice_base <= slice);
             const uint32_t hit = 31 - __clz(m);  // lane 0 always holds
             lo += hit * step;
             n = min(step, n - hit * step);
         }
-        const HubRow row = p.hub_rows[lo];
+        const HubRow row = p.hub_rows[half + lo];
         if (row.n_slices == 0) continue;  // did not fit: its own warp has done it
         if (row.batch != batch) { batch = row.batch; load_params(); }
         const FrontierEntry fe = p.frontier[row.vertex];
-        const uint32_t deg = fe.deg, len = hub_slice_len(deg, p.hub_slice);
+        const uint32_t deg = fe.deg, len = hub_slice_len(deg, AGAIN ? kHubDegree : p.hub_slice);
         const uint64_t first = (uint64_t)(slice - row.slice_base) * len;
         uint32_t begin = (uint32_t)min((uint64_t)deg, first), end = (uint32_t)min((uint64_t)deg, first + len);
-        float guess = p.hub_guess[lo];
-        uint32_t *shared_thr = p.hub_thr + lo;
+        float guess = AGAIN ? __uint_as_float(0x7F800000u) : p.hub_guess[lo];
+        uint32_t *shared_thr = p.hub_thr + half + lo;
         double best_key;
         uint32_t best_pos;
         bool mine = true;  // this warp finishes the row
         for (bool whole = row.n_slices == 1;; whole = true) {
-            topk_stream(p, hop, fe, begin, end, k, lane, best_key, best_pos, s_queue + warp * 64, guess, shared_thr);
+            topk_stream(p, hop, fe, begin, end, k, lane, best_key, best_pos, s_queue + warp * kQueue, guess, shared_thr);
             if (!whole) {
                 const uint64_t at = (uint64_t)slice * k;
                 if ((uint32_t)lane < k) { p.hub_key[at + lane] = best_key; p.hub_pos[at + lane] = best_pos; }
                 __threadfence();
                 __syncwarp();
                 uint32_t before = 0;
-                if (lane == 0) { before = atomicAdd(p.hub_done + lo, 1u); __threadfence(); }
+                if (lane == 0) { before = atomicAdd(p.hub_done + half + lo, 1u); __threadfence(); }
                 mine = __shfl_sync(0xffffffffu, before, 0) == row.n_slices - 1;
                 if (!mine) break;
                 __syncwarp();  // lane 0's fence comes before the other lanes' reads
@@ -1128,8 +1192,11 @@ k_pick_hub_slices(const SampleParams *pa, uint32_t hop, uint32_t k) {
                     topk_insert_chunk(ck, cp, best_key, best_pos, k, lane);
                 }
             }
-            if (__shfl_sync(0xffffffffu, best_key, k - 1) <= (double)guess) break;
-            // the guess was too low: the whole row once more without one
+            if (AGAIN || __shfl_sync(0xffffffffu, best_key, k - 1) <= (double)guess) break;
+            // The guess was too low: the row once more without one, by this warp if the queue is full.
+            // (What was found bounds the k-th best key from above, if k were found.)
+            const float bound = __double2float_ru(__shfl_sync(0xffffffffu, best_key, k - 1));
+            if (queue_long_row(p, 1, row.batch, row.vertex, deg, bound, lane)) { mine = false; break; }
             begin = 0; end = deg; guess = __uint_as_float(0x7F800000u); shared_thr = nullptr;
         }
         if (!mine) continue;
@@ -1183,8 +1250,10 @@ void launch_pick(int mode, uint32_t k, uint64_t frontier_est, uint32_t n_batches
         const uint64_t blocks = std::min<uint64_t>((frontier_est + kWeightedThreads / 32 - 1) / (kWeightedThreads / 32),
                                                    std::max<uint64_t>(1, (uint64_t)kSMs * 128 / n_batches));
         launch_chained(k_pick<32, kPickWeighted>, dim3((uint32_t)std::max<uint64_t>(1, blocks), n_batches), dim3(kWeightedThreads), st, pa, hop, k);
-        // rows longer than kHubDegree were only queued: a warp per slice of them
-        launch_chained(k_pick_hub_slices, dim3((uint32_t)kSMs * 16), dim3(kWeightedThreads), st, pa, hop, k);
+        // rows longer than kHubDegree were only queued: a warp per slice of them, and once more for
+        // those whose guess was too low (none as a rule: 2 us)
+        launch_chained(k_pick_hub_slices<false>, dim3((uint32_t)kSMs * 16), dim3(kWeightedThreads), st, pa, hop, k);
+        launch_chained(k_pick_hub_slices<true>, dim3((uint32_t)kSMs * 4), dim3(kWeightedThreads), st, pa, hop, k);
     } else if (k > 32) {
         launch_chained(k_pick<32, kPickLarge>, dim3(blocks_for(frontier_est, 4), n_batches), dim3(128), st, pa, hop, k);
     } else {
@@ -1367,9 +1436,9 @@ int32_t ensure_scratch(ag_sampler *s, uint64_t n_seeds) {
         carve(&s->tiles, G * s->n_tiles * sizeof(TileDesc));
         carve(&s->stage_dev, stage);
         if (hubs) {
-            carve(&s->hub_rows, hubs * sizeof(HubRow)); carve(&s->hub_count, 8);
+            carve(&s->hub_rows, 2 * hubs * sizeof(HubRow)); carve(&s->hub_count, 16);
             carve(&s->hub_key, hubs * hop_k * 8); carve(&s->hub_pos, hubs * hop_k * 4);
-            carve(&s->hub_thr, hubs * 4); carve(&s->hub_done, hubs * 4); carve(&s->hub_guess, hubs * 4);
+            carve(&s->hub_thr, 2 * hubs * 4); carve(&s->hub_done, 2 * hubs * 4); carve(&s->hub_guess, hubs * 4);
         }
         if (!pass) {
             AG_CUDA(workspace_alloc(&base, off));

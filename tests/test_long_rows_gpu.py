@@ -26,28 +26,41 @@ def _hub_graph(degrees, n, seed, weights=None):
         w[rng.random(len(w)) < 0.9995] = 0.0
         for value in (-1.0, np.inf, np.nan, 1e-42, 3.3e38, 1e-30):
             w[rng.integers(0, len(w), 50)] = value
+    elif weights == "pareto":  # no mean: the sampled weights say little about the keys
+        w = (1.0 + rng.pareto(0.5, len(src))).astype(np.float32)
+    elif weights in ("heavy", "few"):  # a row's first position far above the rest; eight positive ones and zeros
+        at = np.arange(len(src)) - np.searchsorted(src, src)
+        w = np.where(at == 0, 1e6, 1.0) if weights == "heavy" else np.where(at % 61 == 0, 1.0, 0.0) * (at < 8 * 61)
+        w = w.astype(np.float32)
+    elif weights == "comb":  # positive exactly where a row's mean weight is sampled
+        at = np.arange(len(src)) - np.searchsorted(src, src)
+        w = (at % np.maximum(np.bincount(src)[src] // 512, 1) == 0).astype(np.float32)
     return csr_from_edges(n, src, dst, w)
 
 
 DEGREES = [2047, 2048, 2049, 4096, 4097, 31, 33, 70_000, 530_001, 9000, 0, 1, 16, 15]
+# and at the edges of a chunk, of the rows that start from a guessed threshold and of its sample
+WEIGHTED_DEGREES = DEGREES + [32, 64, 65, 127, 128, 129, 160, 511, 512, 513, 1500]
 
 
-@pytest.mark.parametrize("weights", ["lognormal", "equal", "odd"])
-@pytest.mark.parametrize("fanout,rng_mode", [([15, 4], "wyrand_exact"), ([32], "wyrand_exact"), ([1, 1, 2], "wyrand_exact")])
-def test_weighted(weights, fanout, rng_mode):
+@pytest.mark.parametrize("weights", ["lognormal", "equal", "odd", "pareto", "heavy", "few", "comb"])
+@pytest.mark.parametrize("fanout", [[15, 4], [32], [1, 1, 2]])
+def test_weighted(weights, fanout):
+    """With "heavy", "few" and "comb" the guessed threshold is below the k-th best key of most long
+    rows, with "comb" of those above 1024 that stay with a warp too: they are streamed once more."""
     import aethergraph_b200 as ag
     from oracle import ago
 
     n = 4000
-    off, dst, w = _hub_graph(DEGREES, n, 3, weights)
+    off, dst, w = _hub_graph(WEIGHTED_DEGREES, n, 3, weights)
     g = ag.Graph.from_csr(off, dst, w)
-    cfg = ag.SamplingConfig(num_neighbors=fanout, weighted=True, seed=11, rng_mode=rng_mode)
+    cfg = ag.SamplingConfig(num_neighbors=fanout, weighted=True, seed=11)
     o = ago.Sampler(off, dst, fanout, weights=w, weighted=True, seed=11)
     s = ag.NeighborSampler(g, cfg)
-    for count in (len(DEGREES), 1, 60):
+    for count in (len(WEIGHTED_DEGREES), 1, 60):
         seeds = np.arange(count, dtype=np.uint32)[::-1].copy()
         assert_same_subgraph(s.sample(seeds).raw_u32(), o.sample(seeds))
-    batches = [np.arange(len(DEGREES) - i, dtype=np.uint32) for i in range(8)]
+    batches = [np.arange(len(WEIGHTED_DEGREES) - i, dtype=np.uint32) for i in range(8)]
     for i, sg in enumerate(ag.ParallelBatchSampler(g, cfg, group=8).sample_batches(batches)):
         o.reseed(ago.batch_seed(11, i))
         assert_same_subgraph(sg.raw_u32(), o.sample(batches[i]), ctx=f"batch {i}: ")
