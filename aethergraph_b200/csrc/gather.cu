@@ -111,7 +111,8 @@ __device__ __forceinline__ const uint8_t *shard_row(const ag_shard_table *t, uin
 }
 
 // Vector path: row_bytes % 16 == 0 and the payload base is 16-byte aligned.
-// LPR lanes share a row; vecs = row_bytes / 16.
+// LPR lanes share a row; vecs = row_bytes / 16.  Five blocks per SM (48 registers): with four, f16
+// rows of 256 took 10.4 us instead of 9.2 (20 K rows) and 127 instead of 119 (500 K).
 template <int DTYPE, int LPR>
 __device__ __forceinline__ void gather_vec_rows(GatherArgs &a, uint64_t first) {
     constexpr int kRowsPerBlock = kThreads / LPR;
@@ -162,7 +163,7 @@ __device__ __forceinline__ void gather_vec_rows(GatherArgs &a, uint64_t first) {
 }
 
 template <int DTYPE, int LPR>
-__global__ void __launch_bounds__(kThreads)
+__global__ void __launch_bounds__(kThreads, 5)
 k_gather_vec(GatherArgs a, const GatherArgs *group, uint64_t first) {
     chain_sync();
     if (group) a = group[blockIdx.y];  // one batch of a group per grid row
@@ -173,7 +174,7 @@ k_gather_vec(GatherArgs a, const GatherArgs *group, uint64_t first) {
 // The rows of several stores of one dtype (node types) in one launch: grid row y is the
 // batch, z the store, whose arguments are group[z * stride + y].
 template <int DTYPE>
-__global__ void __launch_bounds__(kThreads)
+__global__ void __launch_bounds__(kThreads, 5)
 k_gather_stores(const GatherArgs *group, uint32_t stride) {
     chain_sync();
     GatherArgs a = group[(uint64_t)blockIdx.z * stride + blockIdx.y];
