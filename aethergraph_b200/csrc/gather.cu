@@ -18,6 +18,7 @@
 // count) without a host round trip.
 #include <algorithm>
 #include <mutex>
+#include <type_traits>
 
 #include <cub/device/device_radix_sort.cuh>
 #include <cuda_fp16.h>
@@ -400,14 +401,16 @@ __global__ void k_encode_i8(const float *__restrict__ src, uint64_t rows, uint64
 // Rows that are not a whole number of 16-byte vectors (or not 16-byte aligned): a row is
 // split into units of UNIT elements, the largest power of two up to four that divides the
 // row's length and that the bases' alignment allows, so that a unit is one aligned load of
-// UNIT * element bytes and one aligned store of UNIT floats.  A group of 2^lpr_log2 lanes
-// owns a row and walks its units; consecutive lanes touch consecutive bytes, and
-// kUnitRows x kUnitCols units are in flight per lane before any of them is stored.
+// UNIT * element bytes and one aligned store of UNIT floats.  Row by row: a group of
+// 2^lpr_log2 lanes owns a row and walks its units; consecutive lanes touch consecutive bytes,
+// and kUnitRows x kUnitCols units are in flight per lane before any of them is stored.  Or
+// flat, whatever row a unit is in (launch_units says which).
 //
-// A thread per element (a 64-bit division, an id and a 2-byte load for every float) took
+// A thread per element (a 64-bit division, an id and a 2-byte load for every float) takes
 // 127 us for 200 003 rows of 100 f16 (1.0 TB/s), bound by the instructions of the division
-// and of the decode; now 39 us.  100 M values: dim 301 bf16 625 -> 224 us, dim 50 f32 635 ->
-// 248 us, dim 33 int8 619 -> 275 us, dim 602 f16 643 -> 172 us; dim 1 f32 (20 M) 196 -> 141 us.
+// and of the decode; in units 28 us.  100 M values: dim 301 bf16 600 and 212 us, dim 50 f32 610
+// and 171, dim 602 f16 619 and 164 us.
+
 constexpr int kUnitRows = 4, kUnitCols = 2;
 
 template <int BYTES> struct UnitWord;
@@ -441,7 +444,19 @@ __device__ __forceinline__ uint32_t unit_decode(W w, int e, float scale) {
     return DTYPE == AG_BF16 ? h << 16 : __float_as_uint(f16_to_f32_bits(h));
 }
 
-template <int DTYPE, int UNIT, bool SHARDED>
+// Decodes a unit and stores its UNIT floats.
+template <int DTYPE, int UNIT, typename W>
+__device__ __forceinline__ void store_unit(float *dst, W w, float scale) {
+    uint32_t f[UNIT];
+#pragma unroll
+    for (int e = 0; e < UNIT; ++e) f[e] = unit_decode<DTYPE>(w, e, scale);
+    if constexpr (UNIT == 4) st_stream_v4(dst, make_uint4(f[0], f[1], f[2], f[3]));
+    else if constexpr (UNIT == 2) st_stream_v2(dst, make_uint2(f[0], f[1]));
+    else st_stream_u32(dst, f[0]);
+}
+
+// STEPPED: the steps of a row are shared out over the grid's z.
+template <int DTYPE, int UNIT, bool SHARDED, bool STEPPED>
 __global__ void __launch_bounds__(kThreads)
 k_gather_units(GatherArgs a, const GatherArgs *__restrict__ group, uint32_t lpr_log2) {
     constexpr int kElem = DTYPE == AG_F32 ? 4 : DTYPE == AG_I8 ? 1 : 2, kBytes = kElem * UNIT;
@@ -471,7 +486,7 @@ k_gather_units(GatherArgs a, const GatherArgs *__restrict__ group, uint32_t lpr_
                 }
             }
         }
-        for (uint32_t v0 = lane; v0 < units; v0 += lpr * kUnitCols) {
+        for (uint32_t v0 = (STEPPED ? blockIdx.z * lpr * kUnitCols : 0u) + lane; v0 < units; v0 += (STEPPED ? gridDim.z : 1u) * lpr * kUnitCols) {
             W val[kUnitRows][kUnitCols];
             float scale[kUnitRows][kUnitCols];
 #pragma unroll
@@ -494,15 +509,52 @@ k_gather_units(GatherArgs a, const GatherArgs *__restrict__ group, uint32_t lpr_
                 for (int c = 0; c < kUnitCols; ++c) {
                     const uint32_t v = v0 + c * lpr;
                     if (v >= units) continue;
-                    float *dst = a.out + r * a.dim + (uint64_t)v * UNIT;
-                    uint32_t f[UNIT];
-#pragma unroll
-                    for (int e = 0; e < UNIT; ++e) f[e] = unit_decode<DTYPE>(val[u][c], e, scale[u][c]);
-                    if constexpr (UNIT == 4) st_stream_v4(dst, make_uint4(f[0], f[1], f[2], f[3]));
-                    else if constexpr (UNIT == 2) st_stream_v2(dst, make_uint2(f[0], f[1]));
-                    else st_stream_u32(dst, f[0]);
+                    store_unit<DTYPE, UNIT>(a.out + r * a.dim + (uint64_t)v * UNIT, val[u][c], scale[u][c]);
                 }
             }
+        }
+    }
+}
+
+// The same rows unit by unit, whatever row a unit is in: a block takes FLIGHT * 256 consecutive
+// units of the output, every lane FLIGHT of them.
+template <int DTYPE, int UNIT, bool SHARDED, int FLIGHT>
+__global__ void __launch_bounds__(kThreads)
+k_gather_flat(GatherArgs a, const GatherArgs *__restrict__ group) {
+    constexpr int kElem = DTYPE == AG_F32 ? 4 : DTYPE == AG_I8 ? 1 : 2, kBytes = kElem * UNIT;
+    using W = typename UnitWord<kBytes>::T;
+    if (group) a = group[blockIdx.y];
+    if (!a.payload) return;
+    const uint64_t n = a.n_dev ? min((uint64_t)*a.n_dev, a.n) : a.n;
+    if (a.ids_off) a.ids = (const uint32_t *)a.ids + *a.ids_off;
+    const uint32_t units = a.dim / UNIT, blocks_per_row = (a.dim + kQuantBlock - 1) / kQuantBlock;
+    const uint64_t total = n * units;
+    for (uint64_t base = blockIdx.x * (uint64_t)(kThreads * FLIGHT); base < total; base += gridDim.x * (uint64_t)(kThreads * FLIGHT)) {
+        // 32-bit divisions, but for what lies beyond 2^32 units
+        const uint64_t from = FLIGHT == 1 ? base + threadIdx.x : base;
+        const uint64_t row0 = from <= 0xFFFFFFFFull ? (uint32_t)from / units : from / units;
+        const uint32_t rest = (uint32_t)(from - row0 * units) + (FLIGHT == 1 ? 0u : threadIdx.x);
+        W val[FLIGHT];
+        float scale[FLIGHT];
+#pragma unroll
+        for (int u = 0; u < FLIGHT; ++u) {
+            val[u] = W{};  // a row outside the store decodes to zeros
+            scale[u] = 0.f;
+            if (base + u * kThreads + threadIdx.x >= total) continue;
+            const uint32_t off = rest + u * kThreads, r = FLIGHT == 1 ? 0u : off / units, v = off - r * units;
+            const uint64_t id = load_id(a.ids, a.ids64, row0 + r), local = id - a.row_begin;
+            if (id >= a.row_begin && local < a.rows) {
+                const uint8_t *row = SHARDED ? shard_row(a.shards, id, a.row_bytes) : a.payload + local * a.row_bytes;
+                val[u] = load_unit<kBytes, !SHARDED>(row + (uint64_t)v * kBytes);
+                if (DTYPE == AG_I8) scale[u] = __ldg(a.scales + local * blocks_per_row + v * UNIT / kQuantBlock);
+            } else if (v == 0) {
+                atomicOr(a.err, kErrBadId);
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < FLIGHT; ++u) {
+            const uint64_t g = base + u * kThreads + threadIdx.x;
+            if (g < total) store_unit<DTYPE, UNIT>(a.out + g * UNIT, val[u], scale[u]);
         }
     }
 }
@@ -529,22 +581,48 @@ uint32_t unit_lpr_log2(uint32_t units) {
     return best;
 }
 
-// n: rows per batch the grid is sized for; max_blocks: over all batches.
+// n: rows per batch the grid is sized for.  Which kernel, by f32 / f16 launches of a CUDA graph, us:
+//   * few units: flat, one unit per lane, all of them resident at once.  A lane that walks a row
+//     takes its latency step after step: 1 row of 4099 f32 68 row-wise on one block, 2.0 in steps,
+//     1.8 flat; 300 x 602 f32 9.6 / 2.9 / 2.2; 1000 x 5 3.6 row-wise, 1.8 flat.
+//   * short rows, and many rows that a lane group would take in a single step, so that half of its
+//     loads in flight are missing: flat, four units per lane.  1 M x 5 f32 33 row-wise, 16 flat;
+//     1 M x 100 f16 (25 units) 146 and 108, 10 K 3.4 and 3.6; 1 M x 17 43 and 46, 1 M x 33 71 and 85.
+//   * the others row by row: one id and one address per lane and row.  A lane walks its row in
+//     steps of two units; where that leaves the GPU idle (long rows, few of them) the steps go to
+//     blocks of their own, up to two per SM: 1000 x 4099 f32 196 without, 14 with.
+constexpr uint32_t kShortRow = 16;
+template <int DTYPE, int UNIT, bool SHARDED>
+void launch_units(const GatherArgs &a, const GatherArgs *group, uint32_t n_batches, uint64_t n, uint32_t units, cudaStream_t st) {
+    const uint64_t cap = ((uint64_t)kSMs * 64 + n_batches - 1) / n_batches, total = n * units;
+    auto blocks_for = [&](uint64_t items, uint64_t per) { return (uint32_t)std::max<uint64_t>(1, std::min((items + per - 1) / per, cap)); };
+    const uint32_t lg = unit_lpr_log2(units);
+    if (total * n_batches <= (uint64_t)kSMs * kThreads * (units <= kShortRow ? 8 : 5)) {
+        k_gather_flat<DTYPE, UNIT, SHARDED, 1><<<dim3(blocks_for(total, kThreads), n_batches), kThreads, 0, st>>>(a, group);
+    } else if (units <= kShortRow || (units <= (1u << lg) && total * n_batches > (uint64_t)kSMs * kThreads * 16)) {
+        k_gather_flat<DTYPE, UNIT, SHARDED, 4><<<dim3(blocks_for(total, kThreads * 4), n_batches), kThreads, 0, st>>>(a, group);
+    } else {
+        const uint32_t blocks = blocks_for(n, (uint64_t)(kThreads >> lg) * kUnitRows);
+        const uint64_t steps = (units + (kUnitCols << lg) - 1) / (kUnitCols << lg), room = (uint64_t)kSMs * 2 / ((uint64_t)blocks * n_batches);
+        const uint32_t z = (uint32_t)std::max<uint64_t>(1, std::min(steps, room));
+        if (z > 1) k_gather_units<DTYPE, UNIT, SHARDED, true><<<dim3(blocks, n_batches, z), kThreads, 0, st>>>(a, group, lg);
+        else k_gather_units<DTYPE, UNIT, SHARDED, false><<<dim3(blocks, n_batches), kThreads, 0, st>>>(a, group, lg);
+    }
+}
+
 template <int DTYPE>
 cudaError_t launch_units(const GatherArgs &a, const GatherArgs *group, uint32_t n_batches, uint64_t n, uint32_t dim, uint32_t unit,
                          bool sharded, cudaStream_t st) {
-    const uint32_t lg = unit_lpr_log2(dim / unit);
-    const uint64_t per = (uint64_t)(kThreads >> lg) * kUnitRows, need = (n + per - 1) / per;
-    const uint64_t cap = ((uint64_t)kSMs * 64 + n_batches - 1) / n_batches;
-    const dim3 grid((uint32_t)std::max<uint64_t>(1, std::min(need, cap)), n_batches);
-#define AG_LAUNCH_UNITS(U) do { if (sharded) k_gather_units<DTYPE, U, true><<<grid, kThreads, 0, st>>>(a, group, lg); \
-                                else k_gather_units<DTYPE, U, false><<<grid, kThreads, 0, st>>>(a, group, lg); } while (0)
+    auto launch = [&](auto width) {
+        constexpr int kUnit = decltype(width)::value;
+        if (sharded) launch_units<DTYPE, kUnit, true>(a, group, n_batches, n, dim / kUnit, st);
+        else launch_units<DTYPE, kUnit, false>(a, group, n_batches, n, dim / kUnit, st);
+    };
     if constexpr (DTYPE != AG_F32) {
-        if (unit == 4) { AG_LAUNCH_UNITS(4); return cudaGetLastError(); }
+        if (unit == 4) { launch(std::integral_constant<int, 4>{}); return cudaGetLastError(); }
     }
-    if (unit == 2) AG_LAUNCH_UNITS(2);
-    else AG_LAUNCH_UNITS(1);
-#undef AG_LAUNCH_UNITS
+    if (unit == 2) launch(std::integral_constant<int, 2>{});
+    else launch(std::integral_constant<int, 1>{});
     return cudaGetLastError();
 }
 

@@ -40,6 +40,33 @@ def test_rows_and_offsets(dtype, dim):
         assert (got[:shift] == 7).all() and (got[shift + rows * dim:] == 7).all()
 
 
+@pytest.mark.parametrize("dtype,dim,rows", [
+    ("f32", 5, 30_000), ("f32", 5, 70_001), ("f32", 1, 400_003), ("bf16", 6, 200_001), ("i8", 9, 50_000),  # short rows: few units, many
+    ("f16", 100, 7000), ("f16", 100, 9001), ("f32", 25, 20_011), ("i8", 128 - 4, 13_001),                   # one step of a lane group
+    ("f32", 17, 30_011), ("bf16", 33, 20_003), ("i8", 301, 1999), ("f16", 602, 3001),                       # row by row
+    ("f32", 4099, 1), ("f32", 4099, 101), ("f16", 4099, 300), ("i8", 1023, 777), ("bf16", 8190, 40),        # steps on blocks of their own
+])
+def test_launch_forms(dtype, dim, rows):
+    """Few units, short rows, row by row, rows in steps: every element, and ids outside the store."""
+    import torch
+
+    import aethergraph_b200 as ag
+
+    n = 300
+    rng = np.random.default_rng(rows)
+    store = ag.FeatureStore.from_array(rng.standard_normal((n, dim)).astype(np.float32), dtype)
+    ids = rng.integers(0, n, rows)
+    want = torch.from_numpy(_decoded(store, n, dim, dtype)).cuda()[torch.from_numpy(ids).cuda()]
+    assert torch.equal(store.gather(torch.from_numpy(ids).cuda()).view(torch.int32), want.view(torch.int32))
+    store.check()
+    bad = np.unique(rng.integers(0, rows, 5))
+    ids[bad] = n + bad
+    want[torch.from_numpy(bad).cuda()] = 0
+    assert torch.equal(store.gather(torch.from_numpy(ids).cuda()).view(torch.int32), want.view(torch.int32))
+    with pytest.raises(ValueError):
+        store.check()
+
+
 @pytest.mark.parametrize("dtype,dim", [("f16", 100), ("bf16", 301), ("f32", 50), ("i8", 100)])
 def test_batches_of_a_chain(dtype, dim):
     import torch
