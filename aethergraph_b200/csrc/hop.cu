@@ -60,13 +60,14 @@ k_hop_replace(const uint64_t *__restrict__ offsets, const uint32_t *__restrict__
 
 // Decisions t in [fanout, degree) of one row, four per generator call (draw t is word t % 4
 // of block t / 4): `who` of `of` threads, each taking every of-th block of four.
-__device__ __forceinline__ void reservoir_scan(uint64_t seed, uint32_t layer, uint64_t node, uint64_t degree, uint32_t fanout,
+template <typename T>
+__device__ __forceinline__ void reservoir_scan(uint64_t seed, uint32_t layer, uint64_t node, T degree, uint32_t fanout,
                                                uint32_t who, uint32_t of, uint32_t *last) {
-    for (uint64_t g = (fanout >> 2) + who; g * 4 < degree; g += of) {
+    for (T g = (fanout >> 2) + who; g * 4 < degree; g += of) {
         const uint4 r = philox4x32_10(seed, layer, node, (uint32_t)g);
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
-            const uint64_t t = g * 4 + e;
+            const T t = g * 4 + e;
             const uint32_t word = e == 0 ? r.x : e == 1 ? r.y : e == 2 ? r.z : r.w;
             if (t < fanout || t >= degree) continue;
             const uint32_t j = word % (uint32_t)(t + 1);
@@ -75,10 +76,14 @@ __device__ __forceinline__ void reservoir_scan(uint64_t seed, uint32_t layer, ui
     }
 }
 
-// Bound by the generator and the remainder, about 45 instructions a decision when each draw
-// had a generator call of its own and now a third of that, and by the longest row: a warp
-// each, a row of 150 K neighbours alone took longer than 100 K ordinary ones.  300 K rows of
-// a 4 M vertex / 100 M edge R-MAT graph, fanout 25: 674 -> 118 us; 100 rows: 25 -> 19 us.
+// Rows of hundreds of neighbours: bound by the generator and the remainder, about 45 instructions
+// a decision with a generator call each and a third of that with four per call; and by the
+// longest row: a row of 150 K neighbours takes one warp longer than 100 K ordinary rows take
+// the GPU.  Rows with at most 32 decisions: latency, so a decision per lane (100 K rows of 40
+// neighbours, fanout 25: 33 us, 41 with four per call), one barrier a round, and 45 registers
+// instead of 48 for the row in 32 bits.  300 K rows of a 4 M vertex / 100 M edge R-MAT graph,
+// fanout 25: 92 us, 290 and more with a warp per row and a call per decision; 300 K rows of 300
+// neighbours 231 and 372, of 10 neighbours 62 and 61 (fanout 8: 86 and 79).
 __global__ void __launch_bounds__(kHopThreads)
 k_hop_reservoir(const uint64_t *__restrict__ offsets, const uint32_t *__restrict__ neighbors, uint64_t num_nodes,
                 uint64_t num_edges, const uint64_t *__restrict__ nodes, uint32_t *__restrict__ output,
@@ -92,37 +97,39 @@ k_hop_reservoir(const uint64_t *__restrict__ offsets, const uint32_t *__restrict
         node = nodes[row];
         hop_row(offsets, num_nodes, num_edges, node, begin, degree);
     };
+    if (threadIdx.x == 0) s_longs = 0;
+    __syncthreads();
     for (uint64_t base = (uint64_t)blockIdx.x * round; base < node_count; base += (uint64_t)gridDim.x * round) {
-        __syncthreads();
-        if (threadIdx.x == 0) s_longs = 0;
-        __syncthreads();
+        bool left = false;  // a row of this warp is left to the block
         for (uint32_t i = warp; i < round && base + i < node_count; i += kWarps) {
-            const uint64_t row = base + i;
-            uint32_t *out = output + row * fanout;
-            uint64_t node, begin, degree;
-            row_of(row, node, begin, degree);
-            uint32_t taken = 0;
-            if (degree == 0) {
-                taken = 0;
-            } else if ((uint64_t)fanout >= degree) {
-                for (uint64_t t = lane; t < degree; t += 32) out[t] = ld_stream_u32(neighbors + begin + t);
-                taken = (uint32_t)degree;
-            } else if (degree >= kHopLong) {
+            uint32_t *out = output + (base + i) * fanout;
+            uint64_t node, begin, length;
+            row_of(base + i, node, begin, length);
+            if (length >= kHopLong) {  // more than any fanout of this kernel
                 if (lane == 0) s_long[atomicAdd(&s_longs, 1u)] = i;
+                left = true;
                 continue;
-            } else {
+            }
+            const uint32_t degree = (uint32_t)length, taken = min(degree, fanout);
+            uint32_t from = lane;  // this lane's neighbour
+            if (degree > fanout) {
                 s_last[warp][lane] = lane;  // slot j starts with element j
                 __syncwarp();
-                reservoir_scan(seed, layer, node, degree, fanout, lane, 32, s_last[warp]);
+                if (degree <= fanout + 32) {  // a decision per lane
+                    const uint32_t t = fanout + lane;
+                    const uint32_t j = philox_u32(seed, layer, node, t) % (t + 1);
+                    if (t < degree && j < fanout) atomicMax(&s_last[warp][j], t);
+                } else {
+                    reservoir_scan(seed, layer, node, degree, fanout, lane, 32, s_last[warp]);
+                }
                 __syncwarp();
-                if (lane < fanout) out[lane] = ld_stream_u32(neighbors + begin + s_last[warp][lane]);
-                taken = fanout;
+                from = s_last[warp][lane];
                 __syncwarp();
             }
-            for (uint32_t t = taken + lane; t < fanout; t += 32) out[t] = AG_SAMPLE_PAD;
-            if (lane == 0) counts[row] = taken;
+            if (lane < fanout) out[lane] = lane < taken ? ld_stream_u32(neighbors + begin + from) : AG_SAMPLE_PAD;
+            if (lane == 0) counts[base + i] = taken;
         }
-        __syncthreads();
+        if (!__syncthreads_or(left)) continue;
         for (uint32_t l = 0; l < s_longs; ++l) {
             const uint64_t row = base + s_long[l];
             uint64_t node, begin, degree;
@@ -135,6 +142,8 @@ k_hop_reservoir(const uint64_t *__restrict__ offsets, const uint32_t *__restrict
             if (threadIdx.x == 0) counts[row] = fanout;
             __syncthreads();
         }
+        if (threadIdx.x == 0) s_longs = 0;
+        __syncthreads();
     }
 }
 
@@ -152,8 +161,9 @@ extern "C" int32_t ag_sample_hop_reservoir(const ag_graph *g, const uint64_t *no
     if (node_count == 0) return AG_OK;
     DeviceGuard guard(g->device);
     if (!guard.ok) return AG_ERR_CUDA;
-    // a row per warp while that does not fill the GPU (8 blocks of 8 warps per SM), four beyond
-    const uint32_t round = fanout > 32 || node_count <= (uint64_t)kSMs * 64 ? kHopThreads / 32 : kHopRows;
+    // A row per warp up to twice what fills the GPU (8 blocks of 8 warps per SM), four beyond: 15 K
+    // rows of 1500 neighbours 42 us, 57 with four; 100 K rows of 10 neighbours 36 us, 31 with four.
+    const uint32_t round = fanout > 32 || node_count <= (uint64_t)kSMs * 128 ? kHopThreads / 32 : kHopRows;
     const uint64_t blocks = std::min<uint64_t>((node_count + round - 1) / round, (uint64_t)kSMs * 32);
     if (fanout > 32)
         k_hop_replace<<<(uint32_t)blocks, kHopThreads, 0, (cudaStream_t)stream>>>(

@@ -1,4 +1,5 @@
-"""One-hop Philox sampling of rows around the length where a block takes over from a warp,
+"""One-hop Philox sampling of rows around the lengths where a warp takes over from a decision per
+lane and a block from a warp, in launches of one and of four rows per warp,
 against the CPU oracle."""
 import numpy as np
 import pytest
@@ -7,11 +8,11 @@ from helpers import csr_from_edges
 
 pytestmark = pytest.mark.gpu
 
-DEGREES = [2047, 2048, 2049, 5, 33, 34, 6, 100_003, 7, 0, 1, 2, 4, 3000]
+DEGREES = [2047, 2048, 2049, 5, 33, 34, 6, 100_003, 7, 0, 1, 2, 4, 3000, 37, 38, 39, 40, 64, 65]
 
 
 @pytest.mark.parametrize("fanout", [1, 5, 6, 7, 32, 40])
-@pytest.mark.parametrize("copies", [1, 900])
+@pytest.mark.parametrize("copies", [1, 900, 1500])
 def test_long_rows(fanout, copies):
     import aethergraph_b200 as ag
     from aethergraph_b200.sampler import reservoir_hop
