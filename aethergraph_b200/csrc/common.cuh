@@ -161,9 +161,12 @@ constexpr int kPackedSmall = 4032, kPackedMedium = 8128, kPackedLarge = 16320;
 // predecessor's results (griddepcontrol.wait; a no-op for a plain launch).  The
 // kernels of a loader's chain do NOT release their successor early: measured, successor
 // blocks parked in SM slots take those slots from the gather of a neighbouring chain and
-// the whole pipeline gets slower.  A chain that runs alone has no such neighbour, and
-// chain_release (after chain_sync, once all blocks have called it) lets the next kernel
-// be launched while this one works; it still waits for all of this one's results.
+// the whole pipeline gets slower.  Other chains (`alone`: one batch of a handle that is no
+// loader's) call chain_release, after chain_sync: once all blocks have, the next kernel is
+// launched while this one works; it still waits for all of this one's results.  Such handles
+// may share the GPU all the same: 24 batches of 1024 seeds with rows of 256 bf16 take 2.89 ms one
+// after the other (2.90 without the release), 1.95 on two streams (1.97), 1.97 on three (1.99) and
+// 2.19 ms from four threads (2.17), all within the runs' spread.
 //
 // A dependent kernel can be resident before its predecessor has written what it reads, and a
 // read-only load promises data that does not change while the kernel is resident: neither the

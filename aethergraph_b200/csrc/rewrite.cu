@@ -185,10 +185,12 @@ namespace {
 // the counts are scanned, writes them behind the stretches before it (second walk).
 //
 // Rows differ by five orders of magnitude (a hub of an R-MAT graph of 64 M edges has
-// over 100 K neighbours, most vertices a few), so a warp per row left the two walks to
+// over 100 K neighbours, most vertices a few), so a warp per row leaves the two walks to
 // the warp with the longest one: 200 seeds, fanouts 10, 5 on that graph reach 3200 nodes
-// and 5.7 M positions, 2660 + 3080 us at 4 % of the warps busy.  Now 39 + 44 us (107 + 84
-// before the filter and the shuffled row search below), bound by the probes of the node table.
+// and 5.7 M positions, 2660 + 3080 us at 4 % of the warps busy; in equal stretches 39 + 44 us.
+// Bound by latency: half of the warps resident, 36 and 47 % of the issue slots used, 6 % of the
+// DRAM rate; a warp waits nine cycles an issue for loads, four at the barriers of the filter
+// (counting walk) or seven for loads (filling walk).
 // One block per SM, so that the filter below is built once for 32 warps and the counts that
 // are scanned are one per block (256-thread blocks: 55 + 48 us, of it 25 us for the scan of
 // 4736 warp counts and up to 10 us for building the filter in waves of blocks).

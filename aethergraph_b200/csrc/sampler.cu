@@ -304,7 +304,7 @@ __device__ __forceinline__ void pick_large(const SampleParams &p, uint32_t hop, 
     }
 }
 
-// Weighted sampling without replacement, fanout <= 32, one warp per vertex.
+// Weighted sampling without replacement, fanout <= 32, one warp per vertex or slice of its row.
 // Selection follows sampler.rs:1418-1469: one 64-bit draw per row position in
 // row order, key = -ln(u) / w in f64 with u = ((bits >> 11) + 1) * 2^-53
 // (sampler.rs:52-55), +inf for a weight that is not finite and positive; the k
@@ -312,10 +312,6 @@ __device__ __forceinline__ void pick_large(const SampleParams &p, uint32_t hop, 
 // order; the reference's own order comes from Rust's select_nth_unstable_by and
 // is not defined by its source tree.  The warp streams the row 32 positions at a
 // time and keeps the k best so far sorted across its lanes.
-// Weighted picks (sampler.rs:1418-1469): every position of a row with deg > k gets
-// the key -ln(u) / w from its own draw; the k smallest (key, position) win and are
-// emitted in ascending order.  A warp streams 32 positions at a time and keeps the
-// current best k sorted across its lanes.
 
 // Compare-exchange with the lane `stride` away; this lane keeps the smaller pair if `small`.
 __device__ __forceinline__ void warp_exchange(double &key, uint32_t &pos, int stride, bool small) {
@@ -1251,7 +1247,7 @@ void launch_pick(int mode, uint32_t k, uint64_t frontier_est, uint32_t n_batches
                                                    std::max<uint64_t>(1, (uint64_t)kSMs * 128 / n_batches));
         launch_chained(k_pick<32, kPickWeighted>, dim3((uint32_t)std::max<uint64_t>(1, blocks), n_batches), dim3(kWeightedThreads), st, pa, hop, k);
         // rows longer than kHubDegree were only queued: a warp per slice of them, and once more for
-        // those whose guess was too low (none as a rule: 2 us)
+        // those whose guess was too low (as a rule none)
         launch_chained(k_pick_hub_slices<false>, dim3((uint32_t)kSMs * 16), dim3(kWeightedThreads), st, pa, hop, k);
         launch_chained(k_pick_hub_slices<true>, dim3((uint32_t)kSMs * 4), dim3(kWeightedThreads), st, pa, hop, k);
     } else if (k > 32) {
@@ -1534,14 +1530,14 @@ extern "C" int32_t ag_sampler_reseed(ag_sampler *s, uint64_t seed) {
     return AG_OK;
 }
 
+void ag::sampler_set_pipelined(ag_sampler *s) { s->pipelined = true; }
+
 // A loader's worker threads wait for their chains by polling the event and yielding
 // the core between polls instead of spinning inside the runtime: with three workers
 // per GPU and eight GPUs per host the spinning waits alone would occupy most of the
 // host's cores, which the consumer's own thread needs; on an idle core a yield returns
 // at once, so nothing is lost when there are cores to spare.  (Sleeping on the event
 // — cudaEventBlockingSync — was measured too: -9 % on one GPU, the wake-up is too slow.)
-void ag::sampler_set_pipelined(ag_sampler *s) { s->pipelined = true; }
-
 int32_t ag::sampler_set_yielding_wait(ag_sampler *s, bool on) {
     s->yield_wait = on;
     return AG_OK;

@@ -840,9 +840,10 @@ def run_device(args, w):
                                          "also copied to pinned host memory: PCIe-bound"}},
             "sharded": sharded, "int8_payload": int8_leg, "secondary": secondary,
             # one launch chain per group of batches (the batch is blockIdx.y): hops + 1 assign (the
-            # first inserts the seeds, up to 2048 a batch; more: a launch of its own), hops pick,
-            # gather (sharded: + key, sorted gather, overflow)
-            "gpu_launches": world * chains * (2 * hops + (2 if bs <= 2048 else 3) + (3 if sharded_main else 0)),
+            # first inserts the seeds, up to 2048 a batch; more: a launch of its own), hops pick
+            # (weighted: + two for the slices of long rows), gather (sharded: + key, sorted gather,
+            # overflow)
+            "gpu_launches": world * chains * ((4 if w["weighted"] else 2) * hops + (2 if bs <= 2048 else 3) + (3 if sharded_main else 0)),
         }
         print(json.dumps(line), flush=True)
     if world > 1:
