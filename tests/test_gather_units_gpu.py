@@ -67,6 +67,24 @@ def test_launch_forms(dtype, dim, rows):
         store.check()
 
 
+@pytest.mark.parametrize("dtype,dim,rows", [("f32", 5, 1000), ("bf16", 5, 70_001), ("f16", 100, 9001), ("f16", 33, 20_003), ("f32", 4099, 101)])
+def test_launch_forms_of_a_sharded_view(dtype, dim, rows):
+    import torch
+
+    import aethergraph_b200 as ag
+    from aethergraph_b200 import synth
+
+    n, world = 301, 3
+    whole = synth.features(n, dim, dtype, 7)
+    ids = torch.from_numpy(np.random.default_rng(rows).integers(0, n, rows)).cuda()
+    want = torch.from_numpy(_decoded(whole, n, dim, dtype)).cuda()[ids]
+    for layout in ("range", "cyclic"):
+        shards = [synth.features_shard(n, dim, dtype, 7, r, world, layout) for r in range(world)]
+        view = ag.FeatureStore.view_sharded(shards, 1)
+        assert torch.equal(view.gather(ids).view(torch.int32), want.view(torch.int32))
+        view.check()
+
+
 @pytest.mark.parametrize("dtype,dim", [("f16", 100), ("bf16", 301), ("f32", 50), ("i8", 100)])
 def test_batches_of_a_chain(dtype, dim):
     import torch
